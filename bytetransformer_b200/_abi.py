@@ -61,6 +61,7 @@ SIGNATURES = {
     "bt_destroy": (_i, [_vp]),
     "bt_set_layer_weights": (_i, [_vp, _i, C.POINTER(bt_layer_weights)]),
     "bt_workspace_bytes": (_i, [_vp, _i, _i, C.POINTER(_sz)]),
+    "bt_workspace_bytes_bias": (_i, [_vp, _i, _i, C.POINTER(_sz)]),
     "bt_workspace_bytes_packed": (_i, [_vp, _i, _i, C.POINTER(_sz)]),
     "bt_last_error": (C.c_char_p, [_vp]),
     "bt_device_status": (_i, [_vp, _vp, C.POINTER(_i)]),

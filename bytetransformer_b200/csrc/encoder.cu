@@ -324,9 +324,10 @@ static int run_gemm(bt_handle h, int kind, const __half* A, const void* W, __hal
 struct GeneralMask {
   const __half* mask = nullptr;
   const __half* bias = nullptr;
-  const int* kv_bound = nullptr;  // per (sequence, query tile): leading keys that matter (launch_mask_key_bound)
-  const uint32_t* bits = nullptr; // the mask as bits (launch_mask_bits), or null
+  const int* kv_bound = nullptr;  // per (sequence, query tile): leading keys that matter (launch_mask_bits)
+  const uint32_t* bits = nullptr; // the mask as bits, from the same launch
   const int* bits_flag = nullptr;
+  const void* bias_tiles = nullptr; // the bias as launch_bias_tiles lays it out, or null
 };
 
 static int run_mha(bt_handle h, const __half* qkv, __half* ctx, const int* batch_idx, int B, int max_len, int rows,
@@ -350,6 +351,7 @@ static int run_mha(bt_handle h, const __half* qkv, __half* ctx, const int* batch
     a.gen_kv_bound = gm->kv_bound;
     a.gen_bits = gm->bits;
     a.gen_bits_flag = gm->bits_flag;
+    a.gen_bias_tiles = gm->bias_tiles;
     a.gen_inv_scale = sqrtf(static_cast<float>(h->cfg.size_per_head)) * h->cfg.tao;
   }
   cudaError_t e;
@@ -565,30 +567,35 @@ static int stack_general(bt_handle h, int first_layer, int n_layers, const void*
   cudaError_t e;
   {
     LaunchScope scope(h, BT_PROF_OFFSETS, stream);
-    e = launch_uniform_offsets(ws.batch_idx, B, S, stream, ws.mask_bits_flag);
+    // the key bounds, filled in by the next launch, lie in the packed-index region, which is free on this path:
+    // B * ceil(S/128) <= B * S ints
+    e = launch_uniform_offsets(ws.batch_idx, B, S, stream, ws.mask_bits_flag, ws.word_idx, B * ((S + 127) / 128));
   }
   if (e != cudaSuccess) return fail_cuda(h, e, "offsets launch");
   GeneralMask gm;
   gm.mask = reinterpret_cast<const __half*>(mask);
   gm.bias = reinterpret_cast<const __half*>(attention_bias);
-  // Key tiles that no row of a query tile may see are left out of the attention (once per call; the
-  // packed-index region of the workspace is free on this path: B * ceil(S/128) <= B * S ints).
+  // One pass over the mask per call: a mask of zeros and ones is applied from bits (the attention kernel falls back
+  // to the fp16 mask if the pass meets any other value), and key tiles that no row of a query tile may see are
+  // left out of the attention.
   {
     LaunchScope scope(h, BT_PROF_OFFSETS, stream);
-    e = launch_mask_key_bound(gm.mask, B, S, ws.word_idx, stream);
+    e = launch_mask_bits(gm.mask, B, S, ws.mask_bits, ws.mask_bits_flag, ws.word_idx, stream);
   }
-  if (e != cudaSuccess) return fail_cuda(h, e, "mask key-bound launch");
+  if (e != cudaSuccess) return fail_cuda(h, e, "mask bits launch");
   gm.kv_bound = ws.word_idx;
-  if (gm.bias == nullptr) {
-    // no bias: a mask of zeros and ones is applied from bits (one pre-pass per call; the kernel falls back to
-    // the fp16 mask if the pre-pass meets any other value)
+  gm.bits = ws.mask_bits;
+  gm.bits_flag = ws.mask_bits_flag;
+  // The bias is re-laid for the attention kernel behind the workspace proper when the caller's workspace has room
+  // for it (bt_workspace_bytes_bias); without that room the kernel reads it where it is.
+  if (gm.bias != nullptr && workspace_bytes >= need.bytes + bias_tiles_bytes(h->cfg.head_num, S)) {
+    void* tiles = reinterpret_cast<uint8_t*>(base) + (need.bytes - 1024);
     {
       LaunchScope scope(h, BT_PROF_OFFSETS, stream);
-      e = launch_mask_bits(gm.mask, B, S, ws.mask_bits, ws.mask_bits_flag, stream);
+      e = launch_bias_tiles(gm.bias, h->cfg.head_num, S, tiles, stream);
     }
-    if (e != cudaSuccess) return fail_cuda(h, e, "mask bits launch");
-    gm.bits = ws.mask_bits;
-    gm.bits_flag = ws.mask_bits_flag;
+    if (e != cudaSuccess) return fail_cuda(h, e, "bias layout launch");
+    gm.bias_tiles = tiles;
   }
   const __half* cur = reinterpret_cast<const __half*>(input);
   for (int l = 0; l < n_layers; ++l) {
@@ -677,6 +684,13 @@ int bt_workspace_bytes(bt_handle h, int batch_size, int seq_len, size_t* bytes) 
   if (rc != BT_OK) return rc;
   const size_t rows = static_cast<size_t>(batch_size) * seq_len;
   *bytes = carve(nullptr, rows, h->hidden, h->ffn, batch_size + 1, rows).bytes;
+  return BT_OK;
+}
+
+int bt_workspace_bytes_bias(bt_handle h, int batch_size, int seq_len, size_t* bytes) {
+  const int rc = bt_workspace_bytes(h, batch_size, seq_len, bytes);
+  if (rc != BT_OK) return rc;
+  *bytes += bias_tiles_bytes(h->cfg.head_num, seq_len);
   return BT_OK;
 }
 

@@ -135,11 +135,14 @@ restore_rows_kernel(const uint4* __restrict__ packed, uint4* __restrict__ padded
 }
 
 __global__ void __launch_bounds__(256) uniform_offsets_kernel(int* __restrict__ batch_idx, int B, int S,
-                                                              int* __restrict__ clear_flag) {
+                                                              int* __restrict__ clear_flag, int* __restrict__ clear,
+                                                              int n_clear) {
   pdl_launch_dependents();
   pdl_wait();
-  if (clear_flag != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *clear_flag = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= B; i += gridDim.x * blockDim.x) batch_idx[i] = i * S;
+  const int i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  if (clear_flag != nullptr && i0 == 0) *clear_flag = 0;
+  for (int i = i0; i <= B; i += step) batch_idx[i] = i * S;
+  for (int i = i0; i < n_clear; i += step) clear[i] = 0;
 }
 
 // One CTA per sequence.  len = number of entries >= 0.5 in row 0 (the definition of the packed path);
@@ -179,55 +182,21 @@ mask_is_right_padded_kernel(const __half* __restrict__ mask, int B, int S, int* 
   if (threadIdx.x == 0 && s_bad) atomicExch(flag, 0);
 }
 
-// General-mask attention: for every (sequence, tile of 128 query rows) the number of leading keys that
-// matter.  A key whose mask value is exactly 0 gets -10000 added to its score and an exponential of 0,
-// so the key tiles behind the last non-zero mask entry of every row of the query tile can be left out -
-// unless a row has no non-zero entry at all: then all its scores are shifted alike, its softmax runs
-// over ALL keys, and the bound of its tile is the full length.  Thread = one query row, scanned from
-// the end; CTA = one query tile.
-__global__ void __launch_bounds__(128)
-mask_key_bound_kernel(const __half* __restrict__ mask, int S, int* __restrict__ bound) {
-  __shared__ int s_bound;
-  pdl_launch_dependents();
-  pdl_wait();
-  if (threadIdx.x == 0) s_bound = 0;
-  __syncthreads();
-  const int b = blockIdx.y;
-  const int row = blockIdx.x * 128 + threadIdx.x;
-  if (row < S) {
-    const __half* m = mask + (static_cast<size_t>(b) * S + row) * S;
-    const __half zero = __float2half(0.f);
-    int last = -1;
-    int j = S - 1;
-    if ((S & 7) == 0) {
-      // 16-byte steps while the vector is all zero
-      for (; j >= 7 && last < 0; j -= 8) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(m + j - 7));
-        if ((v.x | v.y | v.z | v.w) & 0x7FFF7FFFu) {  // some half is not +-0
-          for (int k = j; k > j - 8; --k)
-            if (__hne(m[k], zero)) {
-              last = k;
-              break;
-            }
-        }
-      }
-    } else {
-      for (; j >= 0 && last < 0; --j)
-        if (__hne(m[j], zero)) last = j;
-    }
-    atomicMax(&s_bound, last < 0 ? S : last + 1);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) bound[b * gridDim.x + blockIdx.x] = s_bound;
-}
-
-// The mask of the general path as one bit per (query, key): bit k of a row's word k/32 is set iff
-// mask[row, k] == 1.  `flag` (zero beforehand) is raised when some entry is neither 0 nor 1: the attention
-// kernel then keeps adding the fp16 mask itself.  Warp per mask row; a row's words are `stride_words`
-// apart (a multiple of 4, so that the 128 bits of a key tile are one aligned 16-byte load).
+// The mask of the general path, read once per call.  Two things come out of the one pass:
+//  * one bit per (query, key): bit k of a row's word k/32 is set iff mask[row, k] == 1.  `flag` (zero
+//    beforehand) is raised when some entry is neither 0 nor 1: the attention kernel then keeps adding the
+//    fp16 mask itself;
+//  * `bound` (zero beforehand): for every (sequence, tile of 128 query rows) the number of leading keys that
+//    matter.  A key whose mask value is exactly 0 gets -10000 added to its score and an exponential of 0, so
+//    the key tiles behind the last non-zero mask entry of every row of the query tile can be left out - unless
+//    a row has no non-zero entry at all: then all its scores are shifted alike, its softmax runs over ALL
+//    keys, and the bound of its tile is the full length.
+// Warp per mask row; a row's words are `stride_words` apart (a multiple of 4, so that the 128 bits of a key
+// tile are one aligned 16-byte load).  HBM-bound: 2 S bytes per row.  (The bound had a kernel of its own,
+// one thread walking each row from its end: for an odd S that was up to S dependent 2-byte loads.)
 __global__ void __launch_bounds__(256)
 mask_bits_kernel(const __half* __restrict__ mask, int S, long long rows, uint32_t* __restrict__ bits,
-                 int stride_words, int* __restrict__ flag) {
+                 int stride_words, int* __restrict__ flag, int* __restrict__ bound) {
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -236,6 +205,7 @@ mask_bits_kernel(const __half* __restrict__ mask, int S, long long rows, uint32_
   const unsigned short* m = reinterpret_cast<const unsigned short*>(mask) + row * S;
   uint32_t* out = bits + row * stride_words;
   bool odd = false;  // an entry that is neither +-0 nor 1
+  int last = -1;     // this lane's last entry that is not +-0
   if ((S & 7) == 0) {
     const int nvec = S >> 3;
     for (int v0 = 0; v0 < nvec; v0 += 32) {
@@ -250,6 +220,8 @@ mask_bits_kernel(const __half* __restrict__ mask, int S, long long rows, uint32_
           byte |= (lo == 0x3c00u ? 1u : 0u) << (2 * i);
           byte |= (hi == 0x3c00u ? 1u : 0u) << (2 * i + 1);
           odd = odd || (lo != 0x3c00u && (lo & 0x7fffu) != 0u) || (hi != 0x3c00u && (hi & 0x7fffu) != 0u);
+          if ((lo & 0x7fffu) != 0u) last = v * 8 + 2 * i;
+          if ((hi & 0x7fffu) != 0u) last = v * 8 + 2 * i + 1;
         }
       }
       uint32_t part = byte << ((lane & 3) * 8);
@@ -258,15 +230,63 @@ mask_bits_kernel(const __half* __restrict__ mask, int S, long long rows, uint32_
       if ((lane & 3) == 0 && v < nvec) out[v >> 2] = part;
     }
   } else {
+#pragma unroll 4
     for (int k0 = 0; k0 < S; k0 += 32) {
       const int k = k0 + lane;
       const uint32_t h = k < S ? m[k] : 0u;
       odd = odd || (h != 0x3c00u && (h & 0x7fffu) != 0u);
+      if ((h & 0x7fffu) != 0u) last = k;
       const uint32_t word = __ballot_sync(0xffffffffu, h == 0x3c00u);
       if (lane == 0) out[k0 >> 5] = word;
     }
   }
   if (__any_sync(0xffffffffu, odd) && lane == 0) atomicOr(flag, 1);
+  last = __reduce_max_sync(0xffffffffu, last);
+  if (lane == 0) {
+    const long long b = row / S;
+    const int q_tile = static_cast<int>(row - b * S) >> 7;
+    atomicMax(bound + b * ((S + 127) >> 7) + q_tile, last < 0 ? S : last + 1);
+  }
+}
+
+// The additive attention bias [heads, S, S] re-laid for the attention kernel, once per call (it is read again by
+// every layer and every sequence): 16-byte units of 8 keys, unit (head, query tile, key / 8, query row) - the
+// 32 rows of a softmax warp are 32 neighbouring units, so one load instruction of a warp covers four whole
+// 128-byte lines.  In the caller's layout a warp's lanes sit 2 S bytes apart (32 lines per instruction), and for
+// S % 8 != 0 only 2-byte loads are aligned.  Rows and keys from S up to the next multiple of 128 are zeros.
+// CTA = one 128 x 128 tile, turned through shared memory.  HBM-bound: 2 S^2 read + 2 ceil128(S)^2 written per head.
+__global__ void __launch_bounds__(256)
+bias_tiles_kernel(const __half* __restrict__ bias, int S, uint4* __restrict__ tiles) {
+  constexpr int kStride = 17;  // 16-byte units per staged row: 16 of data, 1 against bank conflicts
+  __shared__ uint4 buf[128 * kStride];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int q_tile = blockIdx.x, k_tile = blockIdx.y, head = blockIdx.z;
+  const int n_tiles = gridDim.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned short* src = reinterpret_cast<const unsigned short*>(bias) + static_cast<size_t>(head) * S * S;
+  if ((S & 7) == 0) {
+    for (int r = warp * 2 + (lane >> 4); r < 128; r += 16) {
+      const int q = q_tile * 128 + r, k = k_tile * 128 + (lane & 15) * 8;
+      buf[r * kStride + (lane & 15)] = (q < S && k < S)
+                                           ? __ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(q) * S + k))
+                                           : make_uint4(0u, 0u, 0u, 0u);
+    }
+  } else {
+#pragma unroll 4
+    for (int r = warp; r < 128; r += 8) {
+      const int q = q_tile * 128 + r;
+      unsigned short* row = reinterpret_cast<unsigned short*>(buf + r * kStride);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = k_tile * 128 + i * 32 + lane;
+        row[i * 32 + lane] = (q < S && k < S) ? __ldg(src + static_cast<size_t>(q) * S + k) : static_cast<unsigned short>(0);
+      }
+    }
+  }
+  __syncthreads();
+  uint4* dst = tiles + ((static_cast<size_t>(head) * n_tiles + q_tile) * n_tiles + k_tile) * (16 * 128);
+  for (int u = threadIdx.x; u < 16 * 128; u += 256) dst[u] = buf[(u & 127) * kStride + (u >> 7)];
 }
 
 __global__ void set_flag_kernel(int* flag, int v) {
@@ -290,29 +310,38 @@ cudaError_t launch_build_offsets(const __half* mask, int B, int S, int* batch_id
   return launch_pdl(build_offsets_kernel, dim3(1), dim3(kOffThreads), 0, stream, mask, B, S, batch_idx, word_idx);
 }
 
-cudaError_t launch_uniform_offsets(int* batch_idx, int B, int S, cudaStream_t stream, int* clear_flag) {
-  const int grid = (B + 1 + 255) / 256;
-  return launch_pdl(uniform_offsets_kernel, dim3(grid), dim3(256), 0, stream, batch_idx, B, S, clear_flag);
+cudaError_t launch_uniform_offsets(int* batch_idx, int B, int S, cudaStream_t stream, int* clear_flag, int* clear,
+                                   int n_clear) {
+  const int n = B + 1 > n_clear ? B + 1 : n_clear;
+  const int grid = (n + 255) / 256;
+  return launch_pdl(uniform_offsets_kernel, dim3(grid), dim3(256), 0, stream, batch_idx, B, S, clear_flag, clear, n_clear);
 }
 
 int mask_bits_stride_words(int S) { return ((S + 127) / 128) * 4; }
 
-cudaError_t launch_mask_bits(const __half* mask, int B, int S, uint32_t* bits, int* flag_dev, cudaStream_t stream) {
+cudaError_t launch_mask_bits(const __half* mask, int B, int S, uint32_t* bits, int* flag_dev, int* bound_dev,
+                             cudaStream_t stream) {
   if (B <= 0 || S <= 0) return cudaErrorInvalidValue;
   const long long rows = static_cast<long long>(B) * S;
   return launch_pdl(mask_bits_kernel, dim3(static_cast<unsigned>((rows + 7) / 8)), dim3(256), 0, stream, mask, S, rows,
-                    bits, mask_bits_stride_words(S), flag_dev);
+                    bits, mask_bits_stride_words(S), flag_dev, bound_dev);
+}
+
+size_t bias_tiles_bytes(int heads, int S) {
+  const size_t sp = static_cast<size_t>((S + 127) / 128) * 128;
+  return static_cast<size_t>(heads) * sp * sp * 2;
+}
+
+cudaError_t launch_bias_tiles(const __half* bias, int heads, int S, void* tiles, cudaStream_t stream) {
+  if (heads <= 0 || S <= 0) return cudaErrorInvalidValue;
+  const unsigned t = static_cast<unsigned>((S + 127) / 128);
+  return launch_pdl(bias_tiles_kernel, dim3(t, t, heads), dim3(256), 0, stream, bias, S, reinterpret_cast<uint4*>(tiles));
 }
 
 cudaError_t launch_mask_is_right_padded(const __half* mask, int B, int S, int* flag_dev, cudaStream_t stream) {
   cudaError_t e = launch_pdl(set_flag_kernel, dim3(1), dim3(1), 0, stream, flag_dev, 1);
   if (e != cudaSuccess) return e;
   return launch_pdl(mask_is_right_padded_kernel, dim3(B), dim3(256), 0, stream, mask, B, S, flag_dev);
-}
-
-cudaError_t launch_mask_key_bound(const __half* mask, int B, int S, int* bound_dev, cudaStream_t stream) {
-  if (B <= 0 || B > 65535 || S <= 0) return cudaErrorInvalidValue;
-  return launch_pdl(mask_key_bound_kernel, dim3((S + 127) / 128, B), dim3(128), 0, stream, mask, S, bound_dev);
 }
 
 cudaError_t launch_pack_rows(const __half* padded, __half* packed, const int* batch_idx, int B, int S, int hidden,

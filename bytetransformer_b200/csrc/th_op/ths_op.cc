@@ -86,7 +86,8 @@ class LayerEncoder {
     c10::cuda::CUDAGuard guard(input.device());
     Tensor out = torch::empty_like(input);
     size_t bytes = 0;
-    int rc = bt_workspace_bytes(handle_, batch, seq, &bytes);
+    int rc = attention_bias.defined() ? bt_workspace_bytes_bias(handle_, batch, seq, &bytes)
+                                      : bt_workspace_bytes(handle_, batch, seq, &bytes);
     TORCH_CHECK(rc == BT_OK, "bt_workspace_bytes failed: ", bt_last_error(handle_));
     Tensor buf = torch::empty({static_cast<int64_t>(bytes)}, torch::dtype(torch::kInt8).device(input.device()));
     cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();

@@ -214,7 +214,8 @@ class Encoder:
         with torch.cuda.device(self.device):
             out = torch.empty_like(x)
             n = C.c_size_t()
-            self._call("bt_workspace_bytes", self._h, B, S, C.byref(n))
+            self._call("bt_workspace_bytes" if attention_bias is None else "bt_workspace_bytes_bias", self._h, B, S,
+                       C.byref(n))
             ws = self._workspace(n.value)
             self._call("bt_stack_forward_padded_general", self._h, nl, x.data_ptr(), attr_mask.data_ptr(),
                        attention_bias.data_ptr() if attention_bias is not None else None, out.data_ptr(),

@@ -116,6 +116,10 @@ int bt_set_layer_weights(bt_handle h, int layer, const bt_layer_weights* w);
 
 /* `BertTransformer::cal_bufsize()` (bert_transformer.h:193-213). */
 int bt_workspace_bytes(bt_handle h, int batch_size, int seq_len, size_t* bytes);
+/* The same plus room for an attention bias in the layout the attention kernel reads fastest
+ * (head_num * (seq_len rounded up to 128)^2 * 2 bytes).  The general-mask entry points take a
+ * workspace of either size; with an `attention_bias` the larger one is several times faster. */
+int bt_workspace_bytes_bias(bt_handle h, int batch_size, int seq_len, size_t* bytes);
 
 /* Human-readable text of the last host-side error of this handle. */
 const char* bt_last_error(bt_handle h);
@@ -179,7 +183,8 @@ int bt_stack_forward_padded(bt_handle h, int n_layers, const void* input, const 
  * before the softmax (bytetransformer/include/softmax.h:41-45,
  * bytetransformer/src/attention_nofused.cu:78-95, th_op/bert_transformer_ext.h:83-107).  Any
  * [B,S,S] mask is honoured element by element (prefix-LM, block-diagonal, ...), not only row 0.
- * `attention_bias` is fp16 [head_num, seq_len, seq_len] or NULL.  Workspace: bt_workspace_bytes().
+ * `attention_bias` is fp16 [head_num, seq_len, seq_len] or NULL.  Workspace: bt_workspace_bytes() or, with a bias,
+ * bt_workspace_bytes_bias().
  * A key whose mask value is exactly 0 contributes an exponential of 0, so key tiles behind the last
  * non-zero mask entry of a tile of 128 query rows are not computed; a query row whose mask is all
  * zero has every score shifted alike and therefore attends to ALL keys, as the formula says (this

@@ -96,6 +96,37 @@ def test_binary_mask_without_bias_is_applied_from_bits(cuda_device, S, kind):
     _run(cuda_device, 2, 2, S, kind, False, 2, seed=S)
 
 
+@pytest.mark.parametrize("S,kind", [(1, "right_padded"), (77, "causal"), (128, "causal_blank_rows"), (197, "right_padded"),
+                                    (256, "prefix_lm"), (300, "soft"), (1023, "causal")])
+def test_bias_in_tile_layout_equals_bias_in_place(cuda_device, S, kind):
+    """With room behind the workspace the bias is re-laid once per call, without it the kernel reads it where it
+    is: the same terms are added in the same order, so the outputs are the same bits - for odd and even
+    sequence lengths, tails of a tile, rows that see nothing, and masks that the bits cannot stand for."""
+    import ctypes as C
+
+    from bytetransformer_b200.encoder import Encoder
+    g = torch.Generator().manual_seed(S)
+    nh, B = 3, 2
+    enc = Encoder(nh, 64, [to_device_weights(make_layer_weights(nh * 64, g), cuda_device) for _ in range(2)])
+    x = torch.randn(B, S, nh * 64, generator=g).half().to(cuda_device)
+    mask = _masks(kind, B, S, g).half().to(cuda_device)
+    bias = torch.randn(nh, S, S, generator=g).half().to(cuda_device)
+    outs = []
+    for size in ("bt_workspace_bytes", "bt_workspace_bytes_bias"):
+        n = C.c_size_t()
+        enc._call(size, enc._h, B, S, C.byref(n))
+        ws = torch.empty(n.value, dtype=torch.uint8, device=cuda_device)
+        out = torch.empty_like(x)
+        enc._call("bt_stack_forward_padded_general", enc._h, 2, x.data_ptr(), mask.data_ptr(), bias.data_ptr(),
+                  out.data_ptr(), ws.data_ptr(), ws.numel(), B, S, torch.cuda.current_stream().cuda_stream)
+        outs.append(out)
+    torch.cuda.synchronize()
+    assert enc.device_status() == 0
+    assert torch.equal(outs[0], outs[1])
+    assert torch.equal(outs[1], enc.forward_general(x, mask, bias))
+    enc.close()
+
+
 def test_mask_with_other_values_falls_back_to_the_additive_form(cuda_device):
     """(1 - mask) * -10000 for entries like 0.25 or 0.75 cannot be expressed in bits: the pre-pass raises its
     flag and the kernel adds the fp16 mask itself."""
