@@ -124,6 +124,26 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
+// The same for a warp whose 32 lanes all wait (the TMA and MMA roles): one answer for the warp, from a vote.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                               int code) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, status, code)) != 0;
+}
+
+// ------------------------------------------------------------ warp-uniform roles
+// tcgen05 and TMA instructions take their descriptors, addresses and coordinates from uniform registers.  In a
+// branch that one lane takes (`if (lane == 0)`) every operand of every instruction is moved there first, and that
+// cost more than the instruction: a 128 x N x 16 MMA took 91 clocks for any N <= 128 (132 in the GEMM main loop, with
+// its barrier waits), where the tensor core needs 64 at N = 128 and 50 at N = 32.  So the single-thread roles are
+// walked by their whole warp - role, loop bounds and shared values go through uniform_int() - and only the
+// instructions themselves are predicated on an elected lane, all MMAs of a K block and their commit on one
+// election (umma_k_block): 84 clocks per MMA in the main loop, 525 -> 335 clocks per K block of 64 (N <= 128).
+// Because elect.sync needs the whole warp, a warp's lanes must not part ways after a wait that gave up: waits end
+// in a vote (mbar_wait_warp), except in the K loop, which goes on to its end with `ok` remembered (a vote there
+// costs 30 clocks per K block) and votes after it.
+__device__ __forceinline__ int uniform_int(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ uint32_t uniform_u32(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // ----------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
@@ -172,17 +192,44 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// D[tmem] (+)= A[smem] * B[smem], fp16 inputs, fp32 accumulate; issued by ONE thread.
-__device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+// One K block of a GEMM main loop, D[tmem] (+)= A[smem] * B[smem], fp16 inputs, fp32 accumulation: four MMAs of 16 K elements each (operands `astep` / `bstep` descriptor units
+// apart) and the commit that frees the block's stage.  Called by a whole warp; one elect for the five instructions,
+// which are predicated on it.  `accumulate` = 0 overwrites the accumulator with the first product.  PAIR: cta_group::2,
+// the commit arrives on the barrier at the same offset in both CTAs.
+template <bool PAIR>
+__device__ __forceinline__ void umma_k_block(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t astep, uint32_t bstep,
+                                             uint32_t idesc, uint32_t accumulate, uint64_t* bar) {
+#define BT_UMMA_K_BLOCK(GROUP, COMMIT)                                                                       \
+  asm volatile(                                                                                              \
+      "{\n\t"                                                                                                \
+      ".reg .pred p, q, t;\n\t"                                                                              \
+      ".reg .b64 a1, a2, a3, b1, b2, b3, sa, sb;\n\t"                                                        \
+      ".reg .b16 m;\n\t"                                                                                     \
+      "cvt.u64.u32 sa, %3;\n\t"                                                                              \
+      "cvt.u64.u32 sb, %4;\n\t"                                                                              \
+      "add.u64 a1, %1, sa;\n\t"                                                                              \
+      "add.u64 a2, a1, sa;\n\t"                                                                              \
+      "add.u64 a3, a2, sa;\n\t"                                                                              \
+      "add.u64 b1, %2, sb;\n\t"                                                                              \
+      "add.u64 b2, b1, sb;\n\t"                                                                              \
+      "add.u64 b3, b2, sb;\n\t"                                                                              \
+      "mov.b16 m, 3;\n\t"                                                                                    \
+      "elect.sync _|q, 0xffffffff;\n\t"                                                                      \
+      "setp.ne.b32 p, %6, 0;\n\t"                                                                            \
+      "setp.eq.u32 t, 0, 0;\n\t"                                                                             \
+      "@q tcgen05.mma." GROUP ".kind::f16 [%0], %1, %2, %5, p;\n\t"                                          \
+      "@q tcgen05.mma." GROUP ".kind::f16 [%0], a1, b1, %5, t;\n\t"                                          \
+      "@q tcgen05.mma." GROUP ".kind::f16 [%0], a2, b2, %5, t;\n\t"                                          \
+      "@q tcgen05.mma." GROUP ".kind::f16 [%0], a3, b3, %5, t;\n\t"                                          \
+      "@q tcgen05.commit." GROUP ".mbarrier::arrive::one.shared::cluster" COMMIT ";\n\t"                     \
+      "}\n" ::"r"(d_tmem),                                                                                   \
+      "l"(adesc), "l"(bdesc), "r"(astep), "r"(bstep), "r"(idesc), "r"(accumulate), "r"(smem_u32(bar))        \
+      : "memory")
+  if (PAIR)
+    BT_UMMA_K_BLOCK("cta_group::2", ".multicast::cluster.b64 [%7], m");
+  else
+    BT_UMMA_K_BLOCK("cta_group::1", ".b64 [%7]");
+#undef BT_UMMA_K_BLOCK
 }
 // Arrive on `bar` once every tcgen05 operation issued so far by this thread is done.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {

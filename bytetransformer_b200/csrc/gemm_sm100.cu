@@ -280,7 +280,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_int(static_cast<int>(threadIdx.x >> 5));  // warp-uniform roles: see common.cuh
   const int lane = threadIdx.x & 31;
 
   pdl_launch_dependents();
@@ -309,7 +309,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform_u32(*tmem_slot);
 
   const int n_tiles = args.N / BLOCK_N;
   const int splits = kSplitK ? args.split_k : 1;
@@ -331,15 +331,15 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   // `pre_kb` stages get their full byte count armed and their W part requested here, their A
   // part after the wait.
   const int pre_kb = args.early_w ? (num_kb < kStages ? num_kb : kStages) : 0;
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
     int n0 = 0, sp = 0;
     tile_cols(static_cast<int>(blockIdx.x), n0, sp);
     for (int kb = 0; kb < pre_kb; ++kb) {
       uint8_t* sb = smem + kb * Cfg::kStageBytes + kABytes;
-      mbar_arrive_expect_tx(&full_bar[kb], Cfg::kStageBytes);
+      if (elect_one()) mbar_arrive_expect_tx(&full_bar[kb], Cfg::kStageBytes);
 #pragma unroll
       for (int c = 0; c < BLOCK_N / 64; ++c)
-        tma_load_2d(sb + c * (64 * kBlockK * 2), &tm_b, &full_bar[kb], n0 + c * 64, (sp * num_kb + kb) * kBlockK);
+        if (elect_one()) tma_load_2d(sb + c * (64 * kBlockK * 2), &tm_b, &full_bar[kb], n0 + c * 64, (sp * num_kb + kb) * kBlockK);
     }
   } else if (warp >= 2 && EPI != BT_EPI_NONE && args.early_w && args.bias != nullptr) {
     // the bias slice of the first tile, for the same reason
@@ -354,16 +354,16 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   // the row count is known: the first tile's rows lie inside the allocation whether or not they
   // are valid, and a CTA that turns out to have no tile only has to wait for them.
   pdl_wait();
-  if (warp == 0 && lane == 0 && pre_kb > 0) {
+  if (warp == 0 && pre_kb > 0) {
     int n0 = 0, sp = 0;
     const int m0 = tile_cols(static_cast<int>(blockIdx.x), n0, sp) * kBlockM;
     for (int kb = 0; kb < pre_kb; ++kb)
-      tma_load_2d(smem + kb * Cfg::kStageBytes, &tm_a, &full_bar[kb], (sp * num_kb + kb) * kBlockK, m0);
+      if (elect_one()) tma_load_2d(smem + kb * Cfg::kStageBytes, &tm_a, &full_bar[kb], (sp * num_kb + kb) * kBlockK, m0);
   }
   int M = args.m_rows;
   if (args.m_dev != nullptr) {
     const int md = __ldg(args.m_dev);
-    M = md < M ? md : M;
+    M = uniform_int(md < M ? md : M);
   }
   const int m_tiles = (M + kBlockM - 1) / kBlockM;
   const int total_tiles = m_tiles * n_tiles * splits;
@@ -378,7 +378,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
-    if (lane == 0) {
+    {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -387,7 +387,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         // No tile for this CTA after all (fewer valid rows than allocated): wait for the armed
         // stages, so that no copy is in flight at exit.
         for (int kb = 0; kb < pre_kb; ++kb)
-          if (!mbar_wait_bounded(&full_bar[kb], 0u, abort_flag, args.status, kStatusGemmProducerTimeout)) break;
+          if (!mbar_wait_warp(&full_bar[kb], 0u, abort_flag, args.status, kStatusGemmProducerTimeout)) break;
       }
       for (int li = 0; ok && tile_at(li, m0, n0, sp); ++li) {
         for (int i = 0; i < num_kb; ++i) {
@@ -397,16 +397,16 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
           if (li == 0 && i < pre_kb) {
             // armed and requested above (stage == i here)
           } else {
-            if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, abort_flag, args.status,
+            if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, args.status,
                                    kStatusGemmProducerTimeout)) {
               ok = false;
               break;
             }
-            mbar_arrive_expect_tx(&full_bar[stage], Cfg::kStageBytes);
-            tma_load_2d(sa, &tm_a, &full_bar[stage], kb * kBlockK, m0);
+            if (elect_one()) mbar_arrive_expect_tx(&full_bar[stage], Cfg::kStageBytes);
+            if (elect_one()) tma_load_2d(sa, &tm_a, &full_bar[stage], kb * kBlockK, m0);
 #pragma unroll
             for (int c = 0; c < BLOCK_N / 64; ++c)
-              tma_load_2d(sb + c * (64 * kBlockK * 2), &tm_b, &full_bar[stage], n0 + c * 64, kb * kBlockK);
+              if (elect_one()) tma_load_2d(sb + c * (64 * kBlockK * 2), &tm_b, &full_bar[stage], n0 + c * 64, kb * kBlockK);
           }
           if (++stage == kStages) {
             stage = 0;
@@ -417,7 +417,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     }
   } else if (warp == 1) {
     // --------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -425,35 +425,29 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       for (int it = 0; ok && tile_at(it, m0, n0, sp); ++it) {
         const int as = it & 1;
         const uint32_t aphase = (it >> 1) & 1;
-        if (!mbar_wait_bounded(&acc_empty[as], aphase ^ 1u, abort_flag, args.status, kStatusGemmMmaTimeout)) {
+        if (!mbar_wait_warp(&acc_empty[as], aphase ^ 1u, abort_flag, args.status, kStatusGemmMmaTimeout)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        gstamp(args.timing, it, 0);
+        if (lane == 0) gstamp(args.timing, it, 0);
         const uint32_t d_tmem = tmem_base + as * BLOCK_N;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait_bounded(&full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout)) {
-            ok = false;
-            break;
-          }
+          ok &= mbar_wait_bounded(&full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
           const uint32_t sb = sa + kABytes;
-#pragma unroll
-          for (int k = 0; k < kBlockK / 16; ++k) {
-            const uint64_t adesc = smem_desc(args.a_desc_hi, sa + k * args.a_kstep_bytes);
-            const uint64_t bdesc = smem_desc(args.b_desc_hi, sb + k * args.b_kstep_bytes);
-            umma_f16_ss(d_tmem, adesc, bdesc, args.idesc, (kb | k) != 0 ? 1u : 0u);
-          }
-          umma_commit(&empty_bar[stage]);  // frees the smem stage once these MMAs retire
+          // (the commit frees the stage once these MMAs have retired)
+          umma_k_block<false>(d_tmem, smem_desc(args.a_desc_hi, sa), smem_desc(args.b_desc_hi, sb), args.a_kstep_bytes >> 4,
+                       args.b_kstep_bytes >> 4, args.idesc, kb != 0 ? 1u : 0u, &empty_bar[stage]);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if (ok) umma_commit(&acc_full[as]);
-        gstamp(args.timing, it, 1);
+        ok = __all_sync(0xffffffffu, ok) != 0;
+        if (ok && elect_one()) umma_commit(&acc_full[as]);
+        if (lane == 0) gstamp(args.timing, it, 1);
       }
     }
   } else {
@@ -528,17 +522,6 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster_addr), "r"(x), "r"(y)
       : "memory");
 }
-__device__ __forceinline__ void umma_f16_ss_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                                 uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // Arrive on the barrier at this shared-memory offset in BOTH CTAs of the pair once every
 // tcgen05 operation issued so far has retired.
 __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
@@ -572,9 +555,9 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_int(static_cast<int>(threadIdx.x >> 5));  // warp-uniform roles: see common.cuh
   const int lane = threadIdx.x & 31;
-  const uint32_t cta_rank = cluster_ctarank();  // 0 = leader
+  const uint32_t cta_rank = uniform_u32(cluster_ctarank());  // 0 = leader
   const bool leader = cta_rank == 0;
   const int cluster_id = blockIdx.x >> 1;
   const int num_clusters = gridDim.x >> 1;
@@ -603,13 +586,13 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   __syncthreads();
   cluster_sync_all();  // the peer's barriers exist before anything is signalled across the pair
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform_u32(*tmem_slot);
 
   pdl_wait();  // see gemm_f16_kernel
   int M = args.m_rows;
   if (args.m_dev != nullptr) {
     const int md = __ldg(args.m_dev);
-    M = md < M ? md : M;
+    M = uniform_int(md < M ? md : M);
   }
   const int n_tiles = args.N / kTileN;
   const int m_tiles = (M + 2 * kBlockM - 1) / (2 * kBlockM);
@@ -618,9 +601,9 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
-    if (lane == 0) {
-      tma_prefetch_desc(&tm_a);
-      tma_prefetch_desc(&tm_b);
+    {
+      if (elect_one()) tma_prefetch_desc(&tm_a);
+      if (elect_one()) tma_prefetch_desc(&tm_b);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -628,7 +611,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         const int m0 = (tile / n_tiles) * (2 * kBlockM) + static_cast<int>(cta_rank) * kBlockM;
         const int n0 = (tile % n_tiles) * kTileN + static_cast<int>(cta_rank) * 128;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, abort_flag, args.status,
+          if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, args.status,
                                  kStatusGemmProducerTimeout)) {
             ok = false;
             break;
@@ -636,11 +619,11 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
           uint8_t* sa = smem + stage * Cfg::kStageBytes;
           uint8_t* sb = sa + kABytes;
           // the leader announces the bytes of both CTAs; all copies complete on its barrier
-          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * Cfg::kStageBytes);
+          if (leader && elect_one()) mbar_arrive_expect_tx(&full_bar[stage], 2 * Cfg::kStageBytes);
           const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          tma_load_2d_pair(sa, &tm_a, bar, kb * kBlockK, m0);
-          tma_load_2d_pair(sb, &tm_b, bar, n0, kb * kBlockK);
-          tma_load_2d_pair(sb + 64 * kBlockK * 2, &tm_b, bar, n0 + 64, kb * kBlockK);
+          if (elect_one()) tma_load_2d_pair(sa, &tm_a, bar, kb * kBlockK, m0);
+          if (elect_one()) tma_load_2d_pair(sb, &tm_b, bar, n0, kb * kBlockK);
+          if (elect_one()) tma_load_2d_pair(sb + 64 * kBlockK * 2, &tm_b, bar, n0 + 64, kb * kBlockK);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
@@ -650,7 +633,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------- MMA issuer (leader CTA only)
-    if (lane == 0 && leader) {
+    if (leader) {
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -658,35 +641,29 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       for (int tile = cluster_id; tile < total_tiles && ok; tile += num_clusters, ++it) {
         const int as = it & 1;
         const uint32_t aphase = (it >> 1) & 1;
-        if (!mbar_wait_bounded(&acc_empty[as], aphase ^ 1u, abort_flag, args.status, kStatusGemmMmaTimeout)) {
+        if (!mbar_wait_warp(&acc_empty[as], aphase ^ 1u, abort_flag, args.status, kStatusGemmMmaTimeout)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        gstamp(args.timing, it, 0);
+        if (lane == 0) gstamp(args.timing, it, 0);
         const uint32_t d_tmem = tmem_base + as * kTileN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait_bounded(&full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout)) {
-            ok = false;
-            break;
-          }
+          ok &= mbar_wait_bounded(&full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
           const uint32_t sb = sa + kABytes;
-#pragma unroll
-          for (int k = 0; k < kBlockK / 16; ++k) {
-            const uint64_t adesc = smem_desc(args.a_desc_hi, sa + k * args.a_kstep_bytes);
-            const uint64_t bdesc = smem_desc(args.b_desc_hi, sb + k * args.b_kstep_bytes);
-            umma_f16_ss_pair(d_tmem, adesc, bdesc, args.idesc, (kb | k) != 0 ? 1u : 0u);
-          }
-          umma_commit_pair(&empty_bar[stage]);  // frees the stage in both CTAs
+          // (the commit frees the stage once these MMAs have retired)
+          umma_k_block<true>(d_tmem, smem_desc(args.a_desc_hi, sa), smem_desc(args.b_desc_hi, sb), args.a_kstep_bytes >> 4,
+                       args.b_kstep_bytes >> 4, args.idesc, kb != 0 ? 1u : 0u, &empty_bar[stage]);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if (ok) umma_commit_pair(&acc_full[as]);
-        gstamp(args.timing, it, 1);
+        ok = __all_sync(0xffffffffu, ok) != 0;
+        if (ok && elect_one()) umma_commit_pair(&acc_full[as]);
+        if (lane == 0) gstamp(args.timing, it, 1);
       }
     }
   } else {
@@ -1083,7 +1060,7 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   // fp16 vectors of the current tile's 256 columns: bias | gamma | beta (gamma / beta only when they are fp16)
   uint4* vec_s = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(bars) + 256);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_int(static_cast<int>(threadIdx.x >> 5));  // warp-uniform roles: see common.cuh
   const int lane = threadIdx.x & 31;
 
   pdl_launch_dependents();
@@ -1116,13 +1093,13 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform_u32(*tmem_slot);
 
   pdl_wait();  // see gemm_f16_kernel
   int M = args.m_rows;
   if (args.m_dev != nullptr) {
     const int md = __ldg(args.m_dev);
-    M = md < M ? md : M;
+    M = uniform_int(md < M ? md : M);
   }
   const int n_tiles = args.N / kTileN;
   const int m_tiles = (M + kBlockM - 1) / kBlockM;
@@ -1138,25 +1115,25 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
-    if (lane == 0) {
+    {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       int m0 = 0, n0 = 0;
       for (int li = 0; ok && tile_at(li, m0, n0); ++li) {
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, abort_flag, args.status,
+          if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, args.status,
                                  kStatusGemmProducerTimeout)) {
             ok = false;
             break;
           }
           uint8_t* sa = smem + stage * Cfg::kStageBytes;
           uint8_t* sb = sa + kABytes;
-          mbar_arrive_expect_tx(&full_bar[stage], Cfg::kStageBytes);
-          tma_load_2d(sa, &tm_a, &full_bar[stage], kb * kBlockK, m0);
+          if (elect_one()) mbar_arrive_expect_tx(&full_bar[stage], Cfg::kStageBytes);
+          if (elect_one()) tma_load_2d(sa, &tm_a, &full_bar[stage], kb * kBlockK, m0);
 #pragma unroll
           for (int c = 0; c < kTileN / 64; ++c)
-            tma_load_2d(sb + c * (64 * kBlockK * 2), &tm_b, &full_bar[stage], n0 + c * 64, kb * kBlockK);
+            if (elect_one()) tma_load_2d(sb + c * (64 * kBlockK * 2), &tm_b, &full_bar[stage], n0 + c * 64, kb * kBlockK);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
@@ -1166,7 +1143,7 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     }
   } else if (warp == 1) {
     // --------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -1174,35 +1151,29 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       for (int it = 0; ok && tile_at(it, m0, n0); ++it) {
         const int as = it & 1;
         const uint32_t aphase = (it >> 1) & 1;
-        if (!mbar_wait_bounded(&acc_empty[as], aphase ^ 1u, abort_flag, args.status, kStatusGemmMmaTimeout)) {
+        if (!mbar_wait_warp(&acc_empty[as], aphase ^ 1u, abort_flag, args.status, kStatusGemmMmaTimeout)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        gstamp(args.timing, it, 0);
+        if (lane == 0) gstamp(args.timing, it, 0);
         const uint32_t d_tmem = tmem_base + as * kTileN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait_bounded(&full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout)) {
-            ok = false;
-            break;
-          }
+          ok &= mbar_wait_bounded(&full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
           const uint32_t sb = sa + kABytes;
-#pragma unroll
-          for (int k = 0; k < kBlockK / 16; ++k) {
-            const uint64_t adesc = smem_desc(args.a_desc_hi, sa + k * args.a_kstep_bytes);
-            const uint64_t bdesc = smem_desc(args.b_desc_hi, sb + k * args.b_kstep_bytes);
-            umma_f16_ss(d_tmem, adesc, bdesc, args.idesc, (kb | k) != 0 ? 1u : 0u);
-          }
-          umma_commit(&empty_bar[stage]);
+          // (the commit frees the stage once these MMAs have retired)
+          umma_k_block<false>(d_tmem, smem_desc(args.a_desc_hi, sa), smem_desc(args.b_desc_hi, sb), args.a_kstep_bytes >> 4,
+                       args.b_kstep_bytes >> 4, args.idesc, kb != 0 ? 1u : 0u, &empty_bar[stage]);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if (ok) umma_commit(&acc_full[as]);
-        gstamp(args.timing, it, 1);
+        ok = __all_sync(0xffffffffu, ok) != 0;
+        if (ok && elect_one()) umma_commit(&acc_full[as]);
+        if (lane == 0) gstamp(args.timing, it, 1);
       }
     }
   } else {
@@ -1256,9 +1227,9 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   uint4* vec_s = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(bars) + 256);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_int(static_cast<int>(threadIdx.x >> 5));  // warp-uniform roles: see common.cuh
   const int lane = threadIdx.x & 31;
-  const uint32_t cta_rank = cluster_ctarank();  // 0 = leader
+  const uint32_t cta_rank = uniform_u32(cluster_ctarank());  // 0 = leader
   const bool leader = cta_rank == 0;
   const int cluster_id = blockIdx.x >> 1;
   const int num_clusters = gridDim.x >> 1;
@@ -1290,13 +1261,13 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
   __syncthreads();
   cluster_sync_all();  // the peer's barriers exist before anything is signalled across the pair
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform_u32(*tmem_slot);
 
   pdl_wait();  // see gemm_f16_kernel
   int M = args.m_rows;
   if (args.m_dev != nullptr) {
     const int md = __ldg(args.m_dev);
-    M = md < M ? md : M;
+    M = uniform_int(md < M ? md : M);
   }
   const int n_tiles = args.N / kTileN;
   const int m_tiles = (M + 2 * kBlockM - 1) / (2 * kBlockM);
@@ -1305,11 +1276,11 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
 
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
-    if (lane == 0) {
-      tma_prefetch_desc(&tm_a);
-      tma_prefetch_desc(&tm_b);
-      tma_prefetch_desc(&tm_out);
-      tma_prefetch_desc(&tm_res);
+    {
+      if (elect_one()) tma_prefetch_desc(&tm_a);
+      if (elect_one()) tma_prefetch_desc(&tm_b);
+      if (elect_one()) tma_prefetch_desc(&tm_out);
+      if (elect_one()) tma_prefetch_desc(&tm_res);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -1317,7 +1288,7 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
         const int m0 = (tile / n_tiles) * (2 * kBlockM) + static_cast<int>(cta_rank) * kBlockM;
         const int n0 = (tile % n_tiles) * kTileN + static_cast<int>(cta_rank) * 128;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, abort_flag, args.status,
+          if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, args.status,
                                  kStatusGemmProducerTimeout)) {
             ok = false;
             break;
@@ -1325,11 +1296,11 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
           uint8_t* sa = smem + stage * Cfg::kStageBytes;
           uint8_t* sb = sa + kABytes;
           // the leader announces the bytes of both CTAs; all copies complete on its barrier
-          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * Cfg::kStageBytes);
+          if (leader && elect_one()) mbar_arrive_expect_tx(&full_bar[stage], 2 * Cfg::kStageBytes);
           const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          tma_load_2d_pair(sa, &tm_a, bar, kb * kBlockK, m0);
-          tma_load_2d_pair(sb, &tm_b, bar, n0, kb * kBlockK);
-          tma_load_2d_pair(sb + 64 * kBlockK * 2, &tm_b, bar, n0 + 64, kb * kBlockK);
+          if (elect_one()) tma_load_2d_pair(sa, &tm_a, bar, kb * kBlockK, m0);
+          if (elect_one()) tma_load_2d_pair(sb, &tm_b, bar, n0, kb * kBlockK);
+          if (elect_one()) tma_load_2d_pair(sb + 64 * kBlockK * 2, &tm_b, bar, n0 + 64, kb * kBlockK);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
@@ -1339,7 +1310,7 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
     }
   } else if (warp == 1) {
     // ------------------------------------------------- MMA issuer (leader CTA only)
-    if (lane == 0 && leader) {
+    if (leader) {
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -1347,35 +1318,29 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
       for (int tile = cluster_id; tile < total_tiles && ok; tile += num_clusters, ++it) {
         const int as = it & 1;
         const uint32_t aphase = (it >> 1) & 1;
-        if (!mbar_wait_bounded(&acc_empty[as], aphase ^ 1u, abort_flag, args.status, kStatusGemmMmaTimeout)) {
+        if (!mbar_wait_warp(&acc_empty[as], aphase ^ 1u, abort_flag, args.status, kStatusGemmMmaTimeout)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        gstamp(args.timing, it, 0);
+        if (lane == 0) gstamp(args.timing, it, 0);
         const uint32_t d_tmem = tmem_base + as * kTileN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait_bounded(&full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout)) {
-            ok = false;
-            break;
-          }
+          ok &= mbar_wait_bounded(&full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
           const uint32_t sb = sa + kABytes;
-#pragma unroll
-          for (int k = 0; k < kBlockK / 16; ++k) {
-            const uint64_t adesc = smem_desc(args.a_desc_hi, sa + k * args.a_kstep_bytes);
-            const uint64_t bdesc = smem_desc(args.b_desc_hi, sb + k * args.b_kstep_bytes);
-            umma_f16_ss_pair(d_tmem, adesc, bdesc, args.idesc, (kb | k) != 0 ? 1u : 0u);
-          }
-          umma_commit_pair(&empty_bar[stage]);  // frees the stage in both CTAs
+          // (the commit frees the stage once these MMAs have retired)
+          umma_k_block<true>(d_tmem, smem_desc(args.a_desc_hi, sa), smem_desc(args.b_desc_hi, sb), args.a_kstep_bytes >> 4,
+                       args.b_kstep_bytes >> 4, args.idesc, kb != 0 ? 1u : 0u, &empty_bar[stage]);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
         }
-        if (ok) umma_commit_pair(&acc_full[as]);
-        gstamp(args.timing, it, 1);
+        ok = __all_sync(0xffffffffu, ok) != 0;
+        if (ok && elect_one()) umma_commit_pair(&acc_full[as]);
+        if (lane == 0) gstamp(args.timing, it, 1);
       }
     }
   } else {

@@ -120,16 +120,55 @@ __device__ __forceinline__ void add2(float& d0, float& d1, float a0, float a1) {
   unpack_f32x2(add_f32x2(pack_f32x2(d0, d1), pack_f32x2(a0, a1)), d0, d1);
 }
 
-// D[tmem] (+)= A[tmem] * B[smem]: the A operand (P, fp16 pairs) is read from tensor memory.
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
+// S = Q K^T of one 128 x 128 tile (four 16-element K steps, 2 descriptor units apart) and the commit to `bar`;
+// called by a whole warp, one election for the five instructions (see common.cuh).
+__device__ __forceinline__ void umma_s_tile(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint64_t* bar) {
   asm volatile(
       "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      ".reg .pred q, f, t;\n\t"
+      ".reg .b64 a1, a2, a3, b1, b2, b3;\n\t"
+      "add.u64 a1, %1, 2;\n\t"
+      "add.u64 a2, %1, 4;\n\t"
+      "add.u64 a3, %1, 6;\n\t"
+      "add.u64 b1, %2, 2;\n\t"
+      "add.u64 b2, %2, 4;\n\t"
+      "add.u64 b3, %2, 6;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "setp.ne.u32 f, 0, 0;\n\t"
+      "setp.eq.u32 t, 0, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, f;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, t;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, t;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%4];\n\t"
       "}\n" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(smem_u32(bar))
+      : "memory");
+}
+
+// O (+)= P V over the first `steps` <= 8 groups of 16 keys of a tile: the A operand (P, fp16 pairs, 8 columns per
+// step) is read from tensor memory, V (128 descriptor units per step) from shared memory.  Called by a whole warp.
+__device__ __forceinline__ void umma_pv_tile(uint32_t d_tmem, uint32_t p_tmem, uint64_t vdesc, uint32_t idesc,
+                                             uint32_t accumulate, uint32_t steps) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred q, p, t;\n\t"
+      ".reg .b64 b;\n\t"
+      ".reg .b32 a;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "setp.ne.u32 p, %4, 0;\n\t"
+      "setp.eq.u32 t, 0, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+#define BT_PV_STEP(I, A, B)                                                \
+  "add.u32 a, %1, " A ";\n\t"                                              \
+  "add.u64 b, %2, " B ";\n\t"                                              \
+  "setp.gt.and.u32 p, %5, " I ", q;\n\t"                                   \
+  "@p tcgen05.mma.cta_group::1.kind::f16 [%0], [a], b, %3, t;\n\t"
+      BT_PV_STEP("1", "8", "128") BT_PV_STEP("2", "16", "256") BT_PV_STEP("3", "24", "384") BT_PV_STEP("4", "32", "512")
+      BT_PV_STEP("5", "40", "640") BT_PV_STEP("6", "48", "768") BT_PV_STEP("7", "56", "896")
+#undef BT_PV_STEP
+      "}\n" ::"r"(d_tmem),
+      "r"(p_tmem), "l"(vdesc), "r"(idesc), "r"(accumulate), "r"(steps)
       : "memory");
 }
 
@@ -409,8 +448,8 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
   pdl_wait();  // batch_idx and the QKV buffer come from earlier kernels
   const int b = blockIdx.z;
   const int head = blockIdx.y;
-  const int seq_start = __ldg(args.batch_idx + b);
-  const int L = __ldg(args.batch_idx + b + 1) - seq_start;
+  const int seq_start = uniform_int(__ldg(args.batch_idx + b));
+  const int L = uniform_int(__ldg(args.batch_idx + b + 1)) - seq_start;
   const int q0 = blockIdx.x * (kQRows * TILES);
   if (seq_start < 0 || L < 0 || L > args.max_len || seq_start > args.rows - L) {
     // offsets that do not describe rows of the allocation: nothing is read or written for this sequence
@@ -435,13 +474,13 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7 + 3 * kStages);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_int(static_cast<int>(threadIdx.x >> 5));  // warp-uniform roles: see common.cuh
   const int lane = threadIdx.x & 31;
   // General masks: the key tiles behind the last key that any row of this query tile may see are left out
   int kv_rows = L;
   if (GENERAL && args.gen_kv_bound != nullptr) {
     const int bound = __ldg(args.gen_kv_bound + b * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x));
-    kv_rows = bound < L ? (bound > 0 ? bound : 1) : L;
+    kv_rows = uniform_int(bound < L ? (bound > 0 ? bound : 1) : L);
   }
   const int n_kv = (kv_rows + kKvRows - 1) / kKvRows;
 
@@ -467,7 +506,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform_u32(*tmem_slot);
 
   const int col_q = head * kHeadDim;
   const int col_k = args.hidden + head * kHeadDim;
@@ -475,21 +514,21 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
 
   if (warp == 0) {
     // ------------------------------------------------------------------ loads
-    if (lane == 0) {
-      tma_prefetch_desc(&tm_qkv);
+    {
+      if (elect_one()) tma_prefetch_desc(&tm_qkv);
       for (int t = 0; t < n_tiles; ++t) {
-        mbar_arrive_expect_tx(&q_full[t], kTileBytes);
-        tma_load_2d(smem + Cfg::kSmemQ + t * kTileBytes, &tm_qkv, &q_full[t], col_q, seq_start + q0 + t * kQRows);
+        if (elect_one()) mbar_arrive_expect_tx(&q_full[t], kTileBytes);
+        if (elect_one()) tma_load_2d(smem + Cfg::kSmemQ + t * kTileBytes, &tm_qkv, &q_full[t], col_q, seq_start + q0 + t * kQRows);
       }
       int stage = 0;
       uint32_t phase = 0;
       for (int j = 0; j < n_kv; ++j) {
-        if (!mbar_wait_bounded(&kv_empty[stage], phase ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) break;
+        if (!mbar_wait_warp(&kv_empty[stage], phase ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) break;
         const int row = seq_start + j * kKvRows;
-        mbar_arrive_expect_tx(&k_full[stage], kTileBytes);
-        tma_load_2d(smem + Cfg::kSmemK + stage * kTileBytes, &tm_qkv, &k_full[stage], col_k, row);
-        mbar_arrive_expect_tx(&v_full[stage], kTileBytes);
-        tma_load_2d(smem + Cfg::kSmemV + stage * kTileBytes, &tm_qkv, &v_full[stage], col_v, row);
+        if (elect_one()) mbar_arrive_expect_tx(&k_full[stage], kTileBytes);
+        if (elect_one()) tma_load_2d(smem + Cfg::kSmemK + stage * kTileBytes, &tm_qkv, &k_full[stage], col_k, row);
+        if (elect_one()) mbar_arrive_expect_tx(&v_full[stage], kTileBytes);
+        if (elect_one()) tma_load_2d(smem + Cfg::kSmemV + stage * kTileBytes, &tm_qkv, &v_full[stage], col_v, row);
         if (++stage == kStages) {
           stage = 0;
           phase ^= 1u;
@@ -498,7 +537,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issue
-    if (lane == 0) {
+    {
       // K-major operands (Q, K): 8-row groups 1024 B apart.
       constexpr uint64_t kDescK = make_smem_desc_hi(16, 1024);
       // V: MN-major, one 64-wide chunk (LBO unused), 8-key groups 1024 B apart.
@@ -511,24 +550,17 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
       auto issue_s = [&](int t, int stage) {
         const uint32_t sq = s_q + t * kTileBytes;
         const uint32_t sk = s_k + stage * kTileBytes;
-#pragma unroll
-        for (int k = 0; k < kHeadDim / 16; ++k)
-          umma_f16_ss(tmem_base + t * 128, smem_desc(kDescK, sq + k * 32), smem_desc(kDescK, sk + k * 32), kIdescS,
-                      k != 0 ? 1u : 0u);
-        umma_commit(&s_full[t]);
+        umma_s_tile(tmem_base + t * 128, smem_desc(kDescK, sq), smem_desc(kDescK, sk), kIdescS, &s_full[t]);
       };
       auto issue_pv = [&](int t, int stage, bool accumulate) {
         const uint32_t tp = tmem_base + t * 128 + Cfg::kTmemPOff;  // 8 cells (16 keys) per MMA
         const uint32_t sv = s_v + stage * kTileBytes;
-#pragma unroll
-        for (int kk = 0; kk < kKvRows / 16; ++kk)
-          umma_f16_ts(tmem_base + Cfg::kTmemO + t * 64, tp + kk * 8, smem_desc(kDescV, sv + kk * 2048), kIdescO,
-                      (accumulate || kk != 0) ? 1u : 0u);
+        umma_pv_tile(tmem_base + Cfg::kTmemO + t * 64, tp, smem_desc(kDescV, sv), kIdescO, accumulate ? 1u : 0u, kKvRows / 16);
       };
       bool ok = true;
       for (int t = 0; t < n_tiles && ok; ++t)
-        ok = mbar_wait_bounded(&q_full[t], 0, abort_flag, args.status, kStatusMhaMmaTimeout);
-      if (ok) ok = mbar_wait_bounded(&k_full[0], 0, abort_flag, args.status, kStatusMhaMmaTimeout);
+        ok = mbar_wait_warp(&q_full[t], 0, abort_flag, args.status, kStatusMhaMmaTimeout);
+      if (ok) ok = mbar_wait_warp(&k_full[0], 0, abort_flag, args.status, kStatusMhaMmaTimeout);
       if (ok) {
         tc_fence_after();
         for (int t = 0; t < n_tiles; ++t) issue_s(t, 0);
@@ -542,27 +574,27 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
         const bool more = j + 1 < n_kv;
         // ---- tile 0: O0 += P0 V(j), then S0(j+1).  The MMAs of one thread execute in issue
         // order, so S0(j+1) cannot overwrite P0(j) (same columns) before PV0(j) has read it.
-        if (!mbar_wait_bounded(&p_full[0], jpar, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
-        if (!mbar_wait_bounded(&v_full[st], ph, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
+        if (!mbar_wait_warp(&p_full[0], jpar, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
+        if (!mbar_wait_warp(&v_full[st], ph, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
         tc_fence_after();
         issue_pv(0, st, j > 0);
         if (more) {
-          if (!mbar_wait_bounded(&k_full[st_n], ph_n, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
+          if (!mbar_wait_warp(&k_full[st_n], ph_n, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
           tc_fence_after();
           issue_s(0, st_n);
         }
         // ---- tile 1
         if (n_tiles == 2) {
-          if (!mbar_wait_bounded(&p_full[1], jpar, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
+          if (!mbar_wait_warp(&p_full[1], jpar, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
           tc_fence_after();
           issue_pv(1, st, j > 0);
         }
-        umma_commit(&kv_empty[st]);  // every MMA that reads K/V stage `st` has been issued
+        if (elect_one()) umma_commit(&kv_empty[st]);  // every MMA that reads K/V stage `st` has been issued
         if (n_tiles == 2 && more) issue_s(1, st_n);
         st = st_n;
         ph = ph_n;
       }
-      umma_commit(o_done);
+      if (elect_one()) umma_commit(o_done);
     }
   } else {
     // ---------------------------------------------------------------- softmax
@@ -827,10 +859,11 @@ __device__ __forceinline__ void setmaxnreg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-// Bounded wait for the single-thread roles (loader, MMA issuer): between polls the thread sleeps, so that
-// its polling does not take issue slots from the softmax warp that shares its scheduler.
-__device__ __forceinline__ bool mbar_wait_role(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                               int code) {
+// Bounded wait for the roles that one warp walks (loader, MMA issuer; all lanes call it, one answer for the warp):
+// between polls the warp sleeps, so that its polling does not take issue slots from the softmax warp that shares
+// its scheduler.
+__device__ __forceinline__ bool mbar_wait_role_lane(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                                    int code) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   uint32_t polls = 0;
@@ -846,6 +879,10 @@ __device__ __forceinline__ bool mbar_wait_role(uint64_t* bar, uint32_t parity, v
       }
     }
   }
+}
+__device__ __forceinline__ bool mbar_wait_role(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                               int code) {
+  return __all_sync(0xffffffffu, mbar_wait_role_lane(bar, parity, abort_flag, status, code)) != 0;
 }
 
 constexpr int kPersistentThreads = 256;
@@ -882,7 +919,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 5);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_int(static_cast<int>(threadIdx.x >> 5));  // warp-uniform roles: see common.cuh
   const int lane = threadIdx.x & 31;
   const bool smem_ok = (smem_u32(smem) & 1023u) == 0u;
 
@@ -912,7 +949,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform_u32(*tmem_slot);
   pdl_wait();  // batch_idx and the QKV buffer come from earlier kernels
 
   const int G = static_cast<int>(gridDim.x), cta = static_cast<int>(blockIdx.x);
@@ -924,34 +961,37 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
       // fall through to the teardown
     } else if (warp == 4) {
       // ------------------------------------------------------------------ loads
-      // (the whole warp finds the items, lane 0 does the rest)
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       for (int round = 0; ok && decode_item(args, snake_item(round, cta, G), cur_b, cur_first, seq_start, L, qt, head, true);
            ++round) {
-        if (lane == 0) {
+        {
+          L = uniform_int(L);
+          seq_start = uniform_int(seq_start);
+          qt = uniform_int(qt);
+          head = uniform_int(head);
           const int n_kv = (L + kKvRows - 1) / kKvRows;
           const int qb = round % kStages;
           const uint32_t qph = static_cast<uint32_t>(round / kStages) & 1u;
           ok = mbar_wait_role(&q_empty[qb], qph ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout);
           if (ok) {
-          mbar_arrive_expect_tx(&q_full[qb], kTileBytes);
-          tma_load_2d(smem + kSmemQ + qb * kTileBytes, &tm_qkv, &q_full[qb], head * kHeadDim, seq_start + qt * kQRows);
+          if (elect_one()) mbar_arrive_expect_tx(&q_full[qb], kTileBytes);
+          if (elect_one()) tma_load_2d(smem + kSmemQ + qb * kTileBytes, &tm_qkv, &q_full[qb], head * kHeadDim, seq_start + qt * kQRows);
           for (int j = 0; j < n_kv; ++j) {
             const int row = seq_start + j * kKvRows;
             if (!mbar_wait_role(&k_empty[stage], phase ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) {
               ok = false;
               break;
             }
-            mbar_arrive_expect_tx(&k_full[stage], kTileBytes);
-            tma_load_2d(smem + kSmemK + stage * kTileBytes, &tm_qkv, &k_full[stage], args.hidden + head * kHeadDim, row);
+            if (elect_one()) mbar_arrive_expect_tx(&k_full[stage], kTileBytes);
+            if (elect_one()) tma_load_2d(smem + kSmemK + stage * kTileBytes, &tm_qkv, &k_full[stage], args.hidden + head * kHeadDim, row);
             if (!mbar_wait_role(&v_empty[stage], phase ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) {
               ok = false;
               break;
             }
-            mbar_arrive_expect_tx(&v_full[stage], kTileBytes);
-            tma_load_2d(smem + kSmemV + stage * kTileBytes, &tm_qkv, &v_full[stage], 2 * args.hidden + head * kHeadDim,
+            if (elect_one()) mbar_arrive_expect_tx(&v_full[stage], kTileBytes);
+            if (elect_one()) tma_load_2d(smem + kSmemV + stage * kTileBytes, &tm_qkv, &v_full[stage], 2 * args.hidden + head * kHeadDim,
                         row);
             if (++stage == kStages) {
               stage = 0;
@@ -960,11 +1000,9 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
           }
           }
         }
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       }
     } else if (warp == 5) {
       // -------------------------------------------------------------- MMA issue
-      // (the whole warp finds the items, lane 0 does the rest)
       constexpr uint64_t kDescK = make_smem_desc_hi(16, 1024);
       constexpr uint64_t kDescV = make_smem_desc_hi(kTileBytes, 1024);
       constexpr uint32_t kIdescS = make_idesc_f16(128, 128, 0, 0);
@@ -976,20 +1014,16 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
       auto issue_s = [&](int round, int stage) {
         const uint32_t s_q = s_q0 + (round % kStages) * kTileBytes;
         const uint32_t sk = s_k + stage * kTileBytes;
-#pragma unroll
-        for (int k = 0; k < kHeadDim / 16; ++k)
-          umma_f16_ss(tmem_base + kTmemS, smem_desc(kDescK, s_q + k * 32), smem_desc(kDescK, sk + k * 32), kIdescS,
-                      k != 0 ? 1u : 0u);
-        umma_commit(s_full);
-        umma_commit(&k_empty[stage]);
+        umma_s_tile(tmem_base + kTmemS, smem_desc(kDescK, s_q), smem_desc(kDescK, sk), kIdescS, s_full);
+        if (elect_one()) umma_commit(&k_empty[stage]);
       };
       // the item's Q tile is free once its last Q K^T has been issued (and, by the commit, has retired)
-      auto release_q = [&](int round) { umma_commit(&q_empty[round % kStages]); };
+      auto release_q = [&](int round) { if (elect_one()) umma_commit(&q_empty[round % kStages]); };
       auto q_ready = [&](int round) { return static_cast<uint32_t>(round / kStages) & 1u; };
       int st = 0;
       uint32_t ph = 0;
       uint32_t step = 0;
-      // The first S = Q K^T of an item whose predecessor could not issue it ahead (lane 0).
+      // The first S = Q K^T of an item whose predecessor could not issue it ahead.
       auto issue_first_s = [&](int round, int len) -> bool {
         // S(0) overwrites the S columns: the softmax warps must hold the previous item's last S in registers
         if (step > 0 && !mbar_wait_role(s_free, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaMmaTimeout)) return false;
@@ -1000,7 +1034,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
         if (len <= kKvRows) release_q(round);  // the item's last (only) QK^T has been issued
         return true;
       };
-      // Everything else of an item (lane 0): per key tile the NEXT S as soon as the softmax warps hold the
+      // Everything else of an item: per key tile the NEXT S as soon as the softmax warps hold the
       // current one in registers, then O += P V.  On the item's last tile the next S is the first of the
       // CTA's next item, if its Q and K tiles have landed by then (`next_s_issued`): an item boundary then
       // costs the softmax warps no S round trip.  false when a wait gave up.
@@ -1020,7 +1054,8 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
             if (j + 2 == n_kv) release_q(round);
           } else if (have_next) {
             if (!mbar_wait_role(s_free, step & 1u, abort_flag, args.status, kStatusMhaMmaTimeout)) return false;
-            if (mbar_test_wait(&q_full[(round + 1) % kStages], q_ready(round + 1)) && mbar_test_wait(&k_full[st_n], ph_n)) {
+            if (__all_sync(0xffffffffu, mbar_test_wait(&q_full[(round + 1) % kStages], q_ready(round + 1)) &&
+                                            mbar_test_wait(&k_full[st_n], ph_n))) {
               tc_fence_after();
               issue_s(round + 1, st_n);
               if (len_next <= kKvRows) release_q(round + 1);
@@ -1033,35 +1068,29 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
               !mbar_wait_role(&v_full[st], ph, abort_flag, args.status, kStatusMhaMmaTimeout))
             return false;
           tc_fence_after();
-          const uint32_t sv = s_v + st * kTileBytes;
           // only the 16-key steps that hold keys of this sequence
-          const int kk_n = (min(kKvRows, len - j * kKvRows) + 15) >> 4;
-#pragma unroll
-          for (int kk = 0; kk < kKvRows / 16; ++kk)
-            if (kk < kk_n)
-              umma_f16_ts(tmem_base + kTmemO, tmem_base + kTmemP + kk * 8, smem_desc(kDescV, sv + kk * 2048), kIdescO,
-                          (j > 0 || kk != 0) ? 1u : 0u);
-          umma_commit(pv_done);
-          umma_commit(&v_empty[st]);
+          umma_pv_tile(tmem_base + kTmemO, tmem_base + kTmemP, smem_desc(kDescV, s_v + st * kTileBytes), kIdescO, j > 0 ? 1u : 0u,
+                       static_cast<uint32_t>((min(kKvRows, len - j * kKvRows) + 15) >> 4));
+          if (elect_one()) umma_commit(pv_done);
+          if (elect_one()) umma_commit(&v_empty[st]);
           st = st_n;
           ph = ph_n;
         }
-        umma_commit(o_done);
+        if (elect_one()) umma_commit(o_done);
         return true;
       };
       bool ok = true;
       bool have = decode_item(args, snake_item(0, cta, G), cur_b, cur_first, seq_start, L, qt, head, false);
-      int len = L;
+      int len = uniform_int(L);
       bool s_issued = false;  // S(0) of the item about to start has been issued already
       for (int round = 0; ok && have; ++round) {
-        if (lane == 0 && !s_issued) ok = issue_first_s(round, len);
+        if (!s_issued) ok = issue_first_s(round, len);
         // the item after this one is found while this item's first tile is on its way
         const bool have_next = decode_item(args, snake_item(round + 1, cta, G), cur_b, cur_first, seq_start, L, qt, head, false);
-        const int len_next = L;
+        const int len_next = uniform_int(L);
         bool next_s_issued = false;
-        if (lane == 0 && ok) ok = issue_rest(round, len, have_next, len_next, next_s_issued);
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        s_issued = __shfl_sync(0xffffffffu, next_s_issued ? 1 : 0, 0) != 0;
+        if (ok) ok = issue_rest(round, len, have_next, len_next, next_s_issued);
+        s_issued = next_s_issued;
         have = have_next;
         len = len_next;
       }
