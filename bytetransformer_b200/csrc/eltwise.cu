@@ -102,7 +102,11 @@ layernorm_rows_kernel(const void* __restrict__ x_v, const __half* __restrict__ b
     const int md = __ldg(m_dev);
     row_limit = md < m_rows ? md : m_rows;
   }
-  for (long long row = static_cast<long long>(blockIdx.x) * kLnWarps + warp; row < row_limit;
+  // A warp's first row is read before the row count has arrived (it lies inside the allocation either way) and
+  // dropped after the first reduction if it does not exist: in a call of a few rows the count's L2 round trip is a
+  // tenth of the kernel.
+  const long long first_row = static_cast<long long>(blockIdx.x) * kLnWarps + warp;
+  for (long long row = first_row; row < (row == first_row ? m_rows : row_limit);
        row += static_cast<long long>(gridDim.x) * kLnWarps) {
   long long src_row = row;
   if (RESTORE) {
@@ -172,6 +176,7 @@ layernorm_rows_kernel(const void* __restrict__ x_v, const __half* __restrict__ b
     }
   }
   const float mean = warp_sum(sum) / static_cast<float>(hidden);
+  if (!RESTORE && row >= row_limit) break;
   float sq = 0.f;
 #pragma unroll
   for (int it = 0; it < NVEC; ++it) {

@@ -134,6 +134,7 @@ struct bt_encoder_s {
   // tiles; the threshold stood at 100 then.)
   int fused_ln = 1;
   int fused_ln_min_tiles = 40;
+  bool all_rows = false;  // the call in progress computes every allocated row (packed and general-mask entries)
   uint32_t ln_epoch = 0;  // fused LayerNorm launches since the statistics scratch of the current call was zeroed
   bool fused_ln_ffn2_only = false;  // keep the attention-output LayerNorm as its own kernel
   std::vector<cudaEvent_t> ev_pool;
@@ -285,7 +286,7 @@ static int run_gemm(bt_handle h, int kind, const __half* A, const void* W, __hal
     ok = ok && ln != nullptr && h->tmap(&g.tm_out, ln->out_ln, m_rows, N, 64, 32, 2) &&
          h->tmap(&g.tm_res, residual, m_rows, N, 64, 32, 2);
   else if (epi == BT_EPI_BIAS_RESIDUAL_F32OUT)
-    ok = ok && h->tmap(&g.tm_out, out, m_rows, N, 32, 32, 4);
+    ok = ok && h->tmap(&g.tm_out, out, static_cast<uint64_t>(m_rows) * split_k, N, 32, 32, 4);
   else
     ok = ok && h->tmap(&g.tm_out, out, m_rows, N, 64, 32, 2);
   if (!ok) return fail(h, BT_ERR_CUDA, "cuTensorMapEncodeTiled failed (pointer alignment / driver entry point)");
@@ -294,6 +295,7 @@ static int run_gemm(bt_handle h, int kind, const __half* A, const void* W, __hal
   g.residual = residual;
   g.m_dev = m_dev;
   g.m_rows = m_rows;
+  g.all_rows = m_dev == nullptr || h->all_rows;
   g.N = N;
   g.K = K;
   g.epilogue = epi;
@@ -375,8 +377,9 @@ static bool want_fused_ln(bt_handle h, long long rows) {
 // The statistics scratch of the fused LayerNorm (the head of `pre`) holds words tagged with the number
 // of the launch that wrote them; it is zeroed once per call (the caller's workspace starts out with
 // arbitrary contents) and the fused launches of the call are numbered from 1.
-static int prepare_ln_sync(bt_handle h, const Workspace& ws, long long rows, cudaStream_t stream) {
+static int prepare_ln_sync(bt_handle h, const Workspace& ws, long long rows, bool all_rows, cudaStream_t stream) {
   h->ln_epoch = 0;
+  h->all_rows = all_rows;
   if (!want_fused_ln(h, rows)) return BT_OK;
   cudaError_t e = cudaMemsetAsync(ws.pre, 0, ws.ln_stats_bytes, stream);
   return e == cudaSuccess ? BT_OK : fail_cuda(h, e, "memset of the LayerNorm statistics scratch");
@@ -506,7 +509,7 @@ static int stack_padded(bt_handle h, int first_layer, int n_layers, const void* 
   void* base = reinterpret_cast<void*>(align_up(reinterpret_cast<uintptr_t>(workspace), 1024));
   Workspace ws = carve(base, rows, h->hidden, h->ffn, B + 1, rows);
 
-  if ((rc = prepare_ln_sync(h, ws, static_cast<long long>(rows), stream)) != BT_OK) return rc;
+  if ((rc = prepare_ln_sync(h, ws, static_cast<long long>(rows), false, stream)) != BT_OK) return rc;
   pdl_next_launch_plain();  // first kernel of the call: see kernels.h
   cudaError_t e;
   {
@@ -562,7 +565,7 @@ static int stack_general(bt_handle h, int first_layer, int n_layers, const void*
   if (workspace_bytes < need.bytes) return fail(h, BT_ERR_WORKSPACE, "workspace smaller than bt_workspace_bytes()");
   void* base = reinterpret_cast<void*>(align_up(reinterpret_cast<uintptr_t>(workspace), 1024));
   Workspace ws = carve(base, rows, h->hidden, h->ffn, B + 1, rows);
-  if ((rc = prepare_ln_sync(h, ws, static_cast<long long>(rows), stream)) != BT_OK) return rc;
+  if ((rc = prepare_ln_sync(h, ws, static_cast<long long>(rows), true, stream)) != BT_OK) return rc;
   pdl_next_launch_plain();  // first kernel of the call: see kernels.h
   cudaError_t e;
   {
@@ -921,7 +924,7 @@ int bt_stack_forward_packed(bt_handle h, int n_layers, const void* x_packed, con
   void* base = reinterpret_cast<void*>(align_up(reinterpret_cast<uintptr_t>(workspace), 1024));
   Workspace ws = carve(base, static_cast<size_t>(total_tokens), h->hidden, h->ffn, 0, 0);
   {
-    const int rc = prepare_ln_sync(h, ws, total_tokens, stream);
+    const int rc = prepare_ln_sync(h, ws, total_tokens, true, stream);
     if (rc != BT_OK) return rc;
   }
   pdl_next_launch_plain();  // first kernel of the call: see kernels.h
@@ -979,6 +982,7 @@ int bt_gemm(bt_handle h, const void* A, const void* W, void* out, const void* bi
     if (rc != BT_OK) return rc;
   }
   pdl_next_launch_plain();  // W may come straight from the caller's kernel before: see kernels.h
+  h->all_rows = false;
   return run_gemm(h, BT_PROF_GEMM_OTHER, reinterpret_cast<const __half*>(A), W, reinterpret_cast<__half*>(out), bias,
                   reinterpret_cast<const __half*>(residual), m_dev, m_rows, N, K, epilogue, gelu_kind,
                   reinterpret_cast<cudaStream_t>(stream));

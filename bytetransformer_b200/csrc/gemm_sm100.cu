@@ -52,9 +52,11 @@ struct GemmCfg {
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kStages = (BLOCK_N == 256) ? 4 : (BLOCK_N == 128 ? 6 : 8);
   static constexpr int kTmemCols = 2 * BLOCK_N;
-  // Output leaves through per-warp staging rows + TMA bulk stores when a warp's
-  // column share is at least 128 bytes wide (BLOCK_N >= 128).
-  static constexpr bool kTmaStore = BLOCK_N >= 128;
+  // Output leaves through per-warp staging rows + TMA bulk stores when a warp's column share of a row is at
+  // least 128 bytes: 64 fp16 or 32 fp32 columns.
+  static constexpr bool tma_store(int epi) {
+    return BLOCK_N >= 128 || epi == BT_EPI_BIAS_RESIDUAL_F32OUT || epi == kEpiSplitKF32;
+  }
   static constexpr int kStagingBytes = kEpiWarps * kStagingBytesPerWarp;
   static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 /*align slack*/ + 256 /*barriers*/;
 };
@@ -93,7 +95,7 @@ struct GemmArgs {
   // out + s * split_stride floats; range 0 also adds bias and residual
   int split_k;
   long long split_stride;
-  int early_w;  // one-CTA kernel: request the first tile's W blocks before the wait for the kernel before
+  int early_w;  // request the first tile's W blocks before the wait for the kernel before
   long long* timing;  // diagnostics: clock64 stamps per CTA and tile (null = off)
   uint64_t a_desc_hi;
   uint64_t b_desc_hi;
@@ -133,7 +135,6 @@ __device__ __forceinline__ void epilogue_tile(const GemmArgs& args, const CUtens
   constexpr bool kSplitK = (EPI == kEpiSplitKF32);
   constexpr bool kF32Out = (EPI == BT_EPI_BIAS_RESIDUAL_F32OUT) || kSplitK;
   constexpr bool kHasResidual = (EPI == BT_EPI_BIAS_RESIDUAL || EPI == BT_EPI_BIAS_RESIDUAL_F32OUT) || kSplitK;
-  static_assert(!(kSplitK && TMA_STORE), "split-K partials are stored by the threads");
   // 128 bytes of output per row and chunk: 32 fp32 or 64 fp16 columns.
   constexpr int kChunk = kF32Out ? 32 : (kColsPerWarp >= 64 ? 64 : 32);
   constexpr int kNChunks = kColsPerWarp / kChunk;
@@ -227,7 +228,8 @@ __device__ __forceinline__ void epilogue_tile(const GemmArgs& args, const CUtens
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
-        tma_store_2d(tm_out, sbuf, gcol, row0);
+        // (the partial sums of a split lie below one another in the store map: split_stride = m_rows * N)
+        tma_store_2d(tm_out, sbuf, gcol, kSplitK ? split * args.m_rows + row0 : row0);
         tma_store_commit();
       }
     } else if (row_ok) {
@@ -465,14 +467,14 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       if (!mbar_wait_bounded(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
       tc_fence_after();
       if (warp == 2 && lane == 0) gstamp(args.timing, it, 2);
-      epilogue_tile<BLOCK_N, EPI, Cfg::kTmaStore, 1>(args, &tm_out, stg, tmem_base + as * BLOCK_N, m0, n0, M, quarter,
+      epilogue_tile<BLOCK_N, EPI, Cfg::tma_store(EPI), 1>(args, &tm_out, stg, tmem_base + as * BLOCK_N, m0, n0, M, quarter,
                                                   col_half, lane, resv, sp);
       if (warp == 2 && lane == 0) gstamp(args.timing, it, 3);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[as]);
     }
-    if (Cfg::kTmaStore && lane == 0) tma_store_wait_all();  // staging rows must outlive the last bulk store
+    if (Cfg::tma_store(EPI) && lane == 0) tma_store_wait_all();  // staging rows must outlive the last bulk store
   }
 
   // ------------------------------------------------------------------ teardown
@@ -588,46 +590,70 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = uniform_u32(*tmem_slot);
 
+  const int n_tiles = args.N / kTileN;
+  const int num_kb = args.K / kBlockK;
+  // The leading W blocks of the pair's first tile ahead of the dependency wait, its A blocks right behind it (see
+  // gemm_f16_kernel).  Both CTAs' copies complete on the leader's barrier, which the leader arms for both.
+  const int pre_kb = args.early_w ? (num_kb < kStages ? num_kb : kStages) : 0;
+  auto load_w = [&](int stage, int n0, int kb) {
+    uint8_t* sb = smem + stage * Cfg::kStageBytes + kABytes;
+    const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
+    if (elect_one()) tma_load_2d_pair(sb, &tm_b, bar, n0, kb * kBlockK);
+    if (elect_one()) tma_load_2d_pair(sb + 64 * kBlockK * 2, &tm_b, bar, n0 + 64, kb * kBlockK);
+  };
+  auto load_a = [&](int stage, int m0, int kb) {
+    const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
+    if (elect_one()) tma_load_2d_pair(smem + stage * Cfg::kStageBytes, &tm_a, bar, kb * kBlockK, m0);
+  };
+  auto tile_rows = [&](int tile) { return (tile / n_tiles) * (2 * kBlockM) + static_cast<int>(cta_rank) * kBlockM; };
+  auto tile_w_cols = [&](int tile) { return (tile % n_tiles) * kTileN + static_cast<int>(cta_rank) * 128; };
+  if (warp == 0) {
+    if (elect_one()) tma_prefetch_desc(&tm_a);
+    if (elect_one()) tma_prefetch_desc(&tm_b);
+    if (elect_one()) tma_prefetch_desc(&tm_out);
+    for (int kb = 0; kb < pre_kb; ++kb) {
+      if (leader && elect_one()) mbar_arrive_expect_tx(&full_bar[kb], 2 * Cfg::kStageBytes);
+      load_w(kb, tile_w_cols(cluster_id), kb);
+    }
+  }
+
   pdl_wait();  // see gemm_f16_kernel
+  if (warp == 0)
+    for (int kb = 0; kb < pre_kb; ++kb) load_a(kb, tile_rows(cluster_id), kb);
   int M = args.m_rows;
   if (args.m_dev != nullptr) {
     const int md = __ldg(args.m_dev);
     M = uniform_int(md < M ? md : M);
   }
-  const int n_tiles = args.N / kTileN;
   const int m_tiles = (M + 2 * kBlockM - 1) / (2 * kBlockM);
   const int total_tiles = m_tiles * n_tiles;
-  const int num_kb = args.K / kBlockK;
 
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
-    {
-      if (elect_one()) tma_prefetch_desc(&tm_a);
-      if (elect_one()) tma_prefetch_desc(&tm_b);
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = cluster_id; tile < total_tiles && ok; tile += num_clusters) {
-        const int m0 = (tile / n_tiles) * (2 * kBlockM) + static_cast<int>(cta_rank) * kBlockM;
-        const int n0 = (tile % n_tiles) * kTileN + static_cast<int>(cta_rank) * 128;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, args.status,
-                                 kStatusGemmProducerTimeout)) {
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    if (cluster_id >= total_tiles && leader) {
+      // No tile for this pair after all: wait for the armed stages, so that no copy is in flight at exit.
+      for (int kb = 0; kb < pre_kb; ++kb)
+        if (!mbar_wait_warp(&full_bar[kb], 0u, abort_flag, args.status, kStatusGemmProducerTimeout)) break;
+    }
+    for (int tile = cluster_id; tile < total_tiles && ok; tile += num_clusters) {
+      const int m0 = tile_rows(tile), n0 = tile_w_cols(tile);
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (tile != cluster_id || kb >= pre_kb) {  // else armed and requested above (stage == kb)
+          if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, args.status, kStatusGemmProducerTimeout)) {
             ok = false;
             break;
           }
-          uint8_t* sa = smem + stage * Cfg::kStageBytes;
-          uint8_t* sb = sa + kABytes;
           // the leader announces the bytes of both CTAs; all copies complete on its barrier
           if (leader && elect_one()) mbar_arrive_expect_tx(&full_bar[stage], 2 * Cfg::kStageBytes);
-          const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          if (elect_one()) tma_load_2d_pair(sa, &tm_a, bar, kb * kBlockK, m0);
-          if (elect_one()) tma_load_2d_pair(sb, &tm_b, bar, n0, kb * kBlockK);
-          if (elect_one()) tma_load_2d_pair(sb + 64 * kBlockK * 2, &tm_b, bar, n0 + 64, kb * kBlockK);
-          if (++stage == kStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          load_a(stage, m0, kb);
+          load_w(stage, n0, kb);
+        }
+        if (++stage == kStages) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
@@ -1095,16 +1121,38 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   tc_fence_after();
   const uint32_t tmem_base = uniform_u32(*tmem_slot);
 
+  const int n_tiles = args.N / kTileN;
+  const int num_kb = args.K / kBlockK;
+  // The leading W blocks of the first tile ahead of the dependency wait, its A blocks right behind it (see
+  // gemm_f16_kernel).
+  const int pre_kb = args.early_w ? (num_kb < kStages ? num_kb : kStages) : 0;
+  auto load_w = [&](int stage, int n0, int kb) {
+    uint8_t* sb = smem + stage * Cfg::kStageBytes + kABytes;
+#pragma unroll
+    for (int c = 0; c < kTileN / 64; ++c)
+      if (elect_one()) tma_load_2d(sb + c * (64 * kBlockK * 2), &tm_b, &full_bar[stage], n0 + c * 64, kb * kBlockK);
+  };
+  auto load_a = [&](int stage, int m0, int kb) {
+    if (elect_one()) tma_load_2d(smem + stage * Cfg::kStageBytes, &tm_a, &full_bar[stage], kb * kBlockK, m0);
+  };
+  const int first_m0 = (static_cast<int>(blockIdx.x) / n_tiles) * kBlockM;
+  if (warp == 0) {
+    for (int kb = 0; kb < pre_kb; ++kb) {
+      if (elect_one()) mbar_arrive_expect_tx(&full_bar[kb], Cfg::kStageBytes);
+      load_w(kb, (static_cast<int>(blockIdx.x) % n_tiles) * kTileN, kb);
+    }
+  }
+
   pdl_wait();  // see gemm_f16_kernel
+  if (warp == 0)
+    for (int kb = 0; kb < pre_kb; ++kb) load_a(kb, first_m0, kb);
   int M = args.m_rows;
   if (args.m_dev != nullptr) {
     const int md = __ldg(args.m_dev);
     M = uniform_int(md < M ? md : M);
   }
-  const int n_tiles = args.N / kTileN;
   const int m_tiles = (M + kBlockM - 1) / kBlockM;
   const int total_tiles = m_tiles * n_tiles;
-  const int num_kb = args.K / kBlockK;
   auto tile_at = [&](int li, int& m0, int& n0) -> bool {
     const int tile = static_cast<int>(blockIdx.x) + li * static_cast<int>(gridDim.x);
     if (tile >= total_tiles) return false;
@@ -1115,29 +1163,29 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
-    {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      int m0 = 0, n0 = 0;
-      for (int li = 0; ok && tile_at(li, m0, n0); ++li) {
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, args.status,
-                                 kStatusGemmProducerTimeout)) {
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    int m0 = 0, n0 = 0;
+    if (!tile_at(0, m0, n0)) {
+      // No tile for this CTA after all: wait for the armed stages, so that no copy is in flight at exit.
+      for (int kb = 0; kb < pre_kb; ++kb)
+        if (!mbar_wait_warp(&full_bar[kb], 0u, abort_flag, args.status, kStatusGemmProducerTimeout)) break;
+    }
+    for (int li = 0; ok && tile_at(li, m0, n0); ++li) {
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (li != 0 || kb >= pre_kb) {  // else armed and requested above (stage == kb)
+          if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, args.status, kStatusGemmProducerTimeout)) {
             ok = false;
             break;
           }
-          uint8_t* sa = smem + stage * Cfg::kStageBytes;
-          uint8_t* sb = sa + kABytes;
           if (elect_one()) mbar_arrive_expect_tx(&full_bar[stage], Cfg::kStageBytes);
-          if (elect_one()) tma_load_2d(sa, &tm_a, &full_bar[stage], kb * kBlockK, m0);
-#pragma unroll
-          for (int c = 0; c < kTileN / 64; ++c)
-            if (elect_one()) tma_load_2d(sb + c * (64 * kBlockK * 2), &tm_b, &full_bar[stage], n0 + c * 64, kb * kBlockK);
-          if (++stage == kStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          load_a(stage, m0, kb);
+          load_w(stage, n0, kb);
+        }
+        if (++stage == kStages) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
@@ -1263,48 +1311,71 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
   tc_fence_after();
   const uint32_t tmem_base = uniform_u32(*tmem_slot);
 
+  const int n_tiles = args.N / kTileN;
+  const int num_kb = args.K / kBlockK;
+  // The leading W blocks of the pair's first tile ahead of the dependency wait, its A blocks right behind it (see
+  // gemm_f16_kernel).  Both CTAs' copies complete on the leader's barrier, which the leader arms for both.
+  const int pre_kb = args.early_w ? (num_kb < kStages ? num_kb : kStages) : 0;
+  auto load_w = [&](int stage, int n0, int kb) {
+    uint8_t* sb = smem + stage * Cfg::kStageBytes + kABytes;
+    const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
+    if (elect_one()) tma_load_2d_pair(sb, &tm_b, bar, n0, kb * kBlockK);
+    if (elect_one()) tma_load_2d_pair(sb + 64 * kBlockK * 2, &tm_b, bar, n0 + 64, kb * kBlockK);
+  };
+  auto load_a = [&](int stage, int m0, int kb) {
+    const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
+    if (elect_one()) tma_load_2d_pair(smem + stage * Cfg::kStageBytes, &tm_a, bar, kb * kBlockK, m0);
+  };
+  auto tile_rows = [&](int tile) { return (tile / n_tiles) * (2 * kBlockM) + static_cast<int>(cta_rank) * kBlockM; };
+  auto tile_w_cols = [&](int tile) { return (tile % n_tiles) * kTileN + static_cast<int>(cta_rank) * 128; };
+  if (warp == 0) {
+    if (elect_one()) tma_prefetch_desc(&tm_a);
+    if (elect_one()) tma_prefetch_desc(&tm_b);
+    if (elect_one()) tma_prefetch_desc(&tm_out);
+    if (elect_one()) tma_prefetch_desc(&tm_res);
+    for (int kb = 0; kb < pre_kb; ++kb) {
+      if (leader && elect_one()) mbar_arrive_expect_tx(&full_bar[kb], 2 * Cfg::kStageBytes);
+      load_w(kb, tile_w_cols(cluster_id), kb);
+    }
+  }
+
   pdl_wait();  // see gemm_f16_kernel
+  if (warp == 0)
+    for (int kb = 0; kb < pre_kb; ++kb) load_a(kb, tile_rows(cluster_id), kb);
   int M = args.m_rows;
   if (args.m_dev != nullptr) {
     const int md = __ldg(args.m_dev);
     M = uniform_int(md < M ? md : M);
   }
-  const int n_tiles = args.N / kTileN;
   const int m_tiles = (M + 2 * kBlockM - 1) / (2 * kBlockM);
   const int total_tiles = m_tiles * n_tiles;
-  const int num_kb = args.K / kBlockK;
 
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
-    {
-      if (elect_one()) tma_prefetch_desc(&tm_a);
-      if (elect_one()) tma_prefetch_desc(&tm_b);
-      if (elect_one()) tma_prefetch_desc(&tm_out);
-      if (elect_one()) tma_prefetch_desc(&tm_res);
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = cluster_id; tile < total_tiles && ok; tile += num_clusters) {
-        const int m0 = (tile / n_tiles) * (2 * kBlockM) + static_cast<int>(cta_rank) * kBlockM;
-        const int n0 = (tile % n_tiles) * kTileN + static_cast<int>(cta_rank) * 128;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, args.status,
-                                 kStatusGemmProducerTimeout)) {
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    if (cluster_id >= total_tiles && leader) {
+      // No tile for this pair after all: wait for the armed stages, so that no copy is in flight at exit.
+      for (int kb = 0; kb < pre_kb; ++kb)
+        if (!mbar_wait_warp(&full_bar[kb], 0u, abort_flag, args.status, kStatusGemmProducerTimeout)) break;
+    }
+    for (int tile = cluster_id; tile < total_tiles && ok; tile += num_clusters) {
+      const int m0 = tile_rows(tile), n0 = tile_w_cols(tile);
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (tile != cluster_id || kb >= pre_kb) {  // else armed and requested above (stage == kb)
+          if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, args.status, kStatusGemmProducerTimeout)) {
             ok = false;
             break;
           }
-          uint8_t* sa = smem + stage * Cfg::kStageBytes;
-          uint8_t* sb = sa + kABytes;
           // the leader announces the bytes of both CTAs; all copies complete on its barrier
           if (leader && elect_one()) mbar_arrive_expect_tx(&full_bar[stage], 2 * Cfg::kStageBytes);
-          const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          if (elect_one()) tma_load_2d_pair(sa, &tm_a, bar, kb * kBlockK, m0);
-          if (elect_one()) tma_load_2d_pair(sb, &tm_b, bar, n0, kb * kBlockK);
-          if (elect_one()) tma_load_2d_pair(sb + 64 * kBlockK * 2, &tm_b, bar, n0 + 64, kb * kBlockK);
-          if (++stage == kStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          load_a(stage, m0, kb);
+          load_w(stage, n0, kb);
+        }
+        if (++stage == kStages) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
@@ -1570,7 +1641,7 @@ int gemm_pick_split_k(int m_rows, int N, int K, int num_sms) {
   return 1;
 }
 
-int gemm_pick_block_n(int m_rows, int N, int num_sms) {
+int gemm_pick_block_n(int m_rows, int N, int K, int num_sms, bool all_rows) {
   if (g_dbg_force_block_n != 0) return static_cast<int>(g_dbg_force_block_n);
   const int m_tiles = (m_rows + kBlockM - 1) / kBlockM;
   // Prefer the widest tile that still gives every SM at least one tile.
@@ -1578,7 +1649,16 @@ int gemm_pick_block_n(int m_rows, int N, int num_sms) {
   for (int i = 0; i < 3; ++i) {
     const int bn = cands[i];
     if (N % bn != 0) continue;
-    if (static_cast<long long>(m_tiles) * (N / bn) >= num_sms) return bn;
+    const long long tiles = static_cast<long long>(m_tiles) * (N / bn);
+    if (tiles < num_sms) continue;
+    // A 128-column tile's main loop takes hardly longer than a 64-column one's (64 against 54 clocks per MMA), so
+    // with a long K a second wave of 64-column tiles that 128-column ones do not need is the dearer choice: FFN2 of
+    // 8 sequences of 197 tokens (156 tiles of 64 columns or 78 of 128, K = 3072), 12-layer forward 961 us
+    // before, 885 us with this rule and the fp32 sums leaving by bulk store.  Only where every
+    // row is valid: padded rows make no tiles, and 16 sequences of up to 128 tokens, 192 tiles of 64 columns by
+    // their rows and 120 by their tokens, lose 2 % of the forward with 128-column tiles.
+    if (bn == 64 && all_rows && K >= 2048 && N % 128 == 0 && tiles > num_sms) return 128;
+    return bn;
   }
   for (int i = 2; i >= 0; --i)
     if (N % cands[i] == 0) return cands[i];
@@ -1632,7 +1712,7 @@ cudaError_t launch_gemm(const GemmLaunch& g, cudaStream_t stream) {
     a.idesc = make_idesc_f16(kBlockM, 256, 0, 1);
     return launch_ln_gemm(g, a, stream);
   }
-  int bn = g.block_n != 0 ? g.block_n : gemm_pick_block_n(g.m_rows, g.N, g.num_sms);
+  int bn = g.block_n != 0 ? g.block_n : gemm_pick_block_n(g.m_rows, g.N, g.K, g.num_sms, g.all_rows);
   if (bn == 0 || g.N % bn != 0) return cudaErrorInvalidValue;
   a.idesc = make_idesc_f16(kBlockM, bn, 0, 1);
   switch (bn) {
@@ -1665,7 +1745,7 @@ extern "C" int bt_debug_set_gemm_timing(long long* device_buffer) {
 // kernel, 1 = K ranges of an fp32-sum GEMM, 2 = 1 if the pair kernel would take a bias-only GEMM.
 extern "C" int bt_debug_policy(int what, int m_rows, int N, int K, int num_sms) {
   switch (what) {
-    case 0: return bt::gemm_pick_block_n(m_rows, N, num_sms);
+    case 0: return bt::gemm_pick_block_n(m_rows, N, K, num_sms, false);
     case 1: return bt::gemm_pick_split_k(m_rows, N, K, num_sms);
     case 2: {
       bt::GemmLaunch g = {};

@@ -87,6 +87,7 @@ struct GemmLaunch {
   const __half* residual;
   const int* m_dev;  // device int with the number of valid rows, or null
   int m_rows;        // rows allocated in A / out / residual (upper bound of M)
+  bool all_rows = false;  // M is known to be m_rows (a hint for the choice of tile)
   int N;
   int K;
   // fused LayerNorm (BT_EPI_BIAS_RESIDUAL_LAYERNORM): `out` is a scratch of 16 * N/128 bytes per row for the
@@ -109,7 +110,7 @@ struct GemmLaunch {
   int* status;       // device status word
   int num_sms;
 };
-int gemm_pick_block_n(int m_rows, int N, int num_sms);
+int gemm_pick_block_n(int m_rows, int N, int K, int num_sms, bool all_rows);
 cudaError_t launch_gemm(const GemmLaunch& g, cudaStream_t stream);
 
 // ---- fused multi-head attention -----------------------------------------------

@@ -445,23 +445,9 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
   extern __shared__ __align__(1024) uint8_t smem[];
 
   pdl_launch_dependents();
-  pdl_wait();  // batch_idx and the QKV buffer come from earlier kernels
   const int b = blockIdx.z;
   const int head = blockIdx.y;
-  const int seq_start = uniform_int(__ldg(args.batch_idx + b));
-  const int L = uniform_int(__ldg(args.batch_idx + b + 1)) - seq_start;
   const int q0 = blockIdx.x * (kQRows * TILES);
-  if (seq_start < 0 || L < 0 || L > args.max_len || seq_start > args.rows - L) {
-    // offsets that do not describe rows of the allocation: nothing is read or written for this sequence
-    if (threadIdx.x == 0 && args.status != nullptr) atomicCAS(args.status, 0, kStatusBadOffsets);
-    return;
-  }
-  if (q0 >= L) return;  // whole CTA leaves before any barrier / allocation exists
-  if ((smem_u32(smem) & 1023u) != 0u) {
-    if (threadIdx.x == 0 && args.status != nullptr) atomicCAS(args.status, 0, kStatusMhaLoadTimeout + 0x10);
-    return;
-  }
-  const int n_tiles = (TILES == 2 && q0 + kQRows < L) ? 2 : 1;  // query tiles with at least one valid row
 
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kSmemBar);
   uint64_t* q_full = bars;                       // [TILES]
@@ -476,14 +462,6 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
 
   const int warp = uniform_int(static_cast<int>(threadIdx.x >> 5));  // warp-uniform roles: see common.cuh
   const int lane = threadIdx.x & 31;
-  // General masks: the key tiles behind the last key that any row of this query tile may see are left out
-  int kv_rows = L;
-  if (GENERAL && args.gen_kv_bound != nullptr) {
-    const int bound = __ldg(args.gen_kv_bound + b * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x));
-    kv_rows = uniform_int(bound < L ? (bound > 0 ? bound : 1) : L);
-  }
-  const int n_kv = (kv_rows + kKvRows - 1) / kKvRows;
-
   if (threadIdx.x == 0) {
     for (int t = 0; t < TILES; ++t) {
       mbar_init(&q_full[t], 1);
@@ -499,6 +477,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
     *abort_flag = 0;
     fence_mbar_init();
   }
+  if (warp == 0 && lane == 0) tma_prefetch_desc(&tm_qkv);
   if (warp == 1) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
     tmem_relinquish();
@@ -508,14 +487,34 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
   tc_fence_after();
   const uint32_t tmem_base = uniform_u32(*tmem_slot);
 
+  // Everything above is this CTA's own: it runs while the kernel before still does.
+  pdl_wait();  // batch_idx and the QKV buffer come from earlier kernels
+  const int seq_start = uniform_int(__ldg(args.batch_idx + b));
+  const int L = uniform_int(__ldg(args.batch_idx + b + 1)) - seq_start;
+  // offsets that do not describe rows of the allocation: nothing is read or written for this sequence
+  const bool bad_offsets = seq_start < 0 || L < 0 || L > args.max_len || seq_start > args.rows - L;
+  const bool bad_smem = (smem_u32(smem) & 1023u) != 0u;
+  if ((bad_offsets || bad_smem) && threadIdx.x == 0 && args.status != nullptr)
+    atomicCAS(args.status, 0, bad_offsets ? kStatusBadOffsets : kStatusMhaLoadTimeout + 0x10);
+  const bool active = !bad_offsets && !bad_smem && q0 < L;
+  const int n_tiles = (TILES == 2 && q0 + kQRows < L) ? 2 : 1;  // query tiles with at least one valid row
+  // General masks: the key tiles behind the last key that any row of this query tile may see are left out
+  int kv_rows = L;
+  if (GENERAL && args.gen_kv_bound != nullptr) {
+    const int bound = __ldg(args.gen_kv_bound + b * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x));
+    kv_rows = uniform_int(bound < L ? (bound > 0 ? bound : 1) : L);
+  }
+  const int n_kv = (kv_rows + kKvRows - 1) / kKvRows;
+
   const int col_q = head * kHeadDim;
   const int col_k = args.hidden + head * kHeadDim;
   const int col_v = 2 * args.hidden + head * kHeadDim;
 
-  if (warp == 0) {
+  if (!active) {
+    // no rows for this CTA: straight to the teardown
+  } else if (warp == 0) {
     // ------------------------------------------------------------------ loads
     {
-      if (elect_one()) tma_prefetch_desc(&tm_qkv);
       for (int t = 0; t < n_tiles; ++t) {
         if (elect_one()) mbar_arrive_expect_tx(&q_full[t], kTileBytes);
         if (elect_one()) tma_load_2d(smem + Cfg::kSmemQ + t * kTileBytes, &tm_qkv, &q_full[t], col_q, seq_start + q0 + t * kQRows);
