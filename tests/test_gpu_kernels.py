@@ -144,6 +144,48 @@ def test_layernorm_restore(cuda_device):
     assert (got.cpu()[pad] == 0).all()            # exact zeros in padding rows
 
 
+@pytest.mark.parametrize("gb32", [False, True])
+@pytest.mark.parametrize("M,H", [(1, 64), (37, 192), (300, 768), (5, 832), (4096, 768), (4097, 1024)])
+def test_layernorm_of_fp32_sums(cuda_device, M, H, gb32):
+    """fp32 input without bias and residual: a CTA per row up to 4096 rows (widths of one warp, of whole and of part
+    warps), a warp per row above; rows beyond the device-side count stay untouched."""
+    from bytetransformer_b200.encoder import add_bias_residual_layernorm
+    g = torch.Generator().manual_seed(M + H)
+    x = torch.randn(M, H, generator=g) * 3 + 1
+    gamma = torch.empty(H).uniform_(0.5, 1.5, generator=g)
+    beta = torch.empty(H).uniform_(-0.4, 0.4, generator=g)
+    gd, bd = (gamma, beta) if gb32 else (gamma.half(), beta.half())
+    n = max(1, M - 3)
+    m_dev = torch.tensor([n], dtype=torch.int32, device=cuda_device)
+    got = add_bias_residual_layernorm(x.to(cuda_device), None, None, gd.to(cuda_device), bd.to(cuda_device), m_dev=m_dev).cpu()
+    want = torch.nn.functional.layer_norm(x.double(), (H,), gd.double(), bd.double(), eps=1e-6)
+    # fp16 rounding of values up to about 6, and fp32 statistics
+    assert ((got[:n].double() - want[:n]).abs() <= want[:n].abs() * 2.0 ** -11 + 1e-5).all()
+    assert (got[n:] == 0).all()
+
+
+def test_layernorm_of_fp32_sums_restore(cuda_device):
+    from bytetransformer_b200.encoder import add_bias_residual_layernorm_restore, build_offsets
+    B, S, H = 4, 20, 768
+    lens = [7, 20, 0, 1]
+    mask = _mask_from_lens(lens, S)
+    T = sum(lens)
+    g = torch.Generator().manual_seed(17)
+    x = torch.randn(T, H, generator=g) * 2
+    gamma = torch.empty(H).uniform_(0.5, 1.5, generator=g).half()
+    beta = torch.empty(H).uniform_(-0.4, 0.4, generator=g).half()
+    bi, _ = build_offsets(mask.to(cuda_device))
+    got = add_bias_residual_layernorm_restore(x.to(cuda_device), None, None, gamma.to(cuda_device), beta.to(cuda_device),
+                                              bi, B, S).cpu()
+    want = torch.nn.functional.layer_norm(x.double(), (H,), gamma.double(), beta.double(), eps=1e-6)
+    row = 0
+    for b, n in enumerate(lens):
+        w = want[row:row + n]
+        assert ((got[b, :n].double() - w).abs() <= w.abs() * 2.0 ** -11 + 1e-5).all()
+        assert (got[b, n:] == 0).all()
+        row += n
+
+
 @pytest.mark.parametrize("kind", ["erf", "tanh"])
 def test_add_bias_gelu(cuda_device, kind):
     from bytetransformer_b200.encoder import add_bias_gelu_
