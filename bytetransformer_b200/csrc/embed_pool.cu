@@ -30,8 +30,8 @@ embedding_layernorm_kernel(const __half* __restrict__ word_emb, const __half* __
                            const int* __restrict__ type_ids, const int* __restrict__ position_ids,
                            __half* __restrict__ out, int rows, int seq_len, int hidden, int vocab, int max_pos,
                            int n_types, float eps, const int* __restrict__ word_idx, const int* __restrict__ t_dev) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();  // only now: second kernel of a call, see MhaLaunch::early_offsets
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int nvec = hidden >> 3;

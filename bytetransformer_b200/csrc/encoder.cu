@@ -333,8 +333,9 @@ struct GeneralMask {
 };
 
 static int run_mha(bt_handle h, const __half* qkv, __half* ctx, const int* batch_idx, int B, int max_len, int rows,
-                   cudaStream_t stream, const GeneralMask* gm = nullptr) {
+                   cudaStream_t stream, bool in_forward, const GeneralMask* gm = nullptr) {
   MhaLaunch a;
+  a.early_offsets = in_forward;
   if (!h->tmap(&a.tm_qkv, qkv, rows, 3 * static_cast<uint64_t>(h->hidden), 64, 128))
     return fail(h, BT_ERR_CUDA, "cuTensorMapEncodeTiled failed for qkv");
   a.has_tm_ctx = h->tmap(&a.tm_ctx, ctx, rows, static_cast<uint64_t>(h->hidden), 64, 32);
@@ -400,7 +401,7 @@ static int run_layer(bt_handle h, int layer, const __half* x_in, __half* x_out, 
   if ((rc = run_gemm(h, BT_PROF_GEMM_QKV, x_in, w.qkv_kernel, ws.qkv, w.qkv_bias, nullptr, m_dev, rows, 3 * H, H, BT_EPI_BIAS, 0,
                      stream)) != BT_OK)
     return rc;
-  if ((rc = run_mha(h, ws.qkv, ws.ctx, batch_idx, B, S_or_maxlen, rows, stream, gm)) != BT_OK) return rc;
+  if ((rc = run_mha(h, ws.qkv, ws.ctx, batch_idx, B, S_or_maxlen, rows, stream, true, gm)) != BT_OK) return rc;
   // LayerNorm rides in the GEMM kernel (clusters of H/256 CTAs per 128-row tile) once there are
   // enough row tiles to occupy the machine that way; below that the narrow-tile GEMM followed by
   // the row kernel spreads the few rows over more SMs.
@@ -1039,7 +1040,7 @@ int bt_attention(bt_handle h, const void* qkv, void* ctx, const int* batch_idx, 
     if (rc != BT_OK) return rc;
   }
   return run_mha(h, reinterpret_cast<const __half*>(qkv), reinterpret_cast<__half*>(ctx), batch_idx, batch_size,
-                 max_len, rows_allocated, reinterpret_cast<cudaStream_t>(stream));
+                 max_len, rows_allocated, reinterpret_cast<cudaStream_t>(stream), false);
 }
 
 int bt_add_bias_residual_layernorm(const void* x, int x_fp32, const void* bias, const void* residual, const void* gamma,

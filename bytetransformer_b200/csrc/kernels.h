@@ -123,6 +123,10 @@ struct MhaLaunch {
   int batch;
   int max_len;         // upper bound of every sequence length
   int rows = 0;        // rows allocated in qkv / ctx
+  // batch_idx may be read before the dependency wait: the kernel that wrote it has completed when this one can start.
+  // True inside a forward call: the offsets come from the call's first kernel (or from before the call), which is
+  // launched plainly, and the second kernel lets its successor start only after its own dependency wait.
+  bool early_offsets = false;
   int head_num;
   int hidden;          // H = head_num * 64
   float scale_log2e;   // log2(e) / sqrt(64) / tao

@@ -82,6 +82,8 @@ struct MhaArgs {
   int* status;
   int rows;     // rows allocated in qkv / ctx
   int max_len;  // upper bound of every sequence length
+  int tma_out;        // the second tensor map describes ctx: whole 32-row output slabs leave by bulk store
+  int early_offsets;  // batch_idx may be read before the dependency wait (see launch_mha)
   // General-mask variant (GENERAL = true): every sequence has `gen_seq_len` rows; the score of
   // (query q, key k) gets  attn_bias[head, q, k] + (1 - mask[b, q, k]) * -10000  added after scaling,
   // the rule of the reference's unfused softmax (bytetransformer/include/softmax.h:41-45).
@@ -192,21 +194,20 @@ __device__ __forceinline__ float chunk_max(const uint32_t (&v)[32], int cbase, i
   }
   return fmaxf(m0, m1);
 }
-template <bool MASKED>
-__device__ __forceinline__ float tile_row_max(uint32_t t_s, int kv_valid) {
+__device__ __forceinline__ float tile_row_max(uint32_t t_s) {
   uint32_t va[32], vb[32];
   tmem_ld_32x32(t_s, va);
   tmem_ld_wait();
   tmem_ld_32x32(t_s + 32, vb);
-  float mx = chunk_max<MASKED>(va, 0, kv_valid);
+  float mx = chunk_max<false>(va, 0, kKvRows);
   tmem_ld_wait();
   tmem_ld_32x32(t_s + 64, va);
-  mx = fmaxf(mx, chunk_max<MASKED>(vb, 32, kv_valid));
+  mx = fmaxf(mx, chunk_max<false>(vb, 32, kKvRows));
   tmem_ld_wait();
   tmem_ld_32x32(t_s + 96, vb);
-  mx = fmaxf(mx, chunk_max<MASKED>(va, 64, kv_valid));
+  mx = fmaxf(mx, chunk_max<false>(va, 64, kKvRows));
   tmem_ld_wait();
-  return fmaxf(mx, chunk_max<MASKED>(vb, 96, kv_valid));
+  return fmaxf(mx, chunk_max<false>(vb, 96, kKvRows));
 }
 
 // One 32-column chunk of S -> 16 cells of fp16 pairs, plus this chunk's row sum (2^x in fp32, one
@@ -233,27 +234,55 @@ __device__ __forceinline__ float chunk_probs(const uint32_t (&v)[32], int cbase,
 
 // Second pass over one S tile, from the last chunk to the first; P chunk c lands in cells
 // [64 + 16c, 64 + 16c + 16) of the same tile, which lie in chunks that were already read.
-template <bool MASKED>
-__device__ __forceinline__ float tile_probs(uint32_t t_s, int kv_valid, float c, float m_ref) {
+__device__ __forceinline__ float tile_probs(uint32_t t_s, float c, float m_ref) {
   const uint32_t t_p = t_s + 64;
   uint32_t va[32], vb[32], pk[16];
   float l = 0.f;
   tmem_ld_32x32(t_s + 96, va);
   tmem_ld_wait();
   tmem_ld_32x32(t_s + 64, vb);  // in flight while chunk 3 is processed
-  l += chunk_probs<MASKED>(va, 96, kv_valid, c, m_ref, pk);
+  l += chunk_probs<false>(va, 96, kKvRows, c, m_ref, pk);
   tmem_ld_wait();               // chunk 2 is in registers: its cells may now be overwritten
   tmem_st_32x16(t_p + 48, pk);
   tmem_ld_32x32(t_s + 32, va);
-  l += chunk_probs<MASKED>(vb, 64, kv_valid, c, m_ref, pk);
+  l += chunk_probs<false>(vb, 64, kKvRows, c, m_ref, pk);
   tmem_ld_wait();
   tmem_st_32x16(t_p + 32, pk);
   tmem_ld_32x32(t_s, vb);
-  l += chunk_probs<MASKED>(va, 32, kv_valid, c, m_ref, pk);
+  l += chunk_probs<false>(va, 32, kKvRows, c, m_ref, pk);
   tmem_ld_wait();
   tmem_st_32x16(t_p + 16, pk);
-  l += chunk_probs<MASKED>(vb, 0, kv_valid, c, m_ref, pk);
+  l += chunk_probs<false>(vb, 0, kKvRows, c, m_ref, pk);
   tmem_st_32x16(t_p, pk);
+  tmem_st_wait();
+  return l;
+}
+
+// The two passes over a tail tile (kv_valid < 128 keys), by its chunks of 32 keys that hold any: a rolled loop, because
+// the calls that end here are short (a handful of items of a few dozen keys) and run once per SM - chunks without
+// keys and instructions fetched for nothing were half of the kernel's time there.  P cells beyond the last chunk stay
+// what they were; the P V product only runs over the 16-key steps that hold keys.
+__device__ __forceinline__ float tail_row_max(uint32_t t_s, int kv_valid) {
+  float mx = -INFINITY;
+#pragma unroll 1
+  for (int c0 = 0; c0 < kv_valid; c0 += 32) {
+    uint32_t v[32];
+    tmem_ld_32x32(t_s + c0, v);
+    tmem_ld_wait();
+    mx = fmaxf(mx, chunk_max<true>(v, c0, kv_valid));
+  }
+  return mx;
+}
+__device__ __forceinline__ float tail_probs(uint32_t t_s, int kv_valid, float c, float m_ref) {
+  float l = 0.f;
+#pragma unroll 1
+  for (int c0 = (kv_valid - 1) & ~31; c0 >= 0; c0 -= 32) {  // last to first: see tile_probs
+    uint32_t v[32], pk[16];
+    tmem_ld_32x32(t_s + c0, v);
+    tmem_ld_wait();
+    l += chunk_probs<true>(v, c0, kv_valid, c, m_ref, pk);
+    tmem_st_32x16(t_s + 64 + (c0 >> 1), pk);
+  }
   tmem_st_wait();
   return l;
 }
@@ -435,7 +464,7 @@ __device__ __forceinline__ float tile_add_bias_row_max(uint32_t t_s, uint4 (&bia
 // its tile layout (an instantiation of its own: the registers that hold the bias would cost the other two).
 template <int MODE>
 __global__ void __launch_bounds__(MhaCfg::kThreads, 2)
-mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
+mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_ctx, const MhaArgs args) {
   using Cfg = MhaCfg;
   constexpr bool GENERAL = MODE != 0;
   constexpr int TILES = 1;  // query tiles per CTA (the loops over `t` below have one trip)
@@ -466,7 +495,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
     for (int t = 0; t < TILES; ++t) {
       mbar_init(&q_full[t], 1);
       mbar_init(&s_full[t], 1);
-      mbar_init(&p_full[t], 128);
+      mbar_init(&p_full[t], 4);  // one arrival per softmax warp
     }
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&k_full[s], 1);
@@ -487,10 +516,20 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
   tc_fence_after();
   const uint32_t tmem_base = uniform_u32(*tmem_slot);
 
-  // Everything above is this CTA's own: it runs while the kernel before still does.
-  pdl_wait();  // batch_idx and the QKV buffer come from earlier kernels
-  const int seq_start = uniform_int(__ldg(args.batch_idx + b));
-  const int L = uniform_int(__ldg(args.batch_idx + b + 1)) - seq_start;
+  // Everything above is this CTA's own: it runs while the kernel before still does, and so does the round trip
+  // for the offsets where the kernel that wrote them is known to have completed.
+  int off0 = 0, off1 = 0;
+  if (args.early_offsets) {
+    off0 = __ldg(args.batch_idx + b);
+    off1 = __ldg(args.batch_idx + b + 1);
+  }
+  pdl_wait();  // the QKV buffer comes from the kernel before
+  if (!args.early_offsets) {
+    off0 = __ldg(args.batch_idx + b);
+    off1 = __ldg(args.batch_idx + b + 1);
+  }
+  const int seq_start = uniform_int(off0);
+  const int L = uniform_int(off1) - seq_start;
   // offsets that do not describe rows of the allocation: nothing is read or written for this sequence
   const bool bad_offsets = seq_start < 0 || L < 0 || L > args.max_len || seq_start > args.rows - L;
   const bool bad_smem = (smem_u32(smem) & 1023u) != 0u;
@@ -551,10 +590,12 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
         const uint32_t sk = s_k + stage * kTileBytes;
         umma_s_tile(tmem_base + t * 128, smem_desc(kDescK, sq), smem_desc(kDescK, sk), kIdescS, &s_full[t]);
       };
-      auto issue_pv = [&](int t, int stage, bool accumulate) {
+      // `keys`: keys of the tile that exist (only the 16-key steps that hold any are multiplied)
+      auto issue_pv = [&](int t, int stage, bool accumulate, int keys) {
         const uint32_t tp = tmem_base + t * 128 + Cfg::kTmemPOff;  // 8 cells (16 keys) per MMA
         const uint32_t sv = s_v + stage * kTileBytes;
-        umma_pv_tile(tmem_base + Cfg::kTmemO + t * 64, tp, smem_desc(kDescV, sv), kIdescO, accumulate ? 1u : 0u, kKvRows / 16);
+        umma_pv_tile(tmem_base + Cfg::kTmemO + t * 64, tp, smem_desc(kDescV, sv), kIdescO, accumulate ? 1u : 0u,
+                     static_cast<uint32_t>((keys + 15) >> 4));
       };
       bool ok = true;
       for (int t = 0; t < n_tiles && ok; ++t)
@@ -576,7 +617,8 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
         if (!mbar_wait_warp(&p_full[0], jpar, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
         if (!mbar_wait_warp(&v_full[st], ph, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
         tc_fence_after();
-        issue_pv(0, st, j > 0);
+        const int keys = min(kKvRows, L - j * kKvRows);
+        issue_pv(0, st, j > 0, keys);
         if (more) {
           if (!mbar_wait_warp(&k_full[st_n], ph_n, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
           tc_fence_after();
@@ -586,7 +628,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
         if (n_tiles == 2) {
           if (!mbar_wait_warp(&p_full[1], jpar, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
           tc_fence_after();
-          issue_pv(1, st, j > 0);
+          issue_pv(1, st, j > 0, keys);
         }
         if (elect_one()) umma_commit(&kv_empty[st]);  // every MMA that reads K/V stage `st` has been issued
         if (n_tiles == 2 && more) issue_s(1, st_n);
@@ -654,12 +696,12 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
             mx = c * (full_tile ? tile_add_bias_row_max<false>(t_s, bias_q, bt, bw, kv_valid, args.gen_inv_scale)
                                 : tile_add_bias_row_max<true>(t_s, bias_q, bt, bw, kv_valid, args.gen_inv_scale));
           else
-            mx = c * (full_tile ? tile_row_max<false>(t_s, kv_valid) : tile_row_max<true>(t_s, kv_valid));
+            mx = c * (full_tile ? tile_row_max(t_s) : tail_row_max(t_s, kv_valid));
         } else if (GENERAL && use_bits)
           mx = c * (full_tile ? tile_row_max_bits<false>(t_s, kv_valid, bw, bits_neg)
                               : tile_row_max_bits<true>(t_s, kv_valid, bw, bits_neg));
         else
-          mx = c * (full_tile ? tile_row_max<false>(t_s, kv_valid) : tile_row_max<true>(t_s, kv_valid));
+          mx = c * (full_tile ? tile_row_max(t_s) : tail_row_max(t_s, kv_valid));
         if (j == 0) {
           m_ref = mx;
         } else {
@@ -686,8 +728,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
           l_run += full_tile ? tile_probs_bits<false>(t_s, kv_valid, c, m_ref, bw, bits_neg)
                              : tile_probs_bits<true>(t_s, kv_valid, c, m_ref, bw, bits_neg);
         else
-          l_run += full_tile ? tile_probs<false>(t_s, kv_valid, c, m_ref)
-                             : tile_probs<true>(t_s, kv_valid, c, m_ref);
+          l_run += full_tile ? tile_probs(t_s, c, m_ref) : tail_probs(t_s, kv_valid, c, m_ref);
         if (!full_tile && t == 0) {
           // tail tile: blank the V rows of keys that do not belong to this sequence
           // (tile 0's PV is issued before tile 1's, so tile 0's warpgroup does it for both)
@@ -695,7 +736,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
             ok = false;
             break;
           }
-          if (r >= kv_valid) {
+          if (r >= kv_valid && r < ((kv_valid + 15) & ~15)) {
             uint4* vr = reinterpret_cast<uint4*>(smem + Cfg::kSmemV + stage * kTileBytes + r * 128);
 #pragma unroll
             for (int i = 0; i < 8; ++i) vr[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -703,7 +744,8 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
           fence_proxy_async_smem();
         }
         tc_fence_before();
-        mbar_arrive(&p_full[t]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[t]);
         if (++stage == kStages) {
           stage = 0;
           phase ^= 1u;
@@ -712,25 +754,45 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const MhaArgs args) {
       if (ok) ok = mbar_wait_bounded(o_done, 0, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
       tc_fence_after();
       if (ok) {
-        const int q_row = q0 + t * kQRows + r;
+        // O / row sum -> fp16 -> global memory by way of the Q tile, which no MMA reads any more (o_done covers the
+        // last S as well): as in the persistent kernel, a whole 32-row slab leaves by one bulk store, a ragged one by
+        // stores that cover whole 128-byte lines.  Row by row from the threads (32 lines per instruction) it took
+        // 1.0-1.3k clocks of a short item and, with the machine full, 5.3k of a 512-token one.
         const float inv = 1.0f / l_run;
-        uint4* dst = reinterpret_cast<uint4*>(args.ctx + static_cast<size_t>(seq_start + q_row) * args.hidden +
-                                              head * kHeadDim);
+        const int row0 = q0 + t * kQRows + quarter * 32;  // first query row of this warp's slab, within the sequence
+        uint8_t* stage_out = smem + Cfg::kSmemQ + t * kTileBytes + quarter * (32 * 128);
 #pragma unroll
         for (int cb = 0; cb < kHeadDim; cb += 32) {
           uint32_t v[32];
           tmem_ld_32x32(t_o + cb, v);
           tmem_ld_wait();
-          if (q_row < L) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              uint4 w;
-              w.x = pack_half2(__uint_as_float(v[u * 8 + 0]) * inv, __uint_as_float(v[u * 8 + 1]) * inv);
-              w.y = pack_half2(__uint_as_float(v[u * 8 + 2]) * inv, __uint_as_float(v[u * 8 + 3]) * inv);
-              w.z = pack_half2(__uint_as_float(v[u * 8 + 4]) * inv, __uint_as_float(v[u * 8 + 5]) * inv);
-              w.w = pack_half2(__uint_as_float(v[u * 8 + 6]) * inv, __uint_as_float(v[u * 8 + 7]) * inv);
-              dst[(cb >> 3) + u] = w;
-            }
+          for (int u = 0; u < 4; ++u) {
+            uint4 w;
+            w.x = pack_half2(__uint_as_float(v[u * 8 + 0]) * inv, __uint_as_float(v[u * 8 + 1]) * inv);
+            w.y = pack_half2(__uint_as_float(v[u * 8 + 2]) * inv, __uint_as_float(v[u * 8 + 3]) * inv);
+            w.z = pack_half2(__uint_as_float(v[u * 8 + 4]) * inv, __uint_as_float(v[u * 8 + 5]) * inv);
+            w.w = pack_half2(__uint_as_float(v[u * 8 + 6]) * inv, __uint_as_float(v[u * 8 + 7]) * inv);
+            *reinterpret_cast<uint4*>(stage_out + lane * 128 + ((((cb >> 3) + u) ^ (lane & 7)) << 4)) = w;
+          }
+        }
+        const bool whole_slab = args.tma_out != 0 && row0 + 32 <= L;
+        if (whole_slab) fence_proxy_async_smem();
+        __syncwarp();
+        if (whole_slab) {
+          if (lane == 0) {
+            tma_store_2d(&tm_ctx, stage_out, col_q, seq_start + row0);
+            tma_store_commit();
+            tma_store_wait_all();
+          }
+        } else {
+          const int sub = lane >> 3, unit = lane & 7;  // row within a group of four, 16-byte unit of the row
+          __half* out_base = args.ctx + static_cast<size_t>(seq_start + row0) * args.hidden + col_q + unit * 8;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const int row = 4 * k + sub;
+            const uint4 w = *reinterpret_cast<const uint4*>(stage_out + row * 128 + ((unit ^ (row & 7)) << 4));
+            if (row0 + row < L) *reinterpret_cast<uint4*>(out_base + static_cast<size_t>(row) * args.hidden) = w;
           }
         }
       }
@@ -786,6 +848,7 @@ struct MhaPersistentArgs {
   int rows;     // rows allocated in qkv / ctx
   int max_len;  // upper bound of every sequence length
   int tma_out;  // the kernel's second tensor map describes ctx: whole 32-row output slabs leave by bulk store
+  int early_offsets;  // batch_idx may be read before the dependency wait (see launch_mha)
 };
 
 // Finds item n = (sequence b, query tile qt, head h); items are numbered sequence by sequence, inside
@@ -949,7 +1012,10 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = uniform_u32(*tmem_slot);
-  pdl_wait();  // batch_idx and the QKV buffer come from earlier kernels
+  // The offsets' round trip (and, per warp, the search for its first item) goes ahead of the wait for the kernel that
+  // writes the QKV buffer where the kernel that wrote the offsets is known to have completed: only the roles' first
+  // touch of other memory has to come after it.
+  if (!args.early_offsets) pdl_wait();
 
   const int G = static_cast<int>(gridDim.x), cta = static_cast<int>(blockIdx.x);
   int cur_b = 0, cur_first = 0, seq_start = 0, L = 0, qt = 0, head = 0;
@@ -963,8 +1029,9 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int round = 0; ok && decode_item(args, snake_item(round, cta, G), cur_b, cur_first, seq_start, L, qt, head, true);
-           ++round) {
+      bool have = decode_item(args, snake_item(0, cta, G), cur_b, cur_first, seq_start, L, qt, head, true);
+      if (args.early_offsets) pdl_wait();
+      for (int round = 0; ok && have; ++round) {
         {
           L = uniform_int(L);
           seq_start = uniform_int(seq_start);
@@ -999,6 +1066,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
           }
           }
         }
+        have = decode_item(args, snake_item(round + 1, cta, G), cur_b, cur_first, seq_start, L, qt, head, true);
       }
     } else if (warp == 5) {
       // -------------------------------------------------------------- MMA issue
@@ -1320,6 +1388,7 @@ cudaError_t launch_persistent(const MhaLaunch& a, cudaStream_t stream) {
   args.rows = a.rows;
   args.max_len = a.max_len;
   args.tma_out = a.has_tm_ctx ? 1 : 0;
+  args.early_offsets = a.early_offsets ? 1 : 0;
   const long long items_max =
       static_cast<long long>(a.batch) * a.head_num * ((a.max_len + kQRows - 1) / kQRows);  // upper bound
   long long grid = 2LL * sms[dev];
@@ -1341,7 +1410,8 @@ cudaError_t launch_per_item(const MhaLaunch& a, const MhaArgs& args, cudaStream_
     attr_set[dev] = true;
   }
   dim3 grid((a.max_len + kQRows - 1) / kQRows, a.head_num, a.batch);
-  return launch_pdl(mha_fwd_kernel<MODE>, grid, dim3(MhaCfg::kThreads), MhaCfg::kSmemBytes, stream, a.tm_qkv, args);
+  return launch_pdl(mha_fwd_kernel<MODE>, grid, dim3(MhaCfg::kThreads), MhaCfg::kSmemBytes, stream, a.tm_qkv,
+                    a.has_tm_ctx ? a.tm_ctx : a.tm_qkv, args);
 }
 
 }  // namespace
@@ -1356,6 +1426,8 @@ cudaError_t launch_mha(const MhaLaunch& a, cudaStream_t stream) {
   args.status = a.status;
   args.rows = a.rows;
   args.max_len = a.max_len;
+  args.tma_out = a.has_tm_ctx ? 1 : 0;
+  args.early_offsets = a.early_offsets ? 1 : 0;
   args.gen_mask = a.gen_mask;
   args.gen_bias = a.gen_bias;
   args.gen_seq_len = a.max_len;

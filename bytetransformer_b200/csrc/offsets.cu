@@ -104,8 +104,8 @@ build_offsets_kernel(const __half* __restrict__ mask, int B, int S, int* __restr
 __global__ void __launch_bounds__(256)
 pack_rows_kernel(const uint4* __restrict__ padded, uint4* __restrict__ packed, const int* __restrict__ batch_idx,
                  int S, int vec_per_row) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();  // only now: second kernel of a call, see MhaLaunch::early_offsets
   const int b = blockIdx.y;
   const int off = __ldg(batch_idx + b);
   const int len = __ldg(batch_idx + b + 1) - off;
@@ -197,8 +197,8 @@ mask_is_right_padded_kernel(const __half* __restrict__ mask, int B, int S, int* 
 __global__ void __launch_bounds__(256)
 mask_bits_kernel(const __half* __restrict__ mask, int S, long long rows, uint32_t* __restrict__ bits,
                  int stride_words, int* __restrict__ flag, int* __restrict__ bound) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();  // only now: second kernel of a call, see MhaLaunch::early_offsets
   const int lane = threadIdx.x & 31;
   const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
