@@ -1006,6 +1006,8 @@ int bt_gemm_layernorm(bt_handle h, const void* A, const void* W, const void* bia
                                    reinterpret_cast<cudaStream_t>(stream));
   if (me != cudaSuccess) return fail_cuda(h, me, "memset of the LayerNorm statistics scratch");
   LnArgs ln{1u, reinterpret_cast<__half*>(out), gamma, beta, gamma_beta_fp32 != 0, eps};
+  pdl_next_launch_plain();  // as in bt_gemm
+  h->all_rows = false;
   return run_gemm(h, BT_PROF_GEMM_OTHER, reinterpret_cast<const __half*>(A), W, reinterpret_cast<__half*>(scratch_f32),
                   bias, reinterpret_cast<const __half*>(residual), m_dev, m_rows, N, K, BT_EPI_BIAS_RESIDUAL_LAYERNORM, 0,
                   reinterpret_cast<cudaStream_t>(stream), &ln);

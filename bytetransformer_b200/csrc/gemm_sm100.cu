@@ -21,7 +21,8 @@
 //               = MN-major for UMMA, so the reference's [in,out] weight layout is consumed
 //               as is, no transposed copy) into a 128B-swizzled shared-memory ring.
 //   warp 1      allocates tensor memory and (leader only, for the pair kernel) issues the
-//               MMAs from one lane; accumulators are double buffered in tensor memory
+//               MMAs (the warp walks the loop, an elected lane's instructions take effect: see
+//               common.cuh); accumulators are double buffered in tensor memory
 //               (2 x 256 columns) so the epilogue of tile i overlaps the main loop of i+1.
 //   warps 2..9  epilogue: tcgen05.ld -> +bias -> GELU / +residual -> fp16 (or fp32)
 //               -> 128B-swizzled staging rows in shared memory -> TMA bulk store

@@ -19,7 +19,7 @@
 // no counterpart here).  Only `batch_idx` tells where sequences start and end;
 // as in the reference's packed kernels the mask tensor is not consulted again.
 //
-// Common to both kernels: one warp issues TMA loads, one thread issues the tcgen05 MMAs (and its warp
+// Common to both kernels: one warp issues TMA loads, one warp the tcgen05 MMAs (through an elected lane; it also
 // owns the tensor-memory allocation), four softmax warps own one query row per thread.
 //   S = Q K^T      128x128x64, both operands from shared memory -> tensor memory, 128 fp32 columns
 //   P = 2^(c*S-m)  fp16 pairs written to tensor memory with tcgen05.st
@@ -38,14 +38,17 @@
 // past the last row) make the sequence a no-op and set kStatusBadOffsets: nothing outside the
 // buffers is read or written.
 //
-// What the measurements on B200 say about the softmax (it, not the tensor core, bounds both kernels:
-// the MMAs of a 128x128 tile take ~540 clocks when two CTAs interleave them, a tile takes ~1900):
-// the special-function unit delivers one warp-wide ex2 per 4 clocks and scheduler, but a single warp
-// only reaches one per ~10 clocks (two warps 6.9, three 4.9), and tensor memory holds S, O and P for
-// two CTAs, i.e. two softmax warps per scheduler.  Halving the exponential work (ex2.f16x2 runs at
-// half rate, so it gains nothing; a polynomial on the FMA pipe for a quarter of the elements: 5 %
-// slower), 256-row ping-pong tiles and two threads per row with an exchange through shared memory
-// (25 % slower) were measured and dropped.
+// What the measurements on B200 say about the softmax (it, not the tensor core, bounds both kernels: the MMAs of a
+// 128x128 tile take ~540 clocks when two CTAs interleave them): in the persistent kernel a 128-key tile takes 1.6 us
+// (3.1k clocks) per CTA with two CTAs per SM, an item another ~3 us; the tile's tensor-memory loads, maximum, 128
+// exponentials, packing and stores alone, two CTAs per SM and MMAs running beside them, take 1.72k clocks.  Tensor
+// memory holds S, O and P for two CTAs, i.e. two softmax warps per scheduler.  Measured and dropped because they did
+// not help: exponentials partly on the FMA pipe (degree-5 polynomial, packed pairs, one pair in 8 / 4 / 3: 403 / 403 /
+// 421 against 403 us per 79k-token launch), ex2.f16x2, 256-row ping-pong tiles, two threads per row with an exchange
+// through shared memory (25 % slower), reading an item's O out behind the next item's exponentials (level to 5 %
+// slower), items handed out by the loader through shared memory (-1 % at 512 tokens, +0.4 % for one sequence),
+// masking a tail tile by groups of keys under branches (spills 624 bytes; the 128 half-rate compares and selects
+// cost ~1k clocks per tail tile).
 #include "common.cuh"
 #include "kernels.h"
 
@@ -1236,10 +1239,9 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
           m_ref = m_new;
         }
         // ---- probabilities: fp16 pairs for P's own columns, fp32 row sum
-        float l0 = 0.f, l1 = 0.f;
+        float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
         uint32_t pk[64];
 #pragma unroll
-        float l2 = 0.f, l3 = 0.f;
         for (int i = 0; i < 64; ++i) {
           float t0, t1;
           fma2(t0, t1, __uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1]), c, -m_ref);

@@ -48,6 +48,21 @@ def test_embedding_ids_outside_the_tables_are_clamped(cuda_device):
     assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("B,H", [(25, 768), (27, 832), (150, 66), (296, 64), (24, 2560)])
+def test_pooler_four_sequences_per_cta(cuda_device, B, H):
+    """From a CTA for half of the SMs on, four sequences share a CTA (B not a multiple of 4, widths that are not
+    multiples of 64 or of the load batch; 2560 is too wide for it): against a matrix product in 64 bits."""
+    from bytetransformer_b200.encoder import pooler
+    g = torch.Generator().manual_seed(H + B)
+    y = torch.randn(B, 3, H, generator=g).half()
+    W = (torch.randn(H, H, generator=g) * 0.05).half()
+    b = torch.empty(H).uniform_(-0.4, 0.4, generator=g).half()
+    got = pooler(y.to(cuda_device), W.to(cuda_device), b.to(cuda_device)).cpu().double()
+    want = torch.tanh(y[:, 0].double() @ W.double() + b.double())
+    # fp16 rounding of the result, fp32 sums of H products of size about 0.05
+    assert ((got - want).abs() <= want.abs() * 2.0 ** -11 + H * 2.0 ** -24 + 2.0 ** -24).all()
+
+
 @pytest.mark.parametrize("B,S,H", [(1, 5, 64), (7, 33, 768), (16, 128, 1024)])
 def test_pooler(cuda_device, B, S, H):
     from bytetransformer_b200.encoder import pooler

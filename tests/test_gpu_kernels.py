@@ -299,6 +299,44 @@ def test_attention(enc, cuda_device, lens):
     assert got[T:].abs().max().item() == 0.0 if rows > T else True
 
 
+@pytest.mark.parametrize("M", [1, 31, 32, 33, 1536, 1537, 1600])
+def test_gemm_fp32_sums_narrow_tiles(enc, cuda_device, M):
+    """64-column fp32 tiles leave by bulk store slab by slab (whole slabs of 32 rows) or row by row (the last one);
+    from 1537 rows on a long K takes 128-column tiles instead of a second wave of 64-column ones."""
+    from bytetransformer_b200 import _abi
+    g = torch.Generator().manual_seed(M)
+    N, K = 768, 3072
+    a = torch.randn(M, K, generator=g).half().to(cuda_device)
+    w = (torch.randn(K, N, generator=g) * 0.05).half().to(cuda_device)
+    bias = torch.empty(N).uniform_(-0.4, 0.4, generator=g).half().to(cuda_device)
+    res = torch.randn(M, N, generator=g).half().to(cuda_device)
+    got = enc.gemm(a, w, bias, res, epilogue=_abi.BT_EPI_BIAS_RESIDUAL_F32OUT)
+    want = a.double() @ w.double() + bias.double() + res.double()
+    # fp32 accumulation of 3072 products of size about 0.05: far below 1e-3 of a sum of size about 3
+    assert (got.double() - want).abs().max().item() <= 1e-3
+    assert enc.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 31, 32, 33, 64, 65, 96, 97, 127, 128, 129, 160, 255])
+def test_attention_tail_tiles(enc, cuda_device, n):
+    """One CTA per item: a tail tile is walked by the 32-key chunks and 16-key steps that hold keys, and a slab of 32
+    output rows leaves whole or row by row; the second sequence must not be touched by the first one's tail."""
+    import bytetransformer_b200._abi as abi
+    from oracle.bert_oracle import attention_packed
+    g = torch.Generator().manual_seed(n)
+    cu = [0, n, n + 3]
+    qkv = torch.randn(n + 3, 3 * enc.head_num * enc.head_size, generator=g).half()
+    lib = abi.load()
+    lib.bt_debug_set_mha_tiles(1)
+    try:
+        got = enc.attention(qkv.to(cuda_device), torch.tensor(cu, dtype=torch.int32, device=cuda_device), n + 3)
+    finally:
+        lib.bt_debug_set_mha_tiles(0)
+    want = attention_packed(qkv.float(), cu, enc.head_num, enc.head_size)
+    assert enc.device_status() == 0
+    assert_close_fp16(got, want, f"attention tail {n}", max_abs=5e-3, mean_abs=3e-4)
+
+
 def test_attention_twice_bit_identical(enc, cuda_device):
     lens = [300, 77, 129]
     cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]).astype(np.int32), device=cuda_device)
