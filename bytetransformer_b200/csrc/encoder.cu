@@ -125,15 +125,17 @@ struct bt_encoder_s {
   long long launches[BT_PROF_KINDS] = {};
   bool prof_on = false;
   // LayerNorm inside the attention-output / FFN2 GEMM kernel (bt_debug_set_fused_layernorm):
-  // 0 never, 1 from `fused_ln_min_tiles` 128-row tiles (of allocated rows) upwards, 2 always.  Measured on
-  // B200 (12 layers, hidden 768, batch 16 through the padded entry point, ms per forward without / with the
-  // fused kernels): 32 row tiles 1.11 / 1.16, 40 tiles 1.45 / 1.28, 48 tiles 1.42 / 1.31, 64 tiles 1.54 / 1.46,
-  // 80 tiles 2.08 / 1.99, 96 tiles 2.14 / 2.10; at 141-148 tiles per call the fused kernels are worth 3 % of the
-  // forward.  Below ~40 tiles the exchange of row statistics between CTAs lengthens the only wave by more
-  // than the saved LayerNorm launch and fp32 round trip.  (An earlier form of the kernels lost up to 65
-  // tiles; the threshold stood at 100 then.)
+  // 0 never, 1 from `fused_ln_min_tiles` 128-row tiles (of allocated rows) upwards, 2 always.  With few row tiles the
+  // exchange of row statistics between CTAs lengthens the only wave by more than the saved LayerNorm launch and fp32
+  // round trip.  What counts is the valid rows, which the host only knows where every row is computed.  Measured on
+  // B200, 12 layers, hidden 768, us per forward without / with the fused kernels: every row computed (packed and
+  // general-mask entries) 24 tiles 1022 / 1142, 32 tiles 1294 / 1197, 34 tiles 1533 / 1398 (with a bias), 36 tiles
+  // 1513 / 1369, 37 tiles 1445 / 1306, 40 tiles 1462 / 1409; padded batches 40 tiles with 2676, 2989 and 3299 valid rows
+  // 1021 / 1082, 1072 / 1155 and 1312 / 1183, 43 tiles with 3411 1241 / 1173, 48 tiles with 4382 1357 / 1262, 64 tiles
+  // with 3970 1313 / 1231.
   int fused_ln = 1;
-  int fused_ln_min_tiles = 40;
+  int fused_ln_min_tiles = 40;           // some rows are padding
+  int fused_ln_min_tiles_all_rows = 32;  // every allocated row is computed
   bool all_rows = false;  // the call in progress computes every allocated row (packed and general-mask entries)
   uint32_t ln_epoch = 0;  // fused LayerNorm launches since the statistics scratch of the current call was zeroed
   bool fused_ln_ffn2_only = false;  // keep the attention-output LayerNorm as its own kernel
@@ -372,7 +374,9 @@ static int run_mha(bt_handle h, const __half* qkv, __half* ctx, const int* batch
 static bool want_fused_ln(bt_handle h, long long rows) {
   const int H = h->hidden;
   const long long row_tiles = (rows + 127) / 128;
-  return (H % 256 == 0) && H <= 1024 && (h->fused_ln == 2 || (h->fused_ln == 1 && row_tiles >= h->fused_ln_min_tiles));
+  return (H % 256 == 0) && H <= 1024 && (h->fused_ln == 2 || (h->fused_ln == 1 &&
+                                                                     row_tiles >= (h->all_rows ? h->fused_ln_min_tiles_all_rows
+                                                                                               : h->fused_ln_min_tiles)));
 }
 
 // The statistics scratch of the fused LayerNorm (the head of `pre`) holds words tagged with the number
@@ -1024,7 +1028,7 @@ int bt_debug_set_fused_layernorm(bt_handle h, int on) {
     h->fused_ln_ffn2_only = true;
   } else if (on > 3) {
     h->fused_ln = 1;
-    h->fused_ln_min_tiles = on;
+    h->fused_ln_min_tiles = h->fused_ln_min_tiles_all_rows = on;
   } else {
     h->fused_ln = on < 0 ? 0 : on;
   }
