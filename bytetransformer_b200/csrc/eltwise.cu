@@ -218,10 +218,12 @@ __global__ void __launch_bounds__(256)
 layernorm_cta_kernel(const float* __restrict__ x, const void* __restrict__ gamma, const void* __restrict__ beta,
                      __half* __restrict__ out, const int* __restrict__ m_dev, int m_rows,
                      const int* __restrict__ batch_idx, int S, int hidden, float eps, LnSplit split) {
-  __shared__ float red[2][8];
+  // the row, four columns per unit: even and odd units apart (by 64 bytes modulo the banks), so that a lane's eight
+  // columns are two conflict-free reads
+  __shared__ float4 vals[2][kLnMaxVec * 32 + 4];
   pdl_launch_dependents();
   const int v = threadIdx.x;  // this thread's four columns
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31;
   const bool has = v < hidden / 4;
   float g[4] = {}, bt[4] = {};
   if (has) {
@@ -269,24 +271,43 @@ layernorm_cta_kernel(const float* __restrict__ x, const void* __restrict__ gamma
       a.w += p[sp].w;
     }
   }
-  const float wsum = warp_sum((a.x + a.y) + (a.z + a.w));
   // (the row was read before its existence was known: it lies inside the allocation either way)
   if (!RESTORE && row >= row_limit) return;
-  if (lane == 0) red[0][warp] = wsum;
+  if (has) vals[v & 1][v >> 1] = a;
   __syncthreads();
+  // Statistics as layernorm_rows_kernel forms them, by every warp for itself: the same columns per lane in the same
+  // order, so that both forms give the same bits.
+  const int nvec = hidden >> 3;
+  float val[kLnMaxVec][8];
   float sum = 0.f;
-  for (int w = 0; w < n_warps; ++w) sum += red[0][w];
-  const float mean = sum / static_cast<float>(hidden);
+#pragma unroll
+  for (int it = 0; it < kLnMaxVec; ++it) {
+    const int u = it * 32 + lane;
+    if (u < nvec) {
+      const float4 lo = vals[0][u], hi = vals[1][u];
+      val[it][0] = lo.x; val[it][1] = lo.y; val[it][2] = lo.z; val[it][3] = lo.w;
+      val[it][4] = hi.x; val[it][5] = hi.y; val[it][6] = hi.z; val[it][7] = hi.w;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sum += val[it][k];
+    }
+  }
+  const float mean = warp_sum(sum) / static_cast<float>(hidden);
+  float sq = 0.f;
+#pragma unroll
+  for (int it = 0; it < kLnMaxVec; ++it) {
+    if (it * 32 + lane < nvec) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float d = val[it][k] - mean;
+        sq = fmaf(d, d, sq);
+      }
+    }
+  }
+  const float rstd = rsqrtf(warp_sum(sq) / static_cast<float>(hidden) + eps);
   a.x -= mean;
   a.y -= mean;
   a.z -= mean;
   a.w -= mean;
-  const float wsq = warp_sum(has ? fmaf(a.x, a.x, a.y * a.y) + fmaf(a.z, a.z, a.w * a.w) : 0.f);
-  if (lane == 0) red[1][warp] = wsq;
-  __syncthreads();
-  float sq = 0.f;
-  for (int w = 0; w < n_warps; ++w) sq += red[1][w];
-  const float rstd = rsqrtf(sq / static_cast<float>(hidden) + eps);
   if (has)
     *o2 = make_uint2(pack_half2(fmaf(a.x * rstd, g[0], bt[0]), fmaf(a.y * rstd, g[1], bt[1])),
                      pack_half2(fmaf(a.z * rstd, g[2], bt[2]), fmaf(a.w * rstd, g[3], bt[3])));

@@ -186,6 +186,29 @@ def test_layernorm_of_fp32_sums_restore(cuda_device):
         row += n
 
 
+@pytest.mark.parametrize("gb32", [False, True])
+@pytest.mark.parametrize("M,H", [(1, 64), (37, 192), (300, 512), (129, 768), (5, 832), (64, 1024)])
+def test_layernorm_forms_give_the_same_bits(cuda_device, M, H, gb32):
+    """Which form runs depends on the number of rows alone, so a row's result must not: a CTA per row (no bias) and a
+    warp per row (a bias of zeros, which leaves every sum what it is) add the same columns in the same order."""
+    from bytetransformer_b200.encoder import (add_bias_residual_layernorm, add_bias_residual_layernorm_restore,
+                                              build_offsets)
+    g = torch.Generator().manual_seed(7 * M + H)
+    x = (torch.randn(M, H, generator=g) * 3 + 1).to(cuda_device)
+    gamma = torch.empty(H).uniform_(0.5, 1.5, generator=g).to(cuda_device)
+    beta = torch.empty(H).uniform_(-0.4, 0.4, generator=g).to(cuda_device)
+    if not gb32:
+        gamma, beta = gamma.half(), beta.half()
+    zeros = torch.zeros(H, dtype=torch.float16, device=cuda_device)
+    assert torch.equal(add_bias_residual_layernorm(x, None, None, gamma, beta),
+                       add_bias_residual_layernorm(x, zeros, None, gamma, beta))
+    lens = [M // 2, 0, M - M // 2]
+    S = max(lens) + 3
+    bi, _ = build_offsets(_mask_from_lens(lens, S).to(cuda_device))
+    assert torch.equal(add_bias_residual_layernorm_restore(x, None, None, gamma, beta, bi, 3, S),
+                       add_bias_residual_layernorm_restore(x, zeros, None, gamma, beta, bi, 3, S))
+
+
 @pytest.mark.parametrize("kind", ["erf", "tanh"])
 def test_add_bias_gelu(cuda_device, kind):
     from bytetransformer_b200.encoder import add_bias_gelu_
