@@ -1054,6 +1054,7 @@ int bt_add_bias_residual_layernorm(const void* x, int x_fp32, const void* bias, 
                                    int hidden, float eps, void* stream) {
   if (!x || !gamma || !beta || !out || m_rows <= 0 || hidden <= 0 || hidden % 8 != 0 || hidden > 1024)
     return BT_ERR_INVALID_ARG;
+  pdl_next_launch_plain();  // gamma and beta are read ahead of the dependency wait: see kernels.h
   cudaError_t e = launch_layernorm(x, x_fp32 != 0, reinterpret_cast<const __half*>(bias),
                                    reinterpret_cast<const __half*>(residual), gamma, beta, gamma_beta_fp32 != 0,
                                    reinterpret_cast<__half*>(out), m_dev, m_rows, hidden, eps,
@@ -1068,6 +1069,7 @@ int bt_add_bias_residual_layernorm_restore(const void* x, int x_fp32, const void
   if (!x || !gamma || !beta || !out_padded || !batch_idx || batch_size <= 0 || seq_len <= 0 || hidden <= 0 ||
       hidden % 8 != 0 || hidden > 1024)
     return BT_ERR_INVALID_ARG;
+  pdl_next_launch_plain();  // gamma and beta are read ahead of the dependency wait: see kernels.h
   cudaError_t e = launch_layernorm_restore(
       x, x_fp32 != 0, reinterpret_cast<const __half*>(bias),
       reinterpret_cast<const __half*>(residual), gamma, beta, gamma_beta_fp32 != 0,

@@ -17,10 +17,10 @@ namespace bt {
 bool pdl_enabled();
 void set_pdl_enabled(bool on);
 // The calling thread's next launch is serialised the ordinary way (it starts when everything before it
-// on the stream has completed and is visible).  The entry points whose GEMMs read their weights ahead
-// of `griddepcontrol.wait` ask for this for their first kernel: a later kernel of the call can only start
-// once that one has, so nothing a caller's own kernel wrote before the call (the weights, say) can still
-// be in flight when a weight block is requested early.
+// on the stream has completed and is visible).  Kernels that read parameters ahead of `griddepcontrol.wait` - the
+// GEMMs their weights and bias, LayerNorm gamma and beta - rely on it: an entry point asks for it for the first
+// kernel of its call, whichever that is.  A later kernel of the call can only start once that one has, so nothing
+// a caller's own kernel wrote before the call can still be in flight when a parameter is requested early.
 void pdl_next_launch_plain();
 bool pdl_take_attr();  // whether the launch being made gets the attribute (consumes a pending request)
 template <typename... KArgs, typename... Args>

@@ -209,6 +209,42 @@ def test_layernorm_forms_give_the_same_bits(cuda_device, M, H, gb32):
                        add_bias_residual_layernorm_restore(x, zeros, None, gamma, beta, bi, 3, S))
 
 
+@pytest.mark.parametrize("restore", [False, True])
+@pytest.mark.parametrize("fp32_sums", [True, False])
+def test_layernorm_sees_parameters_written_just_before_the_call(cuda_device, restore, fp32_sums):
+    """gamma and beta come from a kernel of this library queued right before the call: it lets its successor start early
+    and is still writing then, and the stand-alone LayerNorm entries must not read a parameter before it is through."""
+    import bytetransformer_b200._abi as abi
+    lib = abi.load()
+    H, M, rows = 768, 40, 30000
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn(M, H, generator=g).to(cuda_device)
+    x = x if fp32_sums else x.half()
+    raw = torch.randn(rows, H, generator=g).half().to(cuda_device)
+    zero = torch.zeros(H, dtype=torch.float16, device=cuda_device)
+    bi = torch.tensor([0, M], dtype=torch.int32, device=cuda_device)
+    out = torch.empty(M, H, dtype=torch.float16, device=cuda_device)
+    gb = torch.nn.functional.gelu(raw[-2:].double())
+    want = torch.nn.functional.layer_norm(x.double(), (H,), gb[0], gb[1], eps=1e-6)
+    stream = torch.cuda.current_stream().cuda_stream
+    for attempt in range(5):
+        buf = raw.clone()  # the last two rows become gamma and beta
+        gamma, beta = buf[-2].data_ptr(), buf[-1].data_ptr()
+        torch.cuda.synchronize()
+        # no kernel of another kind in between, as from a C program; the first takes some microseconds, last rows last
+        assert lib.bt_add_bias_gelu(buf.data_ptr(), zero.data_ptr(), None, rows, H, abi.BT_GELU_ERF, stream) == abi.BT_OK
+        if restore:
+            rc = lib.bt_add_bias_residual_layernorm_restore(x.data_ptr(), int(fp32_sums), None, None, gamma, beta, 0,
+                                                            out.data_ptr(), bi.data_ptr(), 1, M, H, 1e-6, stream)
+        else:
+            rc = lib.bt_add_bias_residual_layernorm(x.data_ptr(), int(fp32_sums), None, None, gamma, beta, 0,
+                                                    out.data_ptr(), None, M, H, 1e-6, stream)
+        assert rc == abi.BT_OK
+        # fp16 rounding of gamma, beta and the result, each of size up to about 4; unwritten parameters would be off by
+        # 0.1 and more
+        assert (out.double() - want).abs().max().item() <= 2e-2, attempt
+
+
 @pytest.mark.parametrize("kind", ["erf", "tanh"])
 def test_add_bias_gelu(cuda_device, kind):
     from bytetransformer_b200.encoder import add_bias_gelu_
