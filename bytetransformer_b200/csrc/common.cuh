@@ -130,6 +130,14 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, status, code)) != 0;
 }
 
+// The wait of a loop that goes on to its end when a wait gave up (a vote per K block costs 30 clocks): `ok` is the
+// lane's answer so far, and a lane that gave up once asks no further barrier - the rest of the loop then takes no
+// time, and the bound stays one bound however many blocks are left.  The loop ends in a vote over `ok`.
+__device__ __forceinline__ bool mbar_wait_latched(bool ok, uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                  int* status, int code, long long max_cycles = (1ll << 31)) {
+  return ok && mbar_wait_bounded(bar, parity, abort_flag, status, code, max_cycles);
+}
+
 // ------------------------------------------------------------ warp-uniform roles
 // tcgen05 and TMA instructions take their descriptors, addresses and coordinates from uniform registers.  In a
 // branch that one lane takes (`if (lane == 0)`) every operand of every instruction is moved there first, and that
@@ -139,8 +147,8 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
 // instructions themselves are predicated on an elected lane, all MMAs of a K block and their commit on one
 // election (umma_k_block): 84 clocks per MMA in the main loop, 525 -> 335 clocks per K block of 64 (N <= 128).
 // Because elect.sync needs the whole warp, a warp's lanes must not part ways after a wait that gave up: waits end
-// in a vote (mbar_wait_warp), except in the K loop, which goes on to its end with `ok` remembered (a vote there
-// costs 30 clocks per K block) and votes after it.
+// in a vote (mbar_wait_warp), except in the K loop, which goes on to its end with `ok` remembered (mbar_wait_latched)
+// and votes after it.
 __device__ __forceinline__ int uniform_int(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ uint32_t uniform_u32(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
 

@@ -436,7 +436,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         if (lane == 0) gstamp(args.timing, it, 0);
         const uint32_t d_tmem = tmem_base + as * BLOCK_N;
         for (int kb = 0; kb < num_kb; ++kb) {
-          ok &= mbar_wait_bounded(&full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
+          ok = mbar_wait_latched(ok, &full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
           const uint32_t sb = sa + kABytes;
@@ -676,7 +676,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         if (lane == 0) gstamp(args.timing, it, 0);
         const uint32_t d_tmem = tmem_base + as * kTileN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          ok &= mbar_wait_bounded(&full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
+          ok = mbar_wait_latched(ok, &full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
           const uint32_t sb = sa + kABytes;
@@ -1208,7 +1208,7 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         if (lane == 0) gstamp(args.timing, it, 0);
         const uint32_t d_tmem = tmem_base + as * kTileN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          ok &= mbar_wait_bounded(&full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
+          ok = mbar_wait_latched(ok, &full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
           const uint32_t sb = sa + kABytes;
@@ -1398,7 +1398,7 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
         if (lane == 0) gstamp(args.timing, it, 0);
         const uint32_t d_tmem = tmem_base + as * kTileN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          ok &= mbar_wait_bounded(&full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
+          ok = mbar_wait_latched(ok, &full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
           const uint32_t sb = sa + kABytes;
