@@ -102,7 +102,8 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 
 // Wait for a phase with an upper bound.  Returns false when the bound ran out
 // or another role of this CTA already gave up (`*abort_flag` non-zero); the
-// caller must then leave its loop and fall through to the common teardown.
+// caller must then leave its loop and fall through to the common teardown.  The
+// answer is the calling lane's own: what a warp waits for goes through the two forms below.
 // The bound is ~2^31 SM cycles (about a second) unless the caller gives another,
 // checked every 256 polls.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity,
@@ -124,10 +125,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
-// The same for a warp whose 32 lanes all wait (the TMA and MMA roles): one answer for the warp, from a vote.
+// The same for a warp whose 32 lanes all wait: one answer for the warp, from a vote.  Every wait of a kernel's roles
+// goes through it (or, in a K loop, through the latched form below): lanes that parted ways where a wait gave up would
+// hang in the next warp-wide instruction (elect.sync, tcgen05.ld, __syncwarp), bound or no bound.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                               int code) {
-  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, status, code)) != 0;
+                                               int code, long long max_cycles = (1ll << 31)) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, status, code, max_cycles)) != 0;
 }
 
 // The wait of a loop that goes on to its end when a wait gave up (a vote per K block costs 30 clocks): `ok` is the
@@ -146,9 +149,8 @@ __device__ __forceinline__ bool mbar_wait_latched(bool ok, uint64_t* bar, uint32
 // walked by their whole warp - role, loop bounds and shared values go through uniform_int() - and only the
 // instructions themselves are predicated on an elected lane, all MMAs of a K block and their commit on one
 // election (umma_k_block): 84 clocks per MMA in the main loop, 525 -> 335 clocks per K block of 64 (N <= 128).
-// Because elect.sync needs the whole warp, a warp's lanes must not part ways after a wait that gave up: waits end
-// in a vote (mbar_wait_warp), except in the K loop, which goes on to its end with `ok` remembered (mbar_wait_latched)
-// and votes after it.
+// Because elect.sync needs the whole warp, a warp's lanes must not part ways after a wait that gave up: see
+// mbar_wait_warp and mbar_wait_latched.
 __device__ __forceinline__ int uniform_int(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ uint32_t uniform_u32(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
 

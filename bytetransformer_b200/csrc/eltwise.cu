@@ -635,16 +635,19 @@ __global__ void __launch_bounds__(64) bounded_wait_selftest_kernel(int* status, 
 }
 
 // A K loop's waits after one of them gave up: 64 waits for a barrier that nothing arrives on.  out[0] = clocks of
-// the first, out[1] = of all, out[2] = lanes that believe a wait succeeded.
-__global__ void __launch_bounds__(32) latched_wait_selftest_kernel(long long max_cycles, long long* out) {
-  __shared__ uint64_t bar;
+// the first, out[1] = of all, out[2] = lanes that believe a wait succeeded.  out[3] = lanes told so by a warp's wait
+// where one lane's barrier has completed its phase and the others' has not.
+__global__ void __launch_bounds__(32) wait_forms_selftest_kernel(long long max_cycles, long long* out) {
+  __shared__ uint64_t bar, done;
   __shared__ int abort_flag_s;
   pdl_launch_dependents();
   pdl_wait();
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
+    mbar_init(&done, 1);
     abort_flag_s = 0;
     fence_mbar_init();
+    mbar_arrive(&done);
   }
   __syncthreads();
   const long long t0 = clock64();
@@ -654,11 +657,17 @@ __global__ void __launch_bounds__(32) latched_wait_selftest_kernel(long long max
     ok = mbar_wait_latched(ok, &bar, 0u, &abort_flag_s, nullptr, 0, max_cycles);
     if (kb == 0) t1 = clock64();
   }
+  const long long t2 = clock64();
   const int lanes = __popc(__ballot_sync(0xffffffffu, ok));
+  abort_flag_s = 0;
+  __syncwarp();
+  const bool got = mbar_wait_warp(threadIdx.x == 5 ? &done : &bar, 0u, &abort_flag_s, nullptr, 0, max_cycles);
+  const int told = __popc(__ballot_sync(0xffffffffu, got));
   if (threadIdx.x == 0) {
     out[0] = t1 - t0;
-    out[1] = clock64() - t0;
+    out[1] = t2 - t0;
     out[2] = lanes;
+    out[3] = told;
   }
 }
 }  // namespace
@@ -669,17 +678,17 @@ cudaError_t launch_bounded_wait_selftest(int* status, long long max_cycles, int*
   return launch_pdl(bounded_wait_selftest_kernel, dim3(1), dim3(64), 0, stream, status, max_cycles, gave_up);
 }
 
-static cudaError_t launch_latched_wait_selftest(long long max_cycles, long long* out, cudaStream_t stream) {
+static cudaError_t launch_wait_forms_selftest(long long max_cycles, long long* out, cudaStream_t stream) {
   if (max_cycles < 1024) max_cycles = 1024;
   if (max_cycles > (1ll << 28)) max_cycles = (1ll << 28);
-  return launch_pdl(latched_wait_selftest_kernel, dim3(1), dim3(32), 0, stream, max_cycles, out);
+  return launch_pdl(wait_forms_selftest_kernel, dim3(1), dim3(32), 0, stream, max_cycles, out);
 }
 
 }  // namespace bt
 
-// Diagnostics hook (tests): see latched_wait_selftest_kernel; `out_dev` holds three long long.
-extern "C" int bt_debug_selftest_latched_wait(long long max_cycles, long long* out_dev, void* stream) {
+// Diagnostics hook (tests): see wait_forms_selftest_kernel; `out_dev` holds four long long.
+extern "C" int bt_debug_selftest_wait_forms(long long max_cycles, long long* out_dev, void* stream) {
   if (out_dev == nullptr) return BT_ERR_INVALID_ARG;
-  return bt::launch_latched_wait_selftest(max_cycles, out_dev, reinterpret_cast<cudaStream_t>(stream)) == cudaSuccess
+  return bt::launch_wait_forms_selftest(max_cycles, out_dev, reinterpret_cast<cudaStream_t>(stream)) == cudaSuccess
              ? BT_OK : BT_ERR_CUDA;
 }

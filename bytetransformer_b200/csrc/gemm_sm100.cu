@@ -465,7 +465,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       const uint32_t aphase = (it >> 1) & 1;
       uint4 resv[kHasResidual ? BLOCK_N / 16 : 1];
       prefetch_residual<BLOCK_N, EPI>(args, m0, n0, M, quarter, col_half, lane, resv, sp);
-      if (!mbar_wait_bounded(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
+      if (!mbar_wait_warp(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
       tc_fence_after();
       if (warp == 2 && lane == 0) gstamp(args.timing, it, 2);
       epilogue_tile<BLOCK_N, EPI, Cfg::tma_store(EPI), 1>(args, &tm_out, stg, tmem_base + as * BLOCK_N, m0, n0, M, quarter,
@@ -707,7 +707,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       const uint32_t aphase = (it >> 1) & 1;
       uint4 resv[kHasResidual ? kTileN / 16 : 1];
       prefetch_residual<kTileN, EPI>(args, m0, n0, M, quarter, col_half, lane, resv);
-      if (!mbar_wait_bounded(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
+      if (!mbar_wait_warp(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
       tc_fence_after();
       if (warp == 2 && lane == 0) gstamp(args.timing, it, 2);
       epilogue_tile<kTileN, EPI, true, Cfg::kStagingBufs>(args, &tm_out, stg, tmem_base + as * kTileN, m0, n0, M,
@@ -805,7 +805,7 @@ __device__ __forceinline__ void ln_epilogue_loop(const GemmArgs& args, const CUt
         vg = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(args.gamma) + n0) + lane);
         vt = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(args.beta) + n0) + lane);
       }
-      if (!mbar_wait_bounded(vec_empty, (it & 1u) ^ 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
+      if (!mbar_wait_warp(vec_empty, (it & 1u) ^ 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
       vec_s[lane] = vb;
       vec_s[32 + lane] = vg;
       vec_s[64 + lane] = vt;
@@ -821,9 +821,9 @@ __device__ __forceinline__ void ln_epilogue_loop(const GemmArgs& args, const CUt
       mbar_arrive_expect_tx(&res_bar[e], kStagingBytesPerWarp);
       tma_load_2d(stg, tm_res, &res_bar[e], gcol0, row0);
     }
-    if (!mbar_wait_bounded(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
+    if (!mbar_wait_warp(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
     tc_fence_after();
-    if (!mbar_wait_bounded(vec_full, it & 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
+    if (!mbar_wait_warp(vec_full, it & 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
     if (warp == 2 && lane == 0) gstamp(args.timing, it, 2);
     const uint4* sbias = vec_s + col_half * (kColsPerThread / 8);
     const uint4* sgamma = vec_s + 32 + col_half * (kColsPerThread / 8);
@@ -840,7 +840,7 @@ __device__ __forceinline__ void ln_epilogue_loop(const GemmArgs& args, const CUt
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         // this thread's 64 residual values of box hh: row `lane` of the swizzled buffer
-        if (!mbar_wait_bounded(&res_bar[e], (static_cast<uint32_t>(it) * 2u + hh) & 1u, abort_flag, args.status,
+        if (!mbar_wait_warp(&res_bar[e], (static_cast<uint32_t>(it) * 2u + hh) & 1u, abort_flag, args.status,
                                kStatusGemmEpilogueTimeout)) {
           res_ok = false;
           break;
@@ -954,13 +954,13 @@ __device__ __forceinline__ void ln_epilogue_loop(const GemmArgs& args, const CUt
           }
       }
       if (__all_sync(0xffffffffu, bad == 0)) break;
-      if (*abort_flag != 0 || clock64() - t0 > (1ll << 31)) {
+      if (__any_sync(0xffffffffu, *abort_flag != 0 || clock64() - t0 > (1ll << 31))) {
         give_up = true;
         break;
       }
       __nanosleep(100);
     }
-    if (__any_sync(0xffffffffu, give_up)) {
+    if (give_up) {
       if (lane == 0) {
         *abort_flag = 1;
         if (args.status != nullptr) atomicCAS(args.status, 0, kStatusGemmEpilogueTimeout);

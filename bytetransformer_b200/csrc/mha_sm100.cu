@@ -672,7 +672,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
             for (int u = 0; u < 8; ++u) bias_q[u] = __ldg(bt + u * 128);
           }
         }
-        if (!mbar_wait_bounded(&s_full[t], jpar, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
+        if (!mbar_wait_warp(&s_full[t], jpar, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
           ok = false;
           break;
         }
@@ -735,7 +735,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
         if (!full_tile && t == 0) {
           // tail tile: blank the V rows of keys that do not belong to this sequence
           // (tile 0's PV is issued before tile 1's, so tile 0's warpgroup does it for both)
-          if (!mbar_wait_bounded(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
+          if (!mbar_wait_warp(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
             ok = false;
             break;
           }
@@ -754,7 +754,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
           phase ^= 1u;
         }
       }
-      if (ok) ok = mbar_wait_bounded(o_done, 0, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
+      if (ok) ok = mbar_wait_warp(o_done, 0, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
       tc_fence_after();
       if (ok) {
         // O / row sum -> fp16 -> global memory by way of the Q tile, which no MMA reads any more (o_done covers the
@@ -1185,7 +1185,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
       float l_run = 0.f;
       for (int j = 0; j < n_kv; ++j, ++step) {
         const int kv_valid = min(kKvRows, L - j * kKvRows);
-        if (!mbar_wait_bounded(s_full, step & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
+        if (!mbar_wait_warp(s_full, step & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
           ok = false;
           break;
         }
@@ -1219,7 +1219,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
           m_ref = m_new;
         } else if (__any_sync(0xffffffffu, (m_new - m_ref) > kRescaleThreshold)) {
           // O belongs to the P V MMAs of the previous key tile until those have retired
-          if (!mbar_wait_bounded(pv_done, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
+          if (!mbar_wait_warp(pv_done, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
             ok = false;
             break;
           }
@@ -1253,7 +1253,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
         l_run += (l0 + l1) + (l2 + l3);
         if (!pv_waited) {
           // P belongs to the P V MMAs of the previous key tile until those have retired
-          if (!mbar_wait_bounded(pv_done, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
+          if (!mbar_wait_warp(pv_done, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
             ok = false;
             break;
           }
@@ -1265,7 +1265,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
         tmem_st_32x16_at<48>(t_p + 48, pk);
         if (kv_valid != kKvRows) {
           // tail tile: blank the V rows of keys that do not belong to this sequence
-          if (!mbar_wait_bounded(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
+          if (!mbar_wait_warp(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
             ok = false;
             break;
           }
@@ -1289,7 +1289,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
       // the next item is found while the last P V of this one runs
       int seq_start_n = 0, L_n = 0, qt_n = 0, head_n = 0;
       have = decode_item(args, snake_item(round + 1, cta, G), cur_b, cur_first, seq_start_n, L_n, qt_n, head_n, false);
-      if (!mbar_wait_bounded(o_done, static_cast<uint32_t>(round) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
+      if (!mbar_wait_warp(o_done, static_cast<uint32_t>(round) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
         ok = false;
         break;
       }

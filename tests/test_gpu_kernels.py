@@ -596,17 +596,17 @@ def test_expired_wait_is_reported_and_the_context_stays_usable(enc, cuda_device)
     assert enc.device_status() == 0
 
 
-def test_a_loop_of_waits_gives_up_once(cuda_device):
+def test_warp_waits_give_up_once_and_together(cuda_device):
     """The K loop of the GEMMs goes on to its end when a wait has run out; the waits that are left must not be polled
-    again: 64 waits for a barrier that nothing arrives on take the bound of one of them."""
+    again: 64 waits for a barrier that nothing arrives on take the bound of one of them.  And a warp gets one answer for a wait: one lane whose barrier is complete does not go on alone."""
     import ctypes as C
 
     from bytetransformer_b200 import _abi
-    fn = _abi.load().bt_debug_selftest_latched_wait
+    fn = _abi.load().bt_debug_selftest_wait_forms
     fn.restype, fn.argtypes = C.c_int, [C.c_longlong, C.c_void_p, C.c_void_p]
-    out = torch.zeros(3, dtype=torch.int64, device=cuda_device)
+    out = torch.zeros(4, dtype=torch.int64, device=cuda_device)
     # the bound is looked at every 256 polls: with the smallest one the first wait takes one such batch
     assert fn(1024, out.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
-    first, total, lanes = out.cpu().tolist()
-    assert lanes == 0
+    first, total, lanes, told = out.cpu().tolist()
+    assert lanes == 0 and told == 0
     assert 1024 <= first <= total <= 4 * first, (first, total)  # polled again, the 63 others would be 63 batches
