@@ -470,7 +470,6 @@ __global__ void __launch_bounds__(MhaCfg::kThreads, 2)
 mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_ctx, const MhaArgs args) {
   using Cfg = MhaCfg;
   constexpr bool GENERAL = MODE != 0;
-  constexpr int TILES = 1;  // query tiles per CTA (the loops over `t` below have one trip)
   constexpr int kStages = Cfg::kStages;
   // the exponent reference may lag the running maximum by at most 2^8
   constexpr float kRescaleThreshold = 8.0f;
@@ -479,27 +478,25 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
   pdl_launch_dependents();
   const int b = blockIdx.z;
   const int head = blockIdx.y;
-  const int q0 = blockIdx.x * (kQRows * TILES);
+  const int q0 = blockIdx.x * kQRows;
 
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kSmemBar);
-  uint64_t* q_full = bars;                       // [TILES]
-  uint64_t* k_full = bars + 2;                   // [kStages]
-  uint64_t* v_full = bars + 2 + kStages;         // [kStages]
-  uint64_t* kv_empty = bars + 2 + 2 * kStages;   // [kStages]
-  uint64_t* s_full = bars + 2 + 3 * kStages;     // [TILES]
-  uint64_t* p_full = bars + 4 + 3 * kStages;     // [TILES]
-  uint64_t* o_done = bars + 6 + 3 * kStages;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7 + 3 * kStages);
+  uint64_t* q_full = bars;
+  uint64_t* k_full = bars + 1;                   // [kStages]
+  uint64_t* v_full = bars + 1 + kStages;         // [kStages]
+  uint64_t* kv_empty = bars + 1 + 2 * kStages;   // [kStages]
+  uint64_t* s_full = bars + 1 + 3 * kStages;
+  uint64_t* p_full = bars + 2 + 3 * kStages;
+  uint64_t* o_done = bars + 3 + 3 * kStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4 + 3 * kStages);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = uniform_int(static_cast<int>(threadIdx.x >> 5));  // warp-uniform roles: see common.cuh
   const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int t = 0; t < TILES; ++t) {
-      mbar_init(&q_full[t], 1);
-      mbar_init(&s_full[t], 1);
-      mbar_init(&p_full[t], 4);  // one arrival per softmax warp
-    }
+    mbar_init(q_full, 1);
+    mbar_init(s_full, 1);
+    mbar_init(p_full, 4);  // one arrival per softmax warp
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&k_full[s], 1);
       mbar_init(&v_full[s], 1);
@@ -539,7 +536,6 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
   if ((bad_offsets || bad_smem) && threadIdx.x == 0 && args.status != nullptr)
     atomicCAS(args.status, 0, bad_offsets ? kStatusBadOffsets : kStatusMhaLoadTimeout + 0x10);
   const bool active = !bad_offsets && !bad_smem && q0 < L;
-  const int n_tiles = (TILES == 2 && q0 + kQRows < L) ? 2 : 1;  // query tiles with at least one valid row
   // General masks: the key tiles behind the last key that any row of this query tile may see are left out
   int kv_rows = L;
   if (GENERAL && args.gen_kv_bound != nullptr) {
@@ -556,251 +552,223 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
     // no rows for this CTA: straight to the teardown
   } else if (warp == 0) {
     // ------------------------------------------------------------------ loads
-    {
-      for (int t = 0; t < n_tiles; ++t) {
-        if (elect_one()) mbar_arrive_expect_tx(&q_full[t], kTileBytes);
-        if (elect_one()) tma_load_2d(smem + Cfg::kSmemQ + t * kTileBytes, &tm_qkv, &q_full[t], col_q, seq_start + q0 + t * kQRows);
-      }
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int j = 0; j < n_kv; ++j) {
-        if (!mbar_wait_warp(&kv_empty[stage], phase ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) break;
-        const int row = seq_start + j * kKvRows;
-        if (elect_one()) mbar_arrive_expect_tx(&k_full[stage], kTileBytes);
-        if (elect_one()) tma_load_2d(smem + Cfg::kSmemK + stage * kTileBytes, &tm_qkv, &k_full[stage], col_k, row);
-        if (elect_one()) mbar_arrive_expect_tx(&v_full[stage], kTileBytes);
-        if (elect_one()) tma_load_2d(smem + Cfg::kSmemV + stage * kTileBytes, &tm_qkv, &v_full[stage], col_v, row);
-        if (++stage == kStages) {
-          stage = 0;
-          phase ^= 1u;
-        }
+    if (elect_one()) mbar_arrive_expect_tx(q_full, kTileBytes);
+    if (elect_one()) tma_load_2d(smem + Cfg::kSmemQ, &tm_qkv, q_full, col_q, seq_start + q0);
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int j = 0; j < n_kv; ++j) {
+      if (!mbar_wait_warp(&kv_empty[stage], phase ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) break;
+      const int row = seq_start + j * kKvRows;
+      if (elect_one()) mbar_arrive_expect_tx(&k_full[stage], kTileBytes);
+      if (elect_one()) tma_load_2d(smem + Cfg::kSmemK + stage * kTileBytes, &tm_qkv, &k_full[stage], col_k, row);
+      if (elect_one()) mbar_arrive_expect_tx(&v_full[stage], kTileBytes);
+      if (elect_one()) tma_load_2d(smem + Cfg::kSmemV + stage * kTileBytes, &tm_qkv, &v_full[stage], col_v, row);
+      if (++stage == kStages) {
+        stage = 0;
+        phase ^= 1u;
       }
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issue
-    {
-      // K-major operands (Q, K): 8-row groups 1024 B apart.
-      constexpr uint64_t kDescK = make_smem_desc_hi(16, 1024);
-      // V: MN-major, one 64-wide chunk (LBO unused), 8-key groups 1024 B apart.
-      constexpr uint64_t kDescV = make_smem_desc_hi(kTileBytes, 1024);
-      constexpr uint32_t kIdescS = make_idesc_f16(128, 128, 0, 0);
-      constexpr uint32_t kIdescO = make_idesc_f16(128, 64, 0, 1);
-      const uint32_t s_q = smem_u32(smem + Cfg::kSmemQ);
-      const uint32_t s_k = smem_u32(smem + Cfg::kSmemK);
-      const uint32_t s_v = smem_u32(smem + Cfg::kSmemV);
-      auto issue_s = [&](int t, int stage) {
-        const uint32_t sq = s_q + t * kTileBytes;
-        const uint32_t sk = s_k + stage * kTileBytes;
-        umma_s_tile(tmem_base + t * 128, smem_desc(kDescK, sq), smem_desc(kDescK, sk), kIdescS, &s_full[t]);
-      };
-      // `keys`: keys of the tile that exist (only the 16-key steps that hold any are multiplied)
-      auto issue_pv = [&](int t, int stage, bool accumulate, int keys) {
-        const uint32_t tp = tmem_base + t * 128 + Cfg::kTmemPOff;  // 8 cells (16 keys) per MMA
-        const uint32_t sv = s_v + stage * kTileBytes;
-        umma_pv_tile(tmem_base + Cfg::kTmemO + t * 64, tp, smem_desc(kDescV, sv), kIdescO, accumulate ? 1u : 0u,
-                     static_cast<uint32_t>((keys + 15) >> 4));
-      };
-      bool ok = true;
-      for (int t = 0; t < n_tiles && ok; ++t)
-        ok = mbar_wait_warp(&q_full[t], 0, abort_flag, args.status, kStatusMhaMmaTimeout);
-      if (ok) ok = mbar_wait_warp(&k_full[0], 0, abort_flag, args.status, kStatusMhaMmaTimeout);
-      if (ok) {
-        tc_fence_after();
-        for (int t = 0; t < n_tiles; ++t) issue_s(t, 0);
-      }
-      int st = 0;
-      uint32_t ph = 0;
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const uint32_t jpar = j & 1;
-        const int st_n = (st + 1 == kStages) ? 0 : st + 1;
-        const uint32_t ph_n = (st + 1 == kStages) ? (ph ^ 1u) : ph;
-        const bool more = j + 1 < n_kv;
-        // ---- tile 0: O0 += P0 V(j), then S0(j+1).  The MMAs of one thread execute in issue
-        // order, so S0(j+1) cannot overwrite P0(j) (same columns) before PV0(j) has read it.
-        if (!mbar_wait_warp(&p_full[0], jpar, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
-        if (!mbar_wait_warp(&v_full[st], ph, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
-        tc_fence_after();
-        const int keys = min(kKvRows, L - j * kKvRows);
-        issue_pv(0, st, j > 0, keys);
-        if (more) {
-          if (!mbar_wait_warp(&k_full[st_n], ph_n, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
-          tc_fence_after();
-          issue_s(0, st_n);
-        }
-        // ---- tile 1
-        if (n_tiles == 2) {
-          if (!mbar_wait_warp(&p_full[1], jpar, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
-          tc_fence_after();
-          issue_pv(1, st, j > 0, keys);
-        }
-        if (elect_one()) umma_commit(&kv_empty[st]);  // every MMA that reads K/V stage `st` has been issued
-        if (n_tiles == 2 && more) issue_s(1, st_n);
-        st = st_n;
-        ph = ph_n;
-      }
-      if (elect_one()) umma_commit(o_done);
+    // K-major operands (Q, K): 8-row groups 1024 B apart.
+    constexpr uint64_t kDescK = make_smem_desc_hi(16, 1024);
+    // V: MN-major, one 64-wide chunk (LBO unused), 8-key groups 1024 B apart.
+    constexpr uint64_t kDescV = make_smem_desc_hi(kTileBytes, 1024);
+    constexpr uint32_t kIdescS = make_idesc_f16(128, 128, 0, 0);
+    constexpr uint32_t kIdescO = make_idesc_f16(128, 64, 0, 1);
+    const uint32_t s_q = smem_u32(smem + Cfg::kSmemQ);
+    const uint32_t s_k = smem_u32(smem + Cfg::kSmemK);
+    const uint32_t s_v = smem_u32(smem + Cfg::kSmemV);
+    auto issue_s = [&](int stage) {
+      umma_s_tile(tmem_base, smem_desc(kDescK, s_q), smem_desc(kDescK, s_k + stage * kTileBytes), kIdescS, s_full);
+    };
+    // `keys`: keys of the tile that exist (only the 16-key steps that hold any are multiplied)
+    auto issue_pv = [&](int stage, bool accumulate, int keys) {
+      umma_pv_tile(tmem_base + Cfg::kTmemO, tmem_base + Cfg::kTmemPOff, smem_desc(kDescV, s_v + stage * kTileBytes), kIdescO,
+                   accumulate ? 1u : 0u, static_cast<uint32_t>((keys + 15) >> 4));
+    };
+    bool ok = mbar_wait_warp(q_full, 0, abort_flag, args.status, kStatusMhaMmaTimeout);
+    if (ok) ok = mbar_wait_warp(&k_full[0], 0, abort_flag, args.status, kStatusMhaMmaTimeout);
+    if (ok) {
+      tc_fence_after();
+      issue_s(0);
     }
+    int st = 0;
+    uint32_t ph = 0;
+    for (int j = 0; j < n_kv && ok; ++j) {
+      const int st_n = (st + 1 == kStages) ? 0 : st + 1;
+      const uint32_t ph_n = (st + 1 == kStages) ? (ph ^ 1u) : ph;
+      // O += P V(j), then S(j+1).  The MMAs of one thread execute in issue order, so S(j+1) cannot overwrite
+      // P(j) (same columns) before P V(j) has read it.
+      if (!mbar_wait_warp(p_full, j & 1, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
+      if (!mbar_wait_warp(&v_full[st], ph, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
+      tc_fence_after();
+      issue_pv(st, j > 0, min(kKvRows, L - j * kKvRows));
+      if (j + 1 < n_kv) {
+        if (!mbar_wait_warp(&k_full[st_n], ph_n, abort_flag, args.status, kStatusMhaMmaTimeout)) break;
+        tc_fence_after();
+        issue_s(st_n);
+      }
+      if (elect_one()) umma_commit(&kv_empty[st]);  // every MMA that reads K/V stage `st` has been issued
+      st = st_n;
+      ph = ph_n;
+    }
+    if (elect_one()) umma_commit(o_done);
   } else {
     // ---------------------------------------------------------------- softmax
-    const int t = (warp - 2) >> 2;  // query tile of this warpgroup
-    if (t < n_tiles) {
-      const int quarter = warp & 3;
-      const int r = quarter * 32 + lane;  // query row inside the tile == TMEM lane
-      const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-      const uint32_t t_s = t_lane + t * 128;
-      const uint32_t t_o = t_lane + Cfg::kTmemO + t * 64;
-      const float c = args.scale_log2e;
-      float m_ref = -INFINITY;  // exponent reference, in log2 units
-      float l_run = 0.f;
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      // binary mask, no bias: applied from bits inside the two softmax passes
-      const bool use_bits = GENERAL && args.gen_bits != nullptr && __ldg(args.gen_bits_flag) == 0;
-      const float bits_neg = -10000.0f * args.gen_inv_scale;
-      for (int j = 0; j < n_kv; ++j) {
-        const uint32_t jpar = j & 1;
-        const int kv_valid = min(kKvRows, L - j * kKvRows);
-        const bool full_tile = kv_valid == kKvRows;
-        uint4 bias_q[MODE == 2 ? 8 : 1];
-        const uint4* bt = nullptr;
-        if constexpr (MODE == 2) {
-          if (use_bits) {
-            const int n_qt = static_cast<int>(gridDim.x);
-            bt = args.gen_bias_tiles + ((static_cast<size_t>(head) * n_qt + blockIdx.x) * n_qt + j) * (16 * 128) + r;
+    const int quarter = warp & 3;
+    const int r = quarter * 32 + lane;  // query row inside the tile == TMEM lane
+    const uint32_t t_s = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t t_o = t_s + Cfg::kTmemO;
+    const float c = args.scale_log2e;
+    float m_ref = -INFINITY;  // exponent reference, in log2 units
+    float l_run = 0.f;
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    // binary mask, no bias: applied from bits inside the two softmax passes
+    const bool use_bits = GENERAL && args.gen_bits != nullptr && __ldg(args.gen_bits_flag) == 0;
+    const float bits_neg = -10000.0f * args.gen_inv_scale;
+    for (int j = 0; j < n_kv; ++j) {
+      const int kv_valid = min(kKvRows, L - j * kKvRows);
+      const bool full_tile = kv_valid == kKvRows;
+      uint4 bias_q[MODE == 2 ? 8 : 1];
+      const uint4* bt = nullptr;
+      if constexpr (MODE == 2) {
+        if (use_bits) {
+          const int n_qt = static_cast<int>(gridDim.x);
+          bt = args.gen_bias_tiles + ((static_cast<size_t>(head) * n_qt + blockIdx.x) * n_qt + j) * (16 * 128) + r;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) bias_q[u] = __ldg(bt + u * 128);
-          }
+          for (int u = 0; u < 8; ++u) bias_q[u] = __ldg(bt + u * 128);
         }
-        if (!mbar_wait_warp(&s_full[t], jpar, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
+      }
+      if (!mbar_wait_warp(s_full, j & 1, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      uint4 bw = make_uint4(~0u, ~0u, ~0u, ~0u);  // a row that does not exist masks nothing
+      if (GENERAL && use_bits) {
+        const int q_row = q0 + r;
+        if (q_row < args.gen_seq_len)
+          bw = __ldg(reinterpret_cast<const uint4*>(args.gen_bits + (static_cast<size_t>(b) * args.gen_seq_len + q_row) *
+                                                                        args.gen_bits_stride) + j);
+      } else if (GENERAL) {
+        const int S = args.gen_seq_len;
+        const int q_row = q0 + r;
+        const bool q_ok = q_row < S;
+        const size_t off = static_cast<size_t>(q_ok ? q_row : 0) * S + static_cast<size_t>(j) * kKvRows;
+        tile_add_mask_bias(t_s, args.gen_mask + static_cast<size_t>(b) * S * S + off,
+                           args.gen_bias != nullptr ? args.gen_bias + static_cast<size_t>(head) * S * S + off : nullptr,
+                           q_ok ? kv_valid : 0, (S & 7) == 0, args.gen_inv_scale);
+      }
+      // pass 1: row maximum (scaled to log2 units)
+      float mx;
+      if constexpr (MODE == 2) {
+        if (use_bits)
+          mx = c * (full_tile ? tile_add_bias_row_max<false>(t_s, bias_q, bt, bw, kv_valid, args.gen_inv_scale)
+                              : tile_add_bias_row_max<true>(t_s, bias_q, bt, bw, kv_valid, args.gen_inv_scale));
+        else
+          mx = c * (full_tile ? tile_row_max(t_s) : tail_row_max(t_s, kv_valid));
+      } else if (GENERAL && use_bits)
+        mx = c * (full_tile ? tile_row_max_bits<false>(t_s, kv_valid, bw, bits_neg)
+                            : tile_row_max_bits<true>(t_s, kv_valid, bw, bits_neg));
+      else
+        mx = c * (full_tile ? tile_row_max(t_s) : tail_row_max(t_s, kv_valid));
+      if (j == 0) {
+        m_ref = mx;
+      } else {
+        const float m_new = fmaxf(m_ref, mx);
+        const bool need = (m_new - m_ref) > kRescaleThreshold;
+        if (__any_sync(0xffffffffu, need)) {
+          // the PV of the previous key tile has retired (S of this tile was issued after it)
+          const float f = ex2_approx(m_ref - m_new);
+#pragma unroll
+          for (int cb = 0; cb < kHeadDim; cb += 32) {
+            uint32_t v[32];
+            tmem_ld_32x32(t_o + cb, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * f);
+            tmem_st_32x32(t_o + cb, v);
+          }
+          l_run *= f;
+          m_ref = m_new;
+        }
+      }
+      // pass 2: probabilities -> fp16 pairs -> tensor memory (over S), row sum
+      if (MODE == 1 && use_bits)
+        l_run += full_tile ? tile_probs_bits<false>(t_s, kv_valid, c, m_ref, bw, bits_neg)
+                           : tile_probs_bits<true>(t_s, kv_valid, c, m_ref, bw, bits_neg);
+      else
+        l_run += full_tile ? tile_probs(t_s, c, m_ref) : tail_probs(t_s, kv_valid, c, m_ref);
+      if (!full_tile) {
+        // tail tile: blank the V rows of keys that do not belong to this sequence
+        if (!mbar_wait_warp(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
           ok = false;
           break;
         }
-        tc_fence_after();
-        uint4 bw = make_uint4(~0u, ~0u, ~0u, ~0u);  // a row that does not exist masks nothing
-        if (GENERAL && use_bits) {
-          const int q_row = q0 + t * kQRows + r;
-          if (q_row < args.gen_seq_len)
-            bw = __ldg(reinterpret_cast<const uint4*>(args.gen_bits + (static_cast<size_t>(b) * args.gen_seq_len + q_row) *
-                                                                          args.gen_bits_stride) + j);
-        } else if (GENERAL) {
-          const int S = args.gen_seq_len;
-          const int q_row = q0 + t * kQRows + r;
-          const bool q_ok = q_row < S;
-          const size_t off = static_cast<size_t>(q_ok ? q_row : 0) * S + static_cast<size_t>(j) * kKvRows;
-          tile_add_mask_bias(t_s, args.gen_mask + static_cast<size_t>(b) * S * S + off,
-                             args.gen_bias != nullptr ? args.gen_bias + static_cast<size_t>(head) * S * S + off : nullptr,
-                             q_ok ? kv_valid : 0, (S & 7) == 0, args.gen_inv_scale);
-        }
-        // pass 1: row maximum (scaled to log2 units)
-        float mx;
-        if constexpr (MODE == 2) {
-          if (use_bits)
-            mx = c * (full_tile ? tile_add_bias_row_max<false>(t_s, bias_q, bt, bw, kv_valid, args.gen_inv_scale)
-                                : tile_add_bias_row_max<true>(t_s, bias_q, bt, bw, kv_valid, args.gen_inv_scale));
-          else
-            mx = c * (full_tile ? tile_row_max(t_s) : tail_row_max(t_s, kv_valid));
-        } else if (GENERAL && use_bits)
-          mx = c * (full_tile ? tile_row_max_bits<false>(t_s, kv_valid, bw, bits_neg)
-                              : tile_row_max_bits<true>(t_s, kv_valid, bw, bits_neg));
-        else
-          mx = c * (full_tile ? tile_row_max(t_s) : tail_row_max(t_s, kv_valid));
-        if (j == 0) {
-          m_ref = mx;
-        } else {
-          const float m_new = fmaxf(m_ref, mx);
-          const bool need = (m_new - m_ref) > kRescaleThreshold;
-          if (__any_sync(0xffffffffu, need)) {
-            // the PV of the previous key tile has retired (S of this tile was issued after it)
-            const float f = ex2_approx(m_ref - m_new);
+        if (r >= kv_valid && r < ((kv_valid + 15) & ~15)) {
+          uint4* vr = reinterpret_cast<uint4*>(smem + Cfg::kSmemV + stage * kTileBytes + r * 128);
 #pragma unroll
-            for (int cb = 0; cb < kHeadDim; cb += 32) {
-              uint32_t v[32];
-              tmem_ld_32x32(t_o + cb, v);
-              tmem_ld_wait();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * f);
-              tmem_st_32x32(t_o + cb, v);
-            }
-            l_run *= f;
-            m_ref = m_new;
-          }
+          for (int i = 0; i < 8; ++i) vr[i] = make_uint4(0u, 0u, 0u, 0u);
         }
-        // pass 2: probabilities -> fp16 pairs -> tensor memory (over S), row sum
-        if (MODE == 1 && use_bits)
-          l_run += full_tile ? tile_probs_bits<false>(t_s, kv_valid, c, m_ref, bw, bits_neg)
-                             : tile_probs_bits<true>(t_s, kv_valid, c, m_ref, bw, bits_neg);
-        else
-          l_run += full_tile ? tile_probs(t_s, c, m_ref) : tail_probs(t_s, kv_valid, c, m_ref);
-        if (!full_tile && t == 0) {
-          // tail tile: blank the V rows of keys that do not belong to this sequence
-          // (tile 0's PV is issued before tile 1's, so tile 0's warpgroup does it for both)
-          if (!mbar_wait_warp(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
-            ok = false;
-            break;
-          }
-          if (r >= kv_valid && r < ((kv_valid + 15) & ~15)) {
-            uint4* vr = reinterpret_cast<uint4*>(smem + Cfg::kSmemV + stage * kTileBytes + r * 128);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) vr[i] = make_uint4(0u, 0u, 0u, 0u);
-          }
-          fence_proxy_async_smem();
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&p_full[t]);
-        if (++stage == kStages) {
-          stage = 0;
-          phase ^= 1u;
-        }
-      }
-      if (ok) ok = mbar_wait_warp(o_done, 0, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
-      tc_fence_after();
-      if (ok) {
-        // O / row sum -> fp16 -> global memory by way of the Q tile, which no MMA reads any more (o_done covers the
-        // last S as well): as in the persistent kernel, a whole 32-row slab leaves by one bulk store, a ragged one by
-        // stores that cover whole 128-byte lines.  Row by row from the threads (32 lines per instruction) it took
-        // 1.0-1.3k clocks of a short item and, with the machine full, 5.3k of a 512-token one.
-        const float inv = 1.0f / l_run;
-        const int row0 = q0 + t * kQRows + quarter * 32;  // first query row of this warp's slab, within the sequence
-        uint8_t* stage_out = smem + Cfg::kSmemQ + t * kTileBytes + quarter * (32 * 128);
-#pragma unroll
-        for (int cb = 0; cb < kHeadDim; cb += 32) {
-          uint32_t v[32];
-          tmem_ld_32x32(t_o + cb, v);
-          tmem_ld_wait();
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint4 w;
-            w.x = pack_half2(__uint_as_float(v[u * 8 + 0]) * inv, __uint_as_float(v[u * 8 + 1]) * inv);
-            w.y = pack_half2(__uint_as_float(v[u * 8 + 2]) * inv, __uint_as_float(v[u * 8 + 3]) * inv);
-            w.z = pack_half2(__uint_as_float(v[u * 8 + 4]) * inv, __uint_as_float(v[u * 8 + 5]) * inv);
-            w.w = pack_half2(__uint_as_float(v[u * 8 + 6]) * inv, __uint_as_float(v[u * 8 + 7]) * inv);
-            *reinterpret_cast<uint4*>(stage_out + lane * 128 + ((((cb >> 3) + u) ^ (lane & 7)) << 4)) = w;
-          }
-        }
-        const bool whole_slab = args.tma_out != 0 && row0 + 32 <= L;
-        if (whole_slab) fence_proxy_async_smem();
-        __syncwarp();
-        if (whole_slab) {
-          if (lane == 0) {
-            tma_store_2d(&tm_ctx, stage_out, col_q, seq_start + row0);
-            tma_store_commit();
-            tma_store_wait_all();
-          }
-        } else {
-          const int sub = lane >> 3, unit = lane & 7;  // row within a group of four, 16-byte unit of the row
-          __half* out_base = args.ctx + static_cast<size_t>(seq_start + row0) * args.hidden + col_q + unit * 8;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int row = 4 * k + sub;
-            const uint4 w = *reinterpret_cast<const uint4*>(stage_out + row * 128 + ((unit ^ (row & 7)) << 4));
-            if (row0 + row < L) *reinterpret_cast<uint4*>(out_base + static_cast<size_t>(row) * args.hidden) = w;
-          }
-        }
+        fence_proxy_async_smem();
       }
       tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+      if (++stage == kStages) {
+        stage = 0;
+        phase ^= 1u;
+      }
     }
+    if (ok) ok = mbar_wait_warp(o_done, 0, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
+    tc_fence_after();
+    if (ok) {
+      // O / row sum -> fp16 -> global memory by way of the Q tile, which no MMA reads any more (o_done covers the
+      // last S as well): as in the persistent kernel, a whole 32-row slab leaves by one bulk store, a ragged one by
+      // stores that cover whole 128-byte lines.  Row by row from the threads (32 lines per instruction) it took
+      // 1.0-1.3k clocks of a short item and, with the machine full, 5.3k of a 512-token one.
+      const float inv = 1.0f / l_run;
+      const int row0 = q0 + quarter * 32;  // first query row of this warp's slab, within the sequence
+      uint8_t* stage_out = smem + Cfg::kSmemQ + quarter * (32 * 128);
+#pragma unroll
+      for (int cb = 0; cb < kHeadDim; cb += 32) {
+        uint32_t v[32];
+        tmem_ld_32x32(t_o + cb, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          uint4 w;
+          w.x = pack_half2(__uint_as_float(v[u * 8 + 0]) * inv, __uint_as_float(v[u * 8 + 1]) * inv);
+          w.y = pack_half2(__uint_as_float(v[u * 8 + 2]) * inv, __uint_as_float(v[u * 8 + 3]) * inv);
+          w.z = pack_half2(__uint_as_float(v[u * 8 + 4]) * inv, __uint_as_float(v[u * 8 + 5]) * inv);
+          w.w = pack_half2(__uint_as_float(v[u * 8 + 6]) * inv, __uint_as_float(v[u * 8 + 7]) * inv);
+          *reinterpret_cast<uint4*>(stage_out + lane * 128 + ((((cb >> 3) + u) ^ (lane & 7)) << 4)) = w;
+        }
+      }
+      const bool whole_slab = args.tma_out != 0 && row0 + 32 <= L;
+      if (whole_slab) fence_proxy_async_smem();
+      __syncwarp();
+      if (whole_slab) {
+        if (lane == 0) {
+          tma_store_2d(&tm_ctx, stage_out, col_q, seq_start + row0);
+          tma_store_commit();
+          tma_store_wait_all();
+        }
+      } else {
+        const int sub = lane >> 3, unit = lane & 7;  // row within a group of four, 16-byte unit of the row
+        __half* out_base = args.ctx + static_cast<size_t>(seq_start + row0) * args.hidden + col_q + unit * 8;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int row = 4 * k + sub;
+          const uint4 w = *reinterpret_cast<const uint4*>(stage_out + row * 128 + ((unit ^ (row & 7)) << 4));
+          if (row0 + row < L) *reinterpret_cast<uint4*>(out_base + static_cast<size_t>(row) * args.hidden) = w;
+        }
+      }
+    }
+    tc_fence_before();
   }
 
   __syncthreads();
