@@ -44,11 +44,18 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ------------------------------------------------- programmatic dependent launch
-// Every kernel of the library starts with pdl_launch_dependents() (the next kernel of the
-// stream may be launched as soon as all CTAs of this one have started) and calls
-// pdl_wait() before its first access to global memory that an earlier kernel may have
-// written or may still read: the wait returns once the preceding kernel has completed
-// and its writes are visible.  Without the launch attribute both are no-ops.
+// pdl_launch_dependents(): the next kernel of the stream may be launched as soon as all CTAs of this one have said so
+// (or have ended).  pdl_wait(): returns once the preceding kernel has completed and its writes are visible; every CTA
+// of every kernel calls it before it ends, so a kernel that has completed tells that all before it have.  Without the
+// launch attribute both are no-ops.  What holds between the kernels of a call:
+//  * The first one is launched the ordinary way (pdl_next_launch_plain), so all that the caller's stream did before the
+//    call is complete and visible to every kernel of the call, before its pdl_wait() too.  Weights, bias, gamma, beta and
+//    a packed call's offsets may therefore be read ahead of the wait.
+//  * Kernels say pdl_launch_dependents() first thing - except those that run second in a call (pack_rows,
+//    embedding_layernorm, mask_bits), which say it after their own pdl_wait().  So from the third kernel on, what the
+//    FIRST kernel of the call wrote is complete and visible ahead of the wait as well: the attention kernels read the
+//    offsets there (MhaLaunch::early_offsets).
+//  * Anything else that an earlier kernel may have written or may still read is touched after pdl_wait() only.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Hint: bring the 128-byte line at `p` into L1 (constants such as bias, gamma and beta, asked for

@@ -994,7 +994,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
   if (warp >= 4) {
     setmaxnreg_dec<40>();
     if (!smem_ok) {
-      // fall through to the teardown
+      pdl_wait();  // then straight to the teardown
     } else if (warp == 4) {
       // ------------------------------------------------------------------ loads
       int stage = 0;

@@ -1,6 +1,6 @@
-"""CPU: what the kernels of a call may take for granted when they start ahead of their predecessor's end.  Kernels that
-read parameters ahead of their dependency wait rely on the call's first kernel being launched the ordinary way; forgotten,
-it would be a race that shows on a device only now and then, so it is looked up in the source."""
+"""CPU: what the kernels of a call may take for granted when they start ahead of their predecessor's end (the rules stand
+in csrc/common.cuh).  Broken, each would be a race that shows on a device only now and then, so the order of the two
+instructions and the plain first launch are looked up in the sources."""
 import os
 import re
 
@@ -16,6 +16,14 @@ def _body(name, start):
     return src[at:src.index("\n}\n", at)]
 
 
+@pytest.mark.parametrize("name,kernel", [("offsets.cu", "pack_rows_kernel("), ("offsets.cu", "mask_bits_kernel("),
+                                         ("embed_pool.cu", "embedding_layernorm_kernel(")])
+def test_second_kernels_of_a_call_trigger_after_their_own_wait(name, kernel):
+    body = _body(name, kernel)
+    assert body.index("pdl_wait();") < body.index("pdl_launch_dependents();")
+    assert "return" not in body[:body.index("pdl_launch_dependents();")]
+
+
 @pytest.mark.parametrize("entry,first", [
     ("static int stack_padded(", "launch_build_offsets("), ("static int stack_general(", "launch_uniform_offsets("),
     ("int bt_stack_forward_packed(", "run_layer("), ("int bt_gemm(", "run_gemm("), ("int bt_gemm_layernorm(", "run_gemm("),
@@ -25,3 +33,9 @@ def _body(name, start):
 def test_first_kernel_of_a_call_that_reads_parameters_early_is_launched_plainly(entry, first):
     body = _body("encoder.cu", entry)
     assert body.index("pdl_next_launch_plain();") < body.index(first)
+
+
+def test_offsets_are_read_early_only_inside_a_forward():
+    src = open(os.path.join(CSRC, "encoder.cu")).read()
+    calls = re.findall(r"run_mha\(h,[^;]*?, (true|false)(?:, gm)?\)", src)
+    assert sorted(calls) == ["false", "true"]  # bt_attention and run_layer
