@@ -112,18 +112,20 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 // caller must then leave its loop and fall through to the common teardown.  The
 // answer is the calling lane's own: what a warp waits for goes through the two forms below.
 // The bound is ~2^31 SM cycles (about a second) unless the caller gives another,
-// checked every 256 polls; once the flag is up, a wait polls once.
+// checked every 256 polls; once the flag is up, a wait ends after nine (not after
+// its first: a look at the flag between two polls that a K loop's wait does need was
+// seen in the GEMMs' time).
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity,
                                                   volatile int* abort_flag, int* status, int code,
                                                   long long max_cycles = (1ll << 31)) {
   if (mbar_try_wait(bar, parity)) return true;
-  if (*abort_flag != 0) return false;
   const long long t0 = clock64();
   uint32_t polls = 0;
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((++polls & 255u) == 0u) {
-      if (*abort_flag != 0) return false;
+    ++polls;
+    if ((polls & 255u) == 8u && *abort_flag != 0) return false;
+    if ((polls & 255u) == 0u) {
       if (clock64() - t0 > max_cycles) {
         *abort_flag = 1;
         if (status != nullptr) atomicCAS(status, 0, code);
@@ -133,16 +135,26 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
-// The same for a warp whose 32 lanes all wait: one answer for the warp, from a vote.  Every wait of a kernel's roles
-// goes through it (or, in a K loop, through the latched form below): lanes that parted ways where a wait gave up would
-// hang in the next warp-wide instruction (elect.sync, tcgen05.ld, __syncwarp), bound or no bound.
+// The same for a warp whose 32 lanes all wait: one answer for the warp, from a vote.  No kernel branches on a lane's
+// own answer: lanes that parted ways where a wait gave up would hang in the next warp-wide instruction (elect.sync,
+// tcgen05.ld, __syncwarp), bound or no bound.  A role votes (this form), goes on to the end of its K loop and votes there
+// (mbar_wait_latched), or goes on regardless (mbar_wait_anyway).
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
                                                int code, long long max_cycles = (1ll << 31)) {
   return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, status, code, max_cycles)) != 0;
 }
 
+// The wait of a role that can go on whatever the answer: where it gives up the status word is set, the CTA's flag is up,
+// later waits end after nine polls, and what the role makes of the bytes that did not arrive is as invalid as the launch's output
+// is then.  For waits in the middle of a tile, where a vote is time: with votes at all waits of the LayerNorm epilogue and
+// the softmax warps a BERT-large forward of 36 row tiles took 1794 us against 1706, a causal one of 1024 tokens 869 / 854.
+__device__ __forceinline__ void mbar_wait_anyway(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                                 int code) {
+  (void)mbar_wait_bounded(bar, parity, abort_flag, status, code);
+}
+
 // The wait of a loop that goes on to its end when a wait gave up (a vote per K block costs 30 clocks): `ok` is the
-// lane's answer so far; the loop ends in a vote over it.  The blocks that are left are polled once each, because the
+// lane's answer so far; the loop ends in a vote over it.  The blocks that are left are polled nine times each, because the
 // flag is up: the time to give up stays one bound however many they are.  (Not polled at all, behind a branch on `ok`,
 // was measured too: a 12-layer forward of one 614-token sequence 581 -> 585 us.)
 __device__ __forceinline__ bool mbar_wait_latched(bool ok, uint64_t* bar, uint32_t parity, volatile int* abort_flag,
@@ -160,7 +172,7 @@ __device__ __forceinline__ bool mbar_wait_latched(bool ok, uint64_t* bar, uint32
 // instructions themselves are predicated on an elected lane, all MMAs of a K block and their commit on one
 // election (umma_k_block): 84 clocks per MMA in the main loop, 525 -> 335 clocks per K block of 64 (N <= 128).
 // Because elect.sync needs the whole warp, a warp's lanes must not part ways after a wait that gave up: see
-// mbar_wait_warp and mbar_wait_latched.
+// the three forms of a warp's wait above.
 __device__ __forceinline__ int uniform_int(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ uint32_t uniform_u32(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
 

@@ -465,7 +465,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       const uint32_t aphase = (it >> 1) & 1;
       uint4 resv[kHasResidual ? BLOCK_N / 16 : 1];
       prefetch_residual<BLOCK_N, EPI>(args, m0, n0, M, quarter, col_half, lane, resv, sp);
-      if (!mbar_wait_warp(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
+      mbar_wait_anyway(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout);
       tc_fence_after();
       if (warp == 2 && lane == 0) gstamp(args.timing, it, 2);
       epilogue_tile<BLOCK_N, EPI, Cfg::tma_store(EPI), 1>(args, &tm_out, stg, tmem_base + as * BLOCK_N, m0, n0, M, quarter,
@@ -707,7 +707,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       const uint32_t aphase = (it >> 1) & 1;
       uint4 resv[kHasResidual ? kTileN / 16 : 1];
       prefetch_residual<kTileN, EPI>(args, m0, n0, M, quarter, col_half, lane, resv);
-      if (!mbar_wait_warp(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
+      mbar_wait_anyway(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout);
       tc_fence_after();
       if (warp == 2 && lane == 0) gstamp(args.timing, it, 2);
       epilogue_tile<kTileN, EPI, true, Cfg::kStagingBufs>(args, &tm_out, stg, tmem_base + as * kTileN, m0, n0, M,
@@ -805,7 +805,7 @@ __device__ __forceinline__ void ln_epilogue_loop(const GemmArgs& args, const CUt
         vg = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(args.gamma) + n0) + lane);
         vt = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(args.beta) + n0) + lane);
       }
-      if (!mbar_wait_warp(vec_empty, (it & 1u) ^ 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
+      mbar_wait_anyway(vec_empty, (it & 1u) ^ 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout);
       vec_s[lane] = vb;
       vec_s[32 + lane] = vg;
       vec_s[64 + lane] = vt;
@@ -821,9 +821,9 @@ __device__ __forceinline__ void ln_epilogue_loop(const GemmArgs& args, const CUt
       mbar_arrive_expect_tx(&res_bar[e], kStagingBytesPerWarp);
       tma_load_2d(stg, tm_res, &res_bar[e], gcol0, row0);
     }
-    if (!mbar_wait_warp(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
+    mbar_wait_anyway(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout);
     tc_fence_after();
-    if (!mbar_wait_warp(vec_full, it & 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout)) break;
+    mbar_wait_anyway(vec_full, it & 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout);
     if (warp == 2 && lane == 0) gstamp(args.timing, it, 2);
     const uint4* sbias = vec_s + col_half * (kColsPerThread / 8);
     const uint4* sgamma = vec_s + 32 + col_half * (kColsPerThread / 8);
@@ -836,15 +836,11 @@ __device__ __forceinline__ void ln_epilogue_loop(const GemmArgs& args, const CUt
     {
       uint32_t raw[2][32];
       tmem_ld_32x32(t_row, raw[0]);
-      bool res_ok = true;
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         // this thread's 64 residual values of box hh: row `lane` of the swizzled buffer
-        if (!mbar_wait_warp(&res_bar[e], (static_cast<uint32_t>(it) * 2u + hh) & 1u, abort_flag, args.status,
-                               kStatusGemmEpilogueTimeout)) {
-          res_ok = false;
-          break;
-        }
+        mbar_wait_anyway(&res_bar[e], (static_cast<uint32_t>(it) * 2u + hh) & 1u, abort_flag, args.status,
+                         kStatusGemmEpilogueTimeout);
         uint4 rres[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q)
@@ -891,7 +887,6 @@ __device__ __forceinline__ void ln_epilogue_loop(const GemmArgs& args, const CUt
           tmem_st_32x32(t_row + c, raw[ci & 1]);
         }
       }
-      if (!res_ok) break;
       float s0, s1, q0, q1;
       unpack_f32x2(sd2, s0, s1);
       unpack_f32x2(sdd2, q0, q1);

@@ -625,7 +625,6 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
     float l_run = 0.f;
     int stage = 0;
     uint32_t phase = 0;
-    bool ok = true;
     // binary mask, no bias: applied from bits inside the two softmax passes
     const bool use_bits = GENERAL && args.gen_bits != nullptr && __ldg(args.gen_bits_flag) == 0;
     const float bits_neg = -10000.0f * args.gen_inv_scale;
@@ -642,10 +641,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
           for (int u = 0; u < 8; ++u) bias_q[u] = __ldg(bt + u * 128);
         }
       }
-      if (!mbar_wait_warp(s_full, j & 1, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
-        ok = false;
-        break;
-      }
+      mbar_wait_anyway(s_full, j & 1, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
       tc_fence_after();
       uint4 bw = make_uint4(~0u, ~0u, ~0u, ~0u);  // a row that does not exist masks nothing
       if (GENERAL && use_bits) {
@@ -704,10 +700,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
         l_run += full_tile ? tile_probs(t_s, c, m_ref) : tail_probs(t_s, kv_valid, c, m_ref);
       if (!full_tile) {
         // tail tile: blank the V rows of keys that do not belong to this sequence
-        if (!mbar_wait_warp(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
-          ok = false;
-          break;
-        }
+        mbar_wait_anyway(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
         if (r >= kv_valid && r < ((kv_valid + 15) & ~15)) {
           uint4* vr = reinterpret_cast<uint4*>(smem + Cfg::kSmemV + stage * kTileBytes + r * 128);
 #pragma unroll
@@ -723,7 +716,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
         phase ^= 1u;
       }
     }
-    if (ok) ok = mbar_wait_warp(o_done, 0, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
+    const bool ok = mbar_wait_warp(o_done, 0, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
     tc_fence_after();
     if (ok) {
       // O / row sum -> fp16 -> global memory by way of the Q tile, which no MMA reads any more (o_done covers the
@@ -1153,10 +1146,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
       float l_run = 0.f;
       for (int j = 0; j < n_kv; ++j, ++step) {
         const int kv_valid = min(kKvRows, L - j * kKvRows);
-        if (!mbar_wait_warp(s_full, step & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
-          ok = false;
-          break;
-        }
+        mbar_wait_anyway(s_full, step & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
         tc_fence_after();
         uint32_t s[128];
         tmem_ld_32x32_at<0>(t_s, s);
@@ -1187,10 +1177,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
           m_ref = m_new;
         } else if (__any_sync(0xffffffffu, (m_new - m_ref) > kRescaleThreshold)) {
           // O belongs to the P V MMAs of the previous key tile until those have retired
-          if (!mbar_wait_warp(pv_done, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
-            ok = false;
-            break;
-          }
+          mbar_wait_anyway(pv_done, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
           tc_fence_after();
           pv_waited = true;
           const float f = ex2_approx(m_ref - m_new);
@@ -1221,10 +1208,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
         l_run += (l0 + l1) + (l2 + l3);
         if (!pv_waited) {
           // P belongs to the P V MMAs of the previous key tile until those have retired
-          if (!mbar_wait_warp(pv_done, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
-            ok = false;
-            break;
-          }
+          mbar_wait_anyway(pv_done, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
           tc_fence_after();
         }
         tmem_st_32x16_at<0>(t_p, pk);
@@ -1233,10 +1217,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
         tmem_st_32x16_at<48>(t_p + 48, pk);
         if (kv_valid != kKvRows) {
           // tail tile: blank the V rows of keys that do not belong to this sequence
-          if (!mbar_wait_warp(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
-            ok = false;
-            break;
-          }
+          mbar_wait_anyway(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
           if (r >= kv_valid) {
             uint4* vr = reinterpret_cast<uint4*>(smem + kSmemV + stage * kTileBytes + r * 128);
 #pragma unroll
@@ -1253,7 +1234,6 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
           phase ^= 1u;
         }
       }
-      if (!ok) break;
       // the next item is found while the last P V of this one runs
       int seq_start_n = 0, L_n = 0, qt_n = 0, head_n = 0;
       have = decode_item(args, snake_item(round + 1, cta, G), cur_b, cur_first, seq_start_n, L_n, qt_n, head_n, false);
