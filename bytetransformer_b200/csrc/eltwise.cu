@@ -75,12 +75,12 @@ __device__ __forceinline__ void load_gb8(const void* p, int vec, float (&f)[8]) 
 // RESTORE = false: rows [0, M) of x -> rows [0, M) of out.
 // RESTORE = true : grid covers the B*S padded rows; row (b,i) reads packed row
 //                  batch_idx[b]+i when i < len_b, else writes zeros.
-template <bool RESTORE, bool GB_FP32, bool X_FP32, int NVEC, bool SPLIT>
+template <bool RESTORE, bool GB_FP32, bool X_FP32, int NVEC>
 __global__ void __launch_bounds__(kLnWarps * 32)
 layernorm_rows_kernel(const void* __restrict__ x_v, const __half* __restrict__ bias,
                       const __half* __restrict__ residual, const void* __restrict__ gamma,
                       const void* __restrict__ beta, __half* __restrict__ out, const int* __restrict__ m_dev,
-                      int m_rows, const int* __restrict__ batch_idx, int S, int hidden, float eps, LnSplit split) {
+                      int m_rows, const int* __restrict__ batch_idx, int S, int hidden, float eps) {
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -137,22 +137,6 @@ layernorm_rows_kernel(const void* __restrict__ x_v, const __half* __restrict__ b
         const float4 a = __ldg(xf + 2 * v), b = __ldg(xf + 2 * v + 1);
         val[it][0] = a.x; val[it][1] = a.y; val[it][2] = a.z; val[it][3] = a.w;
         val[it][4] = b.x; val[it][5] = b.y; val[it][6] = b.z; val[it][7] = b.w;
-        // the sum arrives in `split.n` <= kLnMaxSplit fp32 parts (K ranges of the GEMM before); the loads of
-        // all parts are independent and issued together
-        if (SPLIT) {
-          float4 c[kLnMaxSplit - 1], d[kLnMaxSplit - 1];
-#pragma unroll
-          for (int sp = 1; sp < kLnMaxSplit; ++sp) {
-            const float4* xs = xf + sp * (split.stride / 4);
-            c[sp - 1] = sp < split.n ? __ldg(xs + 2 * v) : make_float4(0.f, 0.f, 0.f, 0.f);
-            d[sp - 1] = sp < split.n ? __ldg(xs + 2 * v + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
-          }
-#pragma unroll
-          for (int sp = 0; sp < kLnMaxSplit - 1; ++sp) {
-            val[it][0] += c[sp].x; val[it][1] += c[sp].y; val[it][2] += c[sp].z; val[it][3] += c[sp].w;
-            val[it][4] += d[sp].x; val[it][5] += d[sp].y; val[it][6] += d[sp].z; val[it][7] += d[sp].w;
-          }
-        }
       } else {
         unpack8(__ldg(x4 + v), val[it]);
       }
@@ -206,24 +190,27 @@ layernorm_rows_kernel(const void* __restrict__ x_v, const __half* __restrict__ b
   }  // row loop
 }
 
-// The same for the fp32 sums of a call of few rows: one CTA per row, four columns per thread.  Such a kernel is a
-// chain of latencies, not of bytes: a warp per row loads the up to eight partial sums of its columns in three
-// rounds (48 16-byte loads per lane), here every thread has its loads in flight at once; gamma and beta are in
-// registers before the dependency wait, and the code is a tenth of the length (a kernel that runs once per SM fetches
-// every instruction from L2).  Measured, 12 layers, us per forward with a
-// warp / a CTA per row: 1 sequence of 38 tokens (4 and 8 partial sums) 480 / 412, 1 of 614 (2) 638 / 590, 7 up to 93
-// 544 / 493, 16 up to 128 698 / 658, 32 up to 128 (4096 allocated rows) 980 / 975; 8192 rows 1226 / 1226.
-template <bool RESTORE, bool GB_FP32, int SPLITS>
+// The same for the fp32 sums that a GEMM left (no bias, no residual): a CTA holds one row, or ROWS of them, four columns
+// per thread.  Such a kernel is a chain of latencies, not of bytes: a warp per row loads the up to eight partial sums of
+// its columns in three rounds (48 16-byte loads per lane), here every thread has its loads in flight at once; gamma and
+// beta are in registers before the dependency wait, and the code is a tenth of the length (a kernel that runs once per
+// SM fetches every instruction from L2).  One row per CTA shortens the chain most; with more rows the statistics, which
+// every warp forms for itself then, cost more issue slots than they save, and several rows share a CTA, a warp forming
+// the statistics of each.  Measured, us per 12-layer forward, warp per row / one row / four rows per CTA (hidden 768, all
+// rows valid): 88 rows 480 / 412 / -, 984 rows 745 / 708 / -, 1112 rows 687 / 689 / 662, 2008 rows 857 / 873 / 812,
+// 4096 rows 1328 / 1405 / 1273, 8000 rows 2187 / 2460 / 2208.
+template <bool RESTORE, bool GB_FP32, int SPLITS, int ROWS, int NVEC>
 __global__ void __launch_bounds__(256)
 layernorm_cta_kernel(const float* __restrict__ x, const void* __restrict__ gamma, const void* __restrict__ beta,
                      __half* __restrict__ out, const int* __restrict__ m_dev, int m_rows,
                      const int* __restrict__ batch_idx, int S, int hidden, float eps, LnSplit split) {
-  // the row, four columns per unit: even and odd units apart (by 64 bytes modulo the banks), so that a lane's eight
+  // a row's sums, four columns per unit: even and odd units apart (by 64 bytes modulo the banks), so that a lane's eight
   // columns are two conflict-free reads
-  __shared__ float4 vals[2][kLnMaxVec * 32 + 4];
+  __shared__ float4 vals[ROWS][2][NVEC * 32 + 4];
+  __shared__ float2 stats[ROWS];  // mean, 1 / standard deviation
   pdl_launch_dependents();
   const int v = threadIdx.x;  // this thread's four columns
-  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
   const bool has = v < hidden / 4;
   float g[4] = {}, bt[4] = {};
   if (has) {
@@ -240,110 +227,158 @@ layernorm_cta_kernel(const float* __restrict__ x, const void* __restrict__ gamma
     }
   }
   pdl_wait();
-  const int row = blockIdx.x;
-  int src_row = row, row_limit = m_rows;
-  uint2* o2 = reinterpret_cast<uint2*>(out + static_cast<size_t>(row) * hidden) + v;
-  if (RESTORE) {
-    const int b = row / S;
-    const int i = row - b * S;
-    const int off = __ldg(batch_idx + b);
-    if (i >= __ldg(batch_idx + b + 1) - off) {
-      if (has) *o2 = make_uint2(0u, 0u);
-      return;
-    }
-    src_row = off + i;
-  } else if (m_dev != nullptr) {
-    row_limit = __ldg(m_dev);
-  }
-  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (has) {
-    const float4* xr = reinterpret_cast<const float4*>(x + static_cast<size_t>(src_row) * hidden) + v;
-    float4 p[SPLITS];
+  const int row0 = static_cast<int>(blockIdx.x) * ROWS;
+  uint2* o2 = reinterpret_cast<uint2*>(out + static_cast<size_t>(row0) * hidden) + v;
+  int src[ROWS];  // row of x, or -1: a row of zeros, or -2: no such row
+  int row_limit = m_rows;
 #pragma unroll
-    for (int sp = 0; sp < SPLITS; ++sp)
-      p[sp] = (sp == 0 || sp < split.n) ? __ldg(xr + sp * (split.stride / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    a = p[0];
-#pragma unroll
-    for (int sp = 1; sp < SPLITS; ++sp) {
-      a.x += p[sp].x;
-      a.y += p[sp].y;
-      a.z += p[sp].z;
-      a.w += p[sp].w;
+  for (int r = 0; r < ROWS; ++r) {
+    src[r] = (ROWS == 1 || row0 + r < m_rows) ? row0 + r : -2;
+    if (RESTORE && (ROWS == 1 || src[r] >= 0)) {
+      const int b = src[r] / S;
+      const int i = src[r] - b * S;
+      const int off = __ldg(batch_idx + b);
+      src[r] = i < __ldg(batch_idx + b + 1) - off ? off + i : -1;
     }
   }
-  // (the row was read before its existence was known: it lies inside the allocation either way)
-  if (!RESTORE && row >= row_limit) return;
-  if (has) vals[v & 1][v >> 1] = a;
-  __syncthreads();
-  // Statistics as layernorm_rows_kernel forms them, by every warp for itself: the same columns per lane in the same
-  // order, so that both forms give the same bits.
-  const int nvec = hidden >> 3;
-  float val[kLnMaxVec][8];
-  float sum = 0.f;
-#pragma unroll
-  for (int it = 0; it < kLnMaxVec; ++it) {
-    const int u = it * 32 + lane;
-    if (u < nvec) {
-      const float4 lo = vals[0][u], hi = vals[1][u];
-      val[it][0] = lo.x; val[it][1] = lo.y; val[it][2] = lo.z; val[it][3] = lo.w;
-      val[it][4] = hi.x; val[it][5] = hi.y; val[it][6] = hi.z; val[it][7] = hi.w;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) sum += val[it][k];
-    }
+  if (!RESTORE && m_dev != nullptr) row_limit = __ldg(m_dev);
+  if (RESTORE && ROWS == 1 && src[0] < 0) {
+    if (has) *o2 = make_uint2(0u, 0u);
+    return;
   }
-  const float mean = warp_sum(sum) / static_cast<float>(hidden);
-  float sq = 0.f;
+  float4 a[ROWS];
 #pragma unroll
-  for (int it = 0; it < kLnMaxVec; ++it) {
-    if (it * 32 + lane < nvec) {
+  for (int r = 0; r < ROWS; ++r) {
+    a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (has && (ROWS == 1 || src[r] >= 0)) {
+      const float4* xr = reinterpret_cast<const float4*>(x + static_cast<size_t>(src[r]) * hidden) + v;
+      float4 p[SPLITS];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const float d = val[it][k] - mean;
-        sq = fmaf(d, d, sq);
+      for (int sp = 0; sp < SPLITS; ++sp)
+        p[sp] = (sp == 0 || sp < split.n) ? __ldg(xr + sp * (split.stride / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      a[r] = p[0];
+#pragma unroll
+      for (int sp = 1; sp < SPLITS; ++sp) {
+        a[r].x += p[sp].x;
+        a[r].y += p[sp].y;
+        a[r].z += p[sp].z;
+        a[r].w += p[sp].w;
       }
     }
   }
-  const float rstd = rsqrtf(warp_sum(sq) / static_cast<float>(hidden) + eps);
-  a.x -= mean;
-  a.y -= mean;
-  a.z -= mean;
-  a.w -= mean;
-  if (has)
-    *o2 = make_uint2(pack_half2(fmaf(a.x * rstd, g[0], bt[0]), fmaf(a.y * rstd, g[1], bt[1])),
-                     pack_half2(fmaf(a.z * rstd, g[2], bt[2]), fmaf(a.w * rstd, g[3], bt[3])));
+  // (the rows were read before their existence was known: they lie inside the allocation either way)
+  if (!RESTORE) {
+    if (row0 >= row_limit) return;
+#pragma unroll
+    for (int r = 1; r < ROWS; ++r)
+      if (row0 + r >= row_limit) src[r] = -2;
+  }
+  if (has) {
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) vals[r][v & 1][v >> 1] = a[r];
+  }
+  __syncthreads();
+  // Statistics as layernorm_rows_kernel forms them: the same columns per lane in the same order, so that both forms give
+  // the same bits.  One row per CTA: every warp forms them for itself; more: a warp per row.
+  const int nvec = hidden >> 3;
+  auto row_stats = [&](int r) {
+    float val[NVEC][8];
+    float sum = 0.f;
+#pragma unroll
+    for (int it = 0; it < NVEC; ++it) {
+      const int u = it * 32 + lane;
+      if (it + 1 < NVEC || u < nvec) {
+        const float4 lo = vals[r][0][u], hi = vals[r][1][u];
+        val[it][0] = lo.x; val[it][1] = lo.y; val[it][2] = lo.z; val[it][3] = lo.w;
+        val[it][4] = hi.x; val[it][5] = hi.y; val[it][6] = hi.z; val[it][7] = hi.w;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) sum += val[it][k];
+      }
+    }
+    const float mean = warp_sum(sum) / static_cast<float>(hidden);
+    float sq = 0.f;
+#pragma unroll
+    for (int it = 0; it < NVEC; ++it) {
+      if (it + 1 < NVEC || it * 32 + lane < nvec) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float d = val[it][k] - mean;
+          sq = fmaf(d, d, sq);
+        }
+      }
+    }
+    return make_float2(mean, rsqrtf(warp_sum(sq) / static_cast<float>(hidden) + eps));
+  };
+  float2 st[ROWS];
+  if (ROWS == 1) {
+    st[0] = row_stats(0);
+  } else {
+    for (int r = warp; r < ROWS; r += n_warps) {
+      const float2 t = row_stats(r);
+      if (lane == 0) stats[r] = t;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) st[r] = stats[r];
+  }
+  if (!has) return;
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    if (ROWS > 1 && src[r] == -2) continue;
+    const float mean = st[r].x, rstd = st[r].y;
+    o2[r * (hidden / 4)] = (ROWS > 1 && src[r] < 0) ? make_uint2(0u, 0u)
+                                      : make_uint2(pack_half2(fmaf((a[r].x - mean) * rstd, g[0], bt[0]),
+                                                              fmaf((a[r].y - mean) * rstd, g[1], bt[1])),
+                                                   pack_half2(fmaf((a[r].z - mean) * rstd, g[2], bt[2]),
+                                                              fmaf((a[r].w - mean) * rstd, g[3], bt[3])));
+  }
 }
 
-// The CTA-per-row form is ahead by 14 % of a forward at 64 rows and by 0.5 % at 4096, level at 8192 (above); more
-// rows are the warp-per-row form's, whose CTAs walk many rows each.
-constexpr long long kLnCtaMaxRows = 4096;
-bool ln_cta_form(const void* x, bool x_fp32, const __half* bias, const __half* residual, const void* gamma, const void* beta,
-                 long long rows, int hidden) {
-  return x_fp32 && bias == nullptr && residual == nullptr && rows <= kLnCtaMaxRows && hidden % 4 == 0 && hidden <= 1024 &&
+bool ln_cta_possible(const void* x, bool x_fp32, const __half* bias, const __half* residual, const void* gamma,
+                     const void* beta) {
+  return x_fp32 && bias == nullptr && residual == nullptr &&
          ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta)) & 15u) == 0;
 }
-template <bool RESTORE, bool GB_FP32>
+template <bool RESTORE, bool GB_FP32, int NVEC>
 cudaError_t launch_ln_cta(const void* x, const void* gamma, const void* beta, __half* out, const int* m_dev, int rows,
-                          const int* batch_idx, int S, int hidden, float eps, LnSplit split, cudaStream_t stream) {
+                          const int* batch_idx, int S, int hidden, float eps, LnSplit split, int per_cta,
+                          cudaStream_t stream) {
   const dim3 block((hidden / 4 + 31) / 32 * 32);
   auto go = [&](auto kern) {
-    return launch_pdl(kern, dim3(rows), block, 0, stream, reinterpret_cast<const float*>(x), gamma, beta, out, m_dev, rows,
-                      batch_idx, S, hidden, eps, split);
+    return launch_pdl(kern, dim3((rows + per_cta - 1) / per_cta), block, 0, stream, reinterpret_cast<const float*>(x), gamma,
+                      beta, out, m_dev, rows, batch_idx, S, hidden, eps, split);
   };
-  if (split.n <= 1) return go(layernorm_cta_kernel<RESTORE, GB_FP32, 1>);
-  if (split.n <= 2) return go(layernorm_cta_kernel<RESTORE, GB_FP32, 2>);
-  if (split.n <= 4) return go(layernorm_cta_kernel<RESTORE, GB_FP32, 4>);
-  return go(layernorm_cta_kernel<RESTORE, GB_FP32, kLnMaxSplit>);
+  if constexpr (NVEC > 1) {
+    if (per_cta == 4) return go(layernorm_cta_kernel<RESTORE, GB_FP32, 1, 4, NVEC>);
+  }
+  if constexpr (NVEC <= 3) {
+    if (per_cta == 2) return go(layernorm_cta_kernel<RESTORE, GB_FP32, 1, 2, NVEC>);
+  }
+  if (per_cta != 1) return cudaErrorInvalidValue;
+  if (split.n <= 1) return go(layernorm_cta_kernel<RESTORE, GB_FP32, 1, 1, NVEC>);
+  if (split.n <= 2) return go(layernorm_cta_kernel<RESTORE, GB_FP32, 2, 1, NVEC>);
+  if (split.n <= 4) return go(layernorm_cta_kernel<RESTORE, GB_FP32, 4, 1, NVEC>);
+  return go(layernorm_cta_kernel<RESTORE, GB_FP32, kLnMaxSplit, 1, NVEC>);
+}
+template <bool RESTORE, typename... Args>
+cudaError_t launch_ln_cta_dispatch(bool gb_fp32, int nvec, Args... args) {
+  switch (nvec) {
+    case 1: return gb_fp32 ? launch_ln_cta<RESTORE, true, 1>(args...) : launch_ln_cta<RESTORE, false, 1>(args...);
+    case 2: return gb_fp32 ? launch_ln_cta<RESTORE, true, 2>(args...) : launch_ln_cta<RESTORE, false, 2>(args...);
+    case 3: return gb_fp32 ? launch_ln_cta<RESTORE, true, 3>(args...) : launch_ln_cta<RESTORE, false, 3>(args...);
+    case 4: return gb_fp32 ? launch_ln_cta<RESTORE, true, 4>(args...) : launch_ln_cta<RESTORE, false, 4>(args...);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
-template <bool RESTORE, bool GB_FP32, bool X_FP32, bool SPLIT>
+template <bool RESTORE, bool GB_FP32, bool X_FP32>
 cudaError_t launch_ln_nvec(int nvec_needed, dim3 grid, cudaStream_t stream, const void* x, const __half* bias,
                            const __half* residual, const void* gamma, const void* beta, __half* out,
-                           const int* m_dev, int m_rows, const int* batch_idx, int S, int hidden, float eps,
-                           LnSplit split) {
+                           const int* m_dev, int m_rows, const int* batch_idx, int S, int hidden, float eps) {
 #define BT_LN_CASE(NV)                                                                                        \
   case NV:                                                                                                    \
-    return launch_pdl(layernorm_rows_kernel<RESTORE, GB_FP32, X_FP32, NV, SPLIT>, grid, dim3(kLnWarps * 32), 0, stream,  \
-                      x, bias, residual, gamma, beta, out, m_dev, m_rows, batch_idx, S, hidden, eps, split);
+    return launch_pdl(layernorm_rows_kernel<RESTORE, GB_FP32, X_FP32, NV>, grid, dim3(kLnWarps * 32), 0, stream,  \
+                      x, bias, residual, gamma, beta, out, m_dev, m_rows, batch_idx, S, hidden, eps);
   switch (nvec_needed) {
     BT_LN_CASE(1)
     BT_LN_CASE(2)
@@ -528,19 +563,25 @@ template <bool RESTORE>
 static cudaError_t launch_ln_dispatch(bool gb_fp32, bool x_fp32, int nv, dim3 grid, cudaStream_t stream, const void* x,
                                       const __half* bias, const __half* residual, const void* gamma, const void* beta,
                                       __half* out, const int* m_dev, int m_rows, const int* batch_idx, int S,
-                                      int hidden, float eps, LnSplit split) {
-#define BT_LN_ARGS nv, grid, stream, x, bias, residual, gamma, beta, out, m_dev, m_rows, batch_idx, S, hidden, eps, split
-  if (split.n > 1) {  // fp32 partial sums (checked by the callers)
-    if (gb_fp32) return launch_ln_nvec<RESTORE, true, true, true>(BT_LN_ARGS);
-    return launch_ln_nvec<RESTORE, false, true, true>(BT_LN_ARGS);
-  }
+                                      int hidden, float eps) {
+#define BT_LN_ARGS nv, grid, stream, x, bias, residual, gamma, beta, out, m_dev, m_rows, batch_idx, S, hidden, eps
   if (gb_fp32) {
-    if (x_fp32) return launch_ln_nvec<RESTORE, true, true, false>(BT_LN_ARGS);
-    return launch_ln_nvec<RESTORE, true, false, false>(BT_LN_ARGS);
+    if (x_fp32) return launch_ln_nvec<RESTORE, true, true>(BT_LN_ARGS);
+    return launch_ln_nvec<RESTORE, true, false>(BT_LN_ARGS);
   }
-  if (x_fp32) return launch_ln_nvec<RESTORE, false, true, false>(BT_LN_ARGS);
-  return launch_ln_nvec<RESTORE, false, false, false>(BT_LN_ARGS);
+  if (x_fp32) return launch_ln_nvec<RESTORE, false, true>(BT_LN_ARGS);
+  return launch_ln_nvec<RESTORE, false, false>(BT_LN_ARGS);
 #undef BT_LN_ARGS
+}
+
+int ln_rows_per_cta(long long rows, int hidden, int parts, bool in_forward) {
+  const long long sums = rows * hidden;
+  if (hidden > kLnMaxVec * 256 || rows > 4096) return 0;
+  if (!in_forward && hidden < 512 && rows > 512) return 0;
+  if (rows <= 1024) return (parts <= 1 && hidden >= 512 && sums >= 400 * 768) ? 4 : 1;
+  if (hidden >= 512 && hidden < 640 && rows <= 1536) return 2;
+  if (hidden >= 512) return (in_forward || sums <= 2048 * 768) ? 4 : 0;
+  return (in_forward && hidden >= 256) ? 2 : 0;
 }
 
 cudaError_t launch_layernorm(const void* x, bool x_fp32, const __half* bias, const __half* residual,
@@ -548,13 +589,15 @@ cudaError_t launch_layernorm(const void* x, bool x_fp32, const __half* bias, con
                              int m_rows, int hidden, float eps, cudaStream_t stream, LnSplit split) {
   if (hidden % 8 != 0 || hidden > kLnMaxVec * 256 || m_rows <= 0) return cudaErrorInvalidValue;
   if (split.n > 1 && (!x_fp32 || split.stride % 4 != 0 || split.n > kLnMaxSplit)) return cudaErrorInvalidValue;
-  if (ln_cta_form(x, x_fp32, bias, residual, gamma, beta, m_rows, hidden))
-    return gb_fp32 ? launch_ln_cta<false, true>(x, gamma, beta, out, m_dev, m_rows, nullptr, 0, hidden, eps, split, stream)
-                   : launch_ln_cta<false, false>(x, gamma, beta, out, m_dev, m_rows, nullptr, 0, hidden, eps, split, stream);
   const int nv = (hidden / 8 + 31) / 32;
+  const int per_cta = ln_rows_per_cta(m_rows, hidden, split.n, split.in_forward);
+  if (per_cta != 0 && ln_cta_possible(x, x_fp32, bias, residual, gamma, beta))
+    return launch_ln_cta_dispatch<false>(gb_fp32, nv, x, gamma, beta, out, m_dev, m_rows, static_cast<const int*>(nullptr), 0,
+                                         hidden, eps, split, per_cta, stream);
+  if (split.n > 1) return cudaErrorInvalidValue;  // partial sums come in calls of up to 1024 rows, from aligned buffers
   dim3 grid(ln_grid((m_rows + kLnWarps - 1) / kLnWarps));
   return launch_ln_dispatch<false>(gb_fp32, x_fp32, nv, grid, stream, x, bias, residual, gamma, beta, out, m_dev,
-                                   m_rows, nullptr, 0, hidden, eps, split);
+                                   m_rows, nullptr, 0, hidden, eps);
 }
 
 cudaError_t launch_layernorm_restore(const void* x, bool x_fp32, const __half* bias, const __half* residual,
@@ -565,14 +608,14 @@ cudaError_t launch_layernorm_restore(const void* x, bool x_fp32, const __half* b
   if (split.n > 1 && (!x_fp32 || split.stride % 4 != 0 || split.n > kLnMaxSplit)) return cudaErrorInvalidValue;
   const int nv = (hidden / 8 + 31) / 32;
   const long long rows = static_cast<long long>(B) * S;
-  if (ln_cta_form(x, x_fp32, bias, residual, gamma, beta, rows, hidden))
-    return gb_fp32 ? launch_ln_cta<true, true>(x, gamma, beta, out_padded, nullptr, static_cast<int>(rows), batch_idx, S,
-                                               hidden, eps, split, stream)
-                   : launch_ln_cta<true, false>(x, gamma, beta, out_padded, nullptr, static_cast<int>(rows), batch_idx, S,
-                                                hidden, eps, split, stream);
+  const int per_cta = ln_rows_per_cta(rows, hidden, split.n, split.in_forward);
+  if (per_cta != 0 && ln_cta_possible(x, x_fp32, bias, residual, gamma, beta))
+    return launch_ln_cta_dispatch<true>(gb_fp32, nv, x, gamma, beta, out_padded, static_cast<const int*>(nullptr),
+                                        static_cast<int>(rows), batch_idx, S, hidden, eps, split, per_cta, stream);
+  if (split.n > 1) return cudaErrorInvalidValue;
   dim3 grid(ln_grid((rows + kLnWarps - 1) / kLnWarps));
   return launch_ln_dispatch<true>(gb_fp32, x_fp32, nv, grid, stream, x, bias, residual, gamma, beta, out_padded,
-                                  nullptr, static_cast<int>(rows), batch_idx, S, hidden, eps, split);
+                                  nullptr, static_cast<int>(rows), batch_idx, S, hidden, eps);
 }
 
 cudaError_t launch_add_bias_gelu(__half* x, const __half* bias, const int* m_dev, int m_rows, int n, int gelu_kind,

@@ -436,7 +436,7 @@ static int run_layer(bt_handle h, int layer, const __half* x_in, __half* x_out, 
     {
       LaunchScope scope(h, BT_PROF_LAYERNORM, stream);
       e = launch_layernorm(ws.pre, true, nullptr, nullptr, w.attr_output_layernorm_gamma, w.attr_output_layernorm_beta,
-                           gb32, ws.y, m_dev, rows, H, h->cfg.ln_eps, stream, LnSplit{split_attn, split_stride});
+                           gb32, ws.y, m_dev, rows, H, h->cfg.ln_eps, stream, LnSplit{split_attn, split_stride, true});
     }
     if (e != cudaSuccess) return fail_cuda(h, e, "layernorm launch");
   }
@@ -455,10 +455,10 @@ static int run_layer(bt_handle h, int layer, const __half* x_in, __half* x_out, 
   if (restore_to != nullptr)
     e = launch_layernorm_restore(ws.pre, true, nullptr, nullptr, w.output_layernorm_gamma, w.output_layernorm_beta, gb32,
                                  restore_to, batch_idx, B, S_or_maxlen, H, h->cfg.ln_eps, stream,
-                                 LnSplit{split_ffn2, split_stride});
+                                 LnSplit{split_ffn2, split_stride, true});
   else
     e = launch_layernorm(ws.pre, true, nullptr, nullptr, w.output_layernorm_gamma, w.output_layernorm_beta, gb32, x_out,
-                         m_dev, rows, H, h->cfg.ln_eps, stream, LnSplit{split_ffn2, split_stride});
+                         m_dev, rows, H, h->cfg.ln_eps, stream, LnSplit{split_ffn2, split_stride, true});
   if (e != cudaSuccess) return fail_cuda(h, e, "layernorm launch");
   return BT_OK;
 }

@@ -1738,7 +1738,8 @@ extern "C" int bt_debug_set_gemm_timing(long long* device_buffer) {
   return 0;
 }
 // Host-side shape policies, callable without a device (tests): what 0 = tile width of the one-CTA
-// kernel, 1 = K ranges of an fp32-sum GEMM, 2 = 1 if the pair kernel would take a bias-only GEMM.
+// kernel, 1 = K ranges of an fp32-sum GEMM, 2 = 1 if the pair kernel would take a bias-only GEMM, 3 = rows per CTA of
+// LayerNorm over N columns, K partial sums, inside a forward (4: by itself).
 extern "C" int bt_debug_policy(int what, int m_rows, int N, int K, int num_sms) {
   switch (what) {
     case 0: return bt::gemm_pick_block_n(m_rows, N, K, num_sms, false);
@@ -1753,6 +1754,7 @@ extern "C" int bt_debug_policy(int what, int m_rows, int N, int K, int num_sms) 
       g.num_sms = num_sms;
       return bt::use_pair_kernel(g) ? 1 : 0;
     }
+    case 3: case 4: return bt::ln_rows_per_cta(m_rows, N, K, what == 3);
     default: return -1;
   }
 }

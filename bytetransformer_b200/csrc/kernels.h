@@ -148,7 +148,19 @@ cudaError_t launch_mha(const MhaLaunch& a, cudaStream_t stream);
 struct LnSplit {
   int n = 1;
   long long stride = 0;
+  bool in_forward = false;  // the launch stands between the kernels of a forward
 };
+// How many rows of fp32 sums (no bias, no residual) share a CTA; 0: a warp per row.  `rows` allocated rows, `parts`
+// partial sums per row.  Up to 1024 rows one row per CTA, or four where there are no partial sums to fetch and at least
+// 300k sums (768 columns: 600 rows 4.02 us with one, 3.71 us with four; 300 rows 3.43 and 3.53).  From there to
+// 4096 rows four (two where a CTA has few warps: below 512 columns, below 640 up to 1536 rows) inside a forward, where every launch fetches its
+// code anew and the short chain tells: 12 layers, a warp per row / the form chosen, 256 columns 1496 rows 437 / 441 us
+// (the loss end of it), 3032 rows 517 / 496; 512 columns 1496 rows 601 / 563 (four: 577), 2008 rows 614 / 586 (two: 601); 768 columns 857 / 812; 1024 columns
+// 1144 / 1073; 16 sequences of 128, 1216 tokens of 2048 rows valid, 701 / 645; 32 of 128, 2432 of 4096, 965 / 918.
+// Launched by itself and over and over, the warp per row is ahead from about 1.5M sums (1024 columns, 2048 rows: 5.9
+// against 6.1 us; 768 columns, 2048 rows 5.2 against 4.8) and below 512 columns (256 columns, 1000 rows 3.3 / 3.4, 4096
+// rows 4.4 / 4.9).
+int ln_rows_per_cta(long long rows, int hidden, int parts, bool in_forward);
 cudaError_t launch_layernorm(const void* x, bool x_fp32, const __half* bias, const __half* residual, const void* gamma,
                              const void* beta, bool gb_fp32, __half* out, const int* m_dev, int m_rows,
                              int hidden, float eps, cudaStream_t stream, LnSplit split = LnSplit());

@@ -386,3 +386,26 @@ def test_layernorm_moves_into_the_gemm_at_32_row_tiles_of_valid_rows(cuda_device
     assert d.max().item() <= 8e-3 and d.mean().item() <= 1e-4, (d.max().item(), d.mean().item())
     assert enc.device_status() == 0
     enc.close()
+
+
+@pytest.mark.parametrize("heads", [4, 8, 12, 16])
+def test_rows_do_not_depend_on_the_batch_they_come_in(cuda_device, heads):
+    """With LayerNorm as its own kernel and one attention kernel, a sequence's result is the same bits in a call of 1200
+    rows (two or four rows per LayerNorm CTA) and of 4200 (a warp per row)."""
+    from bytetransformer_b200 import _abi
+    from bytetransformer_b200.encoder import Encoder
+    lib = _abi.load()
+    g = torch.Generator().manual_seed(heads)
+    enc = Encoder(heads, 64, [to_device_weights(make_layer_weights(heads * 64, g), cuda_device) for _ in range(2)])
+    assert lib.bt_debug_set_fused_layernorm(enc._h, 0) == 0
+    x = torch.randn(4200, heads * 64, generator=g).half().to(cuda_device)
+    cu = torch.arange(0, 4201, 100, dtype=torch.int32, device=cuda_device)
+    lib.bt_debug_set_mha_tiles(1)
+    try:
+        few = enc.forward_packed(x[:1200].contiguous(), cu[:13].contiguous(), 100)
+        many = enc.forward_packed(x, cu, 100)
+    finally:
+        lib.bt_debug_set_mha_tiles(0)
+    assert torch.equal(few, many[:1200])
+    assert enc.device_status() == 0
+    enc.close()

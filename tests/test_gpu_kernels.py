@@ -187,9 +187,10 @@ def test_layernorm_of_fp32_sums_restore(cuda_device):
 
 
 @pytest.mark.parametrize("gb32", [False, True])
-@pytest.mark.parametrize("M,H", [(1, 64), (37, 192), (300, 512), (129, 768), (5, 832), (64, 1024)])
+@pytest.mark.parametrize("M,H", [(1, 64), (37, 192), (300, 512), (129, 768), (5, 832), (64, 1024), (512, 256),
+                                 (401, 768), (1022, 832), (1501, 512), (2047, 768), (1535, 1024)])
 def test_layernorm_forms_give_the_same_bits(cuda_device, M, H, gb32):
-    """Which form runs depends on the number of rows alone, so a row's result must not: a CTA per row (no bias) and a
+    """Which form runs depends on the number of rows, so a row's result must not: one or four rows per CTA (no bias) and a
     warp per row (a bias of zeros, which leaves every sum what it is) add the same columns in the same order."""
     from bytetransformer_b200.encoder import (add_bias_residual_layernorm, add_bias_residual_layernorm_restore,
                                               build_offsets)

@@ -50,3 +50,15 @@ def test_k_is_cut_into_as_many_ranges_as_still_fit_the_machine(policy, rows, K, 
 ])
 def test_pair_kernel_takes_over_at_two_tiles_per_sm_pair(policy, rows, N, want):
     assert policy(2, rows, N, 768, SMS) == want
+
+
+@pytest.mark.parametrize("rows,hidden,parts,inside,alone", [
+    (1, 768, 8, 1, 1), (1024, 768, 2, 1, 1),              # partial sums: one row per CTA
+    (399, 768, 1, 1, 1), (400, 768, 1, 4, 4), (512, 256, 1, 1, 1), (513, 256, 1, 1, 0), (1024, 448, 1, 1, 0),
+    (1536, 512, 1, 2, 2), (1537, 512, 1, 4, 4), (1536, 640, 1, 4, 4), (2048, 768, 1, 4, 4), (2049, 768, 1, 4, 0), (4096, 1024, 1, 4, 0), (4096, 512, 1, 4, 0),
+    (1025, 256, 1, 2, 0), (4096, 448, 1, 2, 0), (1025, 192, 1, 0, 0),
+    (4097, 768, 1, 0, 0), (100, 1032, 1, 0, 0),
+])
+def test_rows_that_share_a_layernorm_cta(policy, rows, hidden, parts, inside, alone):
+    assert policy(3, rows, hidden, parts, SMS) == inside
+    assert policy(4, rows, hidden, parts, SMS) == alone
