@@ -132,12 +132,13 @@ embedding_layernorm_kernel(const __half* __restrict__ word_emb, const __half* __
 
 // pooled[b, n] = tanh(sum_k y[b, 0, k] * W[k, n] + bias[n]).  CTA = (64 output columns, SEQ sequences),
 // 256 threads: thread (kg, cp) sums every 8th k (k = kg mod 8) for the column pair cp, so a warp reads
-// one 128-byte line of W per k and 16 loads are in flight per thread; the eight groups meet in shared
+// one 128-byte line of W per k and 16 to 32 loads are in flight per thread; the eight groups meet in shared
 // memory.  The work is tiny (B x H x H): what matters is that no thread walks a long chain of loads.
 //
-// SEQ sequences share a CTA and with it the walk over W: with one sequence each, B CTAs read the same 64 columns
-// from L2, and 32 sequences made 384 CTAs of a chain that four sequences share at the same length: a forward from
-// token ids to pooled vectors of 32 sequences up to 128 tokens 980 us before, 968 us with it.
+// Four sequences that share a CTA share the walk over W, which B CTAs of one sequence each read from L2 again.  That pays
+// from about five CTAs of one sequence per SM on; before, the fewer and longer CTAs are the slower ones.  us per launch
+// with one / four sequences per CTA, hidden 768: 32 sequences 9.4 / 12.6, 48 11.1 / 14.2, 64 15.9 / 15.3, 100 18.9 / 16.0,
+// 256 39.2 / 29.7; hidden 512, 64 8.8 / 10.2, 100 11.2 / 9.2; hidden 1024, 32 15.8 / 18.1, 48 20.5 / 19.5, 100 28.0 / 20.6.
 template <int SEQ>
 __global__ void __launch_bounds__(256)
 pooler_kernel(const __half* __restrict__ y, const __half* __restrict__ W, const __half* __restrict__ bias,
@@ -161,20 +162,29 @@ pooler_kernel(const __half* __restrict__ y, const __half* __restrict__ W, const 
   if (n + 1 < hidden) {  // hidden is even (checked by the launcher)
     const __half2* wp = reinterpret_cast<const __half2*>(W + n);
     const size_t ld2 = static_cast<size_t>(hidden) / 2;  // row stride in half2
-    constexpr int kBatch = 16;  // loads in flight
-    for (int k0 = kg; k0 < hidden; k0 += 8 * kBatch) {
-      __half2 w2[kBatch];
+    if constexpr (SEQ == 1) {
+#pragma unroll 32
+      for (int k = kg; k < hidden; k += 8) {
+        const float2 w = __half22float2(__ldg(wp + static_cast<size_t>(k) * ld2));
+        acc[0][0] = fmaf(xs[k], w.x, acc[0][0]);
+        acc[0][1] = fmaf(xs[k], w.y, acc[0][1]);
+      }
+    } else {
+      constexpr int kBatch = 16;  // loads in flight (asked for by hand: with the loop above four sequences took twice as long)
+      for (int k0 = kg; k0 < hidden; k0 += 8 * kBatch) {
+        __half2 w2[kBatch];
 #pragma unroll
-      for (int i = 0; i < kBatch; ++i)
-        w2[i] = k0 + 8 * i < hidden ? __ldg(wp + static_cast<size_t>(k0 + 8 * i) * ld2) : __half2half2(__half(0.f));
+        for (int i = 0; i < kBatch; ++i)
+          w2[i] = k0 + 8 * i < hidden ? __ldg(wp + static_cast<size_t>(k0 + 8 * i) * ld2) : __half2half2(__half(0.f));
 #pragma unroll
-      for (int i = 0; i < kBatch; ++i) {
-        const float2 w = __half22float2(w2[i]);
-        if (k0 + 8 * i < hidden) {
+        for (int i = 0; i < kBatch; ++i) {
+          const float2 w = __half22float2(w2[i]);
+          if (k0 + 8 * i < hidden) {
 #pragma unroll
-          for (int s = 0; s < SEQ; ++s) {
-            acc[s][0] = fmaf(xs[s * hidden + k0 + 8 * i], w.x, acc[s][0]);
-            acc[s][1] = fmaf(xs[s * hidden + k0 + 8 * i], w.y, acc[s][1]);
+            for (int s = 0; s < SEQ; ++s) {
+              acc[s][0] = fmaf(xs[s * hidden + k0 + 8 * i], w.x, acc[s][0]);
+              acc[s][1] = fmaf(xs[s * hidden + k0 + 8 * i], w.y, acc[s][1]);
+            }
           }
         }
       }
@@ -233,8 +243,8 @@ cudaError_t launch_pooler(const __half* y, const __half* W, const __half* bias, 
   if (B <= 0 || B > 65535 || seq_len <= 0 || hidden <= 0 || hidden > 8192 || hidden % 2 != 0) return cudaErrorInvalidValue;
   const unsigned gx = (hidden + 63) / 64;
   const size_t smem = (static_cast<size_t>(hidden) + 512) * sizeof(float);  // per sequence of a CTA
-  // four sequences per CTA as soon as that leaves a CTA for about half of the SMs
-  if (static_cast<long long>(gx) * ((B + 3) / 4) >= 74 && 4 * smem <= 48 * 1024)
+  // from five CTAs of one sequence per SM on (148 SMs)
+  if (static_cast<long long>(gx) * B >= 5 * 148 && 4 * smem <= 48 * 1024)
     return launch_pdl(pooler_kernel<4>, dim3(gx, (B + 3) / 4), dim3(256), 4 * smem, stream, y, W, bias, pooled, B, seq_len, hidden);
   return launch_pdl(pooler_kernel<1>, dim3(gx, B), dim3(256), smem, stream, y, W, bias, pooled, B, seq_len, hidden);
 }

@@ -48,10 +48,13 @@ def test_embedding_ids_outside_the_tables_are_clamped(cuda_device):
     assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("B,H", [(25, 768), (27, 832), (150, 66), (296, 64), (24, 2560)])
+@pytest.mark.parametrize("B,H", [(25, 768), (27, 832), (150, 66), (296, 64), (24, 2560), (61, 768), (62, 768), (59, 832),
+                                 (371, 66), (743, 64), (18, 2560), (19, 2624)])
 def test_pooler_four_sequences_per_cta(cuda_device, B, H):
-    """From a CTA for half of the SMs on, four sequences share a CTA (B not a multiple of 4, widths that are not
-    multiples of 64 or of the load batch; 2560 is too wide for it): against a matrix product in 64 bits."""
+    """From 740 CTAs of one sequence on, four sequences share a CTA (B not a multiple of 4, widths that are not
+    multiples of 64 or of the load batch, the widest that fits; 2624 is too wide for it; the first four sizes, 61 x 768
+    and 18 x 2560 stay below): against a matrix product in 64 bits, and a sequence's vector is the same bits in a small
+    batch."""
     from bytetransformer_b200.encoder import pooler
     g = torch.Generator().manual_seed(H + B)
     y = torch.randn(B, 3, H, generator=g).half()
@@ -61,6 +64,8 @@ def test_pooler_four_sequences_per_cta(cuda_device, B, H):
     want = torch.tanh(y[:, 0].double() @ W.double() + b.double())
     # fp16 rounding of the result, fp32 sums of H products of size about 0.05
     assert ((got - want).abs() <= want.abs() * 2.0 ** -11 + H * 2.0 ** -24 + 2.0 ** -24).all()
+    few = pooler(y[:5].to(cuda_device), W.to(cuda_device), b.to(cuda_device)).cpu().double()
+    assert torch.equal(few, got[:5])
 
 
 @pytest.mark.parametrize("B,S,H", [(1, 5, 64), (7, 33, 768), (16, 128, 1024)])
