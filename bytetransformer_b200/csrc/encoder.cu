@@ -128,14 +128,16 @@ struct bt_encoder_s {
   // 0 never, 1 from `fused_ln_min_tiles` 128-row tiles (of allocated rows) upwards, 2 always.  With few row tiles the
   // exchange of row statistics between CTAs lengthens the only wave by more than the saved LayerNorm launch and fp32
   // round trip.  What counts is the valid rows, which the host only knows where every row is computed.  Measured on
-  // B200, 12 layers, hidden 768, us per forward without / with the fused kernels: every row computed (packed and
-  // general-mask entries) 24 tiles 1022 / 1142, 32 tiles 1294 / 1197, 34 tiles 1533 / 1398 (with a bias), 36 tiles
-  // 1513 / 1369, 37 tiles 1445 / 1306, 40 tiles 1462 / 1409; padded batches 40 tiles with 2676, 2989 and 3299 valid rows
-  // 1021 / 1082, 1072 / 1155 and 1312 / 1183, 43 tiles with 3411 1241 / 1173, 48 tiles with 4382 1357 / 1262, 64 tiles
-  // with 3970 1313 / 1231.
+  // B200, 12 layers, us per forward without / with the fused kernels.  Every row computed (packed and general-mask
+  // entries), hidden 768: 28 tiles 1245 / 1182, 32 tiles 1280 / 1203, 37 tiles 1452 / 1340; hidden 1024: 32 tiles
+  // 1813 / 1732, 36 tiles 1923 / 1884, 37 tiles 1881 / 2098, 38 tiles 2184 / 2085; hidden 512: 32 tiles 874 / 933,
+  // 37 tiles 965 / 1023, 38 tiles 1055 / 1031; hidden 256: 32 tiles 505 / 599, 39 tiles 613 / 658.  Padded batches, hidden
+  // 768 (measured before LayerNorm of many rows shared CTAs): 40 tiles with 2676, 2989 and 3299 valid rows 1021 / 1082,
+  // 1072 / 1155 and 1312 / 1183, 43 tiles with 3411 1241 / 1173, 48 tiles with 4382 1357 / 1262, 64 tiles with 3970
+  // 1313 / 1231: the line of 40 goes by allocated rows and loses 6-8 % where few of them are valid.
   int fused_ln = 1;
   int fused_ln_min_tiles = 40;           // some rows are padding
-  int fused_ln_min_tiles_all_rows = 32;  // every allocated row is computed
+  int fused_ln_min_tiles_all_rows = 32;  // every allocated row is computed (and see fused_ln_pays)
   bool all_rows = false;  // the call in progress computes every allocated row (packed and general-mask entries)
   uint32_t ln_epoch = 0;  // fused LayerNorm launches since the statistics scratch of the current call was zeroed
   bool fused_ln_ffn2_only = false;  // keep the attention-output LayerNorm as its own kernel
@@ -368,15 +370,22 @@ static int run_mha(bt_handle h, const __half* qkv, __half* ctx, const int* batch
   return BT_OK;
 }
 
-// LayerNorm rides in the attention-output / FFN2 GEMM kernel once there are enough 128-row tiles
-// to occupy the machine with 256-column tiles; below that the narrow-tile GEMM followed by the
-// row kernel spreads the few rows over more SMs.
+// Whether LayerNorm rides in the attention-output / FFN2 GEMM kernels (row tiles of H / 256 CTAs each): below, the
+// narrow-tile GEMM followed by the row kernel spreads the few rows over more SMs.  Where every allocated row is computed
+// that holds from fewer tiles on, if the CTAs are more than half of the SMs - except where the plain GEMM's tiles are just
+// one wave and the clusters, which cannot use every SM, are two (1024 columns, 37 tiles).
+static bool fused_ln_pays(long long row_tiles, int H, int num_sms, bool all_rows, int min_tiles, int min_tiles_all_rows) {
+  if (row_tiles >= min_tiles) return true;
+  const long long ctas = row_tiles * (H / 256);
+  const bool one_wave_of_tiles_only = ctas <= num_sms && ctas + H / 256 > num_sms;
+  return all_rows && row_tiles >= min_tiles_all_rows && 2 * ctas > num_sms && !one_wave_of_tiles_only;
+}
 static bool want_fused_ln(bt_handle h, long long rows) {
   const int H = h->hidden;
   const long long row_tiles = (rows + 127) / 128;
-  return (H % 256 == 0) && H <= 1024 && (h->fused_ln == 2 || (h->fused_ln == 1 &&
-                                                                     row_tiles >= (h->all_rows ? h->fused_ln_min_tiles_all_rows
-                                                                                               : h->fused_ln_min_tiles)));
+  if (H % 256 != 0 || H > 1024 || h->fused_ln == 0) return false;
+  if (h->fused_ln == 2) return true;
+  return fused_ln_pays(row_tiles, H, h->num_sms, h->all_rows, h->fused_ln_min_tiles, h->fused_ln_min_tiles_all_rows);
 }
 
 // The statistics scratch of the fused LayerNorm (the head of `pre`) holds words tagged with the number
@@ -1015,6 +1024,15 @@ int bt_gemm_layernorm(bt_handle h, const void* A, const void* W, const void* bia
   return run_gemm(h, BT_PROF_GEMM_OTHER, reinterpret_cast<const __half*>(A), W, reinterpret_cast<__half*>(scratch_f32),
                   bias, reinterpret_cast<const __half*>(residual), m_dev, m_rows, N, K, BT_EPI_BIAS_RESIDUAL_LAYERNORM, 0,
                   reinterpret_cast<cudaStream_t>(stream), &ln);
+}
+
+// Host-side policy, callable without a device (tests): 1 if LayerNorm runs inside the GEMMs of a forward.
+int bt_debug_fused_layernorm_policy(int rows, int hidden, int num_sms, int all_rows) {
+  bt_encoder_s h;
+  h.hidden = hidden;
+  h.num_sms = num_sms;
+  h.all_rows = all_rows != 0;
+  return want_fused_ln(&h, rows) ? 1 : 0;
 }
 
 // Diagnostics hook: LayerNorm inside the attention-output / FFN2 GEMM kernels: 0 = never (row

@@ -366,16 +366,20 @@ def test_end_to_end_runner_matches_the_device_resident_path(cuda_device):
     enc.close()
 
 
-@pytest.mark.parametrize("tokens,launches", [(3968, 2 * 2), (3969, 0), (4096, 0)])
-def test_layernorm_moves_into_the_gemm_at_32_row_tiles_of_valid_rows(cuda_device, tokens, launches):
-    """Every row of a packed call is valid: from 32 tiles of 128 rows on, LayerNorm runs inside the GEMM kernels (no
-    launches of its own), and the result is that of the separate kernels up to fp16 rounding of the layers' outputs."""
+@pytest.mark.parametrize("heads,tokens,launches", [(12, 3968, 2 * 2), (12, 3969, 0), (12, 4096, 0),
+                                                   (4, 3969, 2 * 2), (4, 4992, 2 * 2), (4, 4993, 0),
+                                                   (8, 4736, 2 * 2), (8, 4737, 0)])
+def test_layernorm_moves_into_the_gemm_at_32_row_tiles_of_valid_rows(cuda_device, heads, tokens, launches):
+    """Every row of a packed call is valid: from 32 tiles of 128 rows on - if their CTAs are more than half of the SMs,
+    else from 40 - LayerNorm runs inside the GEMM kernels (no launches of its own), and the result is that of the
+    separate kernels up to fp16 rounding of the layers' outputs."""
     from bytetransformer_b200 import _abi
     from bytetransformer_b200.encoder import Encoder
     g = torch.Generator().manual_seed(tokens)
-    enc = Encoder(4, 64, [to_device_weights(make_layer_weights(256, g), cuda_device) for _ in range(2)])
-    x = torch.randn(tokens, 256, generator=g).half().to(cuda_device)
-    cu = torch.tensor([0, 500, 512, 1400, 2424, 3448, tokens], dtype=torch.int32, device=cuda_device)
+    enc = Encoder(heads, 64, [to_device_weights(make_layer_weights(heads * 64, g), cuda_device) for _ in range(2)])
+    x = torch.randn(tokens, heads * 64, generator=g).half().to(cuda_device)
+    cu = torch.tensor([0, 500, 512, 1400, 2424, 3448, (3448 + tokens) // 2, tokens], dtype=torch.int32,
+                      device=cuda_device)
     enc.profile_enable(True)
     got = enc.forward_packed(x, cu, 1024)
     assert enc.profile_read()["layernorm"][1] == launches

@@ -62,3 +62,18 @@ def test_pair_kernel_takes_over_at_two_tiles_per_sm_pair(policy, rows, N, want):
 def test_rows_that_share_a_layernorm_cta(policy, rows, hidden, parts, inside, alone):
     assert policy(3, rows, hidden, parts, SMS) == inside
     assert policy(4, rows, hidden, parts, SMS) == alone
+
+
+@pytest.mark.parametrize("tiles,hidden,all_rows,padded", [
+    (31, 768, 0, 0), (32, 768, 1, 0), (39, 768, 1, 0), (40, 768, 1, 1),
+    (31, 1024, 0, 0), (32, 1024, 1, 0), (36, 1024, 1, 0), (37, 1024, 0, 0), (38, 1024, 1, 0), (40, 1024, 1, 1),
+    (37, 512, 0, 0), (38, 512, 1, 0), (40, 512, 1, 1),   # 74 CTAs are half of the SMs
+    (32, 256, 0, 0), (39, 256, 0, 0), (40, 256, 1, 1),
+    (64, 320, 0, 0), (64, 1280, 0, 0),                   # widths without the fused kernels
+])
+def test_layernorm_inside_the_gemm(policy, tiles, hidden, all_rows, padded):
+    from bytetransformer_b200 import _abi
+    fn = _abi.load().bt_debug_fused_layernorm_policy
+    for rows in (tiles * 128, tiles * 128 - 127):
+        assert fn(rows, hidden, SMS, 1) == all_rows
+        assert fn(rows, hidden, SMS, 0) == padded
