@@ -1648,11 +1648,12 @@ int gemm_pick_block_n(int m_rows, int N, int K, int num_sms, bool all_rows) {
     const long long tiles = static_cast<long long>(m_tiles) * (N / bn);
     if (tiles < num_sms) continue;
     // A 128-column tile's main loop takes hardly longer than a 64-column one's (64 against 54 clocks per MMA), so
-    // with a long K a second wave of 64-column tiles that 128-column ones do not need is the dearer choice: FFN2 of
-    // 8 sequences of 197 tokens (156 tiles of 64 columns or 78 of 128, K = 3072), 12-layer forward 961 us
-    // before, 885 us with this rule and the fp32 sums leaving by bulk store.  Only where every
-    // row is valid: padded rows make no tiles, and 16 sequences of up to 128 tokens, 192 tiles of 64 columns by
-    // their rows and 120 by their tokens, lose 2 % of the forward with 128-column tiles.
+    // with a long K a second wave of 64-column tiles that 128-column ones do not need is the dearer choice.  us per launch
+    // of an fp32-sum GEMM with 64- / 128-column tiles over the range of the rule: N = 768, K = 3072, 13 row tiles
+    // 24.7 / 16.8, 18 25.0 / 17.4, 24 25.7 / 18.4 (12, one wave of either: 15.6 / 16.6); N = 768, K = 2048 18.7 / 13.4 to
+    // 19.8 / 14.9; N = 1024, K = 4096, 10 to 18 row tiles 30.7 / 20.2 to 31.6 / 22.0; N = 512, K = 2048, 19 to 37
+    // 18.7 / 13.4 to 19.8 / 14.9.  Only where every row is valid: padded rows make no tiles, and 16 sequences of up to 128
+    // tokens, 192 tiles of 64 columns by their rows and 120 by their tokens, lose 2 % of the forward with 128-column tiles.
     if (bn == 64 && all_rows && K >= 2048 && N % 128 == 0 && tiles > num_sms) return 128;
     return bn;
   }
@@ -1739,11 +1740,12 @@ extern "C" int bt_debug_set_gemm_timing(long long* device_buffer) {
 }
 // Host-side shape policies, callable without a device (tests): what 0 = tile width of the one-CTA
 // kernel, 1 = K ranges of an fp32-sum GEMM, 2 = 1 if the pair kernel would take a bias-only GEMM, 3 = rows per CTA of
-// LayerNorm over N columns, K partial sums, inside a forward (4: by itself).
+// LayerNorm over N columns, K partial sums, inside a forward (4: by itself), 5 = as 0 where every row is valid.
 extern "C" int bt_debug_policy(int what, int m_rows, int N, int K, int num_sms) {
   switch (what) {
     case 0: return bt::gemm_pick_block_n(m_rows, N, K, num_sms, false);
     case 1: return bt::gemm_pick_split_k(m_rows, N, K, num_sms);
+    case 5: return bt::gemm_pick_block_n(m_rows, N, K, num_sms, true);
     case 2: {
       bt::GemmLaunch g = {};
       g.m_rows = m_rows;

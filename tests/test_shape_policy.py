@@ -30,6 +30,21 @@ def test_tile_width_is_the_widest_that_gives_every_sm_a_tile(policy, rows, N, wa
     assert policy(0, rows, N, 768, SMS) == want
 
 
+@pytest.mark.parametrize("rows,N,K,want", [
+    (1536, 768, 3072, 64),   # 12 row tiles: 144 tiles of 64 columns, one wave
+    (1537, 768, 3072, 128),  # 13: 156 would be a second wave, 78 of 128 columns are one
+    (3072, 768, 3072, 128), (3073, 768, 3072, 128),  # 24: 144 tiles of 128; 25: 150, the plain rule again
+    (1537, 768, 768, 64),    # a short K: the second wave is cheap
+    (2304, 512, 2048, 64), (2305, 512, 2048, 128),
+    (1280, 1024, 4096, 128), (1152, 1024, 4096, 64),
+    (1601, 704, 3072, 64), (1793, 704, 3072, 64),    # 704 % 128 != 0
+])
+def test_a_long_k_takes_wide_tiles_instead_of_a_second_wave_where_all_rows_are_valid(policy, rows, N, K, want):
+    assert policy(5, rows, N, K, SMS) == want
+    if (rows, want) != (3073, 128):
+        assert policy(0, rows, N, K, SMS) == 64   # padded rows may make no tiles
+
+
 @pytest.mark.parametrize("rows,K,want", [
     (38, 3072, 8), (256, 3072, 8),        # 12 or 24 tiles of 64 columns: 8 ranges still fit 1.5 x the SMs
     (384, 3072, 4), (512, 3072, 4),
