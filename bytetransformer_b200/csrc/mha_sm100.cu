@@ -63,6 +63,13 @@ constexpr int kKvRows = 128;
 constexpr int kHeadDim = 64;
 constexpr int kTileBytes = 128 * kHeadDim * 2;  // 16 KiB: Q, K or V tile
 
+// The exponent reference of a row may lag its running maximum by at most 2^8; beyond, the row's warp moves the references
+// of its rows to their maxima and rescales O.  Which key tile that happens at shows in the last bits of all 32 rows, so
+// a row behind the last sequence (whatever the buffer holds there) has no say: results are a function of the inputs alone.
+__device__ __forceinline__ float rescale_threshold(int row, int rows_that_exist) {
+  return row < rows_that_exist ? 8.0f : INFINITY;
+}
+
 // One CTA per item: shared-memory and tensor-memory layout.
 struct MhaCfg {
   static constexpr int kStages = 3;
@@ -471,8 +478,6 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
   using Cfg = MhaCfg;
   constexpr bool GENERAL = MODE != 0;
   constexpr int kStages = Cfg::kStages;
-  // the exponent reference may lag the running maximum by at most 2^8
-  constexpr float kRescaleThreshold = 8.0f;
   extern __shared__ __align__(1024) uint8_t smem[];
 
   pdl_launch_dependents();
@@ -518,15 +523,17 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
 
   // Everything above is this CTA's own: it runs while the kernel before still does, and so does the round trip
   // for the offsets where the kernel that wrote them is known to have completed.
-  int off0 = 0, off1 = 0;
+  int off0 = 0, off1 = 0, off_end = 0;
   if (args.early_offsets) {
     off0 = __ldg(args.batch_idx + b);
     off1 = __ldg(args.batch_idx + b + 1);
+    off_end = __ldg(args.batch_idx + gridDim.z);
   }
   pdl_wait();  // the QKV buffer comes from the kernel before
   if (!args.early_offsets) {
     off0 = __ldg(args.batch_idx + b);
     off1 = __ldg(args.batch_idx + b + 1);
+    off_end = __ldg(args.batch_idx + gridDim.z);
   }
   const int seq_start = uniform_int(off0);
   const int L = uniform_int(off1) - seq_start;
@@ -621,6 +628,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
     const uint32_t t_s = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t t_o = t_s + Cfg::kTmemO;
     const float c = args.scale_log2e;
+    const float max_lag = rescale_threshold(seq_start + q0 + r, off_end);
     float m_ref = -INFINITY;  // exponent reference, in log2 units
     float l_run = 0.f;
     int stage = 0;
@@ -675,7 +683,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
         m_ref = mx;
       } else {
         const float m_new = fmaxf(m_ref, mx);
-        const bool need = (m_new - m_ref) > kRescaleThreshold;
+        const bool need = (m_new - m_ref) > max_lag;
         if (__any_sync(0xffffffffu, need)) {
           // the PV of the previous key tile has retired (S of this tile was issued after it)
           const float f = ex2_approx(m_ref - m_new);
@@ -926,7 +934,6 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
   constexpr int kSmemOut = kSmemV + kStages * kTileBytes;
   constexpr int kSmemBar = kSmemOut + kTileBytes;
   constexpr uint32_t kTmemS = 0, kTmemO = 128, kTmemP = 192;
-  constexpr float kRescaleThreshold = 8.0f;
   extern __shared__ __align__(1024) uint8_t smem[];
 
   pdl_launch_dependents();
@@ -1139,9 +1146,11 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
     uint32_t phase = 0;
     uint32_t step = 0;
     bool ok = smem_ok;
+    const int rows_that_exist = __ldg(args.batch_idx + args.batch);
     bool have = decode_item(args, snake_item(0, cta, G), cur_b, cur_first, seq_start, L, qt, head, false);
     for (int round = 0; ok && have; ++round) {
       const int n_kv = (L + kKvRows - 1) / kKvRows;
+      const float max_lag = rescale_threshold(seq_start + qt * kQRows + r, rows_that_exist);
       float m_ref = -INFINITY;
       float l_run = 0.f;
       for (int j = 0; j < n_kv; ++j, ++step) {
@@ -1175,7 +1184,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
         bool pv_waited = (j == 0);  // (first tile of an item: the wait for the previous item's O covered it)
         if (j == 0) {
           m_ref = m_new;
-        } else if (__any_sync(0xffffffffu, (m_new - m_ref) > kRescaleThreshold)) {
+        } else if (__any_sync(0xffffffffu, (m_new - m_ref) > max_lag)) {
           // O belongs to the P V MMAs of the previous key tile until those have retired
           mbar_wait_anyway(pv_done, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
           tc_fence_after();

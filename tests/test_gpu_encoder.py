@@ -413,3 +413,32 @@ def test_rows_do_not_depend_on_the_batch_they_come_in(cuda_device, heads):
     assert torch.equal(few, many[:1200])
     assert enc.device_status() == 0
     enc.close()
+
+
+@pytest.mark.parametrize("B,S,f", [(1, 300, 0.6), (2, 512, 0.6), (8, 256, 0.55), (16, 256, 0.6)])
+def test_results_do_not_depend_on_what_the_workspace_held(cuda_device, B, S, f):
+    """Behind the last sequence's rows the activation buffers hold what earlier calls left, and the last query tile covers
+    some of it.  Neither zeros, nor large values, nor NaN there may show, not in the last bit either (one attention CTA per
+    item and the persistent kernel; sequences of more than one key tile)."""
+    import ctypes as C
+
+    from bytetransformer_b200.encoder import Encoder
+    heads = 12
+    g = torch.Generator().manual_seed(B * S)
+    enc = Encoder(heads, 64, [to_device_weights(make_layer_weights(heads * 64, g), cuda_device) for _ in range(3)])
+    x = torch.randn(B, S, heads * 64, generator=g).half().to(cuda_device)
+    mask = (torch.arange(S) < int(S * f)).half().expand(B, S, S).contiguous().to(cuda_device)
+    n = C.c_size_t()
+    enc._call("bt_workspace_bytes", enc._h, B, S, C.byref(n))
+    outs = []
+    for fill in (0.0, 50.0, float("nan")):
+        ws = torch.randn(n.value // 2, generator=torch.Generator(device=cuda_device).manual_seed(1), device=cuda_device,
+                         dtype=torch.float16) * fill
+        out = torch.empty_like(x)
+        enc._call("bt_stack_forward_padded", enc._h, 3, x.data_ptr(), mask.data_ptr(), out.data_ptr(), ws.data_ptr(),
+                  ws.numel() * 2, B, S, torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        outs.append(out)
+    assert enc.device_status() == 0
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    enc.close()
