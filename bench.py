@@ -204,7 +204,7 @@ def main():
     ap.add_argument("--no-kernel-events", action="store_true", help="do not bracket kernels with events in the timed region")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")
-    ap.add_argument("--no-configs", action="store_true", help="skip the other BASELINE configurations (N = 1 extra key)")
+    ap.add_argument("--no-configs", action="store_true", help="skip the other configurations (N = 1 extra key)")
     ap.add_argument("--token-budget", type=int, default=0)
     ap.add_argument("--e2e-token-budget", type=int, default=0, help="A/B aid: micro-batch budget of the host path")
     ap.add_argument("--fused-ln", type=int, default=-1,
@@ -371,7 +371,7 @@ def main():
         tps, sample, cores, _, _ = cpu_oracle_sample(lengths_for(WORKLOAD), reps=2)
         cpu = {"value": tps, "unit": UNIT, "cores": cores, "kind": "port", "sample": sample}
 
-    # ---- the other BASELINE configurations (rank 0, N = 1 only): extra key, the headline is untouched ----
+    # ---- the other configurations (rank 0, N = 1 only): extra key, the headline is untouched ----
     configs = None
     if rank == 0 and n_gpus == 1 and not args.no_configs and not (args.max_seqs or args.layers):
         from bytetransformer_b200.latency_bench import baseline_configs

@@ -43,7 +43,7 @@ def lengths(batch: int, seq: int, seed: int):
 
 
 def measure_config(name, shape, lens, max_seq, layers=None, iters=20, warmup=5, device=None, peaks=None, enc=None):
-    """One BASELINE configuration through the one-call padded stack (`bt_stack_forward_padded`): median
+    """One configuration through the one-call padded stack (`bt_stack_forward_padded`): median
     milliseconds per forward (CUDA events, L2 flushed before every timed iteration), valid tokens/s,
     algorithmic TFLOP/s and two roofline fractions - of the dense tensor peak, and of HBM bandwidth for the
     bytes every forward has to stream at least once (the layers' weights), which is what bounds the
@@ -92,7 +92,7 @@ def measure_config(name, shape, lens, max_seq, layers=None, iters=20, warmup=5, 
 
 
 def baseline_configs(peaks=None, device=None, iters=20, warmup=5):
-    """The BASELINE configurations that fit one GPU besides the whole-box one, each through the padded
+    """The benchmark configurations that fit one GPU besides the whole-box one, each through the padded
     drop-in entry point: c1 (one layer, batch 16, max_seq 64), c2 (12 layers, batch 1, max_seq 64 / 512 /
     1024 at 0.6 x valid), c3 (12 layers, batch 16, max_seq 512) and c4 (BERT-large, 24 layers, batch 64,
     max_seq 384)."""
@@ -133,7 +133,7 @@ def main():
     ap.add_argument("--front-back", action="store_true",
                     help="also time the embedding + LayerNorm front end (30522-word table) and the pooler for each shape")
     ap.add_argument("--baseline-configs", action="store_true",
-                    help="instead of a sweep: the BASELINE configurations c1-c4 (BERT-base and BERT-large), one JSON line each")
+                    help="instead of a sweep: the benchmark configurations c1-c4 (BERT-base and BERT-large), one JSON line each")
     ap.add_argument("--breakdown", action="store_true",
                     help="add per-kernel-kind microseconds per forward (CUDA events around every launch, L2 warm)")
     args = ap.parse_args()

@@ -2,7 +2,7 @@
 import numpy as np
 import torch
 
-# Tolerances of the fp16 path against the fp32 oracle (stated by the north star):
+# Tolerances of the fp16 path against the fp32 oracle:
 MAX_ABS_TOL = 2e-2
 MEAN_ABS_TOL = 1e-3
 

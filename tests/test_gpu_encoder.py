@@ -180,7 +180,7 @@ def test_config4_bert_large_shapes_sampled(cuda_device):
 
 
 def test_config4_bert_large_full_size(cuda_device):
-    """BASELINE configuration 4 at full size through the padded drop-in entry point: BERT-large (24 layers,
+    """BERT-large at full size through the padded drop-in entry point: BERT-large (24 layers,
     hidden 1024, 16 heads), batch 64, max_seq 384, lengths from the seeded truncated normal (13.7k valid
     tokens: the GEMM + LayerNorm kernels with four column tiles per row tile, 24 layers of error
     accumulation).  The CPU oracle cannot run the whole batch in test time, so:
