@@ -108,9 +108,8 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 }
 
 // Wait for a phase with an upper bound.  Returns false when the bound ran out
-// or another role of this CTA already gave up (`*abort_flag` non-zero); the
-// caller must then leave its loop and fall through to the common teardown.  The
-// answer is the calling lane's own: what a warp waits for goes through the two forms below.
+// or another role of this CTA already gave up (`*abort_flag` non-zero).  The answer
+// is the calling lane's own: what a warp waits for goes through the three forms below.
 // The bound is ~2^31 SM cycles (about a second) unless the caller gives another,
 // checked every 256 polls; once the flag is up, a wait ends after nine (not after
 // its first: a look at the flag between two polls that a K loop's wait does need was
