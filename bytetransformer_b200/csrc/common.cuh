@@ -205,6 +205,36 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// ------------------------------------------------------ cluster launch control
+// A running block takes over a block of its own grid that has not started yet: the hardware cancels that launch and
+// hands its index out.  The answer (16 bytes at `resp`, 16-byte aligned) is counted in bytes on `bar`.  One thread of
+// the block asks; after an answer without a block it must not ask again.
+__device__ __forceinline__ void launch_control_ask(void* resp, uint64_t* bar) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the last answer has been read
+  mbar_arrive_expect_tx(bar, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_u32(resp)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+// The index (x) of the block taken over, or -1 if none was left.
+__device__ __forceinline__ int launch_control_answer(const void* resp) {
+  int x;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b128 r;\n\t"
+      "ld.shared.b128 r, [%1];\n\t"
+      "mov.b32 %0, -1;\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, r;\n\t"
+      "}\n"
+      : "=r"(x)
+      : "r"(smem_u32(resp))
+      : "memory");
+  return x;
+}
+
 // ------------------------------------------------------------------- tcgen05
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_slot, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_slot)),

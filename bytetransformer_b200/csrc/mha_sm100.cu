@@ -805,9 +805,11 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
 // single-thread roles sleep between polls of a barrier so that they leave the issue slots of the
 // schedulers they share with softmax warps alone.
 //
-// Items go to the CTAs in snake order (round k: item k*G + c for even k, k*G + G-1-c for odd k, G CTAs):
-// with sequences sorted by length (longest first), which is how callers batch them, the items of a round
-// get cheaper from first to last, and the snake evens out the per-CTA sums.
+// Items are dealt out as CTAs become free: the grid has a block per item, as many as fit start, and a running CTA that
+// has requested the last key tile of its item takes over a block that has not started (cluster launch control), whose
+// index is its next item.  The two CTAs of an SM do not run at the same speed - the schedulers prefer the older one's
+// warps: 2.45k clocks per key tile against 3.4k in one SM - so an even share of the items leaves the slower one to
+// finish alone, at a third less than the pair's rate.  The loader decodes an item once and hands it to the other roles through a ring in shared memory.
 // ------------------------------------------------------------------------------------------
 struct MhaPersistentArgs {
   __half* ctx;
@@ -828,13 +830,13 @@ struct MhaPersistentArgs {
 // lanes look at 32 sequences at a time (one coalesced read of their offsets, a warp scan of their item
 // counts), because a loop over single sequences pays one L2 round trip per sequence, which with many
 // short sequences cost more than the attention itself.  `cur_b` / `cur_first` is the caller's cursor
-// (first item index of sequence cur_b, the same in all lanes); n never decreases.  A sequence whose
-// offsets are not 0 <= start, 0 <= L <= max_len, start + L <= rows is left out (it yields no items, so
-// nothing is read or written outside the buffers) and, when `report` is set (one warp per CTA),
-// kStatusBadOffsets is recorded.
+// (first item index of sequence cur_b, the same in all lanes).  A sequence whose offsets are not 0 <= start,
+// 0 <= L <= max_len, start + L <= rows is left out (it yields no items, so nothing is read or written outside the
+// buffers) and kStatusBadOffsets is recorded.
 __device__ __forceinline__ bool decode_item(const MhaPersistentArgs& a, int n, int& cur_b, int& cur_first,
-                                            int& seq_start, int& L, int& qt, int& h, bool report) {
+                                            int& seq_start, int& L, int& qt, int& h) {
   const int lane = static_cast<int>(threadIdx.x & 31u);
+  if (n < cur_first) cur_b = cur_first = 0;  // (blocks are taken over in rising order, but nothing says they must be)
   while (cur_b < a.batch) {
     const int b = cur_b + lane;
     int start = 0, len = 0;
@@ -842,7 +844,7 @@ __device__ __forceinline__ bool decode_item(const MhaPersistentArgs& a, int n, i
       start = __ldg(a.batch_idx + b);
       len = __ldg(a.batch_idx + b + 1) - start;
       if (start < 0 || len < 0 || len > a.max_len || start > a.rows - len) {
-        if (report && a.status != nullptr) atomicCAS(a.status, 0, kStatusBadOffsets);
+        if (a.status != nullptr) atomicCAS(a.status, 0, kStatusBadOffsets);
         len = 0;
       }
     }
@@ -870,10 +872,6 @@ __device__ __forceinline__ bool decode_item(const MhaPersistentArgs& a, int n, i
   }
   return false;
 }
-__device__ __forceinline__ int snake_item(int round, int cta, int ctas) {
-  return round * ctas + ((round & 1) ? ctas - 1 - cta : cta);
-}
-
 template <int B>
 __device__ __forceinline__ void tmem_st_32x16_at(uint32_t taddr, const uint32_t (&r)[64]) {
   asm volatile(
@@ -921,9 +919,12 @@ __device__ __forceinline__ bool mbar_wait_role(uint64_t* bar, uint32_t parity, v
 
 constexpr int kPersistentThreads = 256;
 constexpr int kPersistentStages = 2;  // Q, K and V tiles each
-// Q, K, V rings, the softmax warps' output staging (4 x 32 rows x 128 B), barriers
-constexpr int kPersistentSmemBytes = 3 * kPersistentStages * kTileBytes + kTileBytes + 256;
+constexpr int kItemSlots = 4;         // items between the loader and the other roles
+// Q, K, V rings, the softmax warps' output staging (4 x 32 rows x 128 B), barriers and items
+constexpr int kPersistentSmemBytes = 3 * kPersistentStages * kTileBytes + kTileBytes + 512;
 
+// MORE: the grid has more blocks than can be resident, CTAs take over waiting ones.  (Without: one item per CTA.)
+template <bool MORE>
 __global__ void __launch_bounds__(kPersistentThreads, 2)
 mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_ctx,
                       const MhaPersistentArgs args) {
@@ -949,8 +950,14 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
   uint64_t* p_full = s_full + 2;               // P(j) is in tensor memory, V rows blanked (4 arrivals)
   uint64_t* pv_done = s_full + 3;              // O += P(j) V(j) has retired
   uint64_t* o_done = s_full + 4;               // the item's last P V has retired
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 5);
+  uint64_t* item_full = s_full + 5;            // [kItemSlots] an item's description has been written
+  uint64_t* item_empty = item_full + kItemSlots;  // [kItemSlots] read by the MMA warp and the four softmax warps
+  uint64_t* taken_full = item_empty + kItemSlots; // the answer of the launch control has arrived
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(taken_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint8_t* taken = smem + kSmemBar + 256;      // 16 bytes
+  // first row of the sequence, its length, query tile, head; length 0: no more items
+  int4* items = reinterpret_cast<int4*>(smem + kSmemBar + 256 + 16);
 
   const int warp = uniform_int(static_cast<int>(threadIdx.x >> 5));  // warp-uniform roles: see common.cuh
   const int lane = threadIdx.x & 31;
@@ -970,6 +977,11 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
     mbar_init(p_full, 4);
     mbar_init(pv_done, 1);
     mbar_init(o_done, 1);
+    for (int s = 0; s < kItemSlots; ++s) {
+      mbar_init(&item_full[s], 1);
+      mbar_init(&item_empty[s], 5);
+    }
+    mbar_init(taken_full, 1);
     *abort_flag = smem_ok ? 0 : 1;
     fence_mbar_init();
     if (!smem_ok && args.status != nullptr) atomicCAS(args.status, 0, kStatusMhaLoadTimeout + 0x10);
@@ -988,8 +1000,22 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
   // touch of other memory has to come after it.
   if (!args.early_offsets) pdl_wait();
 
-  const int G = static_cast<int>(gridDim.x), cta = static_cast<int>(blockIdx.x);
-  int cur_b = 0, cur_first = 0, seq_start = 0, L = 0, qt = 0, head = 0;
+  // Each role finds the CTA's first item, the block's own, by itself (nothing to hand over while the pipeline is empty);
+  // the n-th taken over, n = 0, 1, ..., comes through slot n % kItemSlots of the ring.
+  int seq_start = 0, L = 0, qt = 0, head = 0;
+  auto own_item = [&](int& cur_b, int& cur_first) {
+    return decode_item(args, static_cast<int>(blockIdx.x), cur_b, cur_first, seq_start, L, qt, head);
+  };
+  auto read_item = [&](uint32_t n) {  // (once item_full has completed)
+    const int4 item = items[n % kItemSlots];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&item_empty[n % kItemSlots]);
+    seq_start = item.x;
+    L = item.y;
+    qt = item.z;
+    head = item.w;
+  };
+  auto item_parity = [](uint32_t n) { return (n / kItemSlots) & 1u; };
 
   if (warp >= 4) {
     setmaxnreg_dec<40>();
@@ -1000,44 +1026,62 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      bool have = decode_item(args, snake_item(0, cta, G), cur_b, cur_first, seq_start, L, qt, head, true);
+      int cur_b = 0, cur_first = 0;
+      bool more = MORE;  // blocks of the grid may still be waiting
+      uint32_t asked = 0;
+      bool have = own_item(cur_b, cur_first);
+      // The grid is sized from an upper bound of the items; a block beyond the last one is taken over as well (cheaper
+      // than letting it start) and the next one asked for.
+      auto take_next = [&]() {
+        have = false;
+        while (more && !have) {
+          if (elect_one()) launch_control_ask(taken, taken_full);
+          if (!mbar_wait_role(taken_full, asked++ & 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) return;
+          const int next = uniform_int(launch_control_answer(taken));
+          more = next >= 0;
+          if (more) have = decode_item(args, next, cur_b, cur_first, seq_start, L, qt, head);
+        }
+      };
       if (args.early_offsets) pdl_wait();
-      for (int round = 0; ok && have; ++round) {
-        {
-          L = uniform_int(L);
-          seq_start = uniform_int(seq_start);
-          qt = uniform_int(qt);
-          head = uniform_int(head);
-          const int n_kv = (L + kKvRows - 1) / kKvRows;
-          const int qb = round % kStages;
-          const uint32_t qph = static_cast<uint32_t>(round / kStages) & 1u;
-          ok = mbar_wait_role(&q_empty[qb], qph ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout);
-          if (ok) {
-          if (elect_one()) mbar_arrive_expect_tx(&q_full[qb], kTileBytes);
-          if (elect_one()) tma_load_2d(smem + kSmemQ + qb * kTileBytes, &tm_qkv, &q_full[qb], head * kHeadDim, seq_start + qt * kQRows);
-          for (int j = 0; j < n_kv; ++j) {
-            const int row = seq_start + j * kKvRows;
-            if (!mbar_wait_role(&k_empty[stage], phase ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) {
-              ok = false;
-              break;
-            }
-            if (elect_one()) mbar_arrive_expect_tx(&k_full[stage], kTileBytes);
-            if (elect_one()) tma_load_2d(smem + kSmemK + stage * kTileBytes, &tm_qkv, &k_full[stage], args.hidden + head * kHeadDim, row);
-            if (!mbar_wait_role(&v_empty[stage], phase ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) {
-              ok = false;
-              break;
-            }
-            if (elect_one()) mbar_arrive_expect_tx(&v_full[stage], kTileBytes);
-            if (elect_one()) tma_load_2d(smem + kSmemV + stage * kTileBytes, &tm_qkv, &v_full[stage], 2 * args.hidden + head * kHeadDim,
-                        row);
-            if (++stage == kStages) {
-              stage = 0;
-              phase ^= 1u;
-            }
-          }
+      if (!have) more = false;  // no item of its own: the blocks behind it have none either, and the other roles are done
+      for (uint32_t n = 0; have; ++n) {
+        L = uniform_int(L);
+        seq_start = uniform_int(seq_start);
+        qt = uniform_int(qt);
+        head = uniform_int(head);
+        const int n_kv = (L + kKvRows - 1) / kKvRows;
+        const int qb = static_cast<int>(n % kStages);
+        ok = mbar_wait_role(&q_empty[qb], ((n / kStages) & 1u) ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout);
+        if (!ok) break;
+        if (elect_one()) mbar_arrive_expect_tx(&q_full[qb], kTileBytes);
+        if (elect_one()) tma_load_2d(smem + kSmemQ + qb * kTileBytes, &tm_qkv, &q_full[qb], head * kHeadDim, seq_start + qt * kQRows);
+        for (int j = 0; j < n_kv; ++j) {
+          const int row = seq_start + j * kKvRows;
+          ok = mbar_wait_role(&k_empty[stage], phase ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout);
+          if (!ok) break;
+          if (elect_one()) mbar_arrive_expect_tx(&k_full[stage], kTileBytes);
+          if (elect_one()) tma_load_2d(smem + kSmemK + stage * kTileBytes, &tm_qkv, &k_full[stage], args.hidden + head * kHeadDim, row);
+          ok = mbar_wait_role(&v_empty[stage], phase ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout);
+          if (!ok) break;
+          if (elect_one()) mbar_arrive_expect_tx(&v_full[stage], kTileBytes);
+          if (elect_one()) tma_load_2d(smem + kSmemV + stage * kTileBytes, &tm_qkv, &v_full[stage], 2 * args.hidden + head * kHeadDim,
+                      row);
+          if (++stage == kStages) {
+            stage = 0;
+            phase ^= 1u;
           }
         }
-        have = decode_item(args, snake_item(round + 1, cta, G), cur_b, cur_first, seq_start, L, qt, head, true);
+        if (!ok) break;
+        // The next item: asked for once this one's last loads are out, i.e. while its last two key tiles are worked on,
+        // and not before, so that a CTA with long items does not hold others back.
+        if (!more) break;
+        take_next();
+        const uint32_t slot = n % kItemSlots;
+        if (!mbar_wait_role(&item_empty[slot], item_parity(n) ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) break;
+        if (lane == 0) {
+          items[slot] = make_int4(seq_start, have ? L : 0, qt, head);
+          mbar_arrive(&item_full[slot]);
+        }
       }
     } else if (warp == 5) {
       // -------------------------------------------------------------- MMA issue
@@ -1074,11 +1118,16 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
       };
       // Everything else of an item: per key tile the NEXT S as soon as the softmax warps hold the
       // current one in registers, then O += P V.  On the item's last tile the next S is the first of the
-      // CTA's next item, if its Q and K tiles have landed by then (`next_s_issued`): an item boundary then
-      // costs the softmax warps no S round trip.  false when a wait gave up.
-      auto issue_rest = [&](int round, int len, bool have_next, int len_next, bool& next_s_issued) -> bool {
+      // CTA's next item, if that is known and its Q and K tiles have landed by then (`next_s_issued`): an item
+      // boundary then costs the softmax warps no S round trip.  false when a wait gave up.
+      auto read_length = [&](int n) -> int {
+        read_item(static_cast<uint32_t>(n));
+        return uniform_int(L);
+      };
+      auto issue_rest = [&](int round, int len, int& len_next, bool& next_s_issued) -> bool {
         const int n_kv = (len + kKvRows - 1) / kKvRows;
         next_s_issued = false;
+        len_next = -1;
         for (int j = 0; j < n_kv; ++j, ++step) {
           const int st_n = (st + 1 == kStages) ? 0 : st + 1;
           const uint32_t ph_n = (st + 1 == kStages) ? (ph ^ 1u) : ph;
@@ -1090,9 +1139,11 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
             tc_fence_after();
             issue_s(round, st_n);
             if (j + 2 == n_kv) release_q(round);
-          } else if (have_next) {
+          } else if (MORE) {
             if (!mbar_wait_role(s_free, step & 1u, abort_flag, args.status, kStatusMhaMmaTimeout)) return false;
-            if (__all_sync(0xffffffffu, mbar_test_wait(&q_full[(round + 1) % kStages], q_ready(round + 1)) &&
+            if (__all_sync(0xffffffffu, mbar_test_wait(&item_full[round % kItemSlots], item_parity(round))))
+              len_next = read_length(round);
+            if (len_next > 0 && __all_sync(0xffffffffu, mbar_test_wait(&q_full[(round + 1) % kStages], q_ready(round + 1)) &&
                                             mbar_test_wait(&k_full[st_n], ph_n))) {
               tc_fence_after();
               issue_s(round + 1, st_n);
@@ -1117,20 +1168,18 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
         if (elect_one()) umma_commit(o_done);
         return true;
       };
-      bool ok = true;
-      bool have = decode_item(args, snake_item(0, cta, G), cur_b, cur_first, seq_start, L, qt, head, false);
-      int len = uniform_int(L);
       bool s_issued = false;  // S(0) of the item about to start has been issued already
-      for (int round = 0; ok && have; ++round) {
-        if (!s_issued) ok = issue_first_s(round, len);
-        // the item after this one is found while this item's first tile is on its way
-        const bool have_next = decode_item(args, snake_item(round + 1, cta, G), cur_b, cur_first, seq_start, L, qt, head, false);
-        const int len_next = uniform_int(L);
-        bool next_s_issued = false;
-        if (ok) ok = issue_rest(round, len, have_next, len_next, next_s_issued);
-        s_issued = next_s_issued;
-        have = have_next;
-        len = len_next;
+      int cur_b = 0, cur_first = 0;
+      // length of the item after the present one, -1 while it is not known, 0 if there is none
+      int len_next = own_item(cur_b, cur_first) ? uniform_int(L) : 0;
+      for (int round = 0; len_next != 0; ++round) {
+        const int len = len_next;
+        if (!s_issued && !issue_first_s(round, len)) break;
+        if (!issue_rest(round, len, len_next, s_issued) || !MORE) break;
+        if (len_next < 0) {
+          if (!mbar_wait_role(&item_full[round % kItemSlots], item_parity(round), abort_flag, args.status, kStatusMhaMmaTimeout)) break;
+          len_next = read_length(round);
+        }
       }
     }
   } else {
@@ -1147,7 +1196,8 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
     uint32_t step = 0;
     bool ok = smem_ok;
     const int rows_that_exist = __ldg(args.batch_idx + args.batch);
-    bool have = decode_item(args, snake_item(0, cta, G), cur_b, cur_first, seq_start, L, qt, head, false);
+    int cur_b = 0, cur_first = 0;
+    bool have = own_item(cur_b, cur_first);
     for (int round = 0; ok && have; ++round) {
       const int n_kv = (L + kKvRows - 1) / kKvRows;
       const float max_lag = rescale_threshold(seq_start + qt * kQRows + r, rows_that_exist);
@@ -1243,9 +1293,6 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
           phase ^= 1u;
         }
       }
-      // the next item is found while the last P V of this one runs
-      int seq_start_n = 0, L_n = 0, qt_n = 0, head_n = 0;
-      have = decode_item(args, snake_item(round + 1, cta, G), cur_b, cur_first, seq_start_n, L_n, qt_n, head_n, false);
       if (!mbar_wait_warp(o_done, static_cast<uint32_t>(round) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout)) {
         ok = false;
         break;
@@ -1303,10 +1350,11 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
         }
       }
       __syncwarp();  // the staging rows are rewritten at the end of the next item
-      seq_start = seq_start_n;
-      L = L_n;
-      qt = qt_n;
-      head = head_n;
+      if (!MORE) break;
+      if (!mbar_wait_warp(&item_full[round % kItemSlots], item_parity(round), abort_flag, args.status, kStatusMhaSoftmaxTimeout))
+        break;
+      read_item(static_cast<uint32_t>(round));
+      have = L > 0;
     }
     if (lane == 0) tma_store_wait_all();  // the staging rows must outlive the last bulk store
     tc_fence_before();
@@ -1329,9 +1377,10 @@ cudaError_t launch_persistent(const MhaLaunch& a, cudaStream_t stream) {
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   if (!attr_set[dev]) {
-    cudaError_t e =
-        cudaFuncSetAttribute(mha_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistentSmemBytes);
-    if (e != cudaSuccess) return e;
+    for (auto kern : {mha_persistent_kernel<false>, mha_persistent_kernel<true>}) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistentSmemBytes);
+      if (e != cudaSuccess) return e;
+    }
     if (cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms[dev] <= 0)
       sms[dev] = 148;
     attr_set[dev] = true;
@@ -1348,12 +1397,15 @@ cudaError_t launch_persistent(const MhaLaunch& a, cudaStream_t stream) {
   args.max_len = a.max_len;
   args.tma_out = a.has_tm_ctx ? 1 : 0;
   args.early_offsets = a.early_offsets ? 1 : 0;
-  const long long items_max =
-      static_cast<long long>(a.batch) * a.head_num * ((a.max_len + kQRows - 1) / kQRows);  // upper bound
-  long long grid = 2LL * sms[dev];
-  if (grid > items_max) grid = items_max;
-  if (grid < 1) grid = 1;
-  return launch_pdl(mha_persistent_kernel, dim3(static_cast<unsigned>(grid)), dim3(kPersistentThreads), kPersistentSmemBytes,
+  // A block per item, by an upper bound: tiles of sequences of max_len, or of sequences that share `rows` rows (each a
+  // fraction of a tile beyond its share).
+  long long tiles = static_cast<long long>(a.batch) * ((a.max_len + kQRows - 1) / kQRows);
+  const long long by_rows = (a.rows + static_cast<long long>(a.batch) * (kQRows - 1)) / kQRows;
+  if (tiles > by_rows) tiles = by_rows;
+  const long long grid = tiles > 0 ? tiles * a.head_num : 1;
+  if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
+  auto kern = grid > 2LL * sms[dev] ? mha_persistent_kernel<true> : mha_persistent_kernel<false>;
+  return launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(kPersistentThreads), kPersistentSmemBytes,
                     stream, a.tm_qkv, a.has_tm_ctx ? a.tm_ctx : a.tm_qkv, args);
 }
 
