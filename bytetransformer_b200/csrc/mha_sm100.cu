@@ -47,8 +47,7 @@
 // 421 against 403 us per 79k-token launch), ex2.f16x2, 256-row ping-pong tiles, two threads per row with an exchange
 // through shared memory (25 % slower), reading an item's O out behind the next item's exponentials (level to 5 %
 // slower), items handed out by the loader through shared memory (-1 % at 512 tokens, +0.4 % for one sequence),
-// masking a tail tile by groups of keys under branches (spills 624 bytes; the 128 half-rate compares and selects
-// cost ~1k clocks per tail tile).
+// masking a tail tile by groups of keys under branches inside the body of the whole tiles (spills 624 bytes).
 #include "common.cuh"
 #include "kernels.h"
 
@@ -795,10 +794,11 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
 // commit) is off the softmax warps' critical path.  With the row in registers the row maximum is exact
 // before the first exponential, and all 128 exponentials are formed before P is touched, by which time
 // the P V MMAs of the previous key tile (the owners of P and O until they retire) are long done.
-// From the first load of S to the last store of P the code is one straight line: keys that do not
-// exist in a sequence's last tile are set to -inf beforehand (probability 0) rather than skipped,
-// because a branch per 32-key chunk cost more (the scheduler cannot overlap across it) than the
-// exponentials it saved.
+// From the first load of S to the last store of P a whole tile is one straight line; a sequence's last tile, unless it
+// is whole, has a rolled loop over its 32-key chunks instead.  (In the straight line the 128 compares and selects of a
+// partial tile took ~1k clocks and its exponentials were formed for keys that do not exist.  us per launch with one body
+// for both / with two: 146 sequences of 16..1024 tokens 320.5 / 298, 64 of up to 384 with 16 heads 60.5 / 55.5, 1200 of 64
+// 195 / 147, 18 of 1024, which have no partial tile, 89.8 / 88.9.)
 //
 // Warps 0-3 softmax (one warpgroup, 216 registers each after setmaxnreg), warp 4 loads, warp 5 issues
 // the MMAs, warps 6-7 only give their registers away (setmaxnreg works on whole warpgroups).  The two
@@ -1207,82 +1207,111 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
         const int kv_valid = min(kKvRows, L - j * kKvRows);
         mbar_wait_anyway(s_full, step & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
         tc_fence_after();
-        uint32_t s[128];
-        tmem_ld_32x32_at<0>(t_s, s);
-        tmem_ld_32x32_at<32>(t_s + 32, s);
-        tmem_ld_32x32_at<64>(t_s + 64, s);
-        tmem_ld_32x32_at<96>(t_s + 96, s);
-        tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(s_free);
-        if (kv_valid != kKvRows) {
-          // last tile of the sequence: keys that do not exist get -inf (probability 0), by selection
-#pragma unroll
-          for (int i = 0; i < 128; ++i) s[i] = (i < kv_valid) ? s[i] : 0xff800000u;
-        }
-        // ---- exact row maximum
-        float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-#pragma unroll
-        for (int i = 0; i < 128; i += 8) {
-          mx0 = max3(mx0, __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
-          mx1 = max3(mx1, __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
-          mx2 = max3(mx2, __uint_as_float(s[i + 4]), __uint_as_float(s[i + 5]));
-          mx3 = max3(mx3, __uint_as_float(s[i + 6]), __uint_as_float(s[i + 7]));
-        }
-        const float m_new = fmaxf(m_ref, c * max3(mx0, mx1, fmaxf(mx2, mx3)));
         bool pv_waited = (j == 0);  // (first tile of an item: the wait for the previous item's O covered it)
-        if (j == 0) {
-          m_ref = m_new;
-        } else if (__any_sync(0xffffffffu, (m_new - m_ref) > max_lag)) {
-          // O belongs to the P V MMAs of the previous key tile until those have retired
+        auto wait_pv = [&]() {  // P and O belong to the P V MMAs of the previous key tile until those have retired
           mbar_wait_anyway(pv_done, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
           tc_fence_after();
           pv_waited = true;
-          const float f = ex2_approx(m_ref - m_new);
+        };
+        // The exponent reference and, where it has fallen too far behind a row's maximum, O
+        auto move_reference = [&](int j, float m_new) {
+          if (j == 0) {
+            m_ref = m_new;
+          } else if (__any_sync(0xffffffffu, (m_new - m_ref) > max_lag)) {
+            wait_pv();
+            const float f = ex2_approx(m_ref - m_new);
 #pragma unroll
-          for (int cb = 0; cb < kHeadDim; cb += 32) {
-            uint32_t v[32];
-            tmem_ld_32x32(t_o + cb, v);
-            tmem_ld_wait();
+            for (int cb = 0; cb < kHeadDim; cb += 32) {
+              uint32_t v[32];
+              tmem_ld_32x32(t_o + cb, v);
+              tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * f);
-            tmem_st_32x32(t_o + cb, v);
+              for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * f);
+              tmem_st_32x32(t_o + cb, v);
+            }
+            l_run *= f;
+            m_ref = m_new;
           }
-          l_run *= f;
-          m_ref = m_new;
-        }
-        // ---- probabilities: fp16 pairs for P's own columns, fp32 row sum
-        float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
-        uint32_t pk[64];
-#pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          float t0, t1;
-          fma2(t0, t1, __uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1]), c, -m_ref);
-          const float p0 = ex2_approx(t0);
-          const float p1 = ex2_approx(t1);
-          if (i & 1) add2(l2, l3, p0, p1); else add2(l0, l1, p0, p1);
-          pk[i] = pack_half2(p0, p1);
-        }
-        l_run += (l0 + l1) + (l2 + l3);
-        if (!pv_waited) {
-          // P belongs to the P V MMAs of the previous key tile until those have retired
-          mbar_wait_anyway(pv_done, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
-          tc_fence_after();
-        }
-        tmem_st_32x16_at<0>(t_p, pk);
-        tmem_st_32x16_at<16>(t_p + 16, pk);
-        tmem_st_32x16_at<32>(t_p + 32, pk);
-        tmem_st_32x16_at<48>(t_p + 48, pk);
+        };
         if (kv_valid != kKvRows) {
-          // tail tile: blank the V rows of keys that do not belong to this sequence
+          // Last tile of the sequence, kv_valid < 128 keys: by chunks of 32 keys, those that hold any, in two passes over
+          // S.  A rolled loop of its own: the straight line below costs the same however few keys there are, plus ~1k
+          // clocks for the 128 selects that a partial tile needs there.
+          const int last = (kv_valid - 1) & ~31;  // first key of the chunk that is masked
+          float mx = -INFINITY;
+#pragma unroll 1
+          for (int c0 = 0; c0 < last; c0 += 32) {
+            uint32_t v[32];
+            tmem_ld_32x32(t_s + c0, v);
+            tmem_ld_wait();
+            mx = fmaxf(mx, chunk_max<false>(v, c0, kv_valid));
+          }
+          uint32_t v[32], pk[16];
+          tmem_ld_32x32(t_s + last, v);
+          tmem_ld_wait();
+          mx = fmaxf(mx, chunk_max<true>(v, last, kv_valid));
+          const float m_new = fmaxf(m_ref, c * mx);
+          move_reference(j, m_new);
+          if (!pv_waited) wait_pv();
+          l_run += chunk_probs<true>(v, last, kv_valid, c, m_ref, pk);
+          tmem_st_32x16(t_p + (last >> 1), pk);
+#pragma unroll 1
+          for (int c0 = 0; c0 < last; c0 += 32) {
+            tmem_ld_32x32(t_s + c0, v);
+            tmem_ld_wait();
+            l_run += chunk_probs<false>(v, c0, kv_valid, c, m_ref, pk);
+            tmem_st_32x16(t_p + (c0 >> 1), pk);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(s_free);
+          // blank the V rows of keys that do not belong to this sequence (as far as they are multiplied)
           mbar_wait_anyway(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
-          if (r >= kv_valid) {
+          if (r >= kv_valid && r < ((kv_valid + 15) & ~15)) {
             uint4* vr = reinterpret_cast<uint4*>(smem + kSmemV + stage * kTileBytes + r * 128);
 #pragma unroll
             for (int i = 0; i < 8; ++i) vr[i] = make_uint4(0u, 0u, 0u, 0u);
           }
           fence_proxy_async_smem();
+        } else {
+          uint32_t s[128];
+          tmem_ld_32x32_at<0>(t_s, s);
+          tmem_ld_32x32_at<32>(t_s + 32, s);
+          tmem_ld_32x32_at<64>(t_s + 64, s);
+          tmem_ld_32x32_at<96>(t_s + 96, s);
+          tmem_ld_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(s_free);
+          // ---- exact row maximum
+          float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+#pragma unroll
+          for (int i = 0; i < 128; i += 8) {
+            mx0 = max3(mx0, __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+            mx1 = max3(mx1, __uint_as_float(s[i + 2]), __uint_as_float(s[i + 3]));
+            mx2 = max3(mx2, __uint_as_float(s[i + 4]), __uint_as_float(s[i + 5]));
+            mx3 = max3(mx3, __uint_as_float(s[i + 6]), __uint_as_float(s[i + 7]));
+          }
+          const float m_new = fmaxf(m_ref, c * max3(mx0, mx1, fmaxf(mx2, mx3)));
+          move_reference(j, m_new);
+          // ---- probabilities: fp16 pairs for P's own columns, fp32 row sum
+          float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
+          uint32_t pk[64];
+#pragma unroll
+          for (int i = 0; i < 64; ++i) {
+            float t0, t1;
+            fma2(t0, t1, __uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1]), c, -m_ref);
+            const float p0 = ex2_approx(t0);
+            const float p1 = ex2_approx(t1);
+            if (i & 1) add2(l2, l3, p0, p1); else add2(l0, l1, p0, p1);
+            pk[i] = pack_half2(p0, p1);
+          }
+          l_run += (l0 + l1) + (l2 + l3);
+          if (!pv_waited) wait_pv();
+          tmem_st_32x16_at<0>(t_p, pk);
+          tmem_st_32x16_at<16>(t_p + 16, pk);
+          tmem_st_32x16_at<32>(t_p + 32, pk);
+          tmem_st_32x16_at<48>(t_p + 48, pk);
         }
         tmem_st_wait();
         tc_fence_before();
