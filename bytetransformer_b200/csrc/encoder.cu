@@ -1014,7 +1014,9 @@ int bt_gemm_layernorm(bt_handle h, const void* A, const void* W, const void* bia
     const int rc = check_device(h);
     if (rc != BT_OK) return rc;
   }
-  // scratch: [m_rows][N/128] tagged partials of 16 bytes, zeroed here; this launch is number 1 on it
+  // scratch: N/128 tagged partials of 16 bytes per row, zeroed here; this launch is number 1 on it.  The kernel moves
+  // a partial as one 16-byte access; the caller's buffer (32 times what is used) may start anywhere.
+  scratch_f32 = reinterpret_cast<void*>(align_up(reinterpret_cast<uintptr_t>(scratch_f32), 16));
   cudaError_t me = cudaMemsetAsync(scratch_f32, 0, static_cast<size_t>(m_rows) * (N / 128) * 16,
                                    reinterpret_cast<cudaStream_t>(stream));
   if (me != cudaSuccess) return fail_cuda(h, me, "memset of the LayerNorm statistics scratch");

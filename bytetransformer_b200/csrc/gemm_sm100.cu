@@ -743,8 +743,8 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 // owns one row and 128 of its columns:
 //   1. v = accumulator + bias + residual, written back to tensor memory, with the sum and
 //      sum of squares of v - s (s = the thread's first value: shifted one-pass statistics);
-//   2. the partial (mean_i, M2_i) goes to a global scratch row (it stays in L2) as two 64-bit
-//      words, each (value bits << 32 | epoch of this launch): an aligned 64-bit store is
+//   2. the partial (mean_i, M2_i) goes to a global scratch (it stays in L2) as two 64-bit
+//      words, side by side with those of the slab's other rows, each (value bits << 32 | epoch of this launch): an aligned 64-bit store is
 //      single-copy atomic, so the tag validates the value and no fence or counter is needed;
 //   3. the thread polls (bounded) the 2 * 2*C words of its row until all carry the epoch and
 //      merges the 2*C partials (equal counts):
@@ -760,13 +760,12 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 // The scratch (16 * N/128 bytes per row) must not hold this launch's epoch in the low half of any
 // word beforehand: the caller zeroes it once and numbers the launches that share it 1, 2, 3, ...
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ void st_relaxed_gpu_u64(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+__device__ __forceinline__ void st_relaxed_gpu_2u64(unsigned long long* p, unsigned long long v0, unsigned long long v1) {
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(v0), "l"(v1) : "memory");
 }
-__device__ __forceinline__ unsigned long long ld_relaxed_gpu_u64(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
+__device__ __forceinline__ void ld_relaxed_gpu_2u64(const unsigned long long* p, unsigned long long& v0,
+                                                    unsigned long long& v1) {
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v0), "=l"(v1) : "l"(p) : "memory");
 }
 // The epilogue warps' loop of the GEMM + LayerNorm kernels (one-CTA and pair form share it): steps 1-4
 // of the description above for every tile that `tile_at(it, m0, n0)` yields (m0 = first of this CTA's 128
@@ -900,49 +899,47 @@ __device__ __forceinline__ void ln_epilogue_loop(const GemmArgs& args, const CUt
     // aligned 64-bit store is single-copy atomic, so a reader that finds this launch's epoch in a word
     // also has its value: no fence, no counter, no second round trip.
     const uint32_t epoch = args.ln_epoch;
-    unsigned long long* words = reinterpret_cast<unsigned long long*>(args.out);
-    if (row_ok) {
-      unsigned long long* wp = words + (static_cast<size_t>(row) * parts + part) * 2;
-      st_relaxed_gpu_u64(wp, (static_cast<unsigned long long>(__float_as_uint(lmean)) << 32) | epoch);
-      st_relaxed_gpu_u64(wp + 1, (static_cast<unsigned long long>(__float_as_uint(m2)) << 32) | epoch);
-    }
+    // The words of a partial's 32 rows lie side by side, so that a warp writes or reads them with one
+    // instruction on four whole lines (the allocation's last slab may have fewer than 32 rows).
+    const int slab_rows = min(32, args.m_rows - row0);
+    unsigned long long* slab_words = reinterpret_cast<unsigned long long*>(args.out) + static_cast<size_t>(row0) * parts * 2;
+    if (row_ok)
+      st_relaxed_gpu_2u64(slab_words + (part * slab_rows + lane) * 2,
+                          (static_cast<unsigned long long>(__float_as_uint(lmean)) << 32) | epoch,
+                          (static_cast<unsigned long long>(__float_as_uint(m2)) << 32) | epoch);
     if (warp == 2 && lane == 0) gstamp(args.timing, it, 5);
     // ---- 3. wait until the row's 2 * parts words all carry this epoch (bounded), then merge.
-    // The partials of the 32 rows of this slab come from the same 2*C warps, so one lane probes its
-    // own row (2 * parts loads per probe, not 64 * parts: letting every lane poll its row was measured
-    // and cost 15 % of the kernel, a pause between probes changed nothing) and only then does every
-    // lane read and validate its row; a lane whose words are not all there yet sends the warp round
-    // again.
+    // A partial's 32 rows are written by one store, so lane p probes partial p of the slab's first row (one load
+    // for the warp) and only when all are there does every lane read and validate its row; a lane whose words
+    // are not all there yet sends the warp round again.  us per launch of 18,944 rows x 768 columns, K = 768 / 3072:
+    // with the words row by row (12 loads over 32 lines each) and one lane probing its own row 59.0 / 91.4, so
+    // 50.7 / 87.9; the wait alone, all CTAs in step, 4.9k and 1.9k clocks.
     float mean = 0.f, rstd = 0.f;
     float pm[8], pq[8];  // N <= 1024: at most 8 partials per row
-    const unsigned long long* rp64 = words + static_cast<size_t>(row_ok ? row : 0) * parts * 2;
     const long long t0 = clock64();
     bool give_up = false;
     while (true) {
-      if (lane == 0 && row_ok) {
+      {
         uint32_t probes = 0;
         while (true) {
-          // all loads are issued before any tag is looked at (no short-circuit: one round trip, not 2*parts)
           uint32_t bad = 0;
-#pragma unroll
-          for (int p = 0; p < 8; ++p)
-            if (p < parts) {
-              const unsigned long long w0 = ld_relaxed_gpu_u64(rp64 + 2 * p);
-              const unsigned long long w1 = ld_relaxed_gpu_u64(rp64 + 2 * p + 1);
-              bad |= (static_cast<uint32_t>(w0) ^ epoch) | (static_cast<uint32_t>(w1) ^ epoch);
-            }
-          if (bad == 0) break;
-          if ((++probes & 15u) == 0u && (*abort_flag != 0 || clock64() - t0 > (1ll << 31))) break;
+          if (lane < parts && row0 < M) {
+            unsigned long long w0, w1;
+            ld_relaxed_gpu_2u64(slab_words + lane * slab_rows * 2, w0, w1);
+            bad = (static_cast<uint32_t>(w0) ^ epoch) | (static_cast<uint32_t>(w1) ^ epoch);
+          }
+          if (__all_sync(0xffffffffu, bad == 0)) break;
+          if ((++probes & 15u) == 0u && __any_sync(0xffffffffu, *abort_flag != 0 || clock64() - t0 > (1ll << 31))) break;
         }
       }
-      __syncwarp();
       uint32_t bad = 0;
       if (row_ok) {
+        // all loads are issued before any tag is looked at: one round trip
 #pragma unroll
         for (int p = 0; p < 8; ++p)
           if (p < parts) {
-            const unsigned long long w0 = ld_relaxed_gpu_u64(rp64 + 2 * p);
-            const unsigned long long w1 = ld_relaxed_gpu_u64(rp64 + 2 * p + 1);
+            unsigned long long w0, w1;
+            ld_relaxed_gpu_2u64(slab_words + (p * slab_rows + lane) * 2, w0, w1);
             bad |= (static_cast<uint32_t>(w0) ^ epoch) | (static_cast<uint32_t>(w1) ^ epoch);
             pm[p] = __uint_as_float(static_cast<uint32_t>(w0 >> 32));
             pq[p] = __uint_as_float(static_cast<uint32_t>(w1 >> 32));

@@ -578,6 +578,22 @@ def _fused_layernorm_case(enc, cuda_device, M, N, K, gb32, m_valid):
     assert enc.device_status() == 0
 
 
+@pytest.mark.parametrize("offset", [0, 4, 8])
+def test_fused_layernorm_scratch_may_start_anywhere(enc, cuda_device, offset):
+    """The statistics scratch of bt_gemm_layernorm needs no alignment of its own (the kernel moves its words 16 bytes at
+    a time); 70 rows end in a slab of six."""
+    M, N, K = 70, 256, 128
+    g = torch.Generator().manual_seed(offset)
+    t = [torch.randn(*s, generator=g).half().to(cuda_device) for s in ((M, K), (K, N), (N,), (M, N), (N,), (N,))]
+    want = enc.gemm_layernorm(*t)
+    out = torch.empty_like(want)
+    scratch = torch.empty(M * N * 4 + 16, dtype=torch.uint8, device=cuda_device)
+    enc._call("bt_gemm_layernorm", enc._h, *[x.data_ptr() for x in t], 0, 1e-6, scratch.data_ptr() + offset, out.data_ptr(), None,
+              M, N, K, torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(out, want)
+    assert enc.device_status() == 0
+
+
 # ---------------------------------------------------------------- failure path
 def test_expired_wait_is_reported_and_the_context_stays_usable(enc, cuda_device):
     """A device-side wait that nothing satisfies (the library's own self-test kernel: an mbarrier
