@@ -134,13 +134,29 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
-// The same for a warp whose 32 lanes all wait: one answer for the warp, from a vote.  No kernel branches on a lane's
-// own answer: lanes that parted ways where a wait gave up would hang in the next warp-wide instruction (elect.sync,
-// tcgen05.ld, __syncwarp), bound or no bound.  A role votes (this form), goes on to the end of its K loop and votes there
+// The same for a warp whose 32 lanes all wait: one answer for the warp.  No kernel branches on a lane's own answer:
+// lanes that parted ways where a wait gave up would hang in the next warp-wide instruction (elect.sync, tcgen05.ld,
+// __syncwarp), bound or no bound.  A role votes (this form), goes on to the end of its K loop and votes there
 // (mbar_wait_latched), or goes on regardless (mbar_wait_anyway).
+// Every branch here is on a vote.  With a branch on the lanes' own answers - a vote behind the loop is too late - the
+// compiler has to take all code behind the wait for code that a part of the warp may run, and forms the operands of the
+// tcgen05 and TMA instructions there lane by lane: a K block of four 128 x 64 x 16 MMAs took 314 clocks behind such a
+// wait and takes 240 behind this one (198 without a wait).
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
                                                int code, long long max_cycles = (1ll << 31)) {
-  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, status, code, max_cycles)) != 0;
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const long long t0 = clock64();
+  uint32_t polls = 0;
+  while (true) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    ++polls;
+    if ((polls & 255u) == 8u && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
+    if ((polls & 255u) == 0u && __any_sync(0xffffffffu, clock64() - t0 > max_cycles)) {
+      *abort_flag = 1;
+      if (status != nullptr) atomicCAS(status, 0, code);
+      return false;
+    }
+  }
 }
 
 // The wait of a role that can go on whatever the answer: where it gives up the status word is set, the CTA's flag is up,
@@ -152,14 +168,16 @@ __device__ __forceinline__ void mbar_wait_anyway(uint64_t* bar, uint32_t parity,
   (void)mbar_wait_bounded(bar, parity, abort_flag, status, code);
 }
 
-// The wait of a loop that goes on to its end when a wait gave up (a vote per K block costs 30 clocks): `ok` is the
-// lane's answer so far; the loop ends in a vote over it.  The blocks that are left are polled nine times each, because the
-// flag is up: the time to give up stays one bound however many they are.  (Not polled at all, behind a branch on `ok`,
-// was measured too: a 12-layer forward of one 614-token sequence 581 -> 585 us.)
-__device__ __forceinline__ bool mbar_wait_latched(bool ok, uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                                  int* status, int code, long long max_cycles = (1ll << 31)) {
-  const bool now = mbar_wait_bounded(bar, parity, abort_flag, status, code, max_cycles);
-  return ok & now;
+// The wait of a K loop, which goes on to its end when a wait gave up: `ok` is the answer so far; the loop ends in a vote
+// over it.  `landed` is what a test of this barrier and phase, made ahead of the MMAs of the block before, said to the lane:
+// the test's latency then passes under the issue of those MMAs (240 -> 218 clocks per K block, see mbar_wait_warp).
+// The blocks that are left after a wait gave up are polled nine times each, because the flag is up: the time to give
+// up stays one bound however many they are.
+__device__ __forceinline__ bool mbar_wait_latched(bool ok, bool landed, uint64_t* bar, uint32_t parity,
+                                                  volatile int* abort_flag, int* status, int code,
+                                                  long long max_cycles = (1ll << 31)) {
+  if (__all_sync(0xffffffffu, landed)) return ok;
+  return mbar_wait_warp(bar, parity, abort_flag, status, code, max_cycles) && ok;
 }
 
 // ------------------------------------------------------------ warp-uniform roles

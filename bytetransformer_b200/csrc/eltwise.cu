@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(32) wait_forms_selftest_kernel(long long max_c
   bool ok = true;
   long long t1 = t0;
   for (int kb = 0; kb < 64; ++kb) {
-    ok = mbar_wait_latched(ok, &bar, 0u, &abort_flag_s, nullptr, 0, max_cycles);
+    ok = mbar_wait_latched(ok, false, &bar, 0u, &abort_flag_s, nullptr, 0, max_cycles);
     if (kb == 0) t1 = clock64();
   }
   const long long t2 = clock64();

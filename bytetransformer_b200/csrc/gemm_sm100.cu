@@ -423,7 +423,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     {
       int stage = 0;
       uint32_t phase = 0;
-      bool ok = true;
+      bool ok = true, landed = false;
       int m0 = 0, n0 = 0, sp = 0;
       for (int it = 0; ok && tile_at(it, m0, n0, sp); ++it) {
         const int as = it & 1;
@@ -436,17 +436,19 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         if (lane == 0) gstamp(args.timing, it, 0);
         const uint32_t d_tmem = tmem_base + as * BLOCK_N;
         for (int kb = 0; kb < num_kb; ++kb) {
-          ok = mbar_wait_latched(ok, &full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
+          ok = mbar_wait_latched(ok, landed, &full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
+          const int cur = stage;
+          const uint32_t sa = smem_u32(smem + cur * Cfg::kStageBytes);
           const uint32_t sb = sa + kABytes;
-          // (the commit frees the stage once these MMAs have retired)
-          umma_k_block<false>(d_tmem, smem_desc(args.a_desc_hi, sa), smem_desc(args.b_desc_hi, sb), args.a_kstep_bytes >> 4,
-                       args.b_kstep_bytes >> 4, args.idesc, kb != 0 ? 1u : 0u, &empty_bar[stage]);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
+          landed = mbar_test_wait(&full_bar[stage], phase);  // the next block, ahead of these MMAs
+          // (the commit frees the stage once these MMAs have retired)
+          umma_k_block<false>(d_tmem, smem_desc(args.a_desc_hi, sa), smem_desc(args.b_desc_hi, sb), args.a_kstep_bytes >> 4,
+                       args.b_kstep_bytes >> 4, args.idesc, kb != 0 ? 1u : 0u, &empty_bar[cur]);
         }
         ok = __all_sync(0xffffffffu, ok) != 0;
         if (ok && elect_one()) umma_commit(&acc_full[as]);
@@ -668,7 +670,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
-      bool ok = true;
+      bool ok = true, landed = false;
       for (int tile = cluster_id; tile < total_tiles && ok; tile += num_clusters, ++it) {
         const int as = it & 1;
         const uint32_t aphase = (it >> 1) & 1;
@@ -680,17 +682,19 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
         if (lane == 0) gstamp(args.timing, it, 0);
         const uint32_t d_tmem = tmem_base + as * kTileN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          ok = mbar_wait_latched(ok, &full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
+          ok = mbar_wait_latched(ok, landed, &full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
+          const int cur = stage;
+          const uint32_t sa = smem_u32(smem + cur * Cfg::kStageBytes);
           const uint32_t sb = sa + kABytes;
-          // (the commit frees the stage once these MMAs have retired)
-          umma_k_block<true>(d_tmem, smem_desc(args.a_desc_hi, sa), smem_desc(args.b_desc_hi, sb), args.a_kstep_bytes >> 4,
-                       args.b_kstep_bytes >> 4, args.idesc, kb != 0 ? 1u : 0u, &empty_bar[stage]);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
+          landed = mbar_test_wait(&full_bar[stage], phase);  // the next block, ahead of these MMAs
+          // (the commit frees the stage once these MMAs have retired)
+          umma_k_block<true>(d_tmem, smem_desc(args.a_desc_hi, sa), smem_desc(args.b_desc_hi, sb), args.a_kstep_bytes >> 4,
+                       args.b_kstep_bytes >> 4, args.idesc, kb != 0 ? 1u : 0u, &empty_bar[cur]);
         }
         ok = __all_sync(0xffffffffu, ok) != 0;
         if (ok && elect_one()) umma_commit_pair(&acc_full[as]);
@@ -1191,7 +1195,7 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     {
       int stage = 0;
       uint32_t phase = 0;
-      bool ok = true;
+      bool ok = true, landed = false;
       int m0 = 0, n0 = 0;
       for (int it = 0; ok && tile_at(it, m0, n0); ++it) {
         const int as = it & 1;
@@ -1204,17 +1208,19 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         if (lane == 0) gstamp(args.timing, it, 0);
         const uint32_t d_tmem = tmem_base + as * kTileN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          ok = mbar_wait_latched(ok, &full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
+          ok = mbar_wait_latched(ok, landed, &full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
+          const int cur = stage;
+          const uint32_t sa = smem_u32(smem + cur * Cfg::kStageBytes);
           const uint32_t sb = sa + kABytes;
-          // (the commit frees the stage once these MMAs have retired)
-          umma_k_block<false>(d_tmem, smem_desc(args.a_desc_hi, sa), smem_desc(args.b_desc_hi, sb), args.a_kstep_bytes >> 4,
-                       args.b_kstep_bytes >> 4, args.idesc, kb != 0 ? 1u : 0u, &empty_bar[stage]);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
+          landed = mbar_test_wait(&full_bar[stage], phase);  // the next block, ahead of these MMAs
+          // (the commit frees the stage once these MMAs have retired)
+          umma_k_block<false>(d_tmem, smem_desc(args.a_desc_hi, sa), smem_desc(args.b_desc_hi, sb), args.a_kstep_bytes >> 4,
+                       args.b_kstep_bytes >> 4, args.idesc, kb != 0 ? 1u : 0u, &empty_bar[cur]);
         }
         ok = __all_sync(0xffffffffu, ok) != 0;
         if (ok && elect_one()) umma_commit(&acc_full[as]);
@@ -1382,7 +1388,7 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
-      bool ok = true;
+      bool ok = true, landed = false;
       for (int tile = cluster_id; tile < total_tiles && ok; tile += num_clusters, ++it) {
         const int as = it & 1;
         const uint32_t aphase = (it >> 1) & 1;
@@ -1394,17 +1400,19 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
         if (lane == 0) gstamp(args.timing, it, 0);
         const uint32_t d_tmem = tmem_base + as * kTileN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          ok = mbar_wait_latched(ok, &full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
+          ok = mbar_wait_latched(ok, landed, &full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
+          const int cur = stage;
+          const uint32_t sa = smem_u32(smem + cur * Cfg::kStageBytes);
           const uint32_t sb = sa + kABytes;
-          // (the commit frees the stage once these MMAs have retired)
-          umma_k_block<true>(d_tmem, smem_desc(args.a_desc_hi, sa), smem_desc(args.b_desc_hi, sb), args.a_kstep_bytes >> 4,
-                       args.b_kstep_bytes >> 4, args.idesc, kb != 0 ? 1u : 0u, &empty_bar[stage]);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
           }
+          landed = mbar_test_wait(&full_bar[stage], phase);  // the next block, ahead of these MMAs
+          // (the commit frees the stage once these MMAs have retired)
+          umma_k_block<true>(d_tmem, smem_desc(args.a_desc_hi, sa), smem_desc(args.b_desc_hi, sb), args.a_kstep_bytes >> 4,
+                       args.b_kstep_bytes >> 4, args.idesc, kb != 0 ? 1u : 0u, &empty_bar[cur]);
         }
         ok = __all_sync(0xffffffffu, ok) != 0;
         if (ok && elect_one()) umma_commit_pair(&acc_full[as]);
