@@ -109,7 +109,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 
 // Wait for a phase with an upper bound.  Returns false when the bound ran out
 // or another role of this CTA already gave up (`*abort_flag` non-zero).  The answer
-// is the calling lane's own: what a warp waits for goes through the three forms below.
+// is the calling lane's own: what a warp waits for goes through the forms below.
 // The bound is ~2^31 SM cycles (about a second) unless the caller gives another,
 // checked every 256 polls; once the flag is up, a wait ends after nine (not after
 // its first: a look at the flag between two polls that a K loop's wait does need was
@@ -160,11 +160,16 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
 }
 
 // The wait of a role that can go on whatever the answer: where it gives up the status word is set, the CTA's flag is up,
-// later waits end after nine polls, and what the role makes of the bytes that did not arrive is as invalid as the launch's output
-// is then.  For waits in the middle of a tile, where a vote is time: with votes at all waits of the LayerNorm epilogue and
-// the softmax warps a BERT-large forward of 36 row tiles took 1794 us against 1706, a causal one of 1024 tokens 869 / 854.
+// later waits end after nine polls, and what the role makes of the bytes that did not arrive is as invalid as the launch's
+// output is then.  For waits in the middle of a tile.  The GEMMs' epilogues use the form whose branches are votes (see
+// above; us per forward, lane form / this one: 16 x 512 1111 / 1097, 16 x 128 595 / 591); the softmax warps of the
+// attention kernels, whose registers are all taken, the lane form (one sequence of 614 tokens 528.3 against 529.8).
 __device__ __forceinline__ void mbar_wait_anyway(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
                                                  int code) {
+  (void)mbar_wait_warp(bar, parity, abort_flag, status, code);
+}
+__device__ __forceinline__ void mbar_wait_anyway_lane(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                                      int code) {
   (void)mbar_wait_bounded(bar, parity, abort_flag, status, code);
 }
 
@@ -183,15 +188,18 @@ __device__ __forceinline__ bool mbar_wait_latched(bool ok, bool landed, uint64_t
 // ------------------------------------------------------------ warp-uniform roles
 // tcgen05 and TMA instructions take their descriptors, addresses and coordinates from uniform registers.  In a
 // branch that one lane takes (`if (lane == 0)`) every operand of every instruction is moved there first, and that
-// cost more than the instruction: a 128 x N x 16 MMA took 91 clocks for any N <= 128 (132 in the GEMM main loop, with
-// its barrier waits), where the tensor core needs 64 at N = 128 and 50 at N = 32.  So the single-thread roles are
-// walked by their whole warp - role, loop bounds and shared values go through uniform_int() - and only the
-// instructions themselves are predicated on an elected lane, all MMAs of a K block and their commit on one
-// election (umma_k_block): 84 clocks per MMA in the main loop, 525 -> 335 clocks per K block of 64 (N <= 128).
+// cost more than the instruction.  So the single-thread roles are
+// walked by their whole warp - role, loop bounds and shared values go through uniform_int(), waits branch on votes - and
+// only the instructions themselves are predicated on an elected lane, all MMAs of a K block and their commit on one
+// election (umma_k_block).  Clocks per K block of four 128 x 64 x 16 MMAs in the main loop: 525 with one lane, 330 with
+// the whole warp and waits that branched on the lanes' own answers, 225 now.
 // Because elect.sync needs the whole warp, a warp's lanes must not part ways after a wait that gave up: see
-// the three forms of a warp's wait above.
-__device__ __forceinline__ int uniform_int(int v) { return __shfl_sync(0xffffffffu, v, 0); }
-__device__ __forceinline__ uint32_t uniform_u32(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+// the forms of a warp's wait above.
+// (A reduction, not a shuffle: its result is born in a uniform register, so a branch on it is one the whole warp takes.
+// us per forward, shuffle / reduction: 16 x 512 causal 1822 / 1787, 16 x 512 1110 / 1097, one of 38 tokens 364.7 / 365.6.)
+// All lanes hold the same value.
+__device__ __forceinline__ uint32_t uniform_u32(uint32_t v) { return __reduce_or_sync(0xffffffffu, v); }
+__device__ __forceinline__ int uniform_int(int v) { return static_cast<int>(uniform_u32(static_cast<uint32_t>(v))); }
 
 // ----------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {

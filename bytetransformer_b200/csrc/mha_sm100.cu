@@ -648,7 +648,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
           for (int u = 0; u < 8; ++u) bias_q[u] = __ldg(bt + u * 128);
         }
       }
-      mbar_wait_anyway(s_full, j & 1, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
+      mbar_wait_anyway_lane(s_full, j & 1, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
       tc_fence_after();
       uint4 bw = make_uint4(~0u, ~0u, ~0u, ~0u);  // a row that does not exist masks nothing
       if (GENERAL && use_bits) {
@@ -707,7 +707,7 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
         l_run += full_tile ? tile_probs(t_s, c, m_ref) : tail_probs(t_s, kv_valid, c, m_ref);
       if (!full_tile) {
         // tail tile: blank the V rows of keys that do not belong to this sequence
-        mbar_wait_anyway(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
+        mbar_wait_anyway_lane(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
         if (r >= kv_valid && r < ((kv_valid + 15) & ~15)) {
           uint4* vr = reinterpret_cast<uint4*>(smem + Cfg::kSmemV + stage * kTileBytes + r * 128);
 #pragma unroll
@@ -891,30 +891,26 @@ __device__ __forceinline__ void setmaxnreg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-// Bounded wait for the roles that one warp walks (loader, MMA issuer; all lanes call it, one answer for the warp):
-// between polls the warp sleeps, so that its polling does not take issue slots from the softmax warp that shares
-// its scheduler.
-__device__ __forceinline__ bool mbar_wait_role_lane(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                                    int code) {
-  if (mbar_try_wait(bar, parity)) return true;
+// Bounded wait for the roles that one warp walks (loader, MMA issuer; all lanes call it, one answer for the warp, every
+// branch on a vote: see mbar_wait_warp): between polls the warp sleeps, so that its polling does not take issue slots
+// from the softmax warp that shares its scheduler.
+__device__ __forceinline__ bool mbar_wait_role(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                               int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   const long long t0 = clock64();
   uint32_t polls = 0;
   while (true) {
     __nanosleep(40);
-    if (mbar_try_wait(bar, parity)) return true;
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     if ((++polls & 63u) == 0u) {
-      if (*abort_flag != 0) return false;
-      if (clock64() - t0 > (1ll << 31)) {
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+      if (__any_sync(0xffffffffu, clock64() - t0 > (1ll << 31))) {
         *abort_flag = 1;
         if (status != nullptr) atomicCAS(status, 0, code);
         return false;
       }
     }
   }
-}
-__device__ __forceinline__ bool mbar_wait_role(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                               int code) {
-  return __all_sync(0xffffffffu, mbar_wait_role_lane(bar, parity, abort_flag, status, code)) != 0;
 }
 
 constexpr int kPersistentThreads = 256;
@@ -1205,11 +1201,11 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
       float l_run = 0.f;
       for (int j = 0; j < n_kv; ++j, ++step) {
         const int kv_valid = min(kKvRows, L - j * kKvRows);
-        mbar_wait_anyway(s_full, step & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
+        mbar_wait_anyway_lane(s_full, step & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
         tc_fence_after();
         bool pv_waited = (j == 0);  // (first tile of an item: the wait for the previous item's O covered it)
         auto wait_pv = [&]() {  // P and O belong to the P V MMAs of the previous key tile until those have retired
-          mbar_wait_anyway(pv_done, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
+          mbar_wait_anyway_lane(pv_done, (step - 1u) & 1u, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
           tc_fence_after();
           pv_waited = true;
         };
@@ -1266,7 +1262,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
           __syncwarp();
           if (lane == 0) mbar_arrive(s_free);
           // blank the V rows of keys that do not belong to this sequence (as far as they are multiplied)
-          mbar_wait_anyway(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
+          mbar_wait_anyway_lane(&v_full[stage], phase, abort_flag, args.status, kStatusMhaSoftmaxTimeout);
           if (r >= kv_valid && r < ((kv_valid + 15) & ~15)) {
             uint4* vr = reinterpret_cast<uint4*>(smem + kSmemV + stage * kTileBytes + r * 128);
 #pragma unroll
