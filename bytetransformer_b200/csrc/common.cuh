@@ -425,8 +425,7 @@ __device__ __forceinline__ float gelu_erf_fast(float x) {
   return fmaf(-0.5f * ax, e, fmaxf(x, 0.f));
 }
 // Two values at once with the packed fp32 instructions of sm_100 (fma.rn.f32x2: one issue slot for two
-// lanes of a 64-bit register pair): the polynomial and the final multiply-add, which are most of the
-// instructions of gelu_erf_fast, take half the issue slots.  Same arithmetic, same results.
+// lanes of a 64-bit register pair).
 __device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -445,22 +444,26 @@ __device__ __forceinline__ unsigned long long add_f32x2(unsigned long long a, un
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+// gelu_erf_fast for two values, with the constants folded together: n = -|x|, clamped, takes the place of z, and the
+// factor 1/2 is in the exponent,
+//   gelu(x) = max(x, 0) + n * 2^q(n),   q(n) = p(-n / sqrt(2)) - 1.
+// Maximum absolute error 6.4e-7 as above.  A NaN stays one (by way of the maximum; n drops it), and an infinity
+// gives what its limit is.  Clocks for the GELU epilogue of a 128 x 256 tile by itself, eight warps: 4322 with the two
+// halvings and the scaling as instructions of their own, 3787 so.
 __device__ __forceinline__ void gelu_erf_fast_pair(float& x0, float& x1) {
-  const float a0 = fabsf(x0), a1 = fabsf(x1);
-  const unsigned long long z = pack_f32x2(fminf(a0 * 0.70710678118654752f, 4.3f), fminf(a1 * 0.70710678118654752f, 4.3f));
-  unsigned long long p = fma_f32x2(pack_f32x2(-0.002677350537851453f, -0.002677350537851453f), z,
-                                   pack_f32x2(0.02833780087530613f, 0.02833780087530613f));
-  p = fma_f32x2(p, z, pack_f32x2(-0.1465892493724823f, -0.1465892493724823f));
-  p = fma_f32x2(p, z, pack_f32x2(-0.9199854135513306f, -0.9199854135513306f));
-  p = fma_f32x2(p, z, pack_f32x2(-1.6274596452713013f, -1.6274596452713013f));
-  p = fma_f32x2(p, z, pack_f32x2(-3.764020948437974e-05f, -3.764020948437974e-05f));
-  float p0, p1, e0, e1;
-  unpack_f32x2(p, p0, p1);
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(p0));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(p1));
-  const unsigned long long r = fma_f32x2(pack_f32x2(-0.5f * a0, -0.5f * a1), pack_f32x2(e0, e1),
-                                         pack_f32x2(fmaxf(x0, 0.f), fmaxf(x1, 0.f)));
-  unpack_f32x2(r, x0, x1);
+  const unsigned long long n = pack_f32x2(fmaxf(-fabsf(x0), -6.0811183f), fmaxf(-fabsf(x1), -6.0811183f));
+  unsigned long long q = fma_f32x2(pack_f32x2(0.00047329318476840854f, 0.00047329318476840854f), n, pack_f32x2(0.007084450218826532f, 0.007084450218826532f));
+  q = fma_f32x2(q, n, pack_f32x2(0.05182712525129318f, 0.05182712525129318f));
+  q = fma_f32x2(q, n, pack_f32x2(-0.4599927067756653f, -0.4599927067756653f));
+  q = fma_f32x2(q, n, pack_f32x2(1.1507877111434937f, 1.1507877111434937f));
+  q = fma_f32x2(q, n, pack_f32x2(-1.000037670135498f, -1.000037670135498f));
+  float q0, q1, e0, e1, m0, m1;
+  unpack_f32x2(q, q0, q1);
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(q0));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(q1));
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(m0) : "f"(x0));
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(m1) : "f"(x1));
+  unpack_f32x2(fma_f32x2(n, pack_f32x2(e0, e1), pack_f32x2(m0, m1)), x0, x1);
 }
 __device__ __forceinline__ float gelu_tanh(float x) {
   // 0.5 x (1 + tanh( sqrt(2/pi) (x + 0.044715 x^3) ))

@@ -46,6 +46,7 @@ constexpr int kGemmThreads = 320;
 constexpr int kEpiWarps = 8;
 constexpr int kABytes = kBlockM * kBlockK * 2;  // 16 KiB
 constexpr int kStagingBytesPerWarp = 32 * 128;  // 32 rows x 128 B
+constexpr int kBiasBytes = 2 * 256 * 2;         // the bias of a tile's columns, for two tiles in turn
 
 template <int BLOCK_N>
 struct GemmCfg {
@@ -59,7 +60,7 @@ struct GemmCfg {
     return BLOCK_N >= 128 || epi == BT_EPI_BIAS_RESIDUAL_F32OUT || epi == kEpiSplitKF32;
   }
   static constexpr int kStagingBytes = kEpiWarps * kStagingBytesPerWarp;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 /*align slack*/ + 256 /*barriers*/;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 /*align slack*/ + 256 /*barriers*/ + kBiasBytes;
 };
 
 // Pair kernel: per CTA 128 rows of A and 128 of the tile's 256 W columns per stage.
@@ -71,7 +72,7 @@ struct PairCfg {
   static constexpr int kTmemCols = 512;
   static constexpr int kStagingBufs = 1;  // per epilogue warp (two were measured: no gain, and they cost a stage)
   static constexpr int kStagingBytes = kStagingBufs * kEpiWarps * kStagingBytesPerWarp;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 + 256;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 + 256 + kBiasBytes;
 };
 
 struct GemmArgs {
@@ -131,7 +132,7 @@ __device__ __forceinline__ void tma_store_wait_read_n() {
 template <int TILE_N, int EPI, bool TMA_STORE, int STG_BUFS>
 __device__ __forceinline__ void epilogue_tile(const GemmArgs& args, const CUtensorMap* tm_out, uint8_t* stg,
                                               uint32_t tmem_acc, int m0, int n0, int M, int quarter, int col_half,
-                                              int lane, const uint4* resv, int split = 0) {
+                                              int lane, const uint4* resv, const uint4* bias_s, int split = 0) {
   constexpr int kColsPerWarp = TILE_N / 2;
   constexpr bool kSplitK = (EPI == kEpiSplitKF32);
   constexpr bool kF32Out = (EPI == BT_EPI_BIAS_RESIDUAL_F32OUT) || kSplitK;
@@ -164,10 +165,9 @@ __device__ __forceinline__ void epilogue_tile(const GemmArgs& args, const CUtens
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[h * 32 + i] = __uint_as_float(raw[ci & 1][h][i]);
     if (EPI != BT_EPI_NONE && (!kSplitK || split == 0)) {
-      const uint4* bp = reinterpret_cast<const uint4*>(args.bias + gcol);
 #pragma unroll
       for (int q = 0; q < kChunk / 8; ++q) {
-        const uint4 b4 = __ldg(bp + q);
+        const uint4 b4 = bias_s[col / 8 + q];
         const __half2* bh = reinterpret_cast<const __half2*>(&b4);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -260,6 +260,36 @@ __device__ __forceinline__ void prefetch_residual(const GemmArgs& args, int m0, 
     for (int q = 0; q < kColsPerWarp / 8; ++q) resv[q] = row_ok ? __ldg(rp + q) : make_uint4(0u, 0u, 0u, 0u);
   }
 }
+
+// The bias of a warp's columns: asked for before the accumulator is waited for (BiasShare holds the lane's share), then put
+// where the warp reads it column by column - read from global memory there, a chunk's loads took a round trip to L2 in
+// the middle of the epilogue.  The four warps of a column half write the same bytes to the same place, so none waits for
+// another.  Two buffers by turns: a warp that has seen the accumulator of tile t + 2 knows that all warps are done with tile t.
+template <int TILE_N>
+struct BiasShare {
+  static constexpr int kPerLane = TILE_N / 64;  // halves
+  alignas(8) __half v[kPerLane];
+  __device__ __forceinline__ void load(const __half* bias, int n0, int col_half, int lane) {
+    const __half* p = bias + n0 + col_half * (TILE_N / 2) + lane * kPerLane;
+    if (kPerLane == 4)
+      *reinterpret_cast<uint2*>(v) = __ldg(reinterpret_cast<const uint2*>(p));
+    else if (kPerLane == 2)
+      *reinterpret_cast<uint32_t*>(v) = __ldg(reinterpret_cast<const uint32_t*>(p));
+    else
+      v[0] = __ldg(p);
+  }
+  // (called by the whole warp)
+  __device__ __forceinline__ void put(__half* bias_s, int col_half, int lane) const {
+    __half* p = bias_s + col_half * (TILE_N / 2) + lane * kPerLane;
+    if (kPerLane == 4)
+      *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(v);
+    else if (kPerLane == 2)
+      *reinterpret_cast<uint32_t*>(p) = *reinterpret_cast<const uint32_t*>(v);
+    else
+      p[0] = v[0];
+    __syncwarp();
+  }
+};
 
 // ------------------------------------------------------------------------------------------
 // One CTA per SM, tile 128 x BLOCK_N.
@@ -461,17 +491,22 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     const int quarter = warp & 3;  // TMEM lane quarter this warp may read
     const int col_half = e >> 2;   // which half of the tile's columns
     uint8_t* stg = smem + kStages * Cfg::kStageBytes + e * kStagingBytesPerWarp;  // 32 rows x 128 B, swizzled
+    __half* bias_bufs = reinterpret_cast<__half*>(reinterpret_cast<uint8_t*>(bars) + 256);
     int m0 = 0, n0 = 0, sp = 0;
     for (int it = 0; tile_at(it, m0, n0, sp); ++it) {
       const int as = it & 1;
       const uint32_t aphase = (it >> 1) & 1;
       uint4 resv[kHasResidual ? BLOCK_N / 16 : 1];
       prefetch_residual<BLOCK_N, EPI>(args, m0, n0, M, quarter, col_half, lane, resv, sp);
+      BiasShare<BLOCK_N> bias;
+      if (EPI != BT_EPI_NONE) bias.load(args.bias, n0, col_half, lane);
       mbar_wait_anyway(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout);
       tc_fence_after();
+      __half* bias_s = bias_bufs + as * 256;
+      if (EPI != BT_EPI_NONE) bias.put(bias_s, col_half, lane);
       if (warp == 2 && lane == 0) gstamp(args.timing, it, 2);
       epilogue_tile<BLOCK_N, EPI, Cfg::tma_store(EPI), 1>(args, &tm_out, stg, tmem_base + as * BLOCK_N, m0, n0, M, quarter,
-                                                  col_half, lane, resv, sp);
+                                                  col_half, lane, resv, reinterpret_cast<const uint4*>(bias_s), sp);
       if (warp == 2 && lane == 0) gstamp(args.timing, it, 3);
       tc_fence_before();
       __syncwarp();
@@ -707,6 +742,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     const int quarter = warp & 3;
     const int col_half = e >> 2;
     uint8_t* stg = smem + kStages * Cfg::kStageBytes + e * (Cfg::kStagingBufs * kStagingBytesPerWarp);
+    __half* bias_bufs = reinterpret_cast<__half*>(reinterpret_cast<uint8_t*>(bars) + 256);
     int it = 0;
     for (int tile = cluster_id; tile < total_tiles; tile += num_clusters, ++it) {
       const int m0 = (tile / n_tiles) * (2 * kBlockM) + static_cast<int>(cta_rank) * kBlockM;
@@ -715,11 +751,16 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       const uint32_t aphase = (it >> 1) & 1;
       uint4 resv[kHasResidual ? kTileN / 16 : 1];
       prefetch_residual<kTileN, EPI>(args, m0, n0, M, quarter, col_half, lane, resv);
+      BiasShare<kTileN> bias;
+      if (EPI != BT_EPI_NONE) bias.load(args.bias, n0, col_half, lane);
       mbar_wait_anyway(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout);
       tc_fence_after();
+      __half* bias_s = bias_bufs + as * 256;
+      if (EPI != BT_EPI_NONE) bias.put(bias_s, col_half, lane);
       if (warp == 2 && lane == 0) gstamp(args.timing, it, 2);
       epilogue_tile<kTileN, EPI, true, Cfg::kStagingBufs>(args, &tm_out, stg, tmem_base + as * kTileN, m0, n0, M,
-                                                          quarter, col_half, lane, resv);
+                                                          quarter, col_half, lane, resv,
+                                                          reinterpret_cast<const uint4*>(bias_s));
       if (warp == 2 && lane == 0) gstamp(args.timing, it, 3);
       tc_fence_before();
       __syncwarp();
@@ -1529,12 +1570,12 @@ cudaError_t launch_pair_epi(const GemmLaunch& g, const GemmArgs& a, cudaStream_t
 }
 
 struct LnGemmCfg {
-  static constexpr int kSmemBytes = GemmCfg<256>::kSmemBytes + 1536;  // + bias / gamma / beta slices of a tile
+  static constexpr int kSmemBytes = GemmCfg<256>::kSmemBytes - kBiasBytes + 1536;  // + bias / gamma / beta slices of a tile
 };
 static_assert(LnGemmCfg::kSmemBytes <= 227 * 1024, "shared memory of the GEMM + LayerNorm kernel");
 
 struct PairLnGemmCfg {
-  static constexpr int kSmemBytes = PairCfg::kSmemBytes + 1536;
+  static constexpr int kSmemBytes = PairCfg::kSmemBytes - kBiasBytes + 1536;
 };
 static_assert(PairLnGemmCfg::kSmemBytes <= 227 * 1024, "shared memory of the pair GEMM + LayerNorm kernel");
 int g_pair_ln_clusters[64] = {};
