@@ -76,6 +76,8 @@ cudaError_t launch_restore_rows(const __half* packed, __half* padded, const int*
 // ---- GEMM ---------------------------------------------------------------------
 // Epilogue of the split-K form of BT_EPI_BIAS_RESIDUAL_F32OUT (internal: chosen through GemmLaunch::split_k).
 constexpr int kEpiSplitKF32 = 64;
+// BT_EPI_BIAS_GELU with GemmLaunch::gelu_kind == BT_GELU_TANH, inside the GEMM kernels
+constexpr int kEpiBiasGeluTanh = 65;
 // Ranges to cut K into for an fp32-sum GEMM of `m_rows` x N over K; 1 = no split.
 int gemm_pick_split_k(int m_rows, int N, int K, int num_sms);
 struct GemmLaunch {
