@@ -342,10 +342,10 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
       : "memory");
 }
 
-// tcgen05.ld 32x32b.x32 into elements [B, B + 32) of a 128-element register array (no address of the array
+// tcgen05.ld 32x32b.x32 into elements [B, B + 32) of a longer register array (no address of the array
 // is formed, so it stays in registers).
-template <int B>
-__device__ __forceinline__ void tmem_ld_32x32_at(uint32_t taddr, uint32_t (&r)[128]) {
+template <int B, int N>
+__device__ __forceinline__ void tmem_ld_32x32_at(uint32_t taddr, uint32_t (&r)[N]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -464,6 +464,17 @@ __device__ __forceinline__ void gelu_erf_fast_pair(float& x0, float& x1) {
   asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(m0) : "f"(x0));
   asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(m1) : "f"(x1));
   unpack_f32x2(fma_f32x2(n, pack_f32x2(e0, e1), pack_f32x2(m0, m1)), x0, x1);
+}
+// a += low half of h, b += high half: mixed-precision additions (one instruction each, no conversion first).
+__device__ __forceinline__ void add_half2(float& a, float& b, uint32_t h) {
+  asm("{\n\t"
+      ".reg .f16 lo, hi;\n\t"
+      "mov.b32 {lo, hi}, %2;\n\t"
+      "add.f32.f16 %0, lo, %0;\n\t"
+      "add.f32.f16 %1, hi, %1;\n\t"
+      "}"
+      : "+f"(a), "+f"(b)
+      : "r"(h));
 }
 __device__ __forceinline__ float gelu_tanh(float x) {
   // 0.5 x (1 + tanh( sqrt(2/pi) (x + 0.044715 x^3) ))

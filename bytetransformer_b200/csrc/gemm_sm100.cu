@@ -784,28 +784,31 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 
 // ------------------------------------------------------------------------------------------
 // GEMM + bias + residual + LayerNorm in one kernel:  y = LN(A*W + bias + residual)*gamma + beta.
-// Same tiles, schedule and main loop as gemm_f16_kernel<256, .>: tile t = (row tile t / C,
-// column tile t % C), C = N/256, tiles round-robin over the CTAs, so the C column tiles of a
-// row tile are worked on by C neighbouring CTAs at about the same time.  The fp32 sums stay
-// in tensor memory; the pre-normalisation tensor never goes to HBM.  Every epilogue thread
-// owns one row and 128 of its columns:
-//   1. v = accumulator + bias + residual, written back to tensor memory, with the sum and
-//      sum of squares of v - s (s = the thread's first value: shifted one-pass statistics);
-//   2. the partial (mean_i, M2_i) goes to a global scratch (it stays in L2) as two 64-bit
-//      words, side by side with those of the slab's other rows, each (value bits << 32 | epoch of this launch): an aligned 64-bit store is
-//      single-copy atomic, so the tag validates the value and no fence or counter is needed;
-//   3. the thread polls (bounded) the 2 * 2*C words of its row until all carry the epoch and
-//      merges the 2*C partials (equal counts):
-//         mean = avg(mean_i),  M2 = sum(M2_i) + 128 * sum((mean_i - mean)^2);
-//   4. second read of tensor memory: normalise, gamma / beta, fp16, staging, TMA store.
+// Main loop as in gemm_f16_kernel: tile t = (row tile t / C, column tile t % C), C = N / tile width, tiles round-robin over
+// the CTAs, so the C column tiles of a row tile are worked on by C neighbouring CTAs at about the same time.  The
+// pre-normalisation tensor never goes to HBM.  An epilogue warp owns 32 rows and 64 columns of the tile (16 warps for 256
+// columns, 12 for 192), a thread one row's 64 values, which stay in its registers from the first touch to the last (20 warps
+// leave 96 registers a thread, which is why two warps of their own deal with the statistics):
+//   1. v = accumulator + bias + residual, with the sum and sum of squares of v - s (s = the thread's first value: shifted
+//      one-pass statistics).  The accumulator goes back to the MMA warp as soon as it has been read;
+//   2. its (mean_i, M2_i) goes to shared memory, where one of two statistics warps merges the row's column groups;
+//   3. that warp publishes the tile's (mean_i, M2_i) to a global scratch (it stays in L2) as two 64-bit
+//      words, side by side with those of the slab's other rows, each (value bits << 32 | epoch of this launch): an aligned
+//      64-bit store is single-copy atomic, so the tag validates the value and no fence or counter is needed.  It polls
+//      (bounded) the 2*C words of the row until all carry the epoch, merges the C partials (equal counts n)
+//         mean = avg(mean_i),  M2 = sum(M2_i) + n * sum((mean_i - mean)^2)
+//      and hands mean and 1 / deviation to the row's threads;
+//   4. normalise, gamma / beta, fp16, staging, TMA store.
+// us per launch of 4,100 rows x 768 columns: with 128 values per thread (8 warps), written back to tensor memory for step 4,
+// K = 768 / 3072 14.4 / 26.2; so LN_768 / LN_3072.
 // Accumulators are double buffered, so 1-4 of a tile overlap the main loop of the CTA's next
 // tile.  A CTA only ever waits for the C CTAs working on the same row tile, and those wait for
 // nothing but that row tile in turn, so the waits are never circular.  Progress does need those
-// C = N/256 neighbouring CTAs to be resident together: the grid never exceeds the SM count and a CTA
+// C neighbouring CTAs to be resident together: the grid never exceeds the SM count and a CTA
 // takes a whole SM, so they are as soon as the kernels before have left; should something else hold
 // SMs for long (another process, a hung kernel on another stream), the wait, bounded like every
 // other wait of the library, gives up and reports kStatusGemmEpilogueTimeout instead of spinning.
-// The scratch (16 * N/128 bytes per row) must not hold this launch's epoch in the low half of any
+// The scratch (16 * C bytes per row) must not hold this launch's epoch in the low half of any
 // word beforehand: the caller zeroes it once and numbers the launches that share it 1, 2, 3, ...
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ void st_relaxed_gpu_2u64(unsigned long long* p, unsigned long long v0, unsigned long long v1) {
@@ -815,323 +818,358 @@ __device__ __forceinline__ void ld_relaxed_gpu_2u64(const unsigned long long* p,
                                                     unsigned long long& v1) {
   asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v0), "=l"(v1) : "l"(p) : "memory");
 }
-// The epilogue warps' loop of the GEMM + LayerNorm kernels (one-CTA and pair form share it): steps 1-4
+// Tile width of the one-CTA GEMM + LayerNorm kernel for this many row tiles on `ctas` CTAs: 192 columns where they take
+// less time than 256, counted in waves of tiles (three quarters as long each).
+__host__ __device__ __forceinline__ int ln_tile_n(int m_tiles, int N, int ctas) {
+  if (N % 192 != 0) return 256;
+  const int waves192 = (m_tiles * (N / 192) + ctas - 1) / ctas, waves256 = (m_tiles * (N / 256) + ctas - 1) / ctas;
+  return 3 * waves192 < 4 * waves256 ? 192 : 256;
+}
+
+constexpr int kLnEpiWarps = 16;
+constexpr int kLnFirstEpiWarp = 4;      // warps 0 and 1 load and multiply, 2 and 3 exchange the statistics
+constexpr int kLnThreads = 32 * (kLnFirstEpiWarp + kLnEpiWarps);
+constexpr int kLnBarBytes = 384;          // barriers and slots
+constexpr int kLnVecBytes = 256 * (4 + 4 + 2);  // gamma | beta | bias of a tile's columns: fp32, fp32, fp16
+constexpr int kLnMaxParts = 5;            // column tiles of a row: N <= 1024, tiles of 192 columns or more
+
+// Barriers between the epilogue warps and the two statistics warps.
+struct LnBars {
+  uint64_t* acc_full;   // [2]
+  uint64_t* vec_full;   // bias / gamma / beta of the tile's columns are in shared memory
+  uint64_t* vec_empty;  // all epilogue warps are done with them
+  uint64_t* part;       // [4] all column groups' partials of a quarter's rows are in the staging buffers
+  uint64_t* stat;       // [4] mean and 1 / deviation of a quarter's rows are there
+  uint64_t* res;        // [kLnEpiWarps] a warp's residual rows have landed in its staging buffer
+};
+__device__ __forceinline__ LnBars ln_bars_at(uint64_t* acc_full) {
+  return LnBars{acc_full, acc_full + 4, acc_full + 5, acc_full + 6, acc_full + 10, acc_full + 14};
+}
+template <int TILE_N>
+__device__ __forceinline__ void init_ln_bars(const LnBars& b) {
+  constexpr int kGroups = TILE_N / 64;
+  mbar_init(b.vec_full, 1);
+  mbar_init(b.vec_empty, 4 * kGroups);
+  for (int q = 0; q < 4; ++q) {
+    mbar_init(&b.part[q], kGroups);
+    mbar_init(&b.stat[q], 1);
+  }
+  for (int w = 0; w < kLnEpiWarps; ++w) mbar_init(&b.res[w], 1);
+}
+// Where a row's partial and then its mean and 1 / deviation lie in a warp's staging buffer, between the reads of the
+// residual and the writes of the output (a 16-byte unit that differs from row to row: four lanes to a bank).
+__device__ __forceinline__ float2* ln_row_slot(uint8_t* stg, int lane) {
+  return reinterpret_cast<float2*>(stg + lane * 128 + ((lane & 7) << 4));
+}
+
+// The epilogue warps' loop of the GEMM + LayerNorm kernels (one-CTA and pair form share it): steps 1, 2 and 4
 // of the description above for every tile that `tile_at(it, m0, n0)` yields (m0 = first of this CTA's 128
-// rows, n0 = first of the tile's 256 columns); `release_acc(as)` hands accumulator buffer `as` back to the
-// MMA issuer.  `stg_base`: 8 staging buffers of 4 KB; `res_bar`: 8 barriers, one per epilogue warp.
-template <class TileAt, class ReleaseAcc>
+// rows, n0 = first of the tile's columns); `release_acc(as)` hands accumulator buffer `as` back to the
+// MMA issuer.  `stg_base`: a staging buffer of 4 KB per warp.
+template <int TILE_N, class TileAt, class ReleaseAcc>
 __device__ __forceinline__ void ln_epilogue_loop(const GemmArgs& args, const CUtensorMap* tm_out,
-                                                 const CUtensorMap* tm_res, uint8_t* stg_base, uint64_t* acc_full,
-                                                 uint64_t* vec_full, uint64_t* vec_empty, uint64_t* res_bar,
-                                                 uint4* vec_s, volatile int* abort_flag, uint32_t tmem_base, int M,
-                                                 int n_tiles, int warp, int lane, TileAt tile_at,
-                                                 ReleaseAcc release_acc) {
-  constexpr int kTileN = 256;
-  constexpr int kColsPerThread = kTileN / 2;  // 128
-  const int e = warp - 2;
+                                                 const CUtensorMap* tm_res, uint8_t* stg_base, const LnBars& bars,
+                                                 const float* vec_s, volatile int* abort_flag, uint32_t tmem_base, int M,
+                                                 int warp, int lane, TileAt tile_at, ReleaseAcc release_acc) {
+  constexpr int kCols = 64;  // columns per thread
+  const int e = warp - kLnFirstEpiWarp;
   const int quarter = warp & 3;
-  const int col_half = e >> 2;
+  const int cg = e >> 2;  // column group
+  if (cg >= TILE_N / kCols) return;
   uint8_t* stg = stg_base + e * kStagingBytesPerWarp;
-  const int parts = 2 * n_tiles;                        // partials per row
-  const float inv_n = 1.0f / static_cast<float>(args.N);
+  uint8_t* srow = stg + lane * 128;
   int m0 = 0, n0 = 0;
   for (int it = 0; tile_at(it, m0, n0); ++it) {
     const int as = it & 1;
     const uint32_t aphase = (it >> 1) & 1;
     const int row0 = m0 + quarter * 32;
-    const int row = row0 + lane;
-    const bool row_ok = row < M;
-    const int gcol0 = n0 + col_half * kColsPerThread;  // first of this thread's 128 columns
-    const int part = 2 * (n0 / kTileN) + col_half;
-    // The first epilogue warp brings the tile's bias / gamma / beta slices into shared memory (every
-    // thread re-reads them, and the residual loads below keep evicting them from L1).
-    if (e == 0) {
-      uint4 vb = __ldg(reinterpret_cast<const uint4*>(args.bias + n0) + lane);
-      uint4 vg = make_uint4(0u, 0u, 0u, 0u), vt = vg;
-      if (!args.gb_fp32) {
-        vg = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(args.gamma) + n0) + lane);
-        vt = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(args.beta) + n0) + lane);
-      }
-      mbar_wait_anyway(vec_empty, (it & 1u) ^ 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout);
-      vec_s[lane] = vb;
-      vec_s[32 + lane] = vg;
-      vec_s[64 + lane] = vt;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(vec_full);
-    }
-    // Residual rows of this warp (32 rows x 128 columns) come through its staging buffer in two
-    // TMA boxes of 64 columns: row-strided 16-byte loads from the threads would cost one L1 tag
-    // look-up per lane and load (4096 per tile), which alone took longer than the main loop.
-    // The first box is requested now, the second when the first has been read.
+    const int gcol0 = n0 + cg * kCols;  // first of this thread's columns
+    // Residual rows of this warp (32 rows x 64 columns) come through its staging buffer by TMA: row-strided 16-byte
+    // loads from the threads would cost one L1 tag look-up per lane and load (4096 per tile), which alone took longer
+    // than the main loop.
     if (lane == 0) {
-      tma_store_wait_read_n<0>();  // the bulk stores of the previous tile have read the buffer
-      mbar_arrive_expect_tx(&res_bar[e], kStagingBytesPerWarp);
-      tma_load_2d(stg, tm_res, &res_bar[e], gcol0, row0);
+      tma_store_wait_read_n<0>();  // the bulk store of the previous tile has read the buffer
+      mbar_arrive_expect_tx(&bars.res[e], kStagingBytesPerWarp);
+      tma_load_2d(stg, tm_res, &bars.res[e], gcol0, row0);
     }
-    mbar_wait_anyway(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout);
+    mbar_wait_anyway(&bars.acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout);
     tc_fence_after();
-    mbar_wait_anyway(vec_full, it & 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout);
-    if (warp == 2 && lane == 0) gstamp(args.timing, it, 2);
-    const uint4* sbias = vec_s + col_half * (kColsPerThread / 8);
-    const uint4* sgamma = vec_s + 32 + col_half * (kColsPerThread / 8);
-    const uint4* sbeta = vec_s + 64 + col_half * (kColsPerThread / 8);
-    const uint32_t t_row = tmem_base + as * kTileN + (static_cast<uint32_t>(quarter * 32) << 16) +
-                           col_half * kColsPerThread;
-    // ---- 1. v = acc + bias + residual -> tensor memory; shifted sums
-    float sd = 0.f, sdd = 0.f, shift0 = 0.f;
-    unsigned long long sd2 = pack_f32x2(0.f, 0.f), sdd2 = sd2, nshift2 = sd2;
+    if (e == 0 && lane == 0) gstamp(args.timing, it, 2);
+    uint32_t v[64];
+    const uint32_t t_row = tmem_base + as * TILE_N + (static_cast<uint32_t>(quarter * 32) << 16) + cg * kCols;
+    tmem_ld_32x32_at<0>(t_row, v);
+    tmem_ld_32x32_at<32>(t_row + 32, v);
+    mbar_wait_anyway(bars.vec_full, it & 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout);
+    mbar_wait_anyway(&bars.res[e], it & 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout);
+    tmem_ld_wait();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) release_acc(as);
+    // ---- 1. v = acc + bias + residual; shifted sums
+    const uint4* sbias = reinterpret_cast<const uint4*>(vec_s + 512) + cg * (kCols / 8);
     {
-      uint32_t raw[2][32];
-      tmem_ld_32x32(t_row, raw[0]);
+      float shift0 = 0.f;
+      unsigned long long sd2 = pack_f32x2(0.f, 0.f), sdd2 = sd2, nshift2 = sd2;
 #pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        // this thread's 64 residual values of box hh: row `lane` of the swizzled buffer
-        mbar_wait_anyway(&res_bar[e], (static_cast<uint32_t>(it) * 2u + hh) & 1u, abort_flag, args.status,
-                         kStatusGemmEpilogueTimeout);
-        uint4 rres[8];
+      for (int q = 0; q < kCols / 8; ++q) {
+        const uint4 r4 = *reinterpret_cast<const uint4*>(srow + ((q ^ (lane & 7)) << 4));
+        const uint4 b4 = sbias[q];
+        const uint32_t rh[4] = {r4.x, r4.y, r4.z, r4.w}, bh[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          rres[q] = *reinterpret_cast<const uint4*>(stg + lane * 128 + ((q ^ (lane & 7)) << 4));
-        if (hh == 0) {
-          fence_proxy_async_smem();  // the reads above precede the next bulk write into the buffer
-          __syncwarp();
-          if (lane == 0) {
-            mbar_arrive_expect_tx(&res_bar[e], kStagingBytesPerWarp);
-            tma_load_2d(stg, tm_res, &res_bar[e], gcol0 + 64, row0);
+        for (int j = 0; j < 4; ++j) {
+          const int i = q * 8 + 2 * j;
+          float v0 = __uint_as_float(v[i]), v1 = __uint_as_float(v[i + 1]);
+          add_half2(v0, v1, bh[j]);
+          add_half2(v0, v1, rh[j]);
+          if (i == 0) {
+            shift0 = v0;
+            nshift2 = pack_f32x2(-v0, -v0);
           }
-        }
-#pragma unroll
-        for (int cj = 0; cj < 2; ++cj) {
-          const int ci = hh * 2 + cj;
-          const int c = ci * 32;
-          tmem_ld_wait();
-          if (ci + 1 < kColsPerThread / 32) tmem_ld_32x32(t_row + c + 32, raw[(ci + 1) & 1]);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint4 b4 = sbias[c / 8 + q];
-            const __half2* bh = reinterpret_cast<const __half2*>(&b4);
-            const __half2* rh = reinterpret_cast<const __half2*>(&rres[cj * 4 + q]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float2 fb = __half22float2(bh[j]);
-              const float2 fr = __half22float2(rh[j]);
-              const unsigned long long br2 = add_f32x2(pack_f32x2(fb.x, fb.y), pack_f32x2(fr.x, fr.y));
-              const unsigned long long v2 = add_f32x2(
-                  pack_f32x2(__uint_as_float(raw[ci & 1][q * 8 + 2 * j]), __uint_as_float(raw[ci & 1][q * 8 + 2 * j + 1])), br2);
-              float v0, v1;
-              unpack_f32x2(v2, v0, v1);
-              if (ci == 0 && q == 0 && j == 0) {
-                shift0 = v0;
-                nshift2 = pack_f32x2(-v0, -v0);
-              }
-              const unsigned long long d2 = add_f32x2(v2, nshift2);
-              sd2 = add_f32x2(sd2, d2);
-              sdd2 = fma_f32x2(d2, d2, sdd2);
-              raw[ci & 1][q * 8 + 2 * j] = __float_as_uint(v0);
-              raw[ci & 1][q * 8 + 2 * j + 1] = __float_as_uint(v1);
-            }
-          }
-          tmem_st_32x32(t_row + c, raw[ci & 1]);
+          const unsigned long long d2 = add_f32x2(pack_f32x2(v0, v1), nshift2);
+          sd2 = add_f32x2(sd2, d2);
+          sdd2 = fma_f32x2(d2, d2, sdd2);
+          v[i] = __float_as_uint(v0);
+          v[i + 1] = __float_as_uint(v1);
         }
       }
       float s0, s1, q0, q1;
       unpack_f32x2(sd2, s0, s1);
       unpack_f32x2(sdd2, q0, q1);
-      sd = s0 + s1;
-      sdd = q0 + q1;
+      const float sd = s0 + s1, sdd = q0 + q1;
+      // ---- 2. (the slot lies in residual columns that a lane reads itself, so no other lane waits for them)
+      *ln_row_slot(stg, lane) =
+          make_float2(shift0 + sd * (1.0f / kCols), fmaxf(sdd - sd * sd * (1.0f / kCols), 0.f));
     }
-    const float lmean = shift0 + sd * (1.0f / kColsPerThread);
-    const float m2 = fmaxf(sdd - sd * sd * (1.0f / kColsPerThread), 0.f);
-    if (warp == 2 && lane == 0) gstamp(args.timing, it, 4);
-    // ---- 2. publish the partial: two 64-bit words, each (value bits << 32 | epoch).  A naturally
-    // aligned 64-bit store is single-copy atomic, so a reader that finds this launch's epoch in a word
-    // also has its value: no fence, no counter, no second round trip.
-    const uint32_t epoch = args.ln_epoch;
-    // The words of a partial's 32 rows lie side by side, so that a warp writes or reads them with one
-    // instruction on four whole lines (the allocation's last slab may have fewer than 32 rows).
-    const int slab_rows = min(32, args.m_rows - row0);
-    unsigned long long* slab_words = reinterpret_cast<unsigned long long*>(args.out) + static_cast<size_t>(row0) * parts * 2;
-    if (row_ok)
-      st_relaxed_gpu_2u64(slab_words + (part * slab_rows + lane) * 2,
-                          (static_cast<unsigned long long>(__float_as_uint(lmean)) << 32) | epoch,
-                          (static_cast<unsigned long long>(__float_as_uint(m2)) << 32) | epoch);
-    if (warp == 2 && lane == 0) gstamp(args.timing, it, 5);
-    // ---- 3. wait until the row's 2 * parts words all carry this epoch (bounded), then merge.
-    // A partial's 32 rows are written by one store, so lane p probes partial p of the slab's first row (one load
-    // for the warp) and only when all are there does every lane read and validate its row; a lane whose words
-    // are not all there yet sends the warp round again.  us per launch of 18,944 rows x 768 columns, K = 768 / 3072:
-    // with the words row by row (12 loads over 32 lines each) and one lane probing its own row 59.0 / 91.4, so
-    // 50.7 / 87.9; the wait alone, all CTAs in step, 4.9k and 1.9k clocks.
-    float mean = 0.f, rstd = 0.f;
-    float pm[8], pq[8];  // N <= 1024: at most 8 partials per row
-    const long long t0 = clock64();
-    bool give_up = false;
-    while (true) {
-      {
-        uint32_t probes = 0;
-        while (true) {
-          uint32_t bad = 0;
-          if (lane < parts && row0 < M) {
-            unsigned long long w0, w1;
-            ld_relaxed_gpu_2u64(slab_words + lane * slab_rows * 2, w0, w1);
-            bad = (static_cast<uint32_t>(w0) ^ epoch) | (static_cast<uint32_t>(w1) ^ epoch);
-          }
-          if (__all_sync(0xffffffffu, bad == 0)) break;
-          if ((++probes & 15u) == 0u && __any_sync(0xffffffffu, *abort_flag != 0 || clock64() - t0 > (1ll << 31))) break;
-        }
-      }
-      uint32_t bad = 0;
-      if (row_ok) {
-        // all loads are issued before any tag is looked at: one round trip
-#pragma unroll
-        for (int p = 0; p < 8; ++p)
-          if (p < parts) {
-            unsigned long long w0, w1;
-            ld_relaxed_gpu_2u64(slab_words + (p * slab_rows + lane) * 2, w0, w1);
-            bad |= (static_cast<uint32_t>(w0) ^ epoch) | (static_cast<uint32_t>(w1) ^ epoch);
-            pm[p] = __uint_as_float(static_cast<uint32_t>(w0 >> 32));
-            pq[p] = __uint_as_float(static_cast<uint32_t>(w1 >> 32));
-          }
-      }
-      if (__all_sync(0xffffffffu, bad == 0)) break;
-      if (__any_sync(0xffffffffu, *abort_flag != 0 || clock64() - t0 > (1ll << 31))) {
-        give_up = true;
-        break;
-      }
-      __nanosleep(100);
-    }
-    if (give_up) {
-      if (lane == 0) {
-        *abort_flag = 1;
-        if (args.status != nullptr) atomicCAS(args.status, 0, kStatusGemmEpilogueTimeout);
-      }
-      break;
-    }
-    if (row_ok) {
-#pragma unroll
-      for (int p = 0; p < 8; ++p)
-        if (p < parts) mean += pm[p];
-      mean *= 1.0f / static_cast<float>(parts);
-      float M2 = 0.f;
-#pragma unroll
-      for (int p = 0; p < 8; ++p)
-        if (p < parts) {
-          const float d = pm[p] - mean;
-          M2 += pq[p] + static_cast<float>(kColsPerThread) * d * d;
-        }
-      rstd = rsqrtf(M2 * inv_n + args.eps);
-    }
-    if (warp == 2 && lane == 0) gstamp(args.timing, it, 6);
-    const float shift = -mean * rstd;
-    const unsigned long long rstd2 = pack_f32x2(rstd, rstd), shift2 = pack_f32x2(shift, shift);
-    tmem_st_wait();  // the write-back of step 1 is complete before tensor memory is read again
-    // ---- 4. normalise, gamma / beta, fp16, store (64 columns = 128 B per row at a time)
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bars.part[quarter]);
+    if (e == 0 && lane == 0) gstamp(args.timing, it, 4);
+    mbar_wait_anyway(&bars.stat[quarter], it & 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout);
+    const float2 stat = *ln_row_slot(stg, lane);
+    if (e == 0 && lane == 0) gstamp(args.timing, it, 6);
+    const float shift = -stat.x * stat.y;
+    const unsigned long long rstd2 = pack_f32x2(stat.y, stat.y), shift2 = pack_f32x2(shift, shift);
+    // ---- 4. normalise, gamma / beta, fp16, store (64 columns = 128 B per row)
+    const float4* sgamma = reinterpret_cast<const float4*>(vec_s + cg * kCols);
+    const float4* sbeta = reinterpret_cast<const float4*>(vec_s + 256 + cg * kCols);
     const bool slab_full = row0 + 32 <= M;
-    {
-      uint32_t raw[2][32];
-      tmem_ld_32x32(t_row, raw[0]);
 #pragma unroll
-      for (int ci = 0; ci < kColsPerThread / 32; ++ci) {
-        const int c = ci * 32;
-        const int hh = ci & 1;  // which half of the current 64-column store chunk
-        uint8_t* srow = stg + lane * 128;
-        if (hh == 0 && slab_full) {
-          if (lane == 0) tma_store_wait_read_n<0>();  // the previous bulk store has read the staging rows
-          __syncwarp();
-        }
-        tmem_ld_wait();
-        if (ci + 1 < kColsPerThread / 32) tmem_ld_32x32(t_row + c + 32, raw[(ci + 1) & 1]);
+    for (int q = 0; q < kCols / 8; ++q) {
+      uint32_t u[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int col8 = gcol0 + c + q * 8;  // first of these 8 columns
-          float g[8], b[8];
-          if (args.gb_fp32) {
-            const float4 g0 = __ldg(reinterpret_cast<const float4*>(args.gamma) + (col8 >> 2));
-            const float4 g1 = __ldg(reinterpret_cast<const float4*>(args.gamma) + (col8 >> 2) + 1);
-            const float4 b0 = __ldg(reinterpret_cast<const float4*>(args.beta) + (col8 >> 2));
-            const float4 b1 = __ldg(reinterpret_cast<const float4*>(args.beta) + (col8 >> 2) + 1);
-            g[0] = g0.x; g[1] = g0.y; g[2] = g0.z; g[3] = g0.w; g[4] = g1.x; g[5] = g1.y; g[6] = g1.z; g[7] = g1.w;
-            b[0] = b0.x; b[1] = b0.y; b[2] = b0.z; b[3] = b0.w; b[4] = b1.x; b[5] = b1.y; b[6] = b1.z; b[7] = b1.w;
-          } else {
-            const uint4 g4 = sgamma[c / 8 + q];
-            const uint4 b4 = sbeta[c / 8 + q];
-            const __half2* gh = reinterpret_cast<const __half2*>(&g4);
-            const __half2* bh = reinterpret_cast<const __half2*>(&b4);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float2 fg = __half22float2(gh[j]);
-              const float2 fb = __half22float2(bh[j]);
-              g[2 * j] = fg.x; g[2 * j + 1] = fg.y;
-              b[2 * j] = fb.x; b[2 * j + 1] = fb.y;
-            }
-          }
-          float y[8];
-#pragma unroll
-          for (int i = 0; i < 8; i += 2) {
-            const unsigned long long n2 = fma_f32x2(
-                pack_f32x2(__uint_as_float(raw[ci & 1][q * 8 + i]), __uint_as_float(raw[ci & 1][q * 8 + i + 1])), rstd2, shift2);
-            unpack_f32x2(fma_f32x2(n2, pack_f32x2(g[i], g[i + 1]), pack_f32x2(b[i], b[i + 1])), y[i], y[i + 1]);
-          }
-          uint4 u;
-          u.x = pack_half2(y[0], y[1]);
-          u.y = pack_half2(y[2], y[3]);
-          u.z = pack_half2(y[4], y[5]);
-          u.w = pack_half2(y[6], y[7]);
-          const int unit = hh * 4 + q;  // 16-byte unit inside the 128-byte row
-          if (slab_full)
-            *reinterpret_cast<uint4*>(srow + ((unit ^ (lane & 7)) << 4)) = u;
-          else if (row_ok)
-            *reinterpret_cast<uint4*>(args.out_ln + static_cast<size_t>(row) * args.N + col8) = u;
-        }
-        if (hh == 1 && slab_full) {
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            tma_store_2d(tm_out, stg, gcol0 + c - 32, row0);
-            tma_store_commit();
-          }
-        }
+      for (int j = 0; j < 4; ++j) {
+        const int i = q * 8 + 2 * j;
+        const float4 g4 = sgamma[2 * q + (j >> 1)], b4 = sbeta[2 * q + (j >> 1)];
+        const unsigned long long n2 =
+            fma_f32x2(pack_f32x2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), rstd2, shift2);
+        float y0, y1;
+        unpack_f32x2(fma_f32x2(n2, (j & 1) ? pack_f32x2(g4.z, g4.w) : pack_f32x2(g4.x, g4.y),
+                               (j & 1) ? pack_f32x2(b4.z, b4.w) : pack_f32x2(b4.x, b4.y)), y0, y1);
+        u[j] = pack_half2(y0, y1);
       }
+      *reinterpret_cast<uint4*>(srow + ((q ^ (lane & 7)) << 4)) = make_uint4(u[0], u[1], u[2], u[3]);
     }
-    if (warp == 2 && lane == 0) gstamp(args.timing, it, 3);
-    tc_fence_before();
+    if (!slab_full && row0 + lane < M) {  // (each lane its own row)
+      __half* op = args.out_ln + static_cast<size_t>(row0 + lane) * args.N + gcol0;
+#pragma unroll 1
+      for (int q = 0; q < kCols / 8; ++q)
+        reinterpret_cast<uint4*>(op)[q] = *reinterpret_cast<const uint4*>(srow + ((q ^ (lane & 7)) << 4));
+    }
+    // (the fence also puts this tile's accesses to the staging rows before the next tile's bulk write into them)
+    fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) {
-      release_acc(as);
-      mbar_arrive(vec_empty);
+      if (slab_full) {
+        tma_store_2d(tm_out, stg, gcol0, row0);
+        tma_store_commit();
+      }
+      mbar_arrive(bars.vec_empty);
     }
+    if (e == 0 && lane == 0) gstamp(args.timing, it, 3);
   }
   if (lane == 0) tma_store_wait_all();
 }
 
-__global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
-                   const __grid_constant__ CUtensorMap tm_out, const __grid_constant__ CUtensorMap tm_res,
-                   const GemmArgs args) {
-  constexpr int kTileN = 256;
-  using Cfg = GemmCfg<kTileN>;
-  constexpr int kStages = Cfg::kStages;
+__device__ __forceinline__ void load8(float (&f)[8], const __half* p) {
+  const uint4 h = __ldg(reinterpret_cast<const uint4*>(p));
+  const __half2* hh = reinterpret_cast<const __half2*>(&h);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 t = __half22float2(hh[j]);
+    f[2 * j] = t.x;
+    f[2 * j + 1] = t.y;
+  }
+}
+__device__ __forceinline__ void load8(float (&f)[8], const float* p) {
+  const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
+  f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * Cfg::kStageBytes + Cfg::kStagingBytes);
+// The statistics warps' loop (`half` 0 or 1: quarters 2 * half and 2 * half + 1, a lane has one row of each): step 3.  The
+// first of them also brings the tile's bias / gamma / beta slices into shared memory.
+template <int TILE_N, class TileAt>
+__device__ __forceinline__ void ln_statistics_loop(const GemmArgs& args, uint8_t* stg_base, const LnBars& bars, float* vec_s,
+                                                   volatile int* abort_flag, int M, int n_tiles, int half, int lane,
+                                                   TileAt tile_at) {
+  constexpr int kGroups = TILE_N / 64;
+  const float inv_n = 1.0f / static_cast<float>(args.N);
+  const float inv_tiles = 1.0f / static_cast<float>(n_tiles);
+  const uint32_t epoch = args.ln_epoch;
+  int m0 = 0, n0 = 0;
+  for (int it = 0; tile_at(it, m0, n0); ++it) {
+    if (half == 0) {
+      float vec[2][8] = {};
+      uint4 bias = make_uint4(0u, 0u, 0u, 0u);
+      if (lane < TILE_N / 8) {
+        const size_t at = n0 + lane * 8;
+        bias = __ldg(reinterpret_cast<const uint4*>(args.bias + at));
+        if (args.gb_fp32) {
+          load8(vec[0], reinterpret_cast<const float*>(args.gamma) + at);
+          load8(vec[1], reinterpret_cast<const float*>(args.beta) + at);
+        } else {
+          load8(vec[0], reinterpret_cast<const __half*>(args.gamma) + at);
+          load8(vec[1], reinterpret_cast<const __half*>(args.beta) + at);
+        }
+      }
+      mbar_wait_anyway(bars.vec_empty, (it & 1u) ^ 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        float4* dst = reinterpret_cast<float4*>(vec_s + k * 256 + lane * 8);
+        dst[0] = make_float4(vec[k][0], vec[k][1], vec[k][2], vec[k][3]);
+        dst[1] = make_float4(vec[k][4], vec[k][5], vec[k][6], vec[k][7]);
+      }
+      reinterpret_cast<uint4*>(vec_s + 512)[lane] = bias;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bars.vec_full);
+    }
+    // The words of a partial's 32 rows lie side by side, so that a warp writes or reads them with one
+    // instruction on four whole lines (the allocation's last slab may have fewer than 32 rows).
+    unsigned long long* words[2];
+    int slab_rows[2];
+    bool row_ok[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int quarter = 2 * half + k;
+      const int row0 = m0 + quarter * 32;
+      slab_rows[k] = min(32, args.m_rows - row0);
+      words[k] = reinterpret_cast<unsigned long long*>(args.out) + static_cast<size_t>(row0) * n_tiles * 2;
+      row_ok[k] = row0 + lane < M;
+      mbar_wait_anyway(&bars.part[quarter], it & 1u, abort_flag, args.status, kStatusGemmEpilogueTimeout);
+      float gm[kGroups], gq[kGroups], mean = 0.f, m2 = 0.f;
+#pragma unroll
+      for (int g = 0; g < kGroups; ++g) {
+        // (quarter q is that of the warps 4 g + q from kLnFirstEpiWarp, a multiple of four, on)
+        const float2 f = *ln_row_slot(stg_base + (g * 4 + quarter) * kStagingBytesPerWarp, lane);
+        gm[g] = f.x;
+        gq[g] = f.y;
+        mean += f.x;
+      }
+      mean *= 1.0f / kGroups;
+#pragma unroll
+      for (int g = 0; g < kGroups; ++g) {
+        const float d = gm[g] - mean;
+        m2 += gq[g] + 64.0f * d * d;
+      }
+      // A naturally aligned 64-bit store is single-copy atomic, so a reader that finds this launch's epoch in a word
+      // also has its value: no fence, no counter, no second round trip.
+      if (row_ok[k])
+        st_relaxed_gpu_2u64(words[k] + ((n0 / TILE_N) * slab_rows[k] + lane) * 2,
+                            (static_cast<unsigned long long>(__float_as_uint(mean)) << 32) | epoch,
+                            (static_cast<unsigned long long>(__float_as_uint(m2)) << 32) | epoch);
+    }
+    if (half == 0 && lane == 0) gstamp(args.timing, it, 5);
+    // Wait until the rows' 2 * n_tiles words all carry this epoch (bounded), then merge.
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int quarter = 2 * half + k;
+      float pm[kLnMaxParts], pq[kLnMaxParts];
+      const long long t0 = clock64();
+      uint32_t probes = 0;
+      while (true) {
+        uint32_t bad = 0;
+        if (row_ok[k]) {
+          // all loads are issued before any tag is looked at: one round trip
+#pragma unroll
+          for (int p = 0; p < kLnMaxParts; ++p)
+            if (p < n_tiles) {
+              unsigned long long w0, w1;
+              ld_relaxed_gpu_2u64(words[k] + (p * slab_rows[k] + lane) * 2, w0, w1);
+              bad |= (static_cast<uint32_t>(w0) ^ epoch) | (static_cast<uint32_t>(w1) ^ epoch);
+              pm[p] = __uint_as_float(static_cast<uint32_t>(w0 >> 32));
+              pq[p] = __uint_as_float(static_cast<uint32_t>(w1 >> 32));
+            }
+        }
+        if (__all_sync(0xffffffffu, bad == 0)) break;
+        if ((++probes & 15u) == 0u && __any_sync(0xffffffffu, *abort_flag != 0 || clock64() - t0 > (1ll << 31))) {
+          if (lane == 0) {
+            *abort_flag = 1;
+            if (args.status != nullptr) atomicCAS(args.status, 0, kStatusGemmEpilogueTimeout);
+          }
+          break;
+        }
+      }
+      float mean = 0.f, rstd = 0.f;
+      if (row_ok[k]) {
+#pragma unroll
+        for (int p = 0; p < kLnMaxParts; ++p)
+          if (p < n_tiles) mean += pm[p];
+        mean *= inv_tiles;
+        float M2 = 0.f;
+#pragma unroll
+        for (int p = 0; p < kLnMaxParts; ++p)
+          if (p < n_tiles) {
+            const float d = pm[p] - mean;
+            M2 += pq[p] + static_cast<float>(TILE_N) * d * d;
+          }
+        rstd = rsqrtf(M2 * inv_n + args.eps);
+      }
+#pragma unroll
+      for (int g = 0; g < kGroups; ++g)
+        *ln_row_slot(stg_base + (g * 4 + quarter) * kStagingBytesPerWarp, lane) = make_float2(mean, rstd);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars.stat[quarter]);
+    }
+  }
+}
+
+// The rows that are there; none where shared memory does not start on the 1,024 bytes that the 128-byte swizzle needs
+// (there is no room to round up in the pair form).
+__device__ __forceinline__ int ln_rows(const GemmArgs& args, const uint8_t* smem) {
+  int M = args.m_rows;
+  if (args.m_dev != nullptr) {
+    const int md = __ldg(args.m_dev);
+    M = md < M ? md : M;
+  }
+  if ((smem_u32(smem) & 1023u) != 0u) {
+    if (threadIdx.x == 0 && args.status != nullptr) atomicCAS(args.status, 0, kStatusGemmProducerTimeout + 0x10);
+    M = 0;
+  }
+  return uniform_int(M);
+}
+
+template <int TILE_N>
+struct LnCfg {
+  static constexpr int kStageBytes = kABytes + TILE_N * kBlockK * 2;
+  static constexpr int kStages = TILE_N == 256 ? 3 : 4;
+  static constexpr int kStagingBytes = (TILE_N / 64) * 4 * kStagingBytesPerWarp;
+  static constexpr int kRingAndStaging = kStages * kStageBytes + kStagingBytes;
+};
+constexpr int kLnRingAndStaging =
+    LnCfg<256>::kRingAndStaging > LnCfg<192>::kRingAndStaging ? LnCfg<256>::kRingAndStaging : LnCfg<192>::kRingAndStaging;
+
+// One width of gemm_f16_ln_kernel, from the barriers on.  `M` valid rows.
+template <int TILE_N>
+__device__ __forceinline__ void ln_gemm_body(const CUtensorMap* tm_a, const CUtensorMap* tm_b, const CUtensorMap* tm_out,
+                                             const CUtensorMap* tm_res, const GemmArgs& args, uint8_t* smem,
+                                             uint64_t* bars, float* vec_s, uint32_t* tmem_slot,
+                                             volatile int* abort_flag, int M, int warp, int lane) {
+  using Cfg = LnCfg<TILE_N>;
+  constexpr int kStages = Cfg::kStages;
   uint64_t* full_bar = bars;                    // [kStages]
   uint64_t* empty_bar = bars + kStages;         // [kStages]
   uint64_t* acc_full = bars + 2 * kStages;      // [2]
   uint64_t* acc_empty = bars + 2 * kStages + 2; // [2]
-  uint64_t* vec_full = bars + 2 * kStages + 4;   // bias / gamma / beta of the tile's columns are in shared memory
-  uint64_t* vec_empty = bars + 2 * kStages + 5;  // all epilogue warps are done with them
-  uint64_t* res_bar = bars + 2 * kStages + 6;    // [kEpiWarps] a warp's residual rows have landed in its staging buffer
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 6 + kEpiWarps);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  // fp16 vectors of the current tile's 256 columns: bias | gamma | beta (gamma / beta only when they are fp16)
-  uint4* vec_s = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(bars) + 256);
-
-  const int warp = uniform_int(static_cast<int>(threadIdx.x >> 5));  // warp-uniform roles: see common.cuh
-  const int lane = threadIdx.x & 31;
-
-  pdl_launch_dependents();
-
+  const LnBars ln_bars = ln_bars_at(acc_full);
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full_bar[s], 1);
@@ -1139,68 +1177,51 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&acc_full[s], 1);
-      mbar_init(&acc_empty[s], kEpiWarps);
+      mbar_init(&acc_empty[s], 4 * (TILE_N / 64));
     }
-    mbar_init(vec_full, 1);
-    mbar_init(vec_empty, kEpiWarps);
-    for (int w = 0; w < kEpiWarps; ++w) mbar_init(&res_bar[w], 1);
-    *abort_flag = 0;
+    init_ln_bars<TILE_N>(ln_bars);
     fence_mbar_init();
-  }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, Cfg::kTmemCols);
-    tmem_relinquish();
-  }
-  if (warp == 0 && lane == 0) {
-    tma_prefetch_desc(&tm_a);
-    tma_prefetch_desc(&tm_b);
-    tma_prefetch_desc(&tm_out);
-    tma_prefetch_desc(&tm_res);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = uniform_u32(*tmem_slot);
 
-  const int n_tiles = args.N / kTileN;
+  const int n_tiles = args.N / TILE_N;
   const int num_kb = args.K / kBlockK;
-  // The leading W blocks of the first tile ahead of the dependency wait, its A blocks right behind it (see
-  // gemm_f16_kernel).
-  const int pre_kb = args.early_w ? (num_kb < kStages ? num_kb : kStages) : 0;
-  auto load_w = [&](int stage, int n0, int kb) {
-    uint8_t* sb = smem + stage * Cfg::kStageBytes + kABytes;
-#pragma unroll
-    for (int c = 0; c < kTileN / 64; ++c)
-      if (elect_one()) tma_load_2d(sb + c * (64 * kBlockK * 2), &tm_b, &full_bar[stage], n0 + c * 64, kb * kBlockK);
-  };
-  auto load_a = [&](int stage, int m0, int kb) {
-    if (elect_one()) tma_load_2d(smem + stage * Cfg::kStageBytes, &tm_a, &full_bar[stage], kb * kBlockK, m0);
-  };
-  const int first_m0 = (static_cast<int>(blockIdx.x) / n_tiles) * kBlockM;
-  if (warp == 0) {
-    for (int kb = 0; kb < pre_kb; ++kb) {
-      if (elect_one()) mbar_arrive_expect_tx(&full_bar[kb], Cfg::kStageBytes);
-      load_w(kb, (static_cast<int>(blockIdx.x) % n_tiles) * kTileN, kb);
-    }
-  }
-
-  pdl_wait();  // see gemm_f16_kernel
-  if (warp == 0)
-    for (int kb = 0; kb < pre_kb; ++kb) load_a(kb, first_m0, kb);
-  int M = args.m_rows;
-  if (args.m_dev != nullptr) {
-    const int md = __ldg(args.m_dev);
-    M = uniform_int(md < M ? md : M);
-  }
   const int m_tiles = (M + kBlockM - 1) / kBlockM;
   const int total_tiles = m_tiles * n_tiles;
   auto tile_at = [&](int li, int& m0, int& n0) -> bool {
     const int tile = static_cast<int>(blockIdx.x) + li * static_cast<int>(gridDim.x);
     if (tile >= total_tiles) return false;
     m0 = (tile / n_tiles) * kBlockM;
-    n0 = (tile % n_tiles) * kTileN;
+    n0 = (tile % n_tiles) * TILE_N;
     return true;
   };
+  // The leading W blocks of the first tile ahead of the dependency wait, its A blocks right behind it (see
+  // gemm_f16_kernel).
+  auto load_w = [&](int stage, int n0, int kb) {
+    uint8_t* sb = smem + stage * Cfg::kStageBytes + kABytes;
+#pragma unroll
+    for (int c = 0; c < TILE_N / 64; ++c)
+      if (elect_one()) tma_load_2d(sb + c * (64 * kBlockK * 2), tm_b, &full_bar[stage], n0 + c * 64, kb * kBlockK);
+  };
+  auto load_a = [&](int stage, int m0, int kb) {
+    if (elect_one()) tma_load_2d(smem + stage * Cfg::kStageBytes, tm_a, &full_bar[stage], kb * kBlockK, m0);
+  };
+  int pre_kb = 0;
+  if (warp == 0) {
+    int m0 = 0, n0 = 0;
+    if (tile_at(0, m0, n0)) {
+      if (args.early_w) pre_kb = num_kb < kStages ? num_kb : kStages;
+      for (int kb = 0; kb < pre_kb; ++kb) {
+        if (elect_one()) mbar_arrive_expect_tx(&full_bar[kb], Cfg::kStageBytes);
+        load_w(kb, n0, kb);
+      }
+    }
+  }
+
+  pdl_wait();  // see gemm_f16_kernel
 
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
@@ -1208,14 +1229,11 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     uint32_t phase = 0;
     bool ok = true;
     int m0 = 0, n0 = 0;
-    if (!tile_at(0, m0, n0)) {
-      // No tile for this CTA after all: wait for the armed stages, so that no copy is in flight at exit.
-      for (int kb = 0; kb < pre_kb; ++kb)
-        if (!mbar_wait_warp(&full_bar[kb], 0u, abort_flag, args.status, kStatusGemmProducerTimeout)) break;
-    }
     for (int li = 0; ok && tile_at(li, m0, n0); ++li) {
       for (int kb = 0; kb < num_kb; ++kb) {
-        if (li != 0 || kb >= pre_kb) {  // else armed and requested above (stage == kb)
+        if (li == 0 && kb < pre_kb) {  // armed above, its W block requested (stage == kb)
+          load_a(stage, m0, kb);
+        } else {
           if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, abort_flag, args.status, kStatusGemmProducerTimeout)) {
             ok = false;
             break;
@@ -1233,6 +1251,7 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   } else if (warp == 1) {
     // --------------------------------------------------------------- MMA issuer
     {
+      constexpr uint32_t kIdesc = make_idesc_f16(kBlockM, TILE_N, 0, 1);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true, landed = false;
@@ -1246,7 +1265,7 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         }
         tc_fence_after();
         if (lane == 0) gstamp(args.timing, it, 0);
-        const uint32_t d_tmem = tmem_base + as * kTileN;
+        const uint32_t d_tmem = tmem_base + as * TILE_N;
         for (int kb = 0; kb < num_kb; ++kb) {
           ok = mbar_wait_latched(ok, landed, &full_bar[stage], phase, abort_flag, args.status, kStatusGemmMmaTimeout);
           tc_fence_after();
@@ -1260,19 +1279,58 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
           landed = mbar_test_wait(&full_bar[stage], phase);  // the next block, ahead of these MMAs
           // (the commit frees the stage once these MMAs have retired)
           umma_k_block<false>(d_tmem, smem_desc(args.a_desc_hi, sa), smem_desc(args.b_desc_hi, sb), args.a_kstep_bytes >> 4,
-                       args.b_kstep_bytes >> 4, args.idesc, kb != 0 ? 1u : 0u, &empty_bar[cur]);
+                       args.b_kstep_bytes >> 4, kIdesc, kb != 0 ? 1u : 0u, &empty_bar[cur]);
         }
         ok = __all_sync(0xffffffffu, ok) != 0;
         if (ok && elect_one()) umma_commit(&acc_full[as]);
         if (lane == 0) gstamp(args.timing, it, 1);
       }
     }
+  } else if (warp < kLnFirstEpiWarp) {
+    // ------------------------------------------------------- row statistics
+    ln_statistics_loop<TILE_N>(args, smem + kStages * Cfg::kStageBytes, ln_bars, vec_s, abort_flag, M, n_tiles, warp - 2,
+                               lane, tile_at);
   } else {
     // ------------------------------------------------------------------ epilogue
-    ln_epilogue_loop(args, &tm_out, &tm_res, smem + kStages * Cfg::kStageBytes, acc_full, vec_full, vec_empty, res_bar,
-                     vec_s, abort_flag, tmem_base, M, n_tiles, warp, lane, tile_at,
-                     [&](int as) { mbar_arrive(&acc_empty[as]); });
+    ln_epilogue_loop<TILE_N>(args, tm_out, tm_res, smem + kStages * Cfg::kStageBytes, ln_bars, vec_s, abort_flag,
+                             tmem_base, M, warp, lane, tile_at, [&](int as) { mbar_arrive(&acc_empty[as]); });
   }
+}
+
+__global__ void __launch_bounds__(kLnThreads, 1)
+gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
+                   const __grid_constant__ CUtensorMap tm_out, const __grid_constant__ CUtensorMap tm_res,
+                   const GemmArgs args) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kLnRingAndStaging);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kLnRingAndStaging + kLnBarBytes - 16);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* vec_s = reinterpret_cast<float*>(smem + kLnRingAndStaging + kLnBarBytes);
+
+  const int warp = uniform_int(static_cast<int>(threadIdx.x >> 5));  // warp-uniform roles: see common.cuh
+  const int lane = threadIdx.x & 31;
+
+  pdl_launch_dependents();
+
+  // The row count is known ahead of the dependency wait (see common.cuh: inside a call this is never the second
+  // kernel), so the tile width can go by the rows that are there instead of those that are allocated.
+  const int M = ln_rows(args, smem);
+  if (threadIdx.x == 0) *abort_flag = 0;
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tm_a);
+    tma_prefetch_desc(&tm_b);
+    tma_prefetch_desc(&tm_out);
+    tma_prefetch_desc(&tm_res);
+  }
+  const int m_tiles = (M + kBlockM - 1) / kBlockM;
+  if (ln_tile_n(m_tiles, args.N, static_cast<int>(gridDim.x)) == 192)
+    ln_gemm_body<192>(&tm_a, &tm_b, &tm_out, &tm_res, args, smem, bars, vec_s, tmem_slot, abort_flag, M, warp, lane);
+  else
+    ln_gemm_body<256>(&tm_a, &tm_b, &tm_out, &tm_res, args, smem, bars, vec_s, tmem_slot, abort_flag, M, warp, lane);
 
   // ------------------------------------------------------------------ teardown
   __syncthreads();
@@ -1281,7 +1339,7 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   }
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    tmem_dealloc(uniform_u32(*tmem_slot), 512);
   }
 }
 
@@ -1293,30 +1351,33 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
 // Tiles go round-robin over the clusters (all resident: the launch asks for no more clusters than fit),
 // and a cluster only waits for clusters working on earlier or the same row tiles: no circular wait.
 // ------------------------------------------------------------------------------------------
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+struct PairLnCfg {
+  static constexpr int kTileN = 256;
+  static constexpr int kStageBytes = PairCfg::kStageBytes;
+  static constexpr int kStages = 5;  // (what 16 staging buffers leave room for)
+  static constexpr int kTmemCols = 512;
+  static constexpr int kStagingBytes = kLnEpiWarps * kStagingBytesPerWarp;
+};
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLnThreads, 1)
 gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                         const __grid_constant__ CUtensorMap tm_out, const __grid_constant__ CUtensorMap tm_res,
                         const GemmArgs args) {
-  using Cfg = PairCfg;
+  using Cfg = PairLnCfg;
   constexpr int kStages = Cfg::kStages;
   constexpr int kTileN = Cfg::kTileN;
 
-  extern __shared__ uint8_t smem_raw[];
-  // Both CTAs of the pair must use identical shared-memory offsets (the MMA and the multicast
-  // commit address the peer by offset); dynamic shared memory starts at the same offset in
-  // every CTA of a launch, so the same round-up applies to both.
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  // (both CTAs of a pair use the same shared-memory offsets: the MMA and the multicast commit address the peer by offset)
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * Cfg::kStageBytes + Cfg::kStagingBytes);
   uint64_t* full_bar = bars;                    // [kStages]  (leader's copy is the live one)
   uint64_t* empty_bar = bars + kStages;         // [kStages]
   uint64_t* acc_full = bars + 2 * kStages;      // [2]
   uint64_t* acc_empty = bars + 2 * kStages + 2; // [2]        (leader's copy is the live one)
-  uint64_t* vec_full = bars + 2 * kStages + 4;   // as in gemm_f16_ln_kernel
-  uint64_t* vec_empty = bars + 2 * kStages + 5;
-  uint64_t* res_bar = bars + 2 * kStages + 6;    // [kEpiWarps]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 6 + kEpiWarps);
+  const LnBars ln_bars = ln_bars_at(acc_full);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(bars) + kLnBarBytes - 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint4* vec_s = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(bars) + 256);
+  float* vec_s = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + kLnBarBytes);
 
   const int warp = uniform_int(static_cast<int>(threadIdx.x >> 5));  // warp-uniform roles: see common.cuh
   const int lane = threadIdx.x & 31;
@@ -1327,6 +1388,8 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
 
   pdl_launch_dependents();
 
+  const int M = ln_rows(args, smem);  // (ahead of the dependency wait, as in gemm_f16_ln_kernel)
+
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full_bar[s], 1);
@@ -1334,11 +1397,9 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&acc_full[s], 1);
-      mbar_init(&acc_empty[s], 2 * kEpiWarps);
+      mbar_init(&acc_empty[s], 2 * kLnEpiWarps);
     }
-    mbar_init(vec_full, 1);
-    mbar_init(vec_empty, kEpiWarps);
-    for (int w = 0; w < kEpiWarps; ++w) mbar_init(&res_bar[w], 1);
+    init_ln_bars<kTileN>(ln_bars);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -1356,9 +1417,11 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
 
   const int n_tiles = args.N / kTileN;
   const int num_kb = args.K / kBlockK;
+  const int m_tiles = (M + 2 * kBlockM - 1) / (2 * kBlockM);
+  const int total_tiles = m_tiles * n_tiles;
   // The leading W blocks of the pair's first tile ahead of the dependency wait, its A blocks right behind it (see
   // gemm_f16_kernel).  Both CTAs' copies complete on the leader's barrier, which the leader arms for both.
-  const int pre_kb = args.early_w ? (num_kb < kStages ? num_kb : kStages) : 0;
+  const int pre_kb = args.early_w && cluster_id < total_tiles ? (num_kb < kStages ? num_kb : kStages) : 0;
   auto load_w = [&](int stage, int n0, int kb) {
     uint8_t* sb = smem + stage * Cfg::kStageBytes + kABytes;
     const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
@@ -1385,24 +1448,11 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
   pdl_wait();  // see gemm_f16_kernel
   if (warp == 0)
     for (int kb = 0; kb < pre_kb; ++kb) load_a(kb, tile_rows(cluster_id), kb);
-  int M = args.m_rows;
-  if (args.m_dev != nullptr) {
-    const int md = __ldg(args.m_dev);
-    M = uniform_int(md < M ? md : M);
-  }
-  const int m_tiles = (M + 2 * kBlockM - 1) / (2 * kBlockM);
-  const int total_tiles = m_tiles * n_tiles;
-
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    if (cluster_id >= total_tiles && leader) {
-      // No tile for this pair after all: wait for the armed stages, so that no copy is in flight at exit.
-      for (int kb = 0; kb < pre_kb; ++kb)
-        if (!mbar_wait_warp(&full_bar[kb], 0u, abort_flag, args.status, kStatusGemmProducerTimeout)) break;
-    }
     for (int tile = cluster_id; tile < total_tiles && ok; tile += num_clusters) {
       const int m0 = tile_rows(tile), n0 = tile_w_cols(tile);
       for (int kb = 0; kb < num_kb; ++kb) {
@@ -1460,7 +1510,7 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue
+    // --------------------------------------------- epilogue and row statistics
     auto tile_at = [&](int it, int& m0, int& n0) -> bool {
       const int tile = cluster_id + it * num_clusters;
       if (tile >= total_tiles) return false;
@@ -1468,9 +1518,13 @@ gemm_f16_pair_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_c
       n0 = (tile % n_tiles) * kTileN;
       return true;
     };
-    ln_epilogue_loop(args, &tm_out, &tm_res, smem + kStages * Cfg::kStageBytes, acc_full, vec_full, vec_empty, res_bar,
-                     vec_s, abort_flag, tmem_base, M, n_tiles, warp, lane, tile_at,
-                     [&](int as) { mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[as]), 0)); });
+    if (warp < kLnFirstEpiWarp)
+      ln_statistics_loop<kTileN>(args, smem + kStages * Cfg::kStageBytes, ln_bars, vec_s, abort_flag, M, n_tiles, warp - 2,
+                                 lane, tile_at);
+    else
+      ln_epilogue_loop<kTileN>(args, &tm_out, &tm_res, smem + kStages * Cfg::kStageBytes, ln_bars, vec_s, abort_flag,
+                               tmem_base, M, warp, lane, tile_at,
+                               [&](int as) { mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[as]), 0)); });
   }
 
   // ------------------------------------------------------------------ teardown
@@ -1573,12 +1627,12 @@ cudaError_t launch_pair_epi(const GemmLaunch& g, const GemmArgs& a, cudaStream_t
 }
 
 struct LnGemmCfg {
-  static constexpr int kSmemBytes = GemmCfg<256>::kSmemBytes - kBiasBytes + 1536;  // + bias / gamma / beta slices of a tile
+  static constexpr int kSmemBytes = kLnRingAndStaging + kLnBarBytes + kLnVecBytes;
 };
 static_assert(LnGemmCfg::kSmemBytes <= 227 * 1024, "shared memory of the GEMM + LayerNorm kernel");
 
 struct PairLnGemmCfg {
-  static constexpr int kSmemBytes = PairCfg::kSmemBytes - kBiasBytes + 1536;
+  static constexpr int kSmemBytes = PairLnCfg::kStages * PairLnCfg::kStageBytes + PairLnCfg::kStagingBytes + kLnBarBytes + kLnVecBytes;
 };
 static_assert(PairLnGemmCfg::kSmemBytes <= 227 * 1024, "shared memory of the pair GEMM + LayerNorm kernel");
 int g_pair_ln_clusters[64] = {};
@@ -1599,7 +1653,7 @@ cudaError_t launch_pair_ln_gemm(const GemmLaunch& g, const GemmArgs& a, cudaStre
   if (g_pair_ln_clusters[dev] == 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * (g.num_sms / 2));
-    cfg.blockDim = dim3(kGemmThreads);
+    cfg.blockDim = dim3(kLnThreads);
     cfg.dynamicSmemBytes = Cfg::kSmemBytes;
     int n = 0;
     // every cluster must be resident (clusters wait for one another's row statistics): without an
@@ -1616,7 +1670,7 @@ cudaError_t launch_pair_ln_gemm(const GemmLaunch& g, const GemmArgs& a, cudaStre
   long long tiles = static_cast<long long>(n_tiles) * m_tiles;
   int clusters = static_cast<int>(tiles < g_pair_ln_clusters[dev] ? tiles : g_pair_ln_clusters[dev]);
   if (clusters < 1) clusters = 1;
-  return launch_pdl(kern, dim3(2 * clusters), dim3(kGemmThreads), Cfg::kSmemBytes, stream, g.tm_a, g.tm_b, g.tm_out,
+  return launch_pdl(kern, dim3(2 * clusters), dim3(kLnThreads), Cfg::kSmemBytes, stream, g.tm_a, g.tm_b, g.tm_out,
                     g.tm_res, a);
 }
 
@@ -1648,10 +1702,10 @@ cudaError_t launch_ln_gemm(const GemmLaunch& g, const GemmArgs& a_in, cudaStream
     attr_set[dev] = true;
   }
   const int m_tiles = (g.m_rows + kBlockM - 1) / kBlockM;
-  const long long tiles = static_cast<long long>(m_tiles) * (g.N / 256);
+  const long long tiles = static_cast<long long>(m_tiles) * (g.N / (g.N % 192 == 0 ? 192 : 256));  // the narrower width's
   int grid = static_cast<int>(tiles < g.num_sms ? tiles : g.num_sms);
   if (grid < 1) grid = 1;
-  return launch_pdl(kern, dim3(grid), dim3(kGemmThreads), Cfg::kSmemBytes, stream, g.tm_a, g.tm_b, g.tm_out, g.tm_res, a);
+  return launch_pdl(kern, dim3(grid), dim3(kLnThreads), Cfg::kSmemBytes, stream, g.tm_a, g.tm_b, g.tm_out, g.tm_res, a);
 }
 
 // The pair kernel needs N % 256 == 0 and pays off once every SM pair gets at least two
