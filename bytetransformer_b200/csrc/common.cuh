@@ -54,7 +54,7 @@ __device__ __forceinline__ bool elect_one() {
 //  * Kernels say pdl_launch_dependents() first thing - except those that run second in a call (pack_rows,
 //    embedding_layernorm, mask_bits), which say it after their own pdl_wait().  So from the third kernel on, what the
 //    FIRST kernel of the call wrote is complete and visible ahead of the wait as well: the attention kernels read the
-//    offsets there (MhaLaunch::early_offsets).
+//    offsets there (MhaLaunch::early_offsets), the GEMM + LayerNorm kernels the row count.
 //  * Anything else that an earlier kernel may have written or may still read is touched after pdl_wait() only.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -140,6 +140,7 @@ struct bt_encoder_s {
   int fused_ln_min_tiles_all_rows = 32;  // every allocated row is computed (and see fused_ln_pays)
   bool all_rows = false;  // the call in progress computes every allocated row (packed and general-mask entries)
   uint32_t ln_epoch = 0;  // fused LayerNorm launches since the statistics scratch of the current call was zeroed
+  bool fused_ln_line_set = false;  // diagnostics have set the two lines above: nothing else decides
   bool fused_ln_ffn2_only = false;  // keep the attention-output LayerNorm as its own kernel
   std::vector<cudaEvent_t> ev_pool;
   size_t ev_used = 0;
@@ -388,13 +389,31 @@ static bool want_fused_ln(bt_handle h, long long rows) {
   return fused_ln_pays(row_tiles, H, h->num_sms, h->all_rows, h->fused_ln_min_tiles, h->fused_ln_min_tiles_all_rows);
 }
 
+// Below that line it pays as soon as the GEMMs of fp32 sums, whose tiles are then 64 columns wide, would need a second wave:
+// the fused kernel's tiles of 128 columns need one.  Where some rows are padding, three fifths are taken to be valid (and
+// the fused kernel fits its tiles to the rows that are there, see ln_tile_n).  us per forward of 12 layers, separate / fused.
+// Every row computed, 768 columns: 12 row tiles 585 / 603, 13 719 / 649; 1024: 9 656 / 692, 10 812 / 763; 512: 18 516 / 518,
+// 19 602 / 552.  Padded, allocated row tiles (valid ones): 768: 20 (12) 575 / 602, 22 (14) 732 / 644; 1024: 16 (9) 629 /
+// 678, 18 (11) 832 / 746; 512: 28 (17) 513 / 525, 32 (19) 621 / 546.  Between one wave of 128-column tiles and the line
+// above, where every row is computed, the separate kernels are kept.
+static bool fused_ln_saves_a_wave(long long row_tiles, int H, int num_sms, bool all_rows) {
+  const long long there = all_rows ? row_tiles : row_tiles * 3 / 5;
+  if (H < 512 || (all_rows && row_tiles * (H / 128) >= num_sms)) return false;
+  return there * (H / 64) > num_sms;
+}
+static bool fuse_ln(bt_handle h, long long rows) {
+  if (want_fused_ln(h, rows)) return true;
+  return h->fused_ln == 1 && !h->fused_ln_line_set && h->hidden % 256 == 0 && h->hidden <= 1024 &&
+         fused_ln_saves_a_wave((rows + 127) / 128, h->hidden, h->num_sms, h->all_rows);
+}
+
 // The statistics scratch of the fused LayerNorm (the head of `pre`) holds words tagged with the number
 // of the launch that wrote them; it is zeroed once per call (the caller's workspace starts out with
 // arbitrary contents) and the fused launches of the call are numbered from 1.
 static int prepare_ln_sync(bt_handle h, const Workspace& ws, long long rows, bool all_rows, cudaStream_t stream) {
   h->ln_epoch = 0;
   h->all_rows = all_rows;
-  if (!want_fused_ln(h, rows)) return BT_OK;
+  if (!fuse_ln(h, rows)) return BT_OK;
   cudaError_t e = cudaMemsetAsync(ws.pre, 0, ws.ln_stats_bytes, stream);
   return e == cudaSuccess ? BT_OK : fail_cuda(h, e, "memset of the LayerNorm statistics scratch");
 }
@@ -415,11 +434,9 @@ static int run_layer(bt_handle h, int layer, const __half* x_in, __half* x_out, 
                      stream)) != BT_OK)
     return rc;
   if ((rc = run_mha(h, ws.qkv, ws.ctx, batch_idx, B, S_or_maxlen, rows, stream, true, gm)) != BT_OK) return rc;
-  // LayerNorm rides in the GEMM kernel (clusters of H/256 CTAs per 128-row tile) once there are
-  // enough row tiles to occupy the machine that way; below that the narrow-tile GEMM followed by
-  // the row kernel spreads the few rows over more SMs.
-  const bool fuse_any = want_fused_ln(h, rows);
-  const bool fuse_ln = fuse_any && !h->fused_ln_ffn2_only;
+  // LayerNorm inside the GEMM kernels, or a GEMM of fp32 sums followed by the row kernel
+  const bool fuse_any = fuse_ln(h, rows);
+  const bool fuse_attn_out = fuse_any && !h->fused_ln_ffn2_only;
   // Few rows: the two GEMMs that feed a LayerNorm cut K into ranges (one fp32 sum each, `rows * H`
   // floats apart in `pre`) and the LayerNorm kernel adds them up.
   auto split_for = [&](int K) {
@@ -431,7 +448,7 @@ static int run_layer(bt_handle h, int layer, const __half* x_in, __half* x_out, 
   const int split_attn = split_for(H), split_ffn2 = split_for(F);
   const long long split_stride = static_cast<long long>(rows) * H;
   cudaError_t e = cudaSuccess;
-  if (fuse_ln) {
+  if (fuse_attn_out) {
     LnArgs ln{++h->ln_epoch, ws.y, w.attr_output_layernorm_gamma, w.attr_output_layernorm_beta, gb32, h->cfg.ln_eps};
     if ((rc = run_gemm(h, BT_PROF_GEMM_ATTN_OUT, ws.ctx, w.attr_output_kernel, reinterpret_cast<__half*>(ws.pre),
                        w.attr_output_bias, x_in, m_dev, rows, H, H, BT_EPI_BIAS_RESIDUAL_LAYERNORM, 0, stream, &ln)) !=
@@ -452,7 +469,7 @@ static int run_layer(bt_handle h, int layer, const __half* x_in, __half* x_out, 
   if ((rc = run_gemm(h, BT_PROF_GEMM_FFN1, ws.y, w.inter_kernel, ws.mid, w.inter_bias, nullptr, m_dev, rows, F, H, BT_EPI_BIAS_GELU,
                      h->cfg.gelu_kind, stream)) != BT_OK)
     return rc;
-  if (fuse_any && restore_to == nullptr) {
+  if (restore_to == nullptr && fuse_any) {
     LnArgs ln{++h->ln_epoch, x_out, w.output_layernorm_gamma, w.output_layernorm_beta, gb32, h->cfg.ln_eps};
     return run_gemm(h, BT_PROF_GEMM_FFN2, ws.mid, w.output_kernel, reinterpret_cast<__half*>(ws.pre), w.output_bias,
                     ws.y, m_dev, rows, H, F, BT_EPI_BIAS_RESIDUAL_LAYERNORM, 0, stream, &ln);
@@ -1028,7 +1045,8 @@ int bt_gemm_layernorm(bt_handle h, const void* A, const void* W, const void* bia
                   reinterpret_cast<cudaStream_t>(stream), &ln);
 }
 
-// Host-side policy, callable without a device (tests): 1 if LayerNorm runs inside the GEMMs of a forward.
+// Host-side policies, callable without a device (tests): 1 if LayerNorm runs inside the GEMMs of a forward, by the lines on
+// row tiles, and with the wave that it may save counted too.
 int bt_debug_fused_layernorm_policy(int rows, int hidden, int num_sms, int all_rows) {
   bt_encoder_s h;
   h.hidden = hidden;
@@ -1037,12 +1055,21 @@ int bt_debug_fused_layernorm_policy(int rows, int hidden, int num_sms, int all_r
   return want_fused_ln(&h, rows) ? 1 : 0;
 }
 
+int bt_debug_fused_layernorm_choice(int rows, int hidden, int num_sms, int all_rows) {
+  bt_encoder_s h;
+  h.hidden = hidden;
+  h.num_sms = num_sms;
+  h.all_rows = all_rows != 0;
+  return fuse_ln(&h, rows) ? 1 : 0;
+}
+
 // Diagnostics hook: LayerNorm inside the attention-output / FFN2 GEMM kernels: 0 = never (row
 // kernel), 1 = when the call has enough 128-row tiles (default), 2 = always; values above 2
 // keep mode 1 and set the tile threshold to that value.
 int bt_debug_set_fused_layernorm(bt_handle h, int on) {
   if (!h) return BT_ERR_INVALID_ARG;
   h->fused_ln_ffn2_only = false;
+  h->fused_ln_line_set = on > 3;
   if (on == 3) {  // mode 1 for the FFN2 GEMM only
     h->fused_ln = 1;
     h->fused_ln_ffn2_only = true;

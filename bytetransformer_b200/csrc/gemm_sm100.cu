@@ -97,6 +97,7 @@ struct GemmArgs {
   int split_k;
   long long split_stride;
   int early_w;  // request the first tile's W blocks before the wait for the kernel before
+  int force_n;  // fused LayerNorm, diagnostics: tile width (0 = ln_tile_n)
   long long* timing;  // diagnostics: clock64 stamps per CTA and tile (null = off)
   uint64_t a_desc_hi;
   uint64_t b_desc_hi;
@@ -290,6 +291,13 @@ struct BiasShare {
   }
 };
 
+// The MMA warp's wait, after its last tile, for the epilogue to hand back the accumulators of the `tiles` tiles it began
+// (two buffers by turns; where a wait gave up, this one ends as quickly as all others).
+__device__ __forceinline__ void wait_accumulators_back(uint64_t* acc_empty, int tiles, volatile int* abort_flag, int* status) {
+  for (int it = tiles < 2 ? 0 : tiles - 2; it < tiles; ++it)
+    mbar_wait_anyway(&acc_empty[it & 1], (it >> 1) & 1, abort_flag, status, kStatusGemmMmaTimeout);
+}
+
 // ------------------------------------------------------------------------------------------
 // One CTA per SM, tile 128 x BLOCK_N.
 // ------------------------------------------------------------------------------------------
@@ -453,7 +461,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true, landed = false;
-      int m0 = 0, n0 = 0, sp = 0;
+      int m0 = 0, n0 = 0, sp = 0, tiles = 0;
       for (int it = 0; ok && tile_at(it, m0, n0, sp); ++it) {
         const int as = it & 1;
         const uint32_t aphase = (it >> 1) & 1;
@@ -482,7 +490,13 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
         ok = __all_sync(0xffffffffu, ok) != 0;
         if (ok && elect_one()) umma_commit(&acc_full[as]);
         if (lane == 0) gstamp(args.timing, it, 1);
+        tiles = it + 1;
       }
+      // Tensor memory goes back as soon as the accumulators have: at the end of the CTA it took 0.6k clocks of the
+      // chain of kernels.
+      wait_accumulators_back(acc_empty, tiles, abort_flag, args.status);
+      tc_fence_after();
+      tmem_dealloc(tmem_base, Cfg::kTmemCols);
     }
   } else {
     // ------------------------------------------------------------------ epilogue
@@ -520,10 +534,6 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     // A wait ran out somewhere: give copies that may still be in flight time to
     // land before the CTA's shared memory is handed to another block.
     for (int i = 0; i < 64; ++i) __nanosleep(2000);
-  }
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem_base, Cfg::kTmemCols);
   }
 }
 
@@ -787,7 +797,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 // Main loop as in gemm_f16_kernel: tile t = (row tile t / C, column tile t % C), C = N / tile width, tiles round-robin over
 // the CTAs, so the C column tiles of a row tile are worked on by C neighbouring CTAs at about the same time.  The
 // pre-normalisation tensor never goes to HBM.  An epilogue warp owns 32 rows and 64 columns of the tile (16 warps for 256
-// columns, 12 for 192), a thread one row's 64 values, which stay in its registers from the first touch to the last (20 warps
+// columns, 12 for 192, 8 for 128), a thread one row's 64 values, which stay in its registers from the first touch to the last (20 warps
 // leave 96 registers a thread, which is why two warps of their own deal with the statistics):
 //   1. v = accumulator + bias + residual, with the sum and sum of squares of v - s (s = the thread's first value: shifted
 //      one-pass statistics).  The accumulator goes back to the MMA warp as soon as it has been read;
@@ -800,7 +810,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
 //      and hands mean and 1 / deviation to the row's threads;
 //   4. normalise, gamma / beta, fp16, staging, TMA store.
 // us per launch of 4,100 rows x 768 columns: with 128 values per thread (8 warps), written back to tensor memory for step 4,
-// K = 768 / 3072 14.4 / 26.2; so LN_768 / LN_3072.
+// K = 768 / 3072 14.5 / 25.0; so 13.6 / 24.6 with 256 columns still and 12.4 / 20.7 with 192 (with the launch's memset).
 // Accumulators are double buffered, so 1-4 of a tile overlap the main loop of the CTA's next
 // tile.  A CTA only ever waits for the C CTAs working on the same row tile, and those wait for
 // nothing but that row tile in turn, so the waits are never circular.  Progress does need those
@@ -818,12 +828,33 @@ __device__ __forceinline__ void ld_relaxed_gpu_2u64(const unsigned long long* p,
                                                     unsigned long long& v1) {
   asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v0), "=l"(v1) : "l"(p) : "memory");
 }
-// Tile width of the one-CTA GEMM + LayerNorm kernel for this many row tiles on `ctas` CTAs: 192 columns where they take
-// less time than 256, counted in waves of tiles (three quarters as long each).
-__host__ __device__ __forceinline__ int ln_tile_n(int m_tiles, int N, int ctas) {
-  if (N % 192 != 0) return 256;
-  const int waves192 = (m_tiles * (N / 192) + ctas - 1) / ctas, waves256 = (m_tiles * (N / 256) + ctas - 1) / ctas;
-  return 3 * waves192 < 4 * waves256 ? 192 : 256;
+// Tile width of the one-CTA GEMM + LayerNorm kernel for this many row tiles on `ctas` CTAs: the width whose waves of tiles
+// take least.  Clocks: a tile's main loop `k_block` per K block of 64, its epilogue `epilogue`; the epilogue of all waves
+// but the last runs under the next wave's main loop, and a wave more costs 1.5k besides.  us per launch with its memset,
+// widths 128 / 192 / 256 (64 columns were measured too: within 0.3 us of 128 at best).  768 columns, K = 768: 12 row tiles
+// 10.9 / 11.4 / 12.7, 25 14.0 / 12.1 / 13.5, 38 14.7 / 15.6 / 13.8, 50 18.2 / 15.9 / 18.2; K = 3072: 12 17.3 / 19.6 /
+// 23.2, 25 25.2 / 20.3 / 24.4, 38 25.8 / 32.3 / 24.9, 50 34.6 / 33.5 / 40.7, 74 41.9 / 39.8 / 49.4.  1024 columns (128 /
+// 256), K = 1024: 16 12.1 / 14.5, 20 15.6 / 14.6, 38 20.7 / 21.5, 64 25.0 / 21.8.
+struct LnWidthCost { int cols, k_block, epilogue; };
+__host__ __device__ __forceinline__ int ln_tile_n(int m_tiles, int N, int K, int ctas) {
+  constexpr LnWidthCost kCosts[3] = {{128, 290, 3700}, {192, 410, 4200}, {256, 520, 5600}};
+  int best = 256;
+  float best_cost = 3.0e38f;
+  const float inv = 1.0f / static_cast<float>(ctas);
+  const float blocks = static_cast<float>(K / kBlockK);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const LnWidthCost w = kCosts[i];
+    if (N % w.cols != 0) continue;
+    const float main = blocks * static_cast<float>(w.k_block), epi = static_cast<float>(w.epilogue);
+    const float waves = ceilf(static_cast<float>(m_tiles * (N / w.cols)) * inv - 1.0e-4f);
+    const float cost = main + epi + (waves - 1.0f) * (fmaxf(main, epi) + 1500.0f);
+    if (cost <= best_cost) {  // (the wider of two that take the same)
+      best_cost = cost;
+      best = w.cols;
+    }
+  }
+  return best;
 }
 
 constexpr int kLnEpiWarps = 16;
@@ -831,7 +862,6 @@ constexpr int kLnFirstEpiWarp = 4;      // warps 0 and 1 load and multiply, 2 an
 constexpr int kLnThreads = 32 * (kLnFirstEpiWarp + kLnEpiWarps);
 constexpr int kLnBarBytes = 384;          // barriers and slots
 constexpr int kLnVecBytes = 256 * (4 + 4 + 2);  // gamma | beta | bias of a tile's columns: fp32, fp32, fp16
-constexpr int kLnMaxParts = 5;            // column tiles of a row: N <= 1024, tiles of 192 columns or more
 
 // Barriers between the epilogue warps and the two statistics warps.
 struct LnBars {
@@ -1012,6 +1042,7 @@ __device__ __forceinline__ void ln_statistics_loop(const GemmArgs& args, uint8_t
                                                    volatile int* abort_flag, int M, int n_tiles, int half, int lane,
                                                    TileAt tile_at) {
   constexpr int kGroups = TILE_N / 64;
+  constexpr int kMaxParts = 1024 / TILE_N;  // column tiles of a row, N <= 1024
   const float inv_n = 1.0f / static_cast<float>(args.N);
   const float inv_tiles = 1.0f / static_cast<float>(n_tiles);
   const uint32_t epoch = args.ln_epoch;
@@ -1082,7 +1113,7 @@ __device__ __forceinline__ void ln_statistics_loop(const GemmArgs& args, uint8_t
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       const int quarter = 2 * half + k;
-      float pm[kLnMaxParts], pq[kLnMaxParts];
+      float pm[kMaxParts], pq[kMaxParts];
       const long long t0 = clock64();
       uint32_t probes = 0;
       while (true) {
@@ -1090,7 +1121,7 @@ __device__ __forceinline__ void ln_statistics_loop(const GemmArgs& args, uint8_t
         if (row_ok[k]) {
           // all loads are issued before any tag is looked at: one round trip
 #pragma unroll
-          for (int p = 0; p < kLnMaxParts; ++p)
+          for (int p = 0; p < kMaxParts; ++p)
             if (p < n_tiles) {
               unsigned long long w0, w1;
               ld_relaxed_gpu_2u64(words[k] + (p * slab_rows[k] + lane) * 2, w0, w1);
@@ -1111,12 +1142,12 @@ __device__ __forceinline__ void ln_statistics_loop(const GemmArgs& args, uint8_t
       float mean = 0.f, rstd = 0.f;
       if (row_ok[k]) {
 #pragma unroll
-        for (int p = 0; p < kLnMaxParts; ++p)
+        for (int p = 0; p < kMaxParts; ++p)
           if (p < n_tiles) mean += pm[p];
         mean *= inv_tiles;
         float M2 = 0.f;
 #pragma unroll
-        for (int p = 0; p < kLnMaxParts; ++p)
+        for (int p = 0; p < kMaxParts; ++p)
           if (p < n_tiles) {
             const float d = pm[p] - mean;
             M2 += pq[p] + static_cast<float>(TILE_N) * d * d;
@@ -1150,12 +1181,12 @@ __device__ __forceinline__ int ln_rows(const GemmArgs& args, const uint8_t* smem
 template <int TILE_N>
 struct LnCfg {
   static constexpr int kStageBytes = kABytes + TILE_N * kBlockK * 2;
-  static constexpr int kStages = TILE_N == 256 ? 3 : 4;
+  static constexpr int kStages = TILE_N == 256 ? 3 : TILE_N == 192 ? 4 : 6;
   static constexpr int kStagingBytes = (TILE_N / 64) * 4 * kStagingBytesPerWarp;
   static constexpr int kRingAndStaging = kStages * kStageBytes + kStagingBytes;
 };
-constexpr int kLnRingAndStaging =
-    LnCfg<256>::kRingAndStaging > LnCfg<192>::kRingAndStaging ? LnCfg<256>::kRingAndStaging : LnCfg<192>::kRingAndStaging;
+constexpr int kLnRingAndStaging = LnCfg<128>::kRingAndStaging;  // the largest of the three
+static_assert(LnCfg<192>::kRingAndStaging <= kLnRingAndStaging && LnCfg<256>::kRingAndStaging <= kLnRingAndStaging, "");
 
 // One width of gemm_f16_ln_kernel, from the barriers on.  `M` valid rows.
 template <int TILE_N>
@@ -1255,7 +1286,7 @@ __device__ __forceinline__ void ln_gemm_body(const CUtensorMap* tm_a, const CUte
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true, landed = false;
-      int m0 = 0, n0 = 0;
+      int m0 = 0, n0 = 0, tiles = 0;
       for (int it = 0; ok && tile_at(it, m0, n0); ++it) {
         const int as = it & 1;
         const uint32_t aphase = (it >> 1) & 1;
@@ -1284,7 +1315,11 @@ __device__ __forceinline__ void ln_gemm_body(const CUtensorMap* tm_a, const CUte
         ok = __all_sync(0xffffffffu, ok) != 0;
         if (ok && elect_one()) umma_commit(&acc_full[as]);
         if (lane == 0) gstamp(args.timing, it, 1);
+        tiles = it + 1;
       }
+      wait_accumulators_back(acc_empty, tiles, abort_flag, args.status);
+      tc_fence_after();
+      tmem_dealloc(tmem_base, 512);
     }
   } else if (warp < kLnFirstEpiWarp) {
     // ------------------------------------------------------- row statistics
@@ -1327,7 +1362,10 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     tma_prefetch_desc(&tm_res);
   }
   const int m_tiles = (M + kBlockM - 1) / kBlockM;
-  if (ln_tile_n(m_tiles, args.N, static_cast<int>(gridDim.x)) == 192)
+  const int tile_n = args.force_n != 0 ? args.force_n : ln_tile_n(m_tiles, args.N, args.K, static_cast<int>(gridDim.x));
+  if (tile_n == 128)
+    ln_gemm_body<128>(&tm_a, &tm_b, &tm_out, &tm_res, args, smem, bars, vec_s, tmem_slot, abort_flag, M, warp, lane);
+  else if (tile_n == 192)
     ln_gemm_body<192>(&tm_a, &tm_b, &tm_out, &tm_res, args, smem, bars, vec_s, tmem_slot, abort_flag, M, warp, lane);
   else
     ln_gemm_body<256>(&tm_a, &tm_b, &tm_out, &tm_res, args, smem, bars, vec_s, tmem_slot, abort_flag, M, warp, lane);
@@ -1336,10 +1374,6 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   __syncthreads();
   if (*abort_flag != 0) {
     for (int i = 0; i < 64; ++i) __nanosleep(2000);
-  }
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(uniform_u32(*tmem_slot), 512);
   }
 }
 
@@ -1674,19 +1708,25 @@ cudaError_t launch_pair_ln_gemm(const GemmLaunch& g, const GemmArgs& a, cudaStre
                     g.tm_res, a);
 }
 
+// The pair form of GEMM + LayerNorm (main loop on SM pairs, half of the W tile per SM) is the faster one where there are
+// waves enough that its coarser tiles fill them; below, the one-CTA form fits its width to the rows.  us per launch with
+// its memset, one-CTA / pair form: 768 columns, K = 3072: 9,400 rows (two waves of 192-column tiles) 39.6 / 43.5, 12,500
+// 54.6 / 51.2, 75,776 300 / 269; K = 768: 18,944 rows (four waves) 28.9 / 30.2, 28,000 41.2 / 40.3, 75,776 101 / 98.  1024
+// columns (no 192; one wave is up to 4,736 rows), K = 4096: 4,100 rows 38.9 / 41.0, 6,200 74.5 / 60.3; K = 1024: 4,100 rows
+// 22.7 / 24.5, 6,400 32.6 / 32.4, 12,500 38.4 / 36.0.  512 columns, K = 2048: 9,400 rows 22.3 / 23.3, 12,500 34.5 / 31.9.
+bool ln_pair_pays(int m_rows, int N, int K, int num_sms) {
+  const long long m_tiles = (m_rows + kBlockM - 1) / kBlockM;
+  if (N % 192 == 0) return m_tiles * (N / 192) > (K >= 2048 ? 2LL : 4LL) * num_sms;
+  return m_tiles * (N / 256) > num_sms;
+}
+
 cudaError_t launch_ln_gemm(const GemmLaunch& g, const GemmArgs& a_in, cudaStream_t stream) {
   using Cfg = LnGemmCfg;
   static bool attr_set[64] = {};
   auto kern = gemm_f16_ln_kernel;
   if (g.N % 256 != 0 || g.N > 1024 || !g.out_ln || !g.gamma || !g.beta || !g.residual || !g.bias || g.ln_epoch == 0)
     return cudaErrorInvalidValue;
-  // The pair form (main loop on SM pairs, half of the W tile per SM) is used where the main loop is the longer
-  // leg of a tile, i.e. for a long K (FFN2, K = 4 x hidden): measured in situ on 69.6k-row launches, 79.5 against
-  // 85 ms of FFN2 kernel time per three steps and +1.3 % on the whole forward.  For a short K (attention output)
-  // the epilogue is the longer leg, and a buffer of the pair's accumulator is only released when the epilogue
-  // warps of BOTH CTAs are done with it: 11 % slower there.  (On 18.9k-row launches, 1800 per step, the gain
-  // on FFN2 was 5 % of its kernel time and the forward did not move.)  Debug key 9: 1 = always, 2 = never.
-  const bool want_pair = g_dbg_ln_pair == 1 || (g_dbg_ln_pair == 0 && g.K >= 2048);
+  const bool want_pair = g_dbg_ln_pair == 1 || (g_dbg_ln_pair == 0 && ln_pair_pays(g.m_rows, g.N, g.K, g.num_sms));
   if (want_pair) {
     GemmArgs ap = a_in;
     ap.idesc = make_idesc_f16(256, 256, 0, 1);
@@ -1702,7 +1742,7 @@ cudaError_t launch_ln_gemm(const GemmLaunch& g, const GemmArgs& a_in, cudaStream
     attr_set[dev] = true;
   }
   const int m_tiles = (g.m_rows + kBlockM - 1) / kBlockM;
-  const long long tiles = static_cast<long long>(m_tiles) * (g.N / (g.N % 192 == 0 ? 192 : 256));  // the narrower width's
+  const long long tiles = static_cast<long long>(m_tiles) * (g.N / 128);  // the narrowest width's
   int grid = static_cast<int>(tiles < g.num_sms ? tiles : g.num_sms);
   if (grid < 1) grid = 1;
   return launch_pdl(kern, dim3(grid), dim3(kLnThreads), Cfg::kSmemBytes, stream, g.tm_a, g.tm_b, g.tm_out, g.tm_res, a);
@@ -1799,6 +1839,7 @@ cudaError_t launch_gemm(const GemmLaunch& g, cudaStream_t stream) {
   a.split_k = 1;
   a.split_stride = 0;
   a.early_w = g_dbg_early_w != 0 ? 1 : 0;
+  a.force_n = g_dbg_force_block_n >= 128 && g.N % g_dbg_force_block_n == 0 ? static_cast<int>(g_dbg_force_block_n) : 0;
   if (g.split_k > 1) {
     if (g.epilogue != BT_EPI_BIAS_RESIDUAL_F32OUT || g.N % 64 != 0 || (g.K / kBlockK) % g.split_k != 0)
       return cudaErrorInvalidValue;

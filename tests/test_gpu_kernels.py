@@ -578,6 +578,27 @@ def _fused_layernorm_case(enc, cuda_device, M, N, K, gb32, m_valid):
     assert enc.device_status() == 0
 
 
+@pytest.mark.parametrize("width", [128, 192, 256])
+@pytest.mark.parametrize("M,K,gb32,m_valid", [
+    (1, 64, False, None),          # one row, one K block
+    (129, 768, True, None),        # a second row tile of one row
+    (300, 448, False, 257),        # fewer blocks than stages; rows that are allocated and not there
+    (4801, 768, False, None),      # 38 row tiles: two waves of 128 and 192 columns, one of 256
+    (2560, 3072, False, 1000),     # the rows that are there decide the width, not the allocated ones
+])
+def test_fused_layernorm_tile_widths(enc, cuda_device, M, K, gb32, m_valid, width):
+    """Every tile width of the one-CTA GEMM + LayerNorm kernel on 768 columns (the widths that all divide it)."""
+    from bytetransformer_b200 import _abi
+    lib = _abi.load()
+    lib.bt_debug_set(9, 2)
+    lib.bt_debug_set(4, width)
+    try:
+        _fused_layernorm_case(enc, cuda_device, M, 768, K, gb32, m_valid)
+    finally:
+        lib.bt_debug_set(4, 0)
+        lib.bt_debug_set(9, 0)
+
+
 @pytest.mark.parametrize("offset", [0, 4, 8])
 def test_fused_layernorm_scratch_may_start_anywhere(enc, cuda_device, offset):
     """The statistics scratch of bt_gemm_layernorm needs no alignment of its own (the kernel moves its words 16 bytes at
@@ -592,6 +613,24 @@ def test_fused_layernorm_scratch_may_start_anywhere(enc, cuda_device, offset):
               M, N, K, torch.cuda.current_stream().cuda_stream)
     assert torch.equal(out, want)
     assert enc.device_status() == 0
+
+
+@pytest.mark.parametrize("N", [64, 128, 768])
+def test_gelu_epilogue_hands_a_nan_on(enc, cuda_device, N):
+    """One NaN among the inputs makes its row NaN and no other; bias values differ from column to column, so a tile that read
+    another tile's would show.  (Values stay below 8, where half a unit of fp16 is 2e-3.)"""
+    from bytetransformer_b200 import _abi
+    M, K = 200, 64
+    g = torch.Generator().manual_seed(N)
+    a = torch.randn(M, K, generator=g).half()
+    w = (torch.randn(K, N, generator=g) * 0.1).half()
+    bias = (torch.randn(N, generator=g) * 0.5).half()
+    a[17, 5] = float("nan")
+    got = enc.gemm(a.to(cuda_device), w.to(cuda_device), bias.to(cuda_device), epilogue=_abi.BT_EPI_BIAS_GELU).cpu()
+    assert got[17].isnan().all()
+    keep = torch.arange(M) != 17
+    want = torch.nn.functional.gelu(a[keep].float() @ w.float() + bias.float())
+    assert_close_fp16(got[keep], want, f"gelu {N}", max_abs=6e-3, mean_abs=4e-4)
 
 
 # ---------------------------------------------------------------- failure path

@@ -92,3 +92,20 @@ def test_layernorm_inside_the_gemm(policy, tiles, hidden, all_rows, padded):
     for rows in (tiles * 128, tiles * 128 - 127):
         assert fn(rows, hidden, SMS, 1) == all_rows
         assert fn(rows, hidden, SMS, 0) == padded
+
+
+@pytest.mark.parametrize("tiles,hidden,all_rows,padded", [
+    (12, 768, 0, 0), (13, 768, 1, 0),                    # 144 and 156 tiles of 64 columns
+    (20, 768, 1, 0), (21, 768, 1, 0), (22, 768, 1, 1),   # three fifths of 21 are 12, of 22 are 13
+    (24, 768, 1, 1), (25, 768, 0, 1), (32, 768, 1, 1),   # 144 and 150 tiles of 128 columns; the line on row tiles
+    (9, 1024, 0, 0), (10, 1024, 1, 0), (16, 1024, 1, 0), (17, 1024, 1, 1), (19, 1024, 0, 1), (38, 1024, 1, 1),
+    (18, 512, 0, 0), (19, 512, 1, 0), (31, 512, 1, 0), (32, 512, 1, 1), (37, 512, 0, 1),
+    (39, 256, 0, 0), (40, 256, 1, 1),
+    (64, 320, 0, 0), (64, 1280, 0, 0),                   # widths without the fused kernels
+])
+def test_layernorm_inside_the_gemm_saves_a_second_wave_of_narrow_tiles(policy, tiles, hidden, all_rows, padded):
+    from bytetransformer_b200 import _abi
+    fn = _abi.load().bt_debug_fused_layernorm_choice
+    for rows in (tiles * 128, tiles * 128 - 127):
+        assert fn(rows, hidden, SMS, 1) == all_rows
+        assert fn(rows, hidden, SMS, 0) == padded
