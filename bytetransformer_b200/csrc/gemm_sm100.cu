@@ -168,13 +168,9 @@ __device__ __forceinline__ void epilogue_tile(const GemmArgs& args, const CUtens
 #pragma unroll
       for (int q = 0; q < kChunk / 8; ++q) {
         const uint4 b4 = bias_s[col / 8 + q];
-        const __half2* bh = reinterpret_cast<const __half2*>(&b4);
+        const uint32_t bh[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = __half22float2(bh[j]);
-          v[q * 8 + 2 * j] += f.x;
-          v[q * 8 + 2 * j + 1] += f.y;
-        }
+        for (int j = 0; j < 4; ++j) add_half2(v[q * 8 + 2 * j], v[q * 8 + 2 * j + 1], bh[j]);
       }
     }
     // (Two instances, not a branch: with both forms in one kernel a 128 x 256 tile's epilogue took 5.7k clocks, by
@@ -192,13 +188,9 @@ __device__ __forceinline__ void epilogue_tile(const GemmArgs& args, const CUtens
 #pragma unroll
       for (int q = 0; q < kChunk / 8; ++q) {
         const uint4 r4 = resv[c / 8 + q];
-        const __half2* rh = reinterpret_cast<const __half2*>(&r4);
+        const uint32_t rh[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 f = __half22float2(rh[j]);
-          v[q * 8 + 2 * j] += f.x;
-          v[q * 8 + 2 * j + 1] += f.y;
-        }
+        for (int j = 0; j < 4; ++j) add_half2(v[q * 8 + 2 * j], v[q * 8 + 2 * j + 1], rh[j]);
       }
     }
     // 8 (or 4) units of 16 bytes per row
