@@ -113,7 +113,7 @@ __device__ __forceinline__ void gstamp(long long* timing, int it, int slot) {
 }
 long long g_dbg_b_lbo = 0, g_dbg_b_sbo = 0, g_dbg_b_kstep = 0, g_dbg_force_block_n = 0, g_dbg_pair_mode = 0;
 long long g_dbg_early_w = 1;  // 1 = W blocks of the first tile requested before the dependency wait
-long long g_dbg_ln_pair = 0;  // GEMM + LayerNorm on SM pairs: 0 = for K >= 2048 (default), 1 = always, anything else = never
+long long g_dbg_ln_pair = 0;  // GEMM + LayerNorm on SM pairs: 0 = by ln_pair_pays (default), 1 = always, anything else = never
 long long g_dbg_split_k = 0;  // 0 = policy, < 0 = never, > 0 = that many ranges whenever the shape allows
 
 // ------------------------------------------------------------------------------------------
@@ -1864,11 +1864,11 @@ cudaError_t launch_gemm(const GemmLaunch& g, cudaStream_t stream) {
 // Diagnostics hook (not part of the stable ABI): overrides descriptor fields of
 // the W operand / the tile width so that encodings can be compared on a device
 // without rebuilding.  key: 1 = LBO bytes, 2 = SBO bytes, 3 = K-step bytes,
-// 4 = forced BLOCK_N of the one-CTA kernel, 5 = pair kernel (0 auto, 1 always when
+// 4 = forced tile width of the one-CTA kernels, 5 = pair kernel (0 auto, 1 always when
 // N % 256 == 0, 2 never), 6 = programmatic dependent launch on (1, default) / off (0),
 // 7 = split-K of the fp32-sum GEMMs (0 policy, < 0 never, > 0 that many K ranges),
 // 8 = W blocks of a CTA's first tile requested before the dependency wait (1, default) or after (0),
-// 9 = GEMM + LayerNorm on SM pairs (0, the default: for K >= 2048; 1 always; 2 never).
+// 9 = GEMM + LayerNorm on SM pairs (0, the default: by ln_pair_pays; 1 always; 2 never).
 // value 0 restores the default for keys 1-5 and 7.
 // Device buffer of 148 x 16 x 8 long long for clock64 stamps of the GEMM kernels (null = off):
 // slots 0/1 MMA warp (accumulator free, last commit), 2/3 epilogue warp 2 (accumulator ready, tile

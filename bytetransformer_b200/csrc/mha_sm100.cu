@@ -7,7 +7,7 @@
 //   mha_fwd_kernel         one CTA per (128 query rows, head, sequence), 192 threads, two CTAs per SM.
 //                          Used while the longest sequence fits two key tiles' worth of work per item
 //                          (max_len <= 192) and for the general-mask variant.
-//   mha_persistent_kernel  persistent CTAs walking a static list of (sequence, query tile, head) items,
+//   mha_persistent_kernel  CTAs that take over waiting (sequence, query tile, head) items,
 //                          256 threads, two CTAs per SM; everything longer.
 // Both run an online softmax over 128-key tiles, so no S x S logits ever reach HBM and any length
 // works.
@@ -782,8 +782,8 @@ mha_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant
 }
 
 // ------------------------------------------------------------------------------------------
-// Persistent kernel: each CTA (256 threads, two per SM) walks a static list of work items
-// (sequence, 128-row query tile, head).  Barriers, tensor memory and the launch are paid once per
+// Persistent kernel: each CTA (256 threads, two per SM) works on one item (sequence, 128-row query tile, head) after
+// another.  Barriers, tensor memory and the launch are paid once per
 // CTA instead of once per item, and the loader runs ahead: the next item's Q/K/V tiles are requested
 // while the current item's last key tiles are still being processed.
 //
