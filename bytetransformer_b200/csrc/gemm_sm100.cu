@@ -46,7 +46,9 @@ constexpr int kGemmThreads = 320;
 constexpr int kEpiWarps = 8;
 constexpr int kABytes = kBlockM * kBlockK * 2;  // 16 KiB
 constexpr int kStagingBytesPerWarp = 32 * 128;  // 32 rows x 128 B
-constexpr int kBiasBytes = 2 * 256 * 2;         // the bias of a tile's columns, for two tiles in turn
+constexpr int kBarBytes = 256;                  // barriers, tensor memory address, flag
+// Every epilogue warp's own copy of the bias of its columns, half of a tile's: see BiasShare.
+constexpr int bias_bytes(int tile_n) { return kEpiWarps * (tile_n / 2) * 2; }
 
 template <int BLOCK_N>
 struct GemmCfg {
@@ -60,7 +62,8 @@ struct GemmCfg {
     return BLOCK_N >= 128 || epi == BT_EPI_BIAS_RESIDUAL_F32OUT || epi == kEpiSplitKF32;
   }
   static constexpr int kStagingBytes = kEpiWarps * kStagingBytesPerWarp;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 /*align slack*/ + 256 /*barriers*/ + kBiasBytes;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + kBarBytes + bias_bytes(BLOCK_N);
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory of the one-CTA GEMM kernel");
 };
 
 // Pair kernel: per CTA 128 rows of A and 128 of the tile's 256 W columns per stage.
@@ -72,7 +75,8 @@ struct PairCfg {
   static constexpr int kTmemCols = 512;
   static constexpr int kStagingBufs = 1;  // per epilogue warp (two were measured: no gain, and they cost a stage)
   static constexpr int kStagingBytes = kStagingBufs * kEpiWarps * kStagingBytesPerWarp;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + 1024 + 256 + kBiasBytes;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + kBarBytes + bias_bytes(kTileN);
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory of the SM-pair GEMM kernel");
 };
 
 struct GemmArgs {
@@ -167,7 +171,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmArgs& args, const CUtens
     if (EPI != BT_EPI_NONE && (!kSplitK || split == 0)) {
 #pragma unroll
       for (int q = 0; q < kChunk / 8; ++q) {
-        const uint4 b4 = bias_s[col / 8 + q];
+        const uint4 b4 = bias_s[c / 8 + q];
         const uint32_t bh[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) add_half2(v[q * 8 + 2 * j], v[q * 8 + 2 * j + 1], bh[j]);
@@ -255,8 +259,12 @@ __device__ __forceinline__ void prefetch_residual(const GemmArgs& args, int m0, 
 
 // The bias of a warp's columns: asked for before the accumulator is waited for (BiasShare holds the lane's share), then put
 // where the warp reads it column by column - read from global memory there, a chunk's loads took a round trip to L2 in
-// the middle of the epilogue.  The four warps of a column half write the same bytes to the same place, so none waits for
-// another.  Two buffers by turns: a warp that has seen the accumulator of tile t + 2 knows that all warps are done with tile t.
+// the middle of the epilogue.  Each warp has a place of its own (bias_slice), so that nothing but its own __syncwarp orders
+// one tile's reads before the next tile's writes: the hand-back of an accumulator to the MMAs orders no memory.
+template <int TILE_N>
+__device__ __forceinline__ __half* bias_slice(uint64_t* bars, int epi_warp) {
+  return reinterpret_cast<__half*>(reinterpret_cast<uint8_t*>(bars) + kBarBytes) + epi_warp * (TILE_N / 2);
+}
 template <int TILE_N>
 struct BiasShare {
   static constexpr int kPerLane = TILE_N / 64;  // halves
@@ -270,9 +278,9 @@ struct BiasShare {
     else
       v[0] = __ldg(p);
   }
-  // (called by the whole warp)
-  __device__ __forceinline__ void put(__half* bias_s, int col_half, int lane) const {
-    __half* p = bias_s + col_half * (TILE_N / 2) + lane * kPerLane;
+  // (called by the whole warp, whose reads of the tile before are behind a __syncwarp)
+  __device__ __forceinline__ void put(__half* bias_s, int lane) const {
+    __half* p = bias_s + lane * kPerLane;
     if (kPerLane == 4)
       *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(v);
     else if (kPerLane == 2)
@@ -290,6 +298,14 @@ __device__ __forceinline__ void wait_accumulators_back(uint64_t* acc_empty, int 
     mbar_wait_anyway(&acc_empty[it & 1], (it >> 1) & 1, abort_flag, status, kStatusGemmMmaTimeout);
 }
 
+// Whether dynamic shared memory starts on the 1,024 bytes that the 128-byte swizzle needs, as it is declared to (there is
+// no room to round up).  If not, the launch computes nothing and the status word says so.
+__device__ __forceinline__ bool smem_aligned(const GemmArgs& args, const uint8_t* smem) {
+  const bool ok = (smem_u32(smem) & 1023u) == 0u;
+  if (!ok && threadIdx.x == 0 && args.status != nullptr) atomicCAS(args.status, 0, kStatusGemmProducerTimeout + 0x10);
+  return ok;
+}
+
 // ------------------------------------------------------------------------------------------
 // One CTA per SM, tile 128 x BLOCK_N.
 // ------------------------------------------------------------------------------------------
@@ -302,8 +318,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   constexpr bool kSplitK = (EPI == kEpiSplitKF32);
   constexpr bool kHasResidual = (EPI == BT_EPI_BIAS_RESIDUAL || EPI == BT_EPI_BIAS_RESIDUAL_F32OUT) || kSplitK;
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const bool smem_ok = smem_aligned(args, smem);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * Cfg::kStageBytes + Cfg::kStagingBytes);
   uint64_t* full_bar = bars;                    // [kStages]
   uint64_t* empty_bar = bars + kStages;         // [kStages]
@@ -362,7 +378,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   // requested before the wait for the kernel before (whose tail they then overlap): the first
   // `pre_kb` stages get their full byte count armed and their W part requested here, their A
   // part after the wait.
-  const int pre_kb = args.early_w ? (num_kb < kStages ? num_kb : kStages) : 0;
+  const int pre_kb = args.early_w && smem_ok ? (num_kb < kStages ? num_kb : kStages) : 0;
   if (warp == 0) {
     int n0 = 0, sp = 0;
     tile_cols(static_cast<int>(blockIdx.x), n0, sp);
@@ -397,6 +413,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     const int md = __ldg(args.m_dev);
     M = uniform_int(md < M ? md : M);
   }
+  if (!smem_ok) M = 0;
   const int m_tiles = (M + kBlockM - 1) / kBlockM;
   const int total_tiles = m_tiles * n_tiles * splits;
   // The li-th tile of this CTA: tiles go round-robin over the CTAs.  With split-K a tile is an
@@ -496,7 +513,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     const int quarter = warp & 3;  // TMEM lane quarter this warp may read
     const int col_half = e >> 2;   // which half of the tile's columns
     uint8_t* stg = smem + kStages * Cfg::kStageBytes + e * kStagingBytesPerWarp;  // 32 rows x 128 B, swizzled
-    __half* bias_bufs = reinterpret_cast<__half*>(reinterpret_cast<uint8_t*>(bars) + 256);
+    __half* bias_s = bias_slice<BLOCK_N>(bars, e);
     int m0 = 0, n0 = 0, sp = 0;
     for (int it = 0; tile_at(it, m0, n0, sp); ++it) {
       const int as = it & 1;
@@ -507,8 +524,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       if (EPI != BT_EPI_NONE) bias.load(args.bias, n0, col_half, lane);
       mbar_wait_anyway(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout);
       tc_fence_after();
-      __half* bias_s = bias_bufs + as * 256;
-      if (EPI != BT_EPI_NONE) bias.put(bias_s, col_half, lane);
+      if (EPI != BT_EPI_NONE) bias.put(bias_s, lane);
       if (warp == 2 && lane == 0) gstamp(args.timing, it, 2);
       epilogue_tile<BLOCK_N, EPI, Cfg::tma_store(EPI), 1>(args, &tm_out, stg, tmem_base + as * BLOCK_N, m0, n0, M, quarter,
                                                   col_half, lane, resv, reinterpret_cast<const uint4*>(bias_s), sp);
@@ -553,7 +569,8 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Hands an accumulator buffer back to the leader.  Relaxed: what the MMAs wait for is that reads of tensor memory are
-// done (tcgen05.wait::ld and the fences around the barrier); no bytes in memory go with it.  A release at cluster scope
+// done (tcgen05.wait::ld and the fences around the barrier); no bytes in memory go with it (what an epilogue warp keeps in
+// shared memory from tile to tile is its own).  A release at cluster scope
 // held the warp for 1-2.6k clocks per tile until its stores before were visible to the peer (18,944 x 3072 x 768 with
 // GELU 108.2 us, relaxed 102.3).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
@@ -587,11 +604,11 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   constexpr int kTileN = Cfg::kTileN;
   constexpr bool kHasResidual = (EPI == BT_EPI_BIAS_RESIDUAL || EPI == BT_EPI_BIAS_RESIDUAL_F32OUT);
 
-  extern __shared__ uint8_t smem_raw[];
   // Both CTAs of the pair must use identical shared-memory offsets (the MMA and the multicast
   // commit address the peer by offset); dynamic shared memory starts at the same offset in
-  // every CTA of a launch, so the same round-up applies to both.
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  // every CTA of a launch.
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const bool smem_ok = smem_aligned(args, smem);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * Cfg::kStageBytes + Cfg::kStagingBytes);
   uint64_t* full_bar = bars;                    // [kStages]  (leader's copy is the live one)
   uint64_t* empty_bar = bars + kStages;         // [kStages]
@@ -637,7 +654,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
   const int num_kb = args.K / kBlockK;
   // The leading W blocks of the pair's first tile ahead of the dependency wait, its A blocks right behind it (see
   // gemm_f16_kernel).  Both CTAs' copies complete on the leader's barrier, which the leader arms for both.
-  const int pre_kb = args.early_w ? (num_kb < kStages ? num_kb : kStages) : 0;
+  const int pre_kb = args.early_w && smem_ok ? (num_kb < kStages ? num_kb : kStages) : 0;
   auto load_w = [&](int stage, int n0, int kb) {
     uint8_t* sb = smem + stage * Cfg::kStageBytes + kABytes;
     const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0);
@@ -668,6 +685,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     const int md = __ldg(args.m_dev);
     M = uniform_int(md < M ? md : M);
   }
+  if (!smem_ok) M = 0;
   const int m_tiles = (M + 2 * kBlockM - 1) / (2 * kBlockM);
   const int total_tiles = m_tiles * n_tiles;
 
@@ -743,7 +761,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     const int quarter = warp & 3;
     const int col_half = e >> 2;
     uint8_t* stg = smem + kStages * Cfg::kStageBytes + e * (Cfg::kStagingBufs * kStagingBytesPerWarp);
-    __half* bias_bufs = reinterpret_cast<__half*>(reinterpret_cast<uint8_t*>(bars) + 256);
+    __half* bias_s = bias_slice<kTileN>(bars, e);
     int it = 0;
     for (int tile = cluster_id; tile < total_tiles; tile += num_clusters, ++it) {
       const int m0 = (tile / n_tiles) * (2 * kBlockM) + static_cast<int>(cta_rank) * kBlockM;
@@ -756,8 +774,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       if (EPI != BT_EPI_NONE) bias.load(args.bias, n0, col_half, lane);
       mbar_wait_anyway(&acc_full[as], aphase, abort_flag, args.status, kStatusGemmEpilogueTimeout);
       tc_fence_after();
-      __half* bias_s = bias_bufs + as * 256;
-      if (EPI != BT_EPI_NONE) bias.put(bias_s, col_half, lane);
+      if (EPI != BT_EPI_NONE) bias.put(bias_s, lane);
       if (warp == 2 && lane == 0) gstamp(args.timing, it, 2);
       epilogue_tile<kTileN, EPI, true, Cfg::kStagingBufs>(args, &tm_out, stg, tmem_base + as * kTileN, m0, n0, M,
                                                           quarter, col_half, lane, resv,
@@ -1155,19 +1172,14 @@ __device__ __forceinline__ void ln_statistics_loop(const GemmArgs& args, uint8_t
   }
 }
 
-// The rows that are there; none where shared memory does not start on the 1,024 bytes that the 128-byte swizzle needs
-// (there is no room to round up in the pair form).
+// The rows that are there; none where shared memory is not aligned.
 __device__ __forceinline__ int ln_rows(const GemmArgs& args, const uint8_t* smem) {
   int M = args.m_rows;
   if (args.m_dev != nullptr) {
     const int md = __ldg(args.m_dev);
     M = md < M ? md : M;
   }
-  if ((smem_u32(smem) & 1023u) != 0u) {
-    if (threadIdx.x == 0 && args.status != nullptr) atomicCAS(args.status, 0, kStatusGemmProducerTimeout + 0x10);
-    M = 0;
-  }
-  return uniform_int(M);
+  return uniform_int(smem_aligned(args, smem) ? M : 0);
 }
 
 template <int TILE_N>
