@@ -185,6 +185,18 @@ __device__ __forceinline__ bool mbar_wait_latched(bool ok, bool landed, uint64_t
   return mbar_wait_warp(bar, parity, abort_flag, status, code, max_cycles) && ok;
 }
 
+// Whether no role of the CTA will touch tensor memory any more: the MMA warp's question after its last tile.  It waits for
+// the epilogue to hand back the accumulators of the `tiles` tiles that were begun (`acc_empty`: two buffers by turns).
+// The answer is the CTA's flag: a wait that gives up raises it (or found it up), the MMA warp's own among them, and the
+// epilogue, which goes on after such a wait (mbar_wait_anyway) with loads of tensor memory and with arrivals that say
+// nothing, raises it ahead of them.  One answer for the warp.
+__device__ __forceinline__ bool accumulators_back(uint64_t* acc_empty, int tiles, volatile int* abort_flag, int* status, int code,
+                                                  long long max_cycles = (1ll << 31)) {
+  for (int it = tiles < 2 ? 0 : tiles - 2; it < tiles; ++it)
+    (void)mbar_wait_warp(&acc_empty[it & 1], (it >> 1) & 1, abort_flag, status, code, max_cycles);
+  return __all_sync(0xffffffffu, *abort_flag == 0) != 0;
+}
+
 // ------------------------------------------------------------ warp-uniform roles
 // tcgen05 and TMA instructions take their descriptors, addresses and coordinates from uniform registers.  In a
 // branch that one lane takes (`if (lane == 0)`) every operand of every instruction is moved there first, and that

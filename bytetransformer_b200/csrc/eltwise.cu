@@ -713,6 +713,33 @@ __global__ void __launch_bounds__(32) wait_forms_selftest_kernel(long long max_c
     out[3] = told;
   }
 }
+// accumulators_back after three tiles (buffer 0 handed back twice, buffer 1 once).  out[k] = lanes told that tensor memory
+// may go: k = 0 all came, 1 all came and the flag is up, 2 the last one of buffer 0 is missing, 3 no tile was begun.
+__global__ void __launch_bounds__(32) accumulators_back_selftest_kernel(long long max_cycles, long long* out) {
+  __shared__ uint64_t acc[2], late[2];
+  __shared__ int abort_flag_s;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&acc[i], 1);
+      mbar_init(&late[i], 1);
+    }
+    abort_flag_s = 0;
+    fence_mbar_init();
+    for (int it = 0; it < 3; ++it) mbar_arrive(&acc[it & 1]);
+    for (int it = 0; it < 2; ++it) mbar_arrive(&late[it & 1]);
+  }
+  __syncthreads();
+  for (int k = 0; k < 4; ++k) {
+    abort_flag_s = k == 1 ? 1 : 0;
+    __syncwarp();
+    const bool may_go = accumulators_back(k == 2 ? late : acc, k == 3 ? 0 : 3, &abort_flag_s, nullptr, 0, max_cycles);
+    const int told = __popc(__ballot_sync(0xffffffffu, may_go));
+    if (threadIdx.x == 0) out[k] = told;
+    __syncwarp();
+  }
+}
 }  // namespace
 
 cudaError_t launch_bounded_wait_selftest(int* status, long long max_cycles, int* gave_up, cudaStream_t stream) {
@@ -727,7 +754,20 @@ static cudaError_t launch_wait_forms_selftest(long long max_cycles, long long* o
   return launch_pdl(wait_forms_selftest_kernel, dim3(1), dim3(32), 0, stream, max_cycles, out);
 }
 
+static cudaError_t launch_accumulators_back_selftest(long long max_cycles, long long* out, cudaStream_t stream) {
+  if (max_cycles < 1024) max_cycles = 1024;
+  if (max_cycles > (1ll << 28)) max_cycles = (1ll << 28);
+  return launch_pdl(accumulators_back_selftest_kernel, dim3(1), dim3(32), 0, stream, max_cycles, out);
+}
+
 }  // namespace bt
+
+// Diagnostics hook (tests): see accumulators_back_selftest_kernel; `out_dev` holds four long long.
+extern "C" int bt_debug_selftest_accumulators_back(long long max_cycles, long long* out_dev, void* stream) {
+  if (out_dev == nullptr) return BT_ERR_INVALID_ARG;
+  return bt::launch_accumulators_back_selftest(max_cycles, out_dev, reinterpret_cast<cudaStream_t>(stream)) == cudaSuccess
+             ? BT_OK : BT_ERR_CUDA;
+}
 
 // Diagnostics hook (tests): see wait_forms_selftest_kernel; `out_dev` holds four long long.
 extern "C" int bt_debug_selftest_wait_forms(long long max_cycles, long long* out_dev, void* stream) {

@@ -31,7 +31,8 @@
 // M is read from device memory (the packed token count is only known on the device), so
 // the host never blocks; the grid is sized from the allocated rows.  Every mbarrier wait
 // is bounded: on expiry the CTA records a code in the status word and all roles drain to
-// a common exit that frees tensor memory.  No TMA load uses cluster multicast.
+// a common exit that frees tensor memory.  (The one-CTA kernels free it ahead of the exit where
+// no wait has run out: see accumulators_back.)  No TMA load uses cluster multicast.
 #include "common.cuh"
 #include "kernels.h"
 #include "../../include/bt_b200.h"
@@ -291,13 +292,6 @@ struct BiasShare {
   }
 };
 
-// The MMA warp's wait, after its last tile, for the epilogue to hand back the accumulators of the `tiles` tiles it began
-// (two buffers by turns; where a wait gave up, this one ends as quickly as all others).
-__device__ __forceinline__ void wait_accumulators_back(uint64_t* acc_empty, int tiles, volatile int* abort_flag, int* status) {
-  for (int it = tiles < 2 ? 0 : tiles - 2; it < tiles; ++it)
-    mbar_wait_anyway(&acc_empty[it & 1], (it >> 1) & 1, abort_flag, status, kStatusGemmMmaTimeout);
-}
-
 // Whether dynamic shared memory starts on the 1,024 bytes that the 128-byte swizzle needs, as it is declared to (there is
 // no room to round up).  If not, the launch computes nothing and the status word says so.
 __device__ __forceinline__ bool smem_aligned(const GemmArgs& args, const uint8_t* smem) {
@@ -424,6 +418,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
     m0 = tile_cols(tile, n0, sp) * kBlockM;
     return true;
   };
+  bool tmem_freed = false;  // (warp 1's answer)
 
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
@@ -503,9 +498,11 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
       }
       // Tensor memory goes back as soon as the accumulators have: at the end of the CTA it took 0.6k clocks of the
       // chain of kernels.
-      wait_accumulators_back(acc_empty, tiles, abort_flag, args.status);
-      tc_fence_after();
-      tmem_dealloc(tmem_base, Cfg::kTmemCols);
+      if (accumulators_back(acc_empty, tiles, abort_flag, args.status, kStatusGemmMmaTimeout)) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, Cfg::kTmemCols);
+        tmem_freed = true;
+      }
     }
   } else {
     // ------------------------------------------------------------------ epilogue
@@ -539,9 +536,13 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant_
   // ------------------------------------------------------------------ teardown
   __syncthreads();
   if (*abort_flag != 0) {
-    // A wait ran out somewhere: give copies that may still be in flight time to
-    // land before the CTA's shared memory is handed to another block.
+    // A wait ran out somewhere: give copies and MMAs that may still be in flight time to
+    // land before the CTA's shared and tensor memory are handed to another block.
     for (int i = 0; i < 64; ++i) __nanosleep(2000);
+    if (warp == 1 && !tmem_freed) {  // (what kept it from being freed raised the flag)
+      tc_fence_after();
+      tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    }
   }
 }
 
@@ -1192,9 +1193,9 @@ struct LnCfg {
 constexpr int kLnRingAndStaging = LnCfg<128>::kRingAndStaging;  // the largest of the three
 static_assert(LnCfg<192>::kRingAndStaging <= kLnRingAndStaging && LnCfg<256>::kRingAndStaging <= kLnRingAndStaging, "");
 
-// One width of gemm_f16_ln_kernel, from the barriers on.  `M` valid rows.
+// One width of gemm_f16_ln_kernel, from the barriers on.  `M` valid rows.  Warp 1 is told whether it has freed tensor memory.
 template <int TILE_N>
-__device__ __forceinline__ void ln_gemm_body(const CUtensorMap* tm_a, const CUtensorMap* tm_b, const CUtensorMap* tm_out,
+__device__ __forceinline__ bool ln_gemm_body(const CUtensorMap* tm_a, const CUtensorMap* tm_b, const CUtensorMap* tm_out,
                                              const CUtensorMap* tm_res, const GemmArgs& args, uint8_t* smem,
                                              uint64_t* bars, float* vec_s, uint32_t* tmem_slot,
                                              volatile int* abort_flag, int M, int warp, int lane) {
@@ -1257,6 +1258,7 @@ __device__ __forceinline__ void ln_gemm_body(const CUtensorMap* tm_a, const CUte
   }
 
   pdl_wait();  // see gemm_f16_kernel
+  bool tmem_freed = false;
 
   if (warp == 0) {
     // ------------------------------------------------------------- TMA producer
@@ -1321,9 +1323,11 @@ __device__ __forceinline__ void ln_gemm_body(const CUtensorMap* tm_a, const CUte
         if (lane == 0) gstamp(args.timing, it, 1);
         tiles = it + 1;
       }
-      wait_accumulators_back(acc_empty, tiles, abort_flag, args.status);
-      tc_fence_after();
-      tmem_dealloc(tmem_base, 512);
+      if (accumulators_back(acc_empty, tiles, abort_flag, args.status, kStatusGemmMmaTimeout)) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, 512);
+        tmem_freed = true;
+      }
     }
   } else if (warp < kLnFirstEpiWarp) {
     // ------------------------------------------------------- row statistics
@@ -1334,6 +1338,7 @@ __device__ __forceinline__ void ln_gemm_body(const CUtensorMap* tm_a, const CUte
     ln_epilogue_loop<TILE_N>(args, tm_out, tm_res, smem + kStages * Cfg::kStageBytes, ln_bars, vec_s, abort_flag,
                              tmem_base, M, warp, lane, tile_at, [&](int as) { mbar_arrive(&acc_empty[as]); });
   }
+  return tmem_freed;
 }
 
 __global__ void __launch_bounds__(kLnThreads, 1)
@@ -1367,17 +1372,22 @@ gemm_f16_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   }
   const int m_tiles = (M + kBlockM - 1) / kBlockM;
   const int tile_n = args.force_n != 0 ? args.force_n : ln_tile_n(m_tiles, args.N, args.K, static_cast<int>(gridDim.x));
+  bool tmem_freed = false;
   if (tile_n == 128)
-    ln_gemm_body<128>(&tm_a, &tm_b, &tm_out, &tm_res, args, smem, bars, vec_s, tmem_slot, abort_flag, M, warp, lane);
+    tmem_freed = ln_gemm_body<128>(&tm_a, &tm_b, &tm_out, &tm_res, args, smem, bars, vec_s, tmem_slot, abort_flag, M, warp, lane);
   else if (tile_n == 192)
-    ln_gemm_body<192>(&tm_a, &tm_b, &tm_out, &tm_res, args, smem, bars, vec_s, tmem_slot, abort_flag, M, warp, lane);
+    tmem_freed = ln_gemm_body<192>(&tm_a, &tm_b, &tm_out, &tm_res, args, smem, bars, vec_s, tmem_slot, abort_flag, M, warp, lane);
   else
-    ln_gemm_body<256>(&tm_a, &tm_b, &tm_out, &tm_res, args, smem, bars, vec_s, tmem_slot, abort_flag, M, warp, lane);
+    tmem_freed = ln_gemm_body<256>(&tm_a, &tm_b, &tm_out, &tm_res, args, smem, bars, vec_s, tmem_slot, abort_flag, M, warp, lane);
 
   // ------------------------------------------------------------------ teardown
   __syncthreads();
   if (*abort_flag != 0) {
     for (int i = 0; i < 64; ++i) __nanosleep(2000);
+    if (warp == 1 && !tmem_freed) {
+      tc_fence_after();
+      tmem_dealloc(*tmem_slot, 512);
+    }
   }
 }
 

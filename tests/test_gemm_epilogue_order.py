@@ -42,3 +42,31 @@ def test_bias_slices_lie_apart_and_inside(tile):
     own = tile // 2 * 2  # half of the tile's columns, two bytes each
     assert all(b - a >= own for a, b in zip(starts, starts[1:])) and starts[0] == 0 and starts[-1] + own <= size
     assert all(s % 16 == 0 for s in starts)  # read 16 bytes at a time
+
+
+@pytest.mark.parametrize("kernel", ["gemm_f16_kernel(const", "ln_gemm_body("])
+def test_tensor_memory_goes_early_only_where_no_wait_has_given_up(kernel):
+    """The epilogue goes on after a wait that gave up, and MMAs may be in flight then: the MMA warp may free tensor memory
+    ahead of the CTA's end only on the answer that every accumulator came back and nobody gave up."""
+    body = _body(kernel)
+    assert body.split("if (*abort_flag != 0)")[0].count("tmem_dealloc(") == 1
+    assert re.search(r"if \(accumulators_back\(acc_empty, tiles, abort_flag, args\.status, kStatusGemmMmaTimeout\)\) \{\s*"
+                     r"tc_fence_after\(\);\s*tmem_dealloc\([^;]*\);\s*tmem_freed = true;\s*\}", body)
+
+
+@pytest.mark.parametrize("kernel", ["gemm_f16_kernel(const", "gemm_f16_ln_kernel(const"])
+def test_tensor_memory_is_freed_behind_the_join_otherwise(kernel):
+    """Whatever keeps it from being freed early raises the flag, so the other place is behind the flag and the drain."""
+    body = _body(kernel)
+    end = body[body.rindex("__syncthreads();"):]
+    flag, drain = end.index("if (*abort_flag != 0) {"), end.index("__nanosleep(2000)")
+    free = end.index("if (warp == 1 && !tmem_freed) {")
+    assert flag < drain < free < end.index("tmem_dealloc(")
+    assert end.count("\n  }") == 1  # one block, the flag's
+
+
+@pytest.mark.parametrize("kernel", ["gemm_f16_pair_kernel(const", "gemm_f16_pair_ln_kernel(const"])
+def test_a_pair_frees_tensor_memory_behind_its_join(kernel):
+    body = _body(kernel)
+    assert body.count("tcgen05.dealloc") == 1
+    assert body.rindex("cluster_sync_all();") < body.index("tcgen05.dealloc")

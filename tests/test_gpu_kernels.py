@@ -666,3 +666,16 @@ def test_warp_waits_give_up_once_and_together(cuda_device):
     first, total, lanes, told = out.cpu().tolist()
     assert lanes == 0 and told == 0
     assert 1024 <= first <= total <= 4 * first, (first, total)  # polled again, the 63 others would be 63 batches
+
+
+def test_tensor_memory_may_go_only_where_every_wait_was_satisfied(cuda_device):
+    """What the GEMMs' MMA warp asks ahead of freeing tensor memory: yes if all accumulators came back (three tiles here, and
+    none), no if a wait of the CTA gave up meanwhile, no if one is missing."""
+    import ctypes as C
+
+    from bytetransformer_b200 import _abi
+    fn = _abi.load().bt_debug_selftest_accumulators_back
+    fn.restype, fn.argtypes = C.c_int, [C.c_longlong, C.c_void_p, C.c_void_p]
+    out = torch.full((4,), -1, dtype=torch.int64, device=cuda_device)
+    assert fn(1024, out.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    assert out.cpu().tolist() == [32, 0, 0, 32]
