@@ -823,6 +823,7 @@ struct MhaPersistentArgs {
   int max_len;  // upper bound of every sequence length
   int tma_out;  // the kernel's second tensor map describes ctx: whole 32-row output slabs leave by bulk store
   int early_offsets;  // batch_idx may be read before the dependency wait (see launch_mha)
+  int take_over;  // the grid has more blocks than are resident
 };
 
 // Finds item n = (sequence b, query tile qt, head h); items are numbered sequence by sequence, inside
@@ -919,7 +920,7 @@ constexpr int kItemSlots = 4;         // items between the loader and the other 
 // Q, K, V rings, the softmax warps' output staging (4 x 32 rows x 128 B), barriers and items
 constexpr int kPersistentSmemBytes = 3 * kPersistentStages * kTileBytes + kTileBytes + 512;
 
-// MORE: the grid has more blocks than can be resident, CTAs take over waiting ones.  (Without: one item per CTA.)
+// MORE: a CTA may work on several items.  (Without: a block for every item there could be, one item per CTA.)
 template <bool MORE>
 __global__ void __launch_bounds__(kPersistentThreads, 2)
 mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_ctx,
@@ -1023,23 +1024,29 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
       uint32_t phase = 0;
       bool ok = true;
       int cur_b = 0, cur_first = 0;
-      bool more = MORE;  // blocks of the grid may still be waiting
+      int item = static_cast<int>(blockIdx.x);  // the one being worked on
       uint32_t asked = 0;
-      bool have = own_item(cur_b, cur_first);
+      bool have = own_item(cur_b, cur_first);  // (if not: the blocks behind have none either, and the other roles are done)
       // The grid is sized from an upper bound of the items; a block beyond the last one is taken over as well (cheaper
-      // than letting it start) and the next one asked for.
+      // than letting it start) and the next one asked for.  Offsets that fall can hold more items than the bound: the CTA
+      // that has the last block goes on with those, and looks at all offsets that way.
       auto take_next = [&]() {
-        have = false;
-        while (more && !have) {
-          if (elect_one()) launch_control_ask(taken, taken_full);
-          if (!mbar_wait_role(taken_full, asked++ & 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) return;
-          const int next = uniform_int(launch_control_answer(taken));
-          more = next >= 0;
-          if (more) have = decode_item(args, next, cur_b, cur_first, seq_start, L, qt, head);
-        }
+        const int blocks = static_cast<int>(gridDim.x);
+        do {
+          have = false;
+          if (item + 1 < blocks) {
+            if (!args.take_over) return;
+            if (elect_one()) launch_control_ask(taken, taken_full);
+            if (!mbar_wait_role(taken_full, asked++ & 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) return;
+            item = uniform_int(launch_control_answer(taken));
+            if (item < 0) return;
+          } else {
+            ++item;
+          }
+          have = decode_item(args, item, cur_b, cur_first, seq_start, L, qt, head);
+        } while (!have && item < blocks);
       };
       if (args.early_offsets) pdl_wait();
-      if (!have) more = false;  // no item of its own: the blocks behind it have none either, and the other roles are done
       for (uint32_t n = 0; have; ++n) {
         L = uniform_int(L);
         seq_start = uniform_int(seq_start);
@@ -1070,7 +1077,7 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
         if (!ok) break;
         // The next item: asked for once this one's last loads are out, i.e. while its last two key tiles are worked on,
         // and not before, so that a CTA with long items does not hold others back.
-        if (!more) break;
+        if (!MORE) break;
         take_next();
         const uint32_t slot = n % kItemSlots;
         if (!mbar_wait_role(&item_empty[slot], item_parity(n) ^ 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) break;
@@ -1423,13 +1430,17 @@ cudaError_t launch_persistent(const MhaLaunch& a, cudaStream_t stream) {
   args.tma_out = a.has_tm_ctx ? 1 : 0;
   args.early_offsets = a.early_offsets ? 1 : 0;
   // A block per item, by an upper bound: tiles of sequences of max_len, or of sequences that share `rows` rows (each a
-  // fraction of a tile beyond its share).
+  // fraction of a tile beyond its share).  The second bound holds for offsets that rise, so it only counts where a CTA can
+  // have several items (see take_next).
   long long tiles = static_cast<long long>(a.batch) * ((a.max_len + kQRows - 1) / kQRows);
+  const long long resident = 2LL * sms[dev];
+  const bool more = tiles * a.head_num > resident;
   const long long by_rows = (a.rows + static_cast<long long>(a.batch) * (kQRows - 1)) / kQRows;
-  if (tiles > by_rows) tiles = by_rows;
+  if (more && tiles > by_rows) tiles = by_rows;
   const long long grid = tiles > 0 ? tiles * a.head_num : 1;
   if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
-  auto kern = grid > 2LL * sms[dev] ? mha_persistent_kernel<true> : mha_persistent_kernel<false>;
+  args.take_over = grid > resident ? 1 : 0;
+  auto kern = more ? mha_persistent_kernel<true> : mha_persistent_kernel<false>;
   return launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(kPersistentThreads), kPersistentSmemBytes,
                     stream, a.tm_qkv, a.has_tm_ctx ? a.tm_ctx : a.tm_qkv, args);
 }

@@ -538,6 +538,51 @@ def test_attention_rejects_offsets_outside_the_allocation(enc, cuda_device, kern
     assert enc.device_status() == 0
 
 
+@pytest.mark.parametrize("repeats,max_len,kernel", [
+    (3, 500, 3), (3, 1024, 3), (20, 500, 3), (3, 500, 1), (20, 500, 1),
+], ids=["one_item_per_block", "blocks_all_resident", "blocks_taken_over", "cta_per_item", "cta_per_item_many"])
+def test_attention_offsets_that_fall_hide_no_sequence(enc, cuda_device, repeats, max_len, kernel):
+    """Where offsets fall, sequences can share rows, and there can be more items than rising offsets would give for
+    these rows.  The last sequence, which shares none, still comes out, as do the repeated ones."""
+    from bytetransformer_b200 import _abi
+    from oracle.bert_oracle import attention_packed
+    cu = [0, 500] * repeats + [600]
+    g = torch.Generator().manual_seed(repeats)
+    qkv = torch.randn(600, 3 * enc.hidden, generator=g).half()
+    want = attention_packed(qkv.float(), [0, 500, 600], enc.head_num, enc.head_size)
+    lib = _abi.load()
+    lib.bt_debug_set_mha_tiles(kernel)
+    try:
+        got = enc.attention(qkv.to(cuda_device), torch.tensor(cu, dtype=torch.int32, device=cuda_device), max_len)
+        assert enc.device_status() == 0x301
+    finally:
+        lib.bt_debug_set_mha_tiles(0)
+    assert_close_fp16(got, want, f"attention, {repeats} falls", max_abs=5e-3, mean_abs=3e-4)
+
+
+@pytest.mark.parametrize("n", [1, 32, 33, 64, 200])
+@pytest.mark.parametrize("kernel", [1, 3], ids=["cta_per_item", "persistent"])
+def test_attention_reports_a_fall_behind_the_last_item(cuda_device, n, kernel):
+    """n sequences of one token (whose output is its V row), then an offset that falls: there are as many items as rising
+    offsets would give, and the fall stands behind the last one, out of sight of the blocks that look for theirs."""
+    from bytetransformer_b200 import _abi
+    from bytetransformer_b200.encoder import Encoder
+    from helpers import make_layer_weights, to_device_weights
+    g = torch.Generator().manual_seed(n)
+    enc = Encoder(4, 64, [to_device_weights(make_layer_weights(256, g), cuda_device)])
+    qkv = torch.randn(n, 3 * enc.hidden, generator=g).half()
+    lib = _abi.load()
+    lib.bt_debug_set_mha_tiles(kernel)
+    try:
+        cu = torch.tensor(list(range(n + 1)) + [n // 2], dtype=torch.int32, device=cuda_device)
+        got = enc.attention(qkv.to(cuda_device), cu, 1)
+        assert enc.device_status() == 0x301
+    finally:
+        lib.bt_debug_set_mha_tiles(0)
+    assert torch.equal(got.cpu(), qkv[:, 2 * enc.hidden:])
+    enc.close()
+
+
 @pytest.mark.parametrize("M,N,K,gb32,m_valid", [
     (128, 256, 64, False, None), (333, 768, 768, False, None), (1000, 768, 3072, True, None),
     (18944, 768, 768, False, None), (700, 1024, 1024, True, 555), (40000, 768, 768, False, 39999), (130, 512, 128, False, 0),
