@@ -397,6 +397,65 @@ def test_attention_tail_tiles(enc, cuda_device, n):
     assert_close_fp16(got, want, f"attention tail {n}", max_abs=5e-3, mean_abs=3e-4)
 
 
+@pytest.mark.parametrize("tail", [1, 31, 32, 33, 63, 64, 65, 95, 96, 97, 111, 112, 113, 127])
+@pytest.mark.parametrize("before", [0, 128], ids=["alone", "behind_a_whole_tile"])
+def test_attention_tail_tiles_of_the_persistent_kernel(enc, cuda_device, tail, before):
+    """Its loop over the 32-key chunks of a partial last key tile, every chunk the last one, whole and not; the second
+    sequence must not be touched by the first one's tail."""
+    from bytetransformer_b200 import _abi
+    from oracle.bert_oracle import attention_packed
+    n = before + tail
+    g = torch.Generator().manual_seed(n)
+    cu = [0, n, n + 3]
+    qkv = (torch.randn(n + 3, 3 * enc.hidden, generator=g) * 1.5).half()  # (a sharp softmax: the reference moves)
+    lib = _abi.load()
+    lib.bt_debug_set_mha_tiles(3)
+    try:
+        got = enc.attention(qkv.to(cuda_device), torch.tensor(cu, dtype=torch.int32, device=cuda_device), n + 3)
+    finally:
+        lib.bt_debug_set_mha_tiles(0)
+    want = attention_packed(qkv.float(), cu, enc.head_num, enc.head_size)
+    assert enc.device_status() == 0
+    assert_close_fp16(got, want, f"attention tail {before} + {tail}", max_abs=8e-3, mean_abs=4e-4)
+
+
+@pytest.mark.parametrize("bad", [None, 9, 63], ids=["sound", "one_bad_offset", "bad_end"])
+def test_attention_blocks_that_are_taken_over(enc, cuda_device, bad):
+    """1824 items for 2232 blocks, of which 296 start by themselves: CTAs take over five or more (the ring
+    between the roles holds four), blocks without an item among them.  Empty sequences, and one whose offset is bad, are
+    stepped over; twice, bit-identical."""
+    from bytetransformer_b200 import _abi
+    from oracle.bert_oracle import attention_packed
+    lens = np.random.RandomState(11).randint(1, 600, 64)
+    lens[[0, 5, 17, 18, 19, 40]] = 0
+    lens[30] = 1024
+    cu = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    T = int(cu[-1])
+    blocks = min(64 * 8, (T + 64 * 127) // 128) * enc.head_num
+    items = int(((lens + 127) // 128).sum()) * enc.head_num
+    assert (items, blocks) == (1824, 2232)
+    g = torch.Generator().manual_seed(64)
+    qkv = torch.randn(T, 3 * enc.hidden, generator=g).half()
+    want = attention_packed(qkv.float(), cu.tolist(), enc.head_num, enc.head_size)
+    rows = torch.ones(T, dtype=torch.bool)
+    if bad is not None:   # the sequences before and behind it are left out
+        for b in (bad - 1, bad):
+            rows[cu[b]:cu[b + 1]] = False
+        cu[bad] = -1
+    dev = [t.to(cuda_device) for t in (qkv, torch.from_numpy(cu))]
+    lib = _abi.load()
+    lib.bt_debug_set_mha_tiles(3)
+    try:
+        got = enc.attention(*dev, 1024)
+        again = enc.attention(*dev, 1024)
+    finally:
+        lib.bt_debug_set_mha_tiles(0)
+    assert enc.device_status() == (0 if bad is None else 0x301)
+    assert torch.equal(got, again)
+    assert_close_fp16(got[rows.to(cuda_device)], want[rows], "attention, blocks taken over", max_abs=5e-3, mean_abs=3e-4)
+    assert got[~rows.to(cuda_device)].abs().sum().item() == 0.0
+
+
 def test_attention_twice_bit_identical(enc, cuda_device):
     lens = [300, 77, 129]
     cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]).astype(np.int32), device=cuda_device)
@@ -639,6 +698,21 @@ def test_fused_layernorm_tile_widths(enc, cuda_device, M, K, gb32, m_valid, widt
     lib.bt_debug_set(4, width)
     try:
         _fused_layernorm_case(enc, cuda_device, M, 768, K, gb32, m_valid)
+    finally:
+        lib.bt_debug_set(4, 0)
+        lib.bt_debug_set(9, 0)
+
+
+@pytest.mark.parametrize("N", [256, 512, 1024])
+@pytest.mark.parametrize("M,K,gb32,m_valid", [(129, 768, True, None), (300, 448, False, 257), (4801, 256, False, None)])
+def test_fused_layernorm_narrowest_tiles(enc, cuda_device, M, N, K, gb32, m_valid):
+    """Tiles of 128 columns of the one-CTA GEMM + LayerNorm kernel: two, four and eight partials to a row."""
+    from bytetransformer_b200 import _abi
+    lib = _abi.load()
+    lib.bt_debug_set(9, 2)
+    lib.bt_debug_set(4, 128)
+    try:
+        _fused_layernorm_case(enc, cuda_device, M, N, K, gb32, m_valid)
     finally:
         lib.bt_debug_set(4, 0)
         lib.bt_debug_set(9, 0)
