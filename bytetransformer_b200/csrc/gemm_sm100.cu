@@ -1737,9 +1737,13 @@ cudaError_t launch_pair_ln_gemm(const GemmLaunch& g, const GemmArgs& a, cudaStre
 // 54.6 / 51.2, 75,776 300 / 269; K = 768: 18,944 rows (four waves) 28.9 / 30.2, 28,000 41.2 / 40.3, 75,776 101 / 98.  1024
 // columns (no 192; one wave is up to 4,736 rows), K = 4096: 4,100 rows 38.9 / 41.0, 6,200 74.5 / 60.3; K = 1024: 4,100 rows
 // 22.7 / 24.5, 6,400 32.6 / 32.4, 12,500 38.4 / 36.0.  512 columns, K = 2048: 9,400 rows 22.3 / 23.3, 12,500 34.5 / 31.9.
+// With a single column tile (256 columns) a long K is what counts, from more than one tile per SM pair on: K = 4096, 11,000
+// rows 38.1 / 32.3, 18,944 46.1 / 40.2; K = 3072 28.8 / 25.5 and 37.6 / 34.0; K = 2048 19.9 / 20.6 and 25.0 / 22.6; 9,400
+// rows, one wave of 128-column tiles, K = 3072 17.4 / 25.2.
 bool ln_pair_pays(int m_rows, int N, int K, int num_sms) {
   const long long m_tiles = (m_rows + kBlockM - 1) / kBlockM;
   if (N % 192 == 0) return m_tiles * (N / 192) > (K >= 2048 ? 2LL : 4LL) * num_sms;
+  if (N == 256 && K >= 2048) return 2 * m_tiles > num_sms;
   return m_tiles * (N / 256) > num_sms;
 }
 
@@ -1910,7 +1914,8 @@ extern "C" int bt_debug_set_gemm_timing(long long* device_buffer) {
 }
 // Host-side shape policies, callable without a device (tests): what 0 = tile width of the one-CTA
 // kernel, 1 = K ranges of an fp32-sum GEMM, 2 = 1 if the pair kernel would take a bias-only GEMM, 3 = rows per CTA of
-// LayerNorm over N columns, K partial sums, inside a forward (4: by itself), 5 = as 0 where every row is valid.
+// LayerNorm over N columns, K partial sums, inside a forward (4: by itself), 5 = as 0 where every row is valid, 6 = 1 if GEMM +
+// LayerNorm runs on SM pairs.
 extern "C" int bt_debug_policy(int what, int m_rows, int N, int K, int num_sms) {
   switch (what) {
     case 0: return bt::gemm_pick_block_n(m_rows, N, K, num_sms, false);
@@ -1927,6 +1932,7 @@ extern "C" int bt_debug_policy(int what, int m_rows, int N, int K, int num_sms) 
       return bt::use_pair_kernel(g) ? 1 : 0;
     }
     case 3: case 4: return bt::ln_rows_per_cta(m_rows, N, K, what == 3);
+    case 6: return bt::ln_pair_pays(m_rows, N, K, num_sms) ? 1 : 0;
     default: return -1;
   }
 }

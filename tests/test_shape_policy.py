@@ -109,3 +109,16 @@ def test_layernorm_inside_the_gemm_saves_a_second_wave_of_narrow_tiles(policy, t
     for rows in (tiles * 128, tiles * 128 - 127):
         assert fn(rows, hidden, SMS, 1) == all_rows
         assert fn(rows, hidden, SMS, 0) == padded
+
+
+@pytest.mark.parametrize("tiles,N,K,pair", [
+    (74, 768, 3072, 0), (75, 768, 3072, 1),              # two waves of 192-column tiles
+    (148, 768, 768, 0), (149, 768, 768, 1),              # four, where K is short
+    (74, 512, 2048, 0), (75, 512, 2048, 1), (75, 512, 512, 1),
+    (37, 1024, 4096, 0), (38, 1024, 4096, 1),
+    (148, 256, 1024, 0), (149, 256, 1024, 1),
+    (74, 256, 2048, 0), (75, 256, 2048, 1), (148, 256, 4096, 1),  # one column tile and a long K
+])
+def test_layernorm_gemm_on_sm_pairs(policy, tiles, N, K, pair):
+    for rows in (tiles * 128, tiles * 128 - 127):
+        assert policy(6, rows, N, K, SMS) == pair
