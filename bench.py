@@ -38,11 +38,11 @@ METRIC = "bert_base_12L_packed_tokens_per_sec"
 UNIT = "tokens/s"
 WORKLOAD = "whole_box_1024x1024"
 # dram__bytes_read.sum + dram__bytes_write.sum per GEMM launch and packed token, mean of the four GEMMs of a layer,
-# from the two ncu captures summarised in profiles/gemm_kernels_microbatch18k.txt (18,645 tokens per launch: 95.2 MB)
-# and profiles/gemm_kernels_microbatch76k.txt (70,734 tokens: 456.4 MB).  The algorithmic bytes of the same launches
+# from the two ncu captures summarised in profiles/gemm_kernels_microbatch18k.txt (18,645 tokens per launch: 94.7 MB)
+# and profiles/gemm_kernels_microbatch76k.txt (70,734 tokens: 456.0 MB).  The algorithmic bytes of the same launches
 # are 7,100 per token; DRAM sees less because a kernel's output is partly still in the 126 MB L2 when the next
 # kernel reads it, the more so the smaller the launch.  Between the two launch sizes the figure is interpolated.
-GEMM_DRAM_BYTES_PER_TOKEN = ((18645, 95.2e6 / 18645), (70734, 456.4e6 / 70734))
+GEMM_DRAM_BYTES_PER_TOKEN = ((18645, 94.7e6 / 18645), (70734, 456.0e6 / 70734))
 
 
 def gemm_dram_bytes_per_launch(tokens_per_launch: float) -> float:
@@ -344,7 +344,7 @@ def main():
         achieved = gemm_flops / (gemm_ms / 1000.0) / 1e12
         # per launch, like `achieved`: this rank's tokens per micro-batch times the captured per-token figure
         traffic = gemm_dram_bytes_per_launch(my_tokens / max(1, len(runner.batches))) if not args.layers else None
-        roofline = {"bound": "tensor", "kernel": "the four GEMMs of a layer: gemm_f16_pair_kernel (QKV, FFN1 + GELU), gemm_f16_ln_kernel (attention output and FFN2, with LayerNorm)", "achieved": achieved,
+        roofline = {"bound": "tensor", "kernel": "the four GEMMs of a layer: gemm_f16_pair_kernel (QKV, FFN1 + GELU), gemm_f16_pair_ln_kernel or gemm_f16_ln_kernel (attention output and FFN2, with LayerNorm)", "achieved": achieved,
                     "peak": peaks["tflops"], "unit": "TFLOP/s", "frac": achieved / peaks["tflops"],
                     "peak_source": peaks["source"] + " sustained bf16 dense", "traffic": traffic,
                     "launches": int(gemm_launches), "avg_launch_ms": gemm_ms / max(1, gemm_launches)}

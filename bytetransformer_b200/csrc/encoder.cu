@@ -125,16 +125,15 @@ struct bt_encoder_s {
   long long launches[BT_PROF_KINDS] = {};
   bool prof_on = false;
   // LayerNorm inside the attention-output / FFN2 GEMM kernel (bt_debug_set_fused_layernorm):
-  // 0 never, 1 from `fused_ln_min_tiles` 128-row tiles (of allocated rows) upwards, 2 always.  With few row tiles the
-  // exchange of row statistics between CTAs lengthens the only wave by more than the saved LayerNorm launch and fp32
-  // round trip.  What counts is the valid rows, which the host only knows where every row is computed.  Measured on
-  // B200, 12 layers, us per forward without / with the fused kernels.  Every row computed (packed and general-mask
-  // entries), hidden 768: 28 tiles 1245 / 1182, 32 tiles 1280 / 1203, 37 tiles 1452 / 1340; hidden 1024: 32 tiles
-  // 1813 / 1732, 36 tiles 1923 / 1884, 37 tiles 1881 / 2098, 38 tiles 2184 / 2085; hidden 512: 32 tiles 874 / 933,
-  // 37 tiles 965 / 1023, 38 tiles 1055 / 1031; hidden 256: 32 tiles 505 / 599, 39 tiles 613 / 658.  Padded batches, hidden
-  // 768 (measured before LayerNorm of many rows shared CTAs): 40 tiles with 2676, 2989 and 3299 valid rows 1021 / 1082,
-  // 1072 / 1155 and 1312 / 1183, 43 tiles with 3411 1241 / 1173, 48 tiles with 4382 1357 / 1262, 64 tiles with 3970
-  // 1313 / 1231: the line of 40 goes by allocated rows and loses 6-8 % where few of them are valid.
+  // 0 never, 1 by the lines below and fused_ln_saves_a_wave (see fuse_ln), 2 always.  With few row tiles the exchange of
+  // row statistics between CTAs lengthens the only wave by more than the saved LayerNorm launch and fp32 round trip.  What
+  // counts is the valid rows, which the host only knows where every row is computed.  The lines were set with an earlier
+  // fused kernel; with the present one they err towards the separate kernels.  us per forward of 12 layers on B200,
+  // separate / fused, every row computed (packed and general-mask entries).  768 columns: 25 row tiles 983 / 867, 28 1047 /
+  // 900, 31 1111 / 952, 32 1128 / 966, 40 1304 / 1183; 1024: 19 1181 / 1126, 31 1636 / 1480, 32 1631 / 1496, 37 1781 /
+  // 1674, 38 2002 / 1748; 512: 37 775 / 662, 38 845 / 773; 256: 32 413 / 411, 36 445 / 420, 39 498 / 447, 40 515 / 451.
+  // Padded batches of 40 tiles, valid share 0.1 / 0.3 / 0.6 / 1: 768 columns 690 / 600, 756 / 654, 993 / 871, 1265 / 1159;
+  // 1024: 959 / 824, 1094 / 949, 1382 / 1221, 1995 / 1749.
   int fused_ln = 1;
   int fused_ln_min_tiles = 40;           // some rows are padding
   int fused_ln_min_tiles_all_rows = 32;  // every allocated row is computed (and see fused_ln_pays)
@@ -371,10 +370,10 @@ static int run_mha(bt_handle h, const __half* qkv, __half* ctx, const int* batch
   return BT_OK;
 }
 
-// Whether LayerNorm rides in the attention-output / FFN2 GEMM kernels (row tiles of H / 256 CTAs each): below, the
-// narrow-tile GEMM followed by the row kernel spreads the few rows over more SMs.  Where every allocated row is computed
-// that holds from fewer tiles on, if the CTAs are more than half of the SMs - except where the plain GEMM's tiles are just
-// one wave and the clusters, which cannot use every SM, are two (1024 columns, 37 tiles).
+// The lines on row tiles from which LayerNorm rides in the attention-output / FFN2 GEMM kernels.  Where every allocated row
+// is computed they lie lower, if the tiles of 256 columns are more than half of the SMs - except where those are just one
+// wave.  (Both conditions were measured with an earlier fused kernel, see fused_ln_min_tiles; where they say no,
+// fused_ln_saves_a_wave has its say.)
 static bool fused_ln_pays(long long row_tiles, int H, int num_sms, bool all_rows, int min_tiles, int min_tiles_all_rows) {
   if (row_tiles >= min_tiles) return true;
   const long long ctas = row_tiles * (H / 256);
@@ -390,12 +389,17 @@ static bool want_fused_ln(bt_handle h, long long rows) {
 }
 
 // Below that line it pays as soon as the GEMMs of fp32 sums, whose tiles are then 64 columns wide, would need a second wave:
-// the fused kernel's tiles of 128 columns need one.  Where some rows are padding, three fifths are taken to be valid (and
-// the fused kernel fits its tiles to the rows that are there, see ln_tile_n).  us per forward of 12 layers, separate / fused.
-// Every row computed, 768 columns: 12 row tiles 585 / 603, 13 719 / 649; 1024: 9 656 / 692, 10 812 / 763; 512: 18 516 / 518,
-// 19 602 / 552.  Padded, allocated row tiles (valid ones): 768: 20 (12) 575 / 602, 22 (14) 732 / 644; 1024: 16 (9) 629 /
-// 678, 18 (11) 832 / 746; 512: 28 (17) 513 / 525, 32 (19) 621 / 546.  Between one wave of 128-column tiles and the line
-// above, where every row is computed, the separate kernels are kept.
+// the fused kernel's tiles of 128 columns need one.  us per forward of 12 layers, separate / fused, every row computed: 768
+// columns: 12 row tiles 575 / 591, 13 705 / 628, 24 844 / 790; 1024: 9 640 / 679, 10 791 / 732, 18 1061 / 958; 512: 18 504 /
+// 506, 19 593 / 535, 36 733 / 634.  Between one wave of 128-column tiles and the line above, where every row is computed, the
+// separate kernels are kept.
+// Where some rows are padding, three fifths are taken to be valid, the mean of the usual batches; the fused kernel fits its
+// tiles to the rows that are there (see ln_tile_n).  What that costs at other shares: below the line full batches lose, 768
+// columns, 13 tiles, share 0.6 / 0.8 / 1: 522 / 540, 573 / 594, 723 / 623; 16 tiles 565 / 582, 726 / 637, 735 / 640; above it
+// sparse ones, 22 tiles, share 0.1 / 0.45 / 0.6 / 1: 533 / 544, 572 / 589, 727 / 636, 805 / 714, from
+// 26 tiles on none: 607 / 573, 653 / 614, 697 / 656, 987 / 865.  1024 columns: 16 tiles, share 0.45 / 0.6 / 1 612 / 656, 812 /
+// 728, 998 / 869; 18 tiles, share 0.1 / 0.45 / 0.6 / 1 581 / 623, 626 / 668, 832 / 736, 1073 / 863; 24 tiles 688 / 664, 796 /
+// 754, 917 / 847, 1290 / 1134.
 static bool fused_ln_saves_a_wave(long long row_tiles, int H, int num_sms, bool all_rows) {
   const long long there = all_rows ? row_tiles : row_tiles * 3 / 5;
   if (H < 512 || (all_rows && row_tiles * (H / 128) >= num_sms)) return false;

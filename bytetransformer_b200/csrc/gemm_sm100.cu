@@ -90,7 +90,7 @@ struct GemmArgs {
   int K;
   int* status;
   // fused LayerNorm (BT_EPI_BIAS_RESIDUAL_LAYERNORM): `out` is the scratch for the row
-  // statistics partials (8 * N/128 bytes per row), `out_ln` the fp16 result
+  // statistics partials (up to 16 * N/128 bytes per row), `out_ln` the fp16 result
   __half* out_ln;
   const void* gamma;
   const void* beta;
@@ -1821,13 +1821,14 @@ int gemm_pick_block_n(int m_rows, int N, int K, int num_sms, bool all_rows) {
     if (N % bn != 0) continue;
     const long long tiles = static_cast<long long>(m_tiles) * (N / bn);
     if (tiles < num_sms) continue;
-    // A 128-column tile's main loop takes hardly longer than a 64-column one's (64 against 54 clocks per MMA), so
-    // with a long K a second wave of 64-column tiles that 128-column ones do not need is the dearer choice.  us per launch
-    // of an fp32-sum GEMM with 64- / 128-column tiles over the range of the rule: N = 768, K = 3072, 13 row tiles
-    // 24.7 / 16.8, 18 25.0 / 17.4, 24 25.7 / 18.4 (12, one wave of either: 15.6 / 16.6); N = 768, K = 2048 18.7 / 13.4 to
-    // 19.8 / 14.9; N = 1024, K = 4096, 10 to 18 row tiles 30.7 / 20.2 to 31.6 / 22.0; N = 512, K = 2048, 19 to 37
-    // 18.7 / 13.4 to 19.8 / 14.9.  Only where every row is valid: padded rows make no tiles, and 16 sequences of up to 128
-    // tokens, 192 tiles of 64 columns by their rows and 120 by their tokens, lose 2 % of the forward with 128-column tiles.
+    // With a long K a second wave of 64-column tiles that 128-column ones do not need is the dearer choice (a K block takes
+    // 225 and 290 clocks).  us per launch of an fp32-sum GEMM with 64- / 128-column tiles: N = 640, K = 2560, 15 row tiles
+    // 14.2 / 11.2, 24 15.2 / 11.6 (14, one wave of either: 9.2 / 11.5); N = 896, K = 3584, 11 to 20 18.4 / 13.8 to 18.9 /
+    // 14.9; N = 768, K = 3072, 13 to 24 16.5 / 12.6 to 17.1 / 13.3; N = 1024, K = 4096, 10 to 18 20.0 / 14.9 to 20.7 / 15.8;
+    // N = 512, K = 2048, 19 12.5 / 10.1.  (At 512, 768 and 1024 columns a forward has LayerNorm inside the GEMM by then: the
+    // rule is left to the other widths and to GEMMs by themselves.)  Only where every row is valid: padded rows make no
+    // tiles, and 16 sequences of up to 128 tokens, 192 tiles of 64 columns by their rows and 120 by their tokens, lost 2 %
+    // of the forward with 128-column tiles.
     if (bn == 64 && all_rows && K >= 2048 && N % 128 == 0 && tiles > num_sms) return 128;
     return bn;
   }
@@ -1879,10 +1880,7 @@ cudaError_t launch_gemm(const GemmLaunch& g, cudaStream_t stream) {
     a.idesc = make_idesc_f16(256, 256, 0, 1);  // M = 256 across the pair
     return launch_pair_epi(g, a, stream);
   }
-  if (g.epilogue == BT_EPI_BIAS_RESIDUAL_LAYERNORM) {
-    a.idesc = make_idesc_f16(kBlockM, 256, 0, 1);
-    return launch_ln_gemm(g, a, stream);
-  }
+  if (g.epilogue == BT_EPI_BIAS_RESIDUAL_LAYERNORM) return launch_ln_gemm(g, a, stream);
   int bn = g.block_n != 0 ? g.block_n : gemm_pick_block_n(g.m_rows, g.N, g.K, g.num_sms, g.all_rows);
   if (bn == 0 || g.N % bn != 0) return cudaErrorInvalidValue;
   a.idesc = make_idesc_f16(kBlockM, bn, 0, 1);
@@ -1906,8 +1904,9 @@ cudaError_t launch_gemm(const GemmLaunch& g, cudaStream_t stream) {
 // 9 = GEMM + LayerNorm on SM pairs (0, the default: by ln_pair_pays; 1 always; 2 never).
 // value 0 restores the default for keys 1-5 and 7.
 // Device buffer of 148 x 16 x 8 long long for clock64 stamps of the GEMM kernels (null = off):
-// slots 0/1 MMA warp (accumulator free, last commit), 2/3 epilogue warp 2 (accumulator ready, tile
-// done), 4..6 LayerNorm kernel only (sums written back, partial published, partials of all peers seen).
+// slots 0/1 MMA warp (accumulator free, last commit), 2/3 first epilogue warp (accumulator ready, tile
+// done), 4..6 LayerNorm kernels only (4 first epilogue warp: its partials are in shared memory, 5 statistics warp 2:
+// partials published, 6 first epilogue warp: mean and 1 / deviation have arrived).
 extern "C" int bt_debug_set_gemm_timing(long long* device_buffer) {
   bt::g_dbg_gemm_timing = device_buffer;
   return 0;

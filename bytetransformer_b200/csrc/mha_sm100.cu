@@ -5,10 +5,9 @@
 // bytetransformer/src/attention_fused_long.cu:171-312 and the grouped-GEMM path
 // of bytetransformer/src/cutlass_attention.cu:150-210 for long ones).  Two kernels:
 //   mha_fwd_kernel         one CTA per (128 query rows, head, sequence), 192 threads, two CTAs per SM.
-//                          Used while the longest sequence fits two key tiles' worth of work per item
-//                          (max_len <= 192) and for the general-mask variant.
+//                          Used for calls of few items and for the general-mask variant.
 //   mha_persistent_kernel  CTAs that take over waiting (sequence, query tile, head) items,
-//                          256 threads, two CTAs per SM; everything longer.
+//                          256 threads, two CTAs per SM; everything else (the lines: launch_mha).
 // Both run an online softmax over 128-key tiles, so no S x S logits ever reach HBM and any length
 // works.
 //
@@ -39,15 +38,14 @@
 // buffers is read or written.
 //
 // What the measurements on B200 say about the softmax (it, not the tensor core, bounds both kernels: the MMAs of a
-// 128x128 tile take ~540 clocks when two CTAs interleave them): in the persistent kernel a 128-key tile takes 1.6 us
-// (3.1k clocks) per CTA with two CTAs per SM, an item another ~3 us; the tile's tensor-memory loads, maximum, 128
+// 128x128 tile take ~540 clocks when two CTAs interleave them): in the persistent kernel a 128-key tile takes 1.4 us
+// (2.7k clocks) per CTA with two CTAs per SM, an item another ~2.2 us; the tile's tensor-memory loads, maximum, 128
 // exponentials, packing and stores alone, two CTAs per SM and MMAs running beside them, take 1.72k clocks.  Tensor
 // memory holds S, O and P for two CTAs, i.e. two softmax warps per scheduler.  Measured and dropped because they did
-// not help: exponentials partly on the FMA pipe (degree-5 polynomial, packed pairs, one pair in 8 / 4 / 3: 403 / 403 /
+// not help (before CTAs took over blocks): exponentials partly on the FMA pipe (degree-5 polynomial, packed pairs, one pair in 8 / 4 / 3: 403 / 403 /
 // 421 against 403 us per 79k-token launch), ex2.f16x2, 256-row ping-pong tiles, two threads per row with an exchange
 // through shared memory (25 % slower), reading an item's O out behind the next item's exponentials (level to 5 %
-// slower), items handed out by the loader through shared memory (-1 % at 512 tokens, +0.4 % for one sequence),
-// masking a tail tile by groups of keys under branches inside the body of the whole tiles (spills 624 bytes).
+// slower), masking a tail tile by groups of keys under branches inside the body of the whole tiles (spills 624 bytes).
 #include "common.cuh"
 #include "kernels.h"
 
@@ -1485,19 +1483,16 @@ cudaError_t launch_mha(const MhaLaunch& a, cudaStream_t stream) {
   args.gen_bias_tiles = tiles ? reinterpret_cast<const uint4*>(a.gen_bias_tiles) : nullptr;
   args.gen_bits_flag = a.gen_bits_flag;
   args.gen_bits_stride = mask_bits_stride_words(a.max_len);
-  // General [B,S,S] mask (+ optional bias): one CTA per (128 query rows, head, sequence).  A persistent-CTA
-  // form of it (mask applied from the bits) was measured slower at batch 16 / 512 tokens (2.36 against 2.19 ms
-  // per 12 layers): 768 items of one to four key tiles fill the 296 CTAs' last round unevenly, while one CTA
-  // per item is balanced by the hardware's block scheduler.
+  // General [B,S,S] mask (+ optional bias): one CTA per (128 query rows, head, sequence).  A persistent form of it (mask
+  // applied from the bits) was measured slower at batch 16 / 512 tokens, 2.36 against 2.19 ms per 12 layers, as long as each
+  // CTA walked a fixed list of items; with blocks that are taken over it has not been tried.
   if (a.gen_mask != nullptr) return tiles ? launch_per_item<2>(a, args, stream) : launch_per_item<1>(a, args, stream);
-  // Measured on B200 (12 heads, 18.9k tokens): the persistent kernel is ahead at every length (sequences
-  // of 64 / 128 / 256 / 384 / 1024 tokens: 70 / 40 / 47 / 57 / 105 us against 77 / 40 / 52 / 62 / 120) and for
-  // few long sequences (one of 614 tokens: 12.8 against 14.0 us; 16 up to 512: 24 against 27); only a handful
-  // of short items, fewer than the persistent CTAs, is served faster by one CTA per item (16 sequences up
-  // to 64 tokens: 7.0 against 8.3 us).
+  // us per launch on B200, 12 heads, one CTA per item / persistent.  18.9k tokens in sequences of 64 / 128 / 256 / 384 / 1024:
+  // 54.8 / 32.6, 32.7 / 21.8, 43.1 / 28.8, 51.8 / 36.8, 97.3 / 79.6; 16 of up to 512 16.3 / 13.7; 25 of up to 128 (300 items
+  // by max_len) 6.79 / 6.69, 24 (288) 5.48 / 5.65; 16 of up to 64 4.14 / 4.70; one of 307 (36) 6.91 / 6.83, of 384 6.86 / 7.07,
+  // of 512 (48) 8.29 / 8.81, of 614 (60) 11.1 / 10.7; two of up to 512 (96) 6.22 / 6.00, of up to 307 (72) 4.53 / 5.06;
+  // 12 of up to 200 (288) 5.72 / 6.19.
   const long long items_max = static_cast<long long>(a.batch) * a.head_num * ((a.max_len + kQRows - 1) / kQRows);
-  // (a few dozen items of a single sequence, e.g. one sequence of 307 tokens = 36 items: 0.622 against 0.641 ms
-  // per 12-layer forward with one CTA per item; from ~100 items of long rows on the persistent kernel is ahead)
   const bool persistent =
       g_dbg_force_kernel == 3 ||
       (g_dbg_force_kernel == 0 && (items_max > 296 || (a.max_len > kQRows && items_max >= 64)));

@@ -253,7 +253,7 @@ int bt_gemm(bt_handle h, const void* A, const void* W, void* out, const void* bi
  * followed by `add_bias_input_layernorm_kernel_launcher`
  * (bytetransformer/src/bert_transformer.cu:102-109 and :115-129):
  * out[M,N] = LayerNorm(A[M,K] * W[K,N] + bias + residual) * gamma + beta.
- * The pre-normalisation sums stay in tensor memory; the N/256 CTAs that share a 128-row tile
+ * The pre-normalisation sums stay in tensor memory; the CTAs (up to N/128) that share a 128-row tile
  * exchange row statistics through `scratch_f32`, a device buffer of m_rows*N*4 bytes whose
  * contents are undefined afterwards (used: 16*N/128 bytes per row, which this call zeroes
  * itself with a memset on `stream`).  N % 256 == 0, N <= 1024, K % 64 == 0.  The waits
