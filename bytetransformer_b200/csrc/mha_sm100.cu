@@ -42,10 +42,11 @@
 // (2.7k clocks) per CTA with two CTAs per SM, an item another ~2.2 us; the tile's tensor-memory loads, maximum, 128
 // exponentials, packing and stores alone, two CTAs per SM and MMAs running beside them, take 1.72k clocks.  Tensor
 // memory holds S, O and P for two CTAs, i.e. two softmax warps per scheduler.  Measured and dropped because they did
-// not help (before CTAs took over blocks): exponentials partly on the FMA pipe (degree-5 polynomial, packed pairs, one pair in 8 / 4 / 3: 403 / 403 /
-// 421 against 403 us per 79k-token launch), ex2.f16x2, 256-row ping-pong tiles, two threads per row with an exchange
-// through shared memory (25 % slower), reading an item's O out behind the next item's exponentials (level to 5 %
-// slower), masking a tail tile by groups of keys under branches inside the body of the whole tiles (spills 624 bytes).
+// not help (before CTAs took over blocks): exponentials partly on the FMA pipe (degree-5 polynomial, packed pairs, one pair
+// in 8 / 4 / 3: 403 / 403 / 421 against 403 us per 79k-token launch), ex2.f16x2, 256-row ping-pong tiles, two threads per
+// row with an exchange through shared memory (25 % slower), reading an item's O out behind the next item's exponentials
+// (level to 5 % slower), masking a tail tile by groups of keys under branches inside the body of the whole tiles (spills
+// 624 bytes).
 #include "common.cuh"
 #include "kernels.h"
 
