@@ -822,7 +822,8 @@ struct MhaPersistentArgs {
   int max_len;  // upper bound of every sequence length
   int tma_out;  // the kernel's second tensor map describes ctx: whole 32-row output slabs leave by bulk store
   int early_offsets;  // batch_idx may be read before the dependency wait (see launch_mha)
-  int take_over;  // the grid has more blocks than are resident
+  int take_over;   // the grid has more blocks than are resident
+  int first_wave;  // blocks that are, or all (see take_next)
 };
 
 // Finds item n = (sequence b, query tile qt, head h); items are numbered sequence by sequence, inside
@@ -1023,27 +1024,38 @@ mha_persistent_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_c
       uint32_t phase = 0;
       bool ok = true;
       int cur_b = 0, cur_first = 0;
-      int item = static_cast<int>(blockIdx.x);  // the one being worked on
       uint32_t asked = 0;
       bool have = own_item(cur_b, cur_first);  // (if not: the blocks behind have none either, and the other roles are done)
       // The grid is sized from an upper bound of the items; a block beyond the last one is taken over as well (cheaper
-      // than letting it start) and the next one asked for.  Offsets that fall can hold more items than the bound: the CTA
-      // that has the last block goes on with those, and looks at all offsets that way.
+      // than letting it start) and the next one asked for.  Offsets that fall can hold more items than the bound: block b
+      // of the first `first_wave` ones, whichever CTA has it, stands for the items b + gridDim, b + gridDim + first_wave, ...
+      // too - its own CTA looks for them when no block is left, and looks at all offsets that way; a CTA that took such a
+      // block over does so right behind it.
+      const int blocks = static_cast<int>(gridDim.x);
+      int beyond = -1;     // the next item behind the blocks to look for
+      bool none_left = false;
       auto take_next = [&]() {
-        const int blocks = static_cast<int>(gridDim.x);
-        do {
-          have = false;
-          if (item + 1 < blocks) {
-            if (!args.take_over) return;
-            if (elect_one()) launch_control_ask(taken, taken_full);
-            if (!mbar_wait_role(taken_full, asked++ & 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) return;
-            item = uniform_int(launch_control_answer(taken));
-            if (item < 0) return;
+        have = false;
+        while (true) {
+          int item = beyond;
+          if (item >= 0) {
+            beyond += args.first_wave;
           } else {
-            ++item;
+            if (none_left) return;
+            if (args.take_over) {
+              if (elect_one()) launch_control_ask(taken, taken_full);
+              if (!mbar_wait_role(taken_full, asked++ & 1u, abort_flag, args.status, kStatusMhaLoadTimeout)) return;
+              item = uniform_int(launch_control_answer(taken));
+            }
+            const int stands_for = item >= 0 ? item : static_cast<int>(blockIdx.x);
+            none_left = item < 0;
+            if (stands_for < args.first_wave) beyond = blocks + stands_for;
+            if (none_left) continue;
           }
           have = decode_item(args, item, cur_b, cur_first, seq_start, L, qt, head);
-        } while (!have && item < blocks);
+          if (have) return;
+          beyond = -1;  // no item behind this one either
+        }
       };
       if (args.early_offsets) pdl_wait();
       for (uint32_t n = 0; have; ++n) {
@@ -1439,6 +1451,7 @@ cudaError_t launch_persistent(const MhaLaunch& a, cudaStream_t stream) {
   const long long grid = tiles > 0 ? tiles * a.head_num : 1;
   if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
   args.take_over = grid > resident ? 1 : 0;
+  args.first_wave = static_cast<int>(grid < resident ? grid : resident);
   auto kern = more ? mha_persistent_kernel<true> : mha_persistent_kernel<false>;
   return launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(kPersistentThreads), kPersistentSmemBytes,
                     stream, a.tm_qkv, a.has_tm_ctx ? a.tm_ctx : a.tm_qkv, args);

@@ -598,8 +598,9 @@ def test_attention_rejects_offsets_outside_the_allocation(enc, cuda_device, kern
 
 
 @pytest.mark.parametrize("repeats,max_len,kernel", [
-    (3, 500, 3), (3, 1024, 3), (20, 500, 3), (3, 500, 1), (20, 500, 1),
-], ids=["one_item_per_block", "blocks_all_resident", "blocks_taken_over", "cta_per_item", "cta_per_item_many"])
+    (3, 500, 3), (3, 1024, 3), (20, 500, 3), (300, 500, 3), (3, 500, 1), (20, 500, 1),
+], ids=["one_item_per_block", "blocks_all_resident", "blocks_taken_over", "many_behind_the_blocks", "cta_per_item",
+        "cta_per_item_many"])
 def test_attention_offsets_that_fall_hide_no_sequence(enc, cuda_device, repeats, max_len, kernel):
     """Where offsets fall, sequences can share rows, and there can be more items than rising offsets would give for
     these rows.  The last sequence, which shares none, still comes out, as do the repeated ones."""
